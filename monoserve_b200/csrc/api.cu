@@ -182,6 +182,7 @@ int forward_locked(monofab_moe* m, const void* xn, const void* x2, void* out, in
   pp.H = H;
   pp.I = I;
   pp.form = m->form;
+  pp.slices = c.fp8 ? 1 : 2;
   pp.tile_cap = m->tile_cap;
   pp.n_experts = E;
   pp.rows_cap = static_cast<int>(m->pairs_cap) - 256;
@@ -236,6 +237,7 @@ int experts_locked(monofab_moe* m, const PlanParams& seg, cudaStream_t st, cudaE
   pp.H = c.hidden;
   pp.I = c.intermediate;
   pp.form = m->form;
+  pp.slices = c.fp8 ? 1 : 2;
   pp.tile_cap = m->tile_cap;
   pp.n_experts = c.experts;
   pp.rows_cap = static_cast<int>(m->pairs_cap) - 256;

@@ -7,6 +7,7 @@
 //             h = bf16(silu(g) * u)                       (kEpiSiluMul)
 //   w2 tile : 128 output rows x the same row block over h, epilogue stores the
 //             fp32 rows y[pos][n] of every routed pair     (kEpiRowsF32)
+// A row block of more than 128 rows takes tiles of two slices (128 features, 256 output rows).
 // A w2 tile may start only when every w13 tile of its row block has stored h:
 // the epilogue warps of w13 tiles count into done[block] (release), and the
 // scheduler waits (bounded) for the count before it hands a w2 tile to the
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
         }
         const GemmTile tile = *t;
         trace_ev(p, 0, it, 1);
-        const int tier = tile.tier_phase & 0xff, phase = tile.tier_phase >> 8;
+        const int tier = tile.tier_phase & 0xff, phase = (tile.tier_phase >> 8) & 0xff;
         const GemmPhaseParams& ph = p.ph[phase];
         int box = 0;
         while ((16 << box) < tile.n) ++box;
@@ -144,6 +145,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
         w.scale = ph.scale ? ph.scale + static_cast<size_t>(tile.expert) * ph.scale_ld : nullptr;
         w.w_fp8 = ph.w_fp8;
         w.fetch = 0;
+        w.slices = tile.tier_phase >> 16;
         w.bias = nullptr;
         w.residual = nullptr;
         w.pair_token = nullptr;
@@ -216,8 +218,9 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
     int n_w2 = 0;
     if (own && lane == 0) own[0] = globaltimer_ns();
     const long long c_begin = own ? clock64() : 0;
+    uint32_t g = 0;   // accumulators used so far
     for (int it = 0;; ++it) {
-      const int slot = it % kWorkSlots, buf = it & 1;
+      const int slot = it % kWorkSlots;
       const long long tw = own ? clock64() : 0;
       if (!mbar_wait_bounded(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
       if (own) sum_work += clock64() - tw;
@@ -225,9 +228,9 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
       trace_ev(p, 2, it, 0);
       if (own && lane == 0 && it == 0) own[1] = globaltimer_ns();
       long long waited[3] = {0, 0, 0};
-      if (!gemm_mma<false>(sh.work[slot], ring, sh.bar, pipe, tmem_base, buf, (it >> 1) & 1, abort_flag,
-                           p.trace ? waited : nullptr))
-        break;
+      const uint32_t slices = sh.work[slot].slices;
+      if (!gemm_mma<false>(sh.work[slot], ring, sh.bar, pipe, tmem_base, g, abort_flag, p.trace ? waited : nullptr)) break;
+      g += slices;
       trace_ev(p, 2, it, 1);
       if (own && lane == 0) {
         sum_wait += waited[0];
@@ -264,8 +267,9 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
     }
   } else {
     // -------------------------------------------------------------- epilogue
+    uint32_t g = 0;
     for (int it = 0;; ++it) {
-      const int slot = it % kWorkSlots, buf = it & 1;
+      const int slot = it % kWorkSlots;
       if (!mbar_wait_bounded(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
       if (!sh.work[slot].valid) break;
       const GemmWork w = sh.work[slot];
@@ -274,14 +278,15 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
       if (warp == 2) trace_ev(p, 3, it, 0);
       unsigned long long* seen =
           (p.trace && blockIdx.x == 0 && warp == 2 && it < 32) ? &p.trace[(3 * 32 + it) * 4 + 3] : nullptr;
-      if (!gemm_epilogue<false>(w, sh.bar, tmem_base, buf, (it >> 1) & 1, abort_flag, seen)) break;
+      if (!gemm_epilogue<false>(w, sh.bar, tmem_base, g, abort_flag, seen)) break;
+      g += w.slices;
       if (warp == 2) trace_ev(p, 3, it, 1);
       if (w.block >= 0) {
         // publish this warp's part of h, then count it into the row block
         __threadfence();
         fence_proxy_async_all();
         __syncwarp();
-        if (lane == 0) atomicAdd(p.done + w.block, 1);
+        if (lane == 0) atomicAdd(p.done + w.block, w.slices);
       }
       if (warp == 2) trace_ev(p, 3, it, 2);
     }

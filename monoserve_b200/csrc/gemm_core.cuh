@@ -5,7 +5,11 @@
 // One tile (the reference's GEMM tile, csrc/fabric/tiles/gemm.cuh:1-18,133-346,
 // csrc/fabric/model_types.h:37-49): 128 weight rows (output features) as the MMA
 // M operand times up to 256 activation rows as the N operand, over a range of
-// 64-element K steps; fp32 accumulation in TMEM.  Both operands are K-major with
+// 64-element K steps; fp32 accumulation in TMEM.  A tile of two slices takes 256 weight rows:
+// both 128-row halves meet the same activation tile of a stage, each with an accumulator buffer.
+// What bounds a prompt's products is the SMs' reads of the L2 (about 10 TB/s in all, whatever the
+// tile): per 128 x 128 x 64 step a tile of n = 128 reads 32 KB, one of n = 256 24 KB, and one of
+// two slices and n = 256 16 KB.  Both operands are K-major with
 // the 128-byte swizzle.  The weight slice is fetched as eight TMA boxes of 16
 // rows, which lets a SwiGLU tile interleave 64 gate rows and 64 up rows in groups
 // of 16: TMEM lane 32q+i (i < 16) then holds gate feature 16q+i and lane 32q+16+i
@@ -76,6 +80,8 @@ struct GemmWork {
                               // partial sums go to column = weight row (kEpiSiluMul always reads two slabs)
   int32_t block;              // row block whose counter the epilogue bumps, or -1
   int32_t w_fp8;              // the weight tensor holds e4m3 bytes: W8A16 (exact e4m3 -> bf16 in shared memory)
+  int32_t slices;             // 1, or 2: two adjacent weight slices (bf16 weights, kEpiAtomicF32 excepted), each with an
+                              // accumulator buffer of its own
   // A fetch record moves fetch_bytes from fetch_src (host-resident weights) to `out` (an HBM staging
   // buffer) through the operand ring, in stages of kFetchStageBytes: no MMA, no accumulator.
   int32_t fetch;
@@ -144,7 +150,7 @@ __device__ __forceinline__ int gemm_stage_count(const GemmWork& w) {
 template <bool kFetch = true>
 __device__ __forceinline__ uint32_t gemm_stage_bytes(const GemmWork& w) {
   if (kFetch && w.fetch) return kFetchStageBytes;
-  return gemm_ksteps(w) * (kATileBytes + w.n * kBlockK * 2);
+  return gemm_ksteps(w) * (w.slices * kATileBytes + w.n * kBlockK * 2);
 }
 
 struct GemmBarriers {
@@ -170,7 +176,7 @@ __device__ __forceinline__ void gemm_barriers_init(GemmBarriers& b) {
 // TMA issue for one tile.  The WHOLE producer warp calls it: every lane keeps
 // the same bookkeeping, lane 0 arms the barrier, and the copies of one stage go
 // out as a single warp-wide instruction (lanes 0..7 the weight boxes, lane 8 the
-// activation box), which costs one issue slot instead of nine.
+// activation box, lanes 16..23 the second slice's), which costs one issue slot instead of nine.
 // Returns false when a wait was abandoned.
 template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,
@@ -183,16 +189,20 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
   // FP8 weights land as raw bytes in the second weight tile (128-byte rows = two K steps, no swizzle)
   const uint32_t a_off = w.w_fp8 ? kATileBytes : 0;
   const uint32_t a_box = 2048;   // bytes of one 16-row box: 128-byte rows either way
-  const uint32_t b_off = ks * kATileBytes;
+  const int slices = w.slices;
+  const uint32_t b_off = ks * slices * kATileBytes;
   const int n_stages = gemm_stage_count<kFetch>(w);
   // SwiGLU tiles of a tensor in the reference row order gather eight 16-row boxes;
   // every other tile is one 128-row box (a packed SwiGLU tensor stores gate/up
   // groups of 16 rows alternately, so its tile starts at row 2 * a_row_lo).
   const bool slab2 = epi_gated(w.epi) || (w.a_packed & 4);
   const bool gather = slab2 && !(w.a_packed & 1);
-  const int a_row = gather ? ((lane & 1) ? w.a_row_hi : w.a_row_lo) + 16 * ((lane & 7) >> 1)
-                           : (slab2 ? 2 * w.a_row_lo : w.a_row_lo);
+  const int second = lane >> 4;   // lanes 16.. bring the second slice's boxes
+  const int a_row = gather ? ((lane & 1) ? w.a_row_hi : w.a_row_lo) + 16 * ((lane & 7) >> 1) + 64 * second
+                           : (slab2 ? 2 * w.a_row_lo : w.a_row_lo) + 128 * second;
   const int n_a = gather ? 8 : 1;
+  const bool brings_a = (lane & 15) < n_a && second < slices;
+  const uint32_t a_at = a_off + second * kATileBytes + (lane & 7) * a_box;
   // read once: the record lives in shared memory and every copy below is a memory barrier to the compiler
   const bool fetch = kFetch && w.fetch != 0;
   const uint32_t fetch_bytes = kFetch ? w.fetch_bytes : 0;
@@ -200,7 +210,7 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
   const CUtensorMap* const a_map = w.a_map;
   const CUtensorMap* const b_map = w.b_map;
   const int a_z = w.a_z, b_row0 = w.b_row0, k0 = w.k0;
-  const uint32_t tx_bytes = kATileBytes + ks * b_bytes;
+  const uint32_t tx_bytes = slices * kATileBytes + ks * b_bytes;
   for (int st = 0; st < n_stages; ++st) {
     uint32_t vb, ve;
     const uint32_t phys = pipe.alloc(size, vb, ve);
@@ -232,8 +242,8 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
     if (lane == 0) mbar_arrive_expect_tx(full, tx_bytes);
     __syncwarp();
     const int x = (k0 + st * ks) * kBlockK;
-    if (lane < n_a) {
-      tma_load_3d(a + a_off + lane * a_box, a_map, full, x, a_row, a_z, pol_w);
+    if (brings_a) {
+      tma_load_3d(a + a_at, a_map, full, x, a_row, a_z, pol_w);
     } else if (lane >= 8 && lane < 8 + ks) {
       tma_load_2d(a + b_off + (lane - 8) * b_bytes, b_map, full, x + (lane - 8) * kBlockK, b_row0, pol_x);
     }
@@ -242,17 +252,61 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
   return true;
 }
 
-// MMA issue for one tile into accumulator buffer `buf`.  The whole MMA warp runs the K loop in
-// step (every lane waits for the stage itself, so the loop needs no warp barrier) and one elected
+// MMA issue for a tile of two slices (bf16 weights): accumulators g and g + 1, eight MMAs a stage.  A loop of its own: the
+// one-slice loop bounds small tiles, and a branch on the slices inside it cost it 100 cycles a stage.
+__device__ __forceinline__ bool gemm_mma_two(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,
+                                             uint32_t tmem_base, uint32_t g, volatile int* abort_flag) {
+  const bool leader = elect_one();
+  const uint32_t b0 = g & 1, b1 = b0 ^ 1;
+  int ok = mbar_wait_bounded(&bar.acc_empty[b0], ((g >> 1) & 1) ^ 1, abort_flag, kWaitBudgetNs);
+  const uint32_t idesc = umma_idesc_bf16(128, w.n);
+  const uint32_t acc0 = tmem_base + b0 * kAccCols, acc1 = tmem_base + b1 * kAccCols;
+  const uint32_t size = gemm_stage_bytes<false>(w), ring_addr = smem_u32(ring);
+  const uint64_t desc0 = umma_desc_sw128(0);
+  const int n_stages = w.k_tiles;
+  for (int kt = 0; kt < n_stages; ++kt) {
+    uint32_t vb, ve;
+    const uint32_t phys = pipe.alloc(size, vb, ve);
+    ok = ok && mbar_wait_bounded(&bar.full[pipe.slot], pipe.parity, abort_flag, kWaitBudgetNs);
+    __syncwarp();   // a lane two laps of the barrier ring behind the leader would wait for a phase that never comes
+    tc_fence_after_sync();
+    const uint64_t da = desc0 + ((ring_addr + phys) >> 4), db = da + (2 * kATileBytes >> 4);
+    if (leader && ok) {
+#pragma unroll
+      for (int k = 0; k < kBlockK / 16; ++k) umma_bf16(acc0, da + 2 * k, db + 2 * k, idesc, (kt | k) != 0);
+    }
+    if (kt == 0) {   // the first slice's MMAs run while the second's accumulator is still being drained
+      ok = ok && mbar_wait_bounded(&bar.acc_empty[b1], (((g + 1) >> 1) & 1) ^ 1, abort_flag, kWaitBudgetNs);
+      tc_fence_after_sync();
+    }
+    if (leader && ok) {
+#pragma unroll
+      for (int k = 0; k < kBlockK / 16; ++k)
+        umma_bf16(acc1, da + (kATileBytes >> 4) + 2 * k, db + 2 * k, idesc, (kt | k) != 0);
+      umma_commit(&bar.empty[pipe.slot]);
+    }
+    pipe.advance();
+  }
+  if (leader && ok) {
+    umma_commit(&bar.acc_full[b0]);
+    umma_commit(&bar.acc_full[b1]);
+  }
+  return __all_sync(0xffffffffu, ok != 0);
+}
+
+// MMA issue for one tile into accumulator g (buffer g & 1).
+// The whole MMA warp runs the K loop in step (every lane waits for the stage itself) and one elected
 // lane issues the four tcgen05.mma and the commit of a stage.  Because the loop is convergent code,
 // its descriptors and addresses are warp-uniform values; with the loop inside a single-lane branch
 // the MMA warp spent twice as long issuing (measured: 67 -> 32 us of a 150 us launch), which is
 // what bounds small-N tiles.
 template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,
-                                         uint32_t tmem_base, int buf, uint32_t acc_parity, volatile int* abort_flag,
+                                         uint32_t tmem_base, uint32_t g, volatile int* abort_flag,
                                          long long* wait_cycles = nullptr) {
+  if (w.slices == 2) return gemm_mma_two(w, ring, bar, pipe, tmem_base, g, abort_flag);
   int ok = 1;
+  const uint32_t buf = g & 1, acc_parity = (g >> 1) & 1;
   const bool leader = elect_one();
   {
     const long long ta = wait_cycles ? clock64() : 0;
@@ -403,11 +457,157 @@ __device__ __forceinline__ float decay_less_one(float z, float coef) {
   return x > -0.25f ? small : large;
 }
 
-// Epilogue of one tile from accumulator buffer `buf` (the four epilogue warps
-// call): everything except handing the buffer back to the MMA warp.
+// One value of kEpiStoreBf16 / the fp32 epilogues / kEpiDecay.
+template <int E>
+__device__ __forceinline__ float epi_value(uint32_t acc, float sc, float bias, float coef) {
+  const float v = __uint_as_float(acc) * sc + bias;
+  return E == kEpiDecay ? decay_less_one(v, coef) : v;
+}
+
+// The chunks (32 accumulator columns = activation rows) of one slice, all of them by epilogue E.  The epilogue is fixed at
+// compile time and a whole chunk has no per-row conditions, so that a chunk's 16 or 32 values are computed side by side:
+// with a branch per row (two activations, rows past the end) a chunk took 1.9 us and the epilogue, one warp per
+// scheduler, bounded the products: 128 rows of a SwiGLU tile 8.2 us, now 2.2.  The next chunk's TMEM load, and the
+// residual's values of the next chunk, are under way while this one is converted and stored.  (The residual loaded where
+// it was added, a 2-byte load behind each 2-byte store, took 0.6 us a row.)
+template <int E>
+__device__ __forceinline__ void epilogue_chunks(const GemmWork& w, uint32_t tacc, int f, int wrow, bool f_ok, float sc,
+                                                float bias, float coef) {
+  const int lane = threadIdx.x & 31;
+  const int n = w.n, rows = w.rows, ld = w.ld_out, c_end = min(n, rows);
+  const bool lo = lane < 16;
+  constexpr bool kGated = E == kEpiSiluMul || E == kEpiGeluMul, kHalf = kGated || E == kEpiStoreBf16;
+  const size_t first = static_cast<size_t>(w.b_row0) * ld + (E == kEpiAtomicF32 && (w.a_packed & 4) ? wrow : f);
+  unsigned short* const out16 = reinterpret_cast<unsigned short*>(w.out) + first;
+  float* const out32 = reinterpret_cast<float*>(w.out) + first;
+  const unsigned short* const res = E == kEpiStoreBf16 && w.residual && f_ok
+      ? reinterpret_cast<const unsigned short*>(w.residual) + static_cast<size_t>(w.b_row0) * w.ld_res + f : nullptr;
+  const int ld_res = w.ld_res;
+  constexpr int kRes = E == kEpiStoreBf16 ? 32 : 1;
+  unsigned short rn[kRes];   // the next chunk's residual values
+  auto load_res = [&](int c0) {
+    if (E != kEpiStoreBf16 || !res) return;
+    const unsigned short* p = res + static_cast<size_t>(c0) * ld_res;
+#pragma unroll
+    for (int j = 0; j < kRes; ++j) rn[j] = c0 + j < rows ? p[static_cast<size_t>(j) * ld_res] : 0;
+  };
+  uint32_t next[32];
+  load_res(0);
+  if (n >= 32) {
+    tmem_ld_32x32(tacc, next);
+  } else {
+    uint32_t r16[16];
+    tmem_ld_32x16(tacc, r16);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      next[j] = r16[j];
+      next[16 + j] = 0;
+    }
+  }
+  if (c_end <= 0) tmem_ld_wait();
+#pragma unroll 1
+  for (int c0 = 0; c0 < c_end; c0 += 32) {
+    uint32_t r[32];
+    unsigned short rv[kRes];
+    __syncwarp();
+    tmem_ld_wait_for(next);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = next[j];
+#pragma unroll
+    for (int j = 0; j < kRes; ++j) rv[j] = rn[j];
+    if (c0 + 32 < c_end) {   // n is a power of two: a whole chunk
+      tmem_ld_32x32(tacc + c0 + 32, next);
+      load_res(c0 + 32);
+    }
+    const bool whole = c0 + 32 <= rows;
+    if constexpr (kGated) {
+      // lanes < 16 own gate rows, lanes >= 16 the matching up rows; exchange halves: the lower lanes take the chunk's
+      // first 16 rows, the upper ones the others
+      float mine[16], other[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        mine[j] = __uint_as_float(lo ? r[j] : r[16 + j]) * sc;
+        other[j] = __shfl_xor_sync(0xffffffffu, __uint_as_float(lo ? r[16 + j] : r[j]) * sc, 16);
+      }
+      unsigned short hv[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float gate = lo ? mine[j] : other[j], up = lo ? other[j] : mine[j];
+        hv[j] = __bfloat16_as_ushort(__float2bfloat16(E == kEpiGeluMul ? gelu_mul(gate, up) : silu_mul(gate, up)));
+      }
+      const int t0 = c0 + (lo ? 0 : 16);
+      unsigned short* const o = out16 + static_cast<size_t>(t0) * ld;
+      if (whole && f_ok) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) o[static_cast<size_t>(j) * ld] = hv[j];
+      } else if (f_ok) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (t0 + j < rows) o[static_cast<size_t>(j) * ld] = hv[j];
+      }
+    } else if constexpr (E == kEpiStoreBf16) {
+      unsigned short hv[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        float v = epi_value<E>(r[j], sc, bias, coef);
+        if (res) v += __bfloat162float(__ushort_as_bfloat16(rv[j]));
+        hv[j] = __bfloat16_as_ushort(__float2bfloat16(v));
+      }
+      unsigned short* const o = out16 + static_cast<size_t>(c0) * ld;
+      if (whole && f_ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) __stcs(o + static_cast<size_t>(j) * ld, hv[j]);
+      } else if (f_ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (c0 + j < rows) __stcs(o + static_cast<size_t>(j) * ld, hv[j]);
+      }
+    } else if constexpr (E == kEpiWeightedAdd) {
+      if (f_ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (c0 + j < rows) {
+            const int m = w.b_row0 + c0 + j;
+            atomicAdd(reinterpret_cast<float*>(w.out) + f + static_cast<size_t>(w.pair_token[m]) * ld,
+                      w.pair_weight[m] * (__uint_as_float(r[j]) * sc));
+          }
+        }
+      }
+    } else if constexpr (E == kEpiAtomicF32) {
+      // a two-slab tile (partial sums of a SwiGLU pair) adds into the column of its weight row
+      if (f_ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (c0 + j < rows) atomicAdd(out32 + static_cast<size_t>(c0 + j) * ld, __uint_as_float(r[j]) * sc + bias);
+      }
+    } else {
+      // fp32 rows; those that are read once, later (per-pair expert outputs, logits) by streaming stores
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = epi_value<E>(r[j], sc, bias, coef);
+      float* const o = out32 + static_cast<size_t>(c0) * ld;
+      if (whole && f_ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (E == kEpiDecay) o[static_cast<size_t>(j) * ld] = v[j];
+          else __stcs(o + static_cast<size_t>(j) * ld, v[j]);
+        }
+      } else if (f_ok) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (c0 + j < rows) __stcs(o + static_cast<size_t>(j) * ld, v[j]);
+      }
+    }
+  }
+}
+
+// Epilogue of one slice of a tile from accumulator buffer `buf` (the four epilogue warps
+// call): everything except handing the buffer back to the MMA warp.  kFetch = false: the expert kernel, which has two
+// epilogues and no fetch records.
 template <bool kFetch = true>
-__device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, GemmBarriers& bar, uint32_t tmem_base, int buf,
-                                                   uint32_t acc_parity, volatile int* abort_flag,
+__device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, int slice, GemmBarriers& bar, uint32_t tmem_base,
+                                                   uint32_t buf, uint32_t acc_parity, volatile int* abort_flag,
                                                    unsigned long long* acc_seen = nullptr) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3;
   if (!mbar_wait_bounded(&bar.acc_full[buf], acc_parity, abort_flag, kWaitBudgetNs)) return false;
@@ -418,121 +618,51 @@ __device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, GemmBarrie
     return true;
   }
   const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * kAccCols;
-  const bool silu = epi_gated(w.epi), gelu = w.epi == kEpiGeluMul;
+  const bool slab2 = epi_gated(w.epi) || (w.a_packed & 4);
   // output feature of this lane, and the weight row its accumulator row came from
   int f, wrow;
-  if (silu || (w.a_packed & 4)) {
-    f = w.a_row_lo + 16 * quad + (lane & 15);
-    wrow = (lane < 16 ? w.a_row_lo : w.a_row_hi) + 16 * quad + (lane & 15);
+  if (slab2) {
+    f = w.a_row_lo + 64 * slice + 16 * quad + (lane & 15);
+    wrow = (lane < 16 ? w.a_row_lo : w.a_row_hi) + 64 * slice + 16 * quad + (lane & 15);
   } else {
-    f = w.a_row_lo + 32 * quad + lane;
+    f = w.a_row_lo + 128 * slice + 32 * quad + lane;
     wrow = f;
   }
   const bool f_ok = f < w.n_limit;
   const float sc = (w.scale && f_ok) ? w.scale[wrow] : 1.f;
-  const float bias = (w.bias && f_ok && w.k0 == 0) ? __bfloat162float(w.bias[f]) : 0.f;
-  for (int c0 = 0; c0 < w.n; c0 += 32) {
-    uint32_t r[32];
-    if (w.n - c0 >= 32) {
-      tmem_ld_32x32(tacc + c0, r);
-    } else {
-      uint32_t r16[16];
-      tmem_ld_32x16(tacc + c0, r16);
-      tmem_ld_wait();
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        r[j] = r16[j];
-        r[16 + j] = 0;
-      }
+  if constexpr (kFetch) {
+    const float bias = (w.bias && f_ok && w.k0 == 0) ? __bfloat162float(w.bias[f]) : 0.f;
+    switch (w.epi) {
+      case kEpiStoreBf16: epilogue_chunks<kEpiStoreBf16>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiSiluMul: epilogue_chunks<kEpiSiluMul>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiGeluMul: epilogue_chunks<kEpiGeluMul>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiWeightedAdd: epilogue_chunks<kEpiWeightedAdd>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiAtomicF32: epilogue_chunks<kEpiAtomicF32>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiDecay:
+        epilogue_chunks<kEpiDecay>(w, tacc, f, wrow, f_ok, sc, bias, f_ok ? w.pair_weight[f] : 0.f);
+        break;
+      default: epilogue_chunks<kEpiStoreF32>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
     }
-    tmem_ld_wait();
-    if (c0 >= w.rows) continue;
-    if (silu) {
-      // lanes < 16 own gate rows, lanes >= 16 the matching up rows; exchange halves
-      const bool lo = lane < 16;
-      const int t0 = c0 + (lo ? 0 : 16);
-      unsigned short* out = reinterpret_cast<unsigned short*>(w.out) + static_cast<size_t>(w.b_row0 + t0) * w.ld_out + f;
-      unsigned short hv[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float mine_keep = __uint_as_float(lo ? r[j] : r[16 + j]) * sc;
-        const float send = __uint_as_float(lo ? r[16 + j] : r[j]) * sc;
-        const float other = __shfl_xor_sync(0xffffffffu, send, 16);
-        const float gate = lo ? mine_keep : other, up = lo ? other : mine_keep;
-        hv[j] = __bfloat16_as_ushort(__float2bfloat16(gelu ? gelu_mul(gate, up) : silu_mul(gate, up)));
-      }
-      if (f_ok) {
-        const int m_hi = w.rows - t0;
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (j < m_hi) out[static_cast<size_t>(j) * w.ld_out] = hv[j];
-      }
-    } else if (w.epi == kEpiStoreBf16) {
-      __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(w.out) + static_cast<size_t>(w.b_row0 + c0) * w.ld_out + f;
-      const __nv_bfloat16* res =
-          w.residual ? w.residual + static_cast<size_t>(w.b_row0 + c0) * w.ld_res + f : nullptr;
-      if (f_ok) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (c0 + j < w.rows) {
-            float v = __uint_as_float(r[j]) * sc + bias;
-            if (res) v += __bfloat162float(res[static_cast<size_t>(j) * w.ld_res]);
-            __stcs(reinterpret_cast<unsigned short*>(out + static_cast<size_t>(j) * w.ld_out),
-                   __bfloat16_as_ushort(__float2bfloat16(v)));
-          }
-        }
-      }
-    } else if (w.epi == kEpiWeightedAdd) {
-      float* out = reinterpret_cast<float*>(w.out) + f;
-      if (f_ok) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (c0 + j < w.rows) {
-            const int m = w.b_row0 + c0 + j;
-            atomicAdd(out + static_cast<size_t>(w.pair_token[m]) * w.ld_out,
-                      w.pair_weight[m] * (__uint_as_float(r[j]) * sc));
-          }
-        }
-      }
-    } else if (w.epi == kEpiAtomicF32) {
-      // a two-slab tile (partial sums of a SwiGLU pair) adds into the column of its weight row
-      float* out = reinterpret_cast<float*>(w.out) + static_cast<size_t>(w.b_row0 + c0) * w.ld_out + ((w.a_packed & 4) ? wrow : f);
-      if (f_ok) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < w.rows) atomicAdd(out + static_cast<size_t>(j) * w.ld_out, __uint_as_float(r[j]) * sc + bias);
-      }
-    } else if (w.epi == kEpiDecay) {
-      float* out = reinterpret_cast<float*>(w.out) + static_cast<size_t>(w.b_row0 + c0) * w.ld_out + f;
-      if (f_ok) {
-        const float coef = w.pair_weight[f];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(decay_less_one(__uint_as_float(r[j]) * sc + bias, coef));
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < w.rows) out[static_cast<size_t>(j) * w.ld_out] = __uint_as_float(r[j]);
-      }
-    } else {
-      // fp32 rows that are read once, later (per-pair expert outputs, logits): streaming stores
-      float* out = reinterpret_cast<float*>(w.out) + static_cast<size_t>(w.b_row0 + c0) * w.ld_out + f;
-      if (f_ok) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (c0 + j < w.rows) __stcs(out + static_cast<size_t>(j) * w.ld_out, __uint_as_float(r[j]) * sc + bias);
-      }
-    }
+  } else if (w.epi == kEpiSiluMul) {
+    epilogue_chunks<kEpiSiluMul>(w, tacc, f, wrow, f_ok, sc, 0.f, 0.f);
+  } else {
+    epilogue_chunks<kEpiRowsF32>(w, tacc, f, wrow, f_ok, sc, 0.f, 0.f);
   }
   tc_fence_before_sync();
   __syncwarp();
   return true;
 }
 
+// The four epilogue warps: every slice of a tile whose first accumulator is g.
 template <bool kFetch = true>
-__device__ __forceinline__ bool gemm_epilogue(const GemmWork& w, GemmBarriers& bar, uint32_t tmem_base, int buf,
-                                              uint32_t acc_parity, volatile int* abort_flag,
-                                              unsigned long long* acc_seen = nullptr) {
-  if (!gemm_epilogue_body<kFetch>(w, bar, tmem_base, buf, acc_parity, abort_flag, acc_seen)) return false;
-  if ((threadIdx.x & 31) == 0) mbar_arrive(&bar.acc_empty[buf]);
+__device__ __forceinline__ bool gemm_epilogue(const GemmWork& w, GemmBarriers& bar, uint32_t tmem_base, uint32_t g,
+                                              volatile int* abort_flag, unsigned long long* acc_seen = nullptr) {
+  const int slices = w.slices;
+#pragma unroll 1
+  for (int i = 0; i < slices; ++i, ++g) {
+    if (!gemm_epilogue_body<kFetch>(w, i, bar, tmem_base, g & 1, (g >> 1) & 1, abort_flag, acc_seen)) return false;
+    if ((threadIdx.x & 31) == 0) mbar_arrive(&bar.acc_empty[g & 1]);
+  }
   return true;
 }
 

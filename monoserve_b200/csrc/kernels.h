@@ -89,6 +89,7 @@ struct PlanParams {
   int* done;                // int32 [block_cap] row-block counters (zeroed here)
   int* status;
   int chunks, E, H, I;
+  int slices;               // 2: tiles of two weight slices may be made (bf16 weights in HBM)
   int form;                 // row-block height of host-resident experts: 16..128; 0 = 256 (one pass up to 256 rows)
   int tile_cap;             // capacity of each tile list
   int block_cap;            // capacity of done[]

@@ -24,7 +24,8 @@ struct GemmTile {
   int32_t rows;       // valid activation rows, 1..n
   int32_t n;          // MMA N = height of the activation box: 16/32/64/128/256
   int32_t z;          // slot of the expert inside its tier's weight tensor
-  int32_t tier_phase; // kTierHost / kTierHot in bits 0..7, phase (0 = w13, 1 = w2) in bits 8..15
+  int32_t tier_phase; // kTierHost / kTierHot in bits 0..7, phase (0 = w13, 1 = w2) in bits 8..15, weight slices (1 or 2)
+                      // in bits 16..23
   int32_t expert;     // expert id (FP8 scale rows)
   int32_t block;      // row block id: w13 tiles count into done[block], w2 tiles wait on it
 };

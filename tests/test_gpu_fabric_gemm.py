@@ -87,6 +87,35 @@ def test_dense_store(fab, where, bm):
     del keep
 
 
+@pytest.mark.parametrize("epi", [EPI_STORE, EPI_SILU_MUL, EPI_F32])
+@pytest.mark.parametrize("rows", [1, 17, 200, 256, 300])
+def test_two_slice_tiles_equal_one_slice_tiles(fab, rows, epi):
+    """Tiles of 256 weight rows (bit 32 of a[3]) do the same arithmetic as two tiles of 128: the same bits.  The last
+    weight slice has no second half, and the last row block is ragged; one-slice tiles follow two-slice ones in a worker."""
+    torch.manual_seed(2)
+    K, N, bm = 448, 5 * 128, 256
+    gated = epi == EPI_SILU_MUL
+    w = (torch.randn(1, N, K, device="cuda") * 0.05).to(torch.bfloat16)
+    x = torch.randn(rows + 256, K, device="cuda").to(torch.bfloat16)[:rows]
+    res = torch.randn(rows, N, device="cuda").to(torch.bfloat16)
+    n_out, step = (N // 2, 64) if gated else (N, 128)
+    wm, xm = weight_map(fab, w.data_ptr(), w.shape), act_map(fab, x, bm)
+    outs = []
+    for two in (0, 1):
+        out = torch.zeros(rows, n_out, device="cuda", dtype=torch.float32 if epi == EPI_F32 else torch.bfloat16)
+        more = dict(residual=res.data_ptr(), ld_res=N) if epi == EPI_STORE else {}
+        args = args_tensor(out=out.data_ptr(), ld_out=n_out, k_tiles=K // 64, epi=epi, bm=bm, n_limit=n_out, up_offset=n_out, **more)
+        tiles = [Tile(KIND_GEMM, i=(n0, m0, min(bm, rows - m0), 0), a=(args.data_ptr(), wm, xm, (two and n0 + step < n_out) << 32))
+                 for _ in range(8) for n0 in range(0, n_out, step << two) for m0 in range(0, rows, bm)]
+        p = Program()
+        run_program(fab, p, p.stage(tiles))
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1])
+    y = x.float() @ w[0].float().t()
+    ref = torch.nn.functional.silu(y[:, :n_out]) * y[:, n_out:] if gated else y + res.float() if epi == EPI_STORE else y
+    assert float((outs[1].float() - ref).norm() / ref.norm()) < 1e-2
+
+
 @pytest.mark.parametrize("where", ["hbm", "cpu"])
 def test_expert_ffn(fab, where):
     """w13 tiles with the SiLU-and-multiply epilogue, then w2 tiles that add

@@ -287,6 +287,29 @@ def test_qwen3_layer_config1_ragged_batch():
 
 
 # ------------------------------------------------------ pack from given routing
+@pytest.mark.parametrize("I", [192, 256])
+def test_row_blocks_at_their_edges(I):
+    """Experts whose row counts lie on the edges of 128- and 256-row blocks, and an odd and an even number of weight slices
+    (a wide block's last tile has one slice when they are odd)."""
+    rows = [1, 128, 129, 255, 256, 257, 384, 385, 512, 0, 640, 700]
+    E, H, P = len(rows), 512, sum(rows)
+    m, wr, w13, w2 = make_layer(P, H, I, E, 1, list(range(E)))
+    g = torch.Generator().manual_seed(3)
+    x = torch.randn(P, H, generator=g).to(torch.bfloat16)
+    m.workspace("xp")[:P * H].copy_(x.flatten().cuda())
+    m.experts(torch.tensor(rows, dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    assert m.status() == 0
+    y, at = m.workspace("y")[:P * H].view(P, H).cpu(), 0
+    for e, n in enumerate(rows):
+        v = x[at:at + n].float() @ w13[e].float().T
+        h = (torch.nn.functional.silu(v[:, :I]) * v[:, I:]).to(torch.bfloat16).float()
+        if n:
+            assert rel_l2(y[at:at + n], h @ w2[e].float().T) < 2e-3, (e, n)   # the rounding of h: 2^-9 of each term
+        at += n
+    m.close()
+
+
 def random_routing(T, E, K, seed):
     g = torch.Generator().manual_seed(seed)
     ids = torch.stack([torch.randperm(E, generator=g)[:K] for _ in range(T)]).to(torch.int32) if T else \
