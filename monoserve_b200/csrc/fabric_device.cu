@@ -1121,7 +1121,7 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
           w.worker_lane = ws.lane;
           w.is_gemm = 0;
           w.is_attn = 0;
-          w.is_wide = tile_is_wide(w.tile.kind);
+          w.is_wide = tile_is_wide(w.tile);
           if (w.tile.kind == kTileAttnPrefill || w.tile.kind == kTileAttnDecode) {
             if (make_attn_work(w.tile, w.attn)) {
               w.is_attn = 1;

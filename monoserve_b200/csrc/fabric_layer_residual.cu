@@ -1,5 +1,6 @@
 // The plain residual of the layer-list decoders, normed before and after each sublayer (fabric_layer_tiles.cuh).
 #include "fabric_layer_tiles.cuh"
+#include "wide_tile.cuh"
 
 namespace mf {
 namespace fab {
@@ -251,21 +252,232 @@ __device__ __noinline__ void residual_rows_ahead(const TileDesc& t, int tid, int
   }
 }
 
-__device__ void tile_residual(const TileDesc& t, int tid, int* scratch) {
+// The same rows through RowStages.  Bound by memory (a row of 2048 with one branch: 16 KB in, 12 KB out); 4096 such rows:
+// 118 -> 68 us, with two branches 174 -> 105.
+template <int NU, bool kTwo>
+__device__ __noinline__ bool residual_bulk(const TileDesc& t, int tid, const LayerCtx& ctx) {
+  __builtin_assume(__isShared(ctx.ring));
+  __builtin_assume(__isShared(ctx.scratch));
+  ResidualArgs A;
+  load_block(A, t.a[0]);
+  const int W = static_cast<int>(A.W), parts0 = static_cast<int>(A.y0_parts), parts1 = kTwo ? static_cast<int>(A.y1_parts) : 0;
+  const int row0 = static_cast<int>(t.i0), rows = static_cast<int>(t.i1);
+  const uint32_t piece = static_cast<uint32_t>(W) * 4;
+  float* const red = reinterpret_cast<float*>(ctx.scratch) + 64;
+  // the weights stay in the ring: what it leaves of the L1 does not hold them from one row to the next
+  constexpr int kWeights = kTwo ? 4 : 2;
+  RowStages pipe(ctx, static_cast<uint32_t>(1 + parts0 + parts1) * piece, rows, tid, kWeights * piece);
+  const float* const weights = reinterpret_cast<const float*>(ctx.ring);   // post_w, w, w0, w1
+  auto fetch = [&](int k, int s) {
+    const size_t r = static_cast<size_t>(row0 + k);
+    uint8_t* to = pipe.stage(s);
+    mbar_arrive_expect_tx(pipe.bar + s, pipe.bytes);
+    bulk_in(to, f32p(A.x) + r * W, piece, pipe.bar + s);
+    for (int q = 0; q < parts0; ++q)
+      bulk_in(to += piece, f32p(A.y0) + (static_cast<size_t>(q) * A.y_rows + r) * W, piece, pipe.bar + s);
+    for (int q = 0; q < parts1; ++q)
+      bulk_in(to += piece, f32p(A.y1) + (static_cast<size_t>(q) * A.y_rows + r) * W, piece, pipe.bar + s);
+  };
+  if (tid == 0) {
+    mbar_expect_tx(pipe.bar, kWeights * piece);   // with the first row
+    const unsigned long long from[4] = {A.post_w, A.w, A.w0, A.w1};
+#pragma unroll
+    for (int i = 0; i < kWeights; ++i) bulk_in(ctx.ring + i * piece, f32p(from[i]), piece, pipe.bar);
+    for (int k = 0; k < pipe.depth; ++k) fetch(k, k);
+  }
+  auto each = [&](auto&& f) {   // f(register piece, first column)
+#pragma unroll
+    for (int i = 0; i < NU; ++i)
+      if ((tid + i * kExecThreads) * 4 < W) f(i, (tid + i * kExecThreads) * 4);
+  };
+  int k = 0;
+  bool ok = true;
+  for (; k < rows; ++k) {
+    const uint32_t r = static_cast<uint32_t>(row0 + k);
+    const int g = A.gather ? reinterpret_cast<const int*>(A.gather)[r] : -1;
+    float x[NU][4], y[NU][4], z[kTwo ? NU : 1][4];
+    float s0 = 0.f, s1 = 0.f;
+    ok = pipe.wait();
+    const float* const in = reinterpret_cast<const float*>(pipe.stage(pipe.at));
+    auto slabs = [&](const float* p, int parts, float (&v)[4]) {
+      ld_vec<4>(p, v);
+      for (int q = 1; q < parts; ++q) {
+        float b[4];
+        ld_vec<4>(p + q * W, b);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] += b[j];
+      }
+    };
+    if (ok)
+      each([&](int i, int c) {
+        ld_vec<4>(in + c, x[i]);
+        slabs(in + W + c, parts0, y[i]);
+        if constexpr (kTwo) slabs(in + (1 + parts0) * W + c, parts1, z[i]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          s0 = fmaf(y[i][j], y[i][j], s0);
+          if constexpr (kTwo) s1 = fmaf(z[i][j], z[i][j], s1);
+        }
+      });
+    // this barrier also carries the decision to go on and the stage's release
+    s0 = warp_sum(s0);
+    s1 = warp_sum(s1);
+    if ((tid & 31) == 0) {
+      red[tid >> 5] = s0;
+      red[4 + (tid >> 5)] = s1;
+    }
+    ok = exec_and(ok);
+    if (!ok) break;
+    if (tid == 0 && k + pipe.depth < rows) {
+      fence_proxy_async_smem();
+      fetch(k + pipe.depth, pipe.at);
+    }
+    pipe.next();
+    s0 = red[0] + red[1] + red[2] + red[3];
+    s1 = red[4] + red[5] + red[6] + red[7];
+    if constexpr (kTwo) {
+      const float inv0 = over_rms(s0, A), inv1 = over_rms(s1, A);
+      s0 = s1 = 0.f;
+      each([&](int i, int c) {
+        float a[4], b[4];
+        ld_vec<4>(weights + 2 * W + c, a);
+        ld_vec<4>(weights + 3 * W + c, b);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          y[i][j] = A.branch_scale * (y[i][j] * inv0 * a[j] + z[i][j] * inv1 * b[j]);
+          s0 = fmaf(y[i][j], y[i][j], s0);
+        }
+      });
+      block_sum2(s0, s1, red + 8, tid);
+    }
+    const float inv = over_rms(s0, A);
+    s0 = s1 = 0.f;
+    each([&](int i, int c) {
+      float w[4];
+      ld_vec<4>(weights + c, w);
+      const size_t at = static_cast<size_t>(r) * W + c;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[i][j] += y[i][j] * inv * w[j];
+        s0 = fmaf(x[i][j], x[i][j], s0);
+      }
+      st_vec<4>(reinterpret_cast<float*>(A.x) + at, x[i]);
+      if (A.sum_out) st_vec<4>(reinterpret_cast<float*>(A.sum_out) + at, x[i]);
+    });
+    block_sum2(s0, s1, red + 16, tid);
+    const float inv_x = over_rms(s0, A);
+    each([&](int i, int c) {
+      float h[4];
+      ld_vec<4>(weights + W + c, h);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = x[i][j] * inv_x * h[j];
+      put_input<4>(A, r, g, c, h);
+    });
+  }
+  pipe.close(tid, ok ? 0 : min(rows - k, pipe.depth));
+  return ok;
+}
+
+// The embedding of rows of at most 512 NU columns, through RowStages as well: the token's row and its position's.
+template <int NU>
+__device__ __noinline__ bool residual_embed(const TileDesc& t, int tid, const LayerCtx& ctx) {
+  __builtin_assume(__isShared(ctx.ring));
+  __builtin_assume(__isShared(ctx.scratch));
+  ResidualArgs A;
+  load_block(A, t.a[0]);
+  const int W = static_cast<int>(A.W), row0 = static_cast<int>(t.i0), rows = static_cast<int>(t.i1);
+  const uint32_t piece = static_cast<uint32_t>(W) * 2;
+  float* const red = reinterpret_cast<float*>(ctx.scratch) + 64;
+  int2* const at = reinterpret_cast<int2*>(ctx.scratch + 128);   // token and position of each row
+  for (int k = tid; k < rows; k += kExecThreads)
+    at[k] = make_int2(reinterpret_cast<const int*>(A.tokens)[row0 + k],
+                      min(reinterpret_cast<const int*>(A.tok_pos)[row0 + k], static_cast<int>(A.max_pos) - 1));
+  RowStages pipe(ctx, (A.pos ? 2 : 1) * piece, rows, tid, 2 * piece);
+  const float* const weights = reinterpret_cast<const float*>(ctx.ring);
+  auto fetch = [&](int k, int s) {
+    uint8_t* const to = pipe.stage(s);
+    const int2 x = at[k];
+    mbar_arrive_expect_tx(pipe.bar + s, pipe.bytes);
+    bulk_in(to, reinterpret_cast<const __nv_bfloat16*>(A.embed) + static_cast<size_t>(x.x) * W, piece, pipe.bar + s);
+    if (A.pos) bulk_in(to + piece, reinterpret_cast<const __nv_bfloat16*>(A.pos) + static_cast<size_t>(x.y) * W, piece, pipe.bar + s);
+  };
+  if (tid == 0) {
+    mbar_expect_tx(pipe.bar, 2 * piece);   // with the first row
+    bulk_in(ctx.ring, f32p(A.w), 2 * piece, pipe.bar);
+    for (int k = 0; k < pipe.depth; ++k) fetch(k, k);
+  }
+  int k = 0;
+  bool ok = true;
+  for (; k < rows; ++k) {
+    const uint32_t r = static_cast<uint32_t>(row0 + k);
+    const int g = A.gather ? reinterpret_cast<const int*>(A.gather)[r] : -1;
+    float x[NU][4], ss = 0.f;
+    ok = pipe.wait();
+    const __nv_bfloat16* const in = reinterpret_cast<const __nv_bfloat16*>(pipe.stage(pipe.at));
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      const int c = (tid + i * kExecThreads) * 4;
+      if (c >= W || !ok) continue;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        x[i][j] = __bfloat162float(in[c + j]) * A.embed_scale + (A.pos ? __bfloat162float(in[W + c + j]) : 0.f);
+        ss = fmaf(x[i][j], x[i][j], ss);
+      }
+      const size_t to = static_cast<size_t>(r) * W + c;
+      st_vec<4>(reinterpret_cast<float*>(A.x) + to, x[i]);
+      if (A.sum_out) st_vec<4>(reinterpret_cast<float*>(A.sum_out) + to, x[i]);
+    }
+    ss = warp_sum(ss);
+    if ((tid & 31) == 0) red[(k & 1) * 4 + (tid >> 5)] = ss;
+    ok = exec_and(ok);
+    if (!ok) break;
+    if (tid == 0 && k + pipe.depth < rows) {
+      fence_proxy_async_smem();
+      fetch(k + pipe.depth, pipe.at);
+    }
+    pipe.next();
+    const float* const sums = red + (k & 1) * 4;
+    const float inv = over_rms(sums[0] + sums[1] + sums[2] + sums[3], A);
+#pragma unroll
+    for (int i = 0; i < NU; ++i) {
+      const int c = (tid + i * kExecThreads) * 4;
+      if (c >= W) continue;
+      float h[4];
+      ld_vec<4>(weights + c, h);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) h[j] = x[i][j] * inv * h[j];
+      put_input<4>(A, r, g, c, h);
+    }
+  }
+  pipe.close(tid, ok ? 0 : min(rows - k, pipe.depth));
+  return ok;
+}
+
+__device__ bool tile_residual(const TileDesc& t, int tid, const LayerCtx& ctx) {
+  int* const scratch = ctx.scratch;
   const ResidualArgs* p = reinterpret_cast<const ResidualArgs*>(t.a[0]);
-  const uint32_t W = __ldcg(&p->W);
-  const bool two = __ldcg(&p->y1_parts) != 0;
-  if (__ldcg(&p->embed) == 0 && (W & 3) == 0 && W <= 2048) {
+  const uint32_t W = __ldcg(&p->W), parts0 = __ldcg(&p->y0_parts), parts1 = __ldcg(&p->y1_parts);
+  const bool two = parts1 != 0, four = (W & 3) == 0, embed = __ldcg(&p->embed) != 0;
+  // two rows in the ring at least, or nothing overlaps
+  const bool bulk = t.i1 >= kBulkRows && parts0 > 0 && (2 * (1 + parts0 + parts1) + (two ? 4 : 2)) * W * 4 <= kWideRingBytes;
+  // (W % 8: whole 16-byte pieces of bf16 rows)
+  if (embed && __ldcg(&p->step) == 0 && t.i1 >= kBulkRows && t.i1 <= 256 && (W & 7) == 0 && W <= 4096 &&
+      ((__ldcg(&p->embed) | __ldcg(&p->pos)) & 15) == 0)
+    return W <= 2048 ? residual_embed<4>(t, tid, ctx) : residual_embed<8>(t, tid, ctx);
+  if (!embed && four && W <= 2048) {
+    if (bulk) return two ? residual_bulk<4, true>(t, tid, ctx) : residual_bulk<4, false>(t, tid, ctx);
     if (two) residual_rows_ahead<4, true>(t, tid, scratch);
     else residual_rows_ahead<4, false>(t, tid, scratch);
-  } else if (__ldcg(&p->embed) == 0 && (W & 3) == 0 && W <= 4096) {
+  } else if (!embed && four && W <= 4096) {
+    if (bulk) return two ? residual_bulk<8, true>(t, tid, ctx) : residual_bulk<8, false>(t, tid, ctx);
     if (two) residual_rows_ahead<8, true>(t, tid, scratch);
     else residual_rows_ahead<8, false>(t, tid, scratch);
-  } else if ((W & 3) == 0) {
+  } else if (four) {
     residual_rows<4>(t, tid, scratch);
   } else {
     residual_rows<1>(t, tid, scratch);
   }
+  return true;
 }
 
 }  // namespace fab

@@ -39,12 +39,19 @@ struct LayerCtx {
 // Runs tile kinds kTileProduct32 .. kTileHeadGate: false for a kind or size these tiles do not take, or when a bounded
 // wait gave up.  All exec threads call it with the same tile.
 __device__ bool run_layer_tile(const TileDesc& t, int tid, const LayerCtx& ctx);
+// Row tiles of at least this many rows bring them through the operand ring (RowStages): a step's few rows would wait for the
+// ring's earlier users and gain nothing.
+constexpr uint32_t kBulkRows = 4, kCombineRows = 16, kLogitsRows = 9;
 // Wide tiles: their exec warps use the operand ring as scratch memory, and TMEM.
-__device__ __forceinline__ bool tile_is_wide(uint32_t kind) {
+__device__ __forceinline__ bool tile_is_wide(const TileDesc& t) {
+  const uint32_t kind = t.kind, rows = t.i1;
+  if (kind == kTileStreams || kind == kTileResidual) return rows >= kBulkRows;
+  if (kind == kTileCombine) return rows >= kCombineRows;
+  if (kind == kTileRouterLogits) return rows >= kLogitsRows && t.i2 == 0 && t.i3 == 0;
   return kind == kTileMemory || kind == kTileScan || kind == kTileGatedMemory || kind == kTileGatedStep || kind == kTileLatentMma || kind == kTileLatentDirect;
 }
 
-__device__ void tile_streams(const TileDesc& t, int tid, int* scratch);
+__device__ bool tile_streams(const TileDesc& t, int tid, const LayerCtx& ctx);
 __device__ void tile_product32(const TileDesc& t, int tid, int* scratch);
 __device__ void tile_gated_act(const TileDesc& t, int tid);
 __device__ void tile_sum_slabs(const TileDesc& t, int tid);
@@ -59,7 +66,7 @@ __device__ bool tile_latent_attn(const TileDesc& t, int tid);
 __device__ bool tile_latent_mma(const TileDesc& t, int tid, const LayerCtx& ctx);
 __device__ bool tile_latent_direct(const TileDesc& t, int tid, const LayerCtx& ctx);
 __device__ void tile_latent_merge(const TileDesc& t, int tid);
-__device__ void tile_residual(const TileDesc& t, int tid, int* scratch);
+__device__ bool tile_residual(const TileDesc& t, int tid, const LayerCtx& ctx);
 __device__ void tile_decay(const TileDesc& t, int tid);
 __device__ bool tile_gated_memory(const TileDesc& t, int tid, uint8_t* ring);
 __device__ bool tile_gated_step(const TileDesc& t, int tid, const LayerCtx& ctx);

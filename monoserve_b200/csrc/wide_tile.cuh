@@ -76,12 +76,58 @@ __device__ __forceinline__ void bulk_in(void* smem, const void* gmem, uint32_t b
                "l"(gmem), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
 }
+// More bytes for the barrier's current phase, without an arrival.
+__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.expect_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
 template <int N>
 __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void tmem_st_done() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void mbar_inval(uint64_t* bar) {
   asm volatile("mbarrier.inval.shared::cta.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
+
+// The rows of a row-wise tile, one after the other through stages of the operand ring.  128 threads cannot hold enough loads
+// of their own in flight to draw an SM's share of the memory bandwidth; bulk copies, issued by thread 0 as far ahead as the
+// ring holds rows, can.  Barriers in the first 2 kRowStages ints of the scratch.
+constexpr uint32_t kWideRingBytes = 216 * 1024;
+constexpr int kRowStages = 12;
+struct RowStages {
+  uint8_t* ring;
+  uint64_t* bar;
+  volatile int* abort_flag;
+  uint32_t bytes, head;    // of a row; of what the tile keeps in front of the stages
+  int depth, rows;
+  int at = 0;              // stage of the current row
+  uint32_t phase = 0;
+
+  // Rows whose stages are not filled yet are for the caller to fetch: the first `depth`, then one per `next`.
+  __device__ __forceinline__ RowStages(const LayerCtx& ctx, uint32_t row_bytes, int n_rows, int tid, uint32_t head_bytes = 0)
+      : ring(ctx.ring), bar(reinterpret_cast<uint64_t*>(ctx.scratch)), abort_flag(ctx.abort_flag), bytes(row_bytes), head(head_bytes),
+        depth(min(min(kRowStages, n_rows), static_cast<int>((kWideRingBytes - head_bytes) / row_bytes))), rows(n_rows) {
+    fence_proxy_async_all();   // the rows may have been written, and the ring used, by plain loads and stores
+    if (tid < depth) mbar_init(bar + tid, 1);
+    fence_barrier_init();
+    exec_sync();
+  }
+  __device__ __forceinline__ uint8_t* stage(int s) const { return ring + head + static_cast<uint32_t>(s) * bytes; }
+  __device__ __forceinline__ bool wait() const { return mbar_wait_bounded(bar + at, phase, abort_flag, kWideWaitNs); }
+  __device__ __forceinline__ void next() {
+    if (++at == depth) {
+      at = 0;
+      phase ^= 1u;
+    }
+  }
+  // After the last row (left == 0), or with `left` rows fetched and not waited for: their copies land, or run out of time.
+  __device__ __forceinline__ void close(int tid, int left) {
+    for (; left > 0; --left) {
+      for (int tries = 0; tries < 1 << 16 && !mbar_try_wait(bar + at, phase); ++tries) {}
+      next();
+    }
+    exec_sync();
+    if (tid < depth) mbar_inval(bar + tid);
+  }
+};
 
 }  // namespace fab
 }  // namespace mf

@@ -295,6 +295,14 @@ class LaneBase:
             return max(1, -(-T // nw))
         return -(-(-(-T // (2 * nw))) // 4) * 4
 
+    def _per_streamed(self, T):
+        """Rows per tile of a stage whose tiles stream their rows through the operand ring: as many as make one round of
+        tiles over the workers (a tile starts with an empty ring), up to 64."""
+        nw = self.fab.num_workers
+        if T <= 4 * nw:
+            return self._per(T)
+        return -(-T // (nw * -(-T // (64 * nw))))
+
     def _one(self, kind, args):
         """The single tile of an expand or plan stage."""
         key = ("one", kind)

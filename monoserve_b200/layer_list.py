@@ -814,7 +814,7 @@ class LayerListLane(LaneBase):
             if split:
                 f.update(split=self.split)
         args = self._dev("StreamArgs" if streams else "ResidualArgs", **f)
-        s = p.stage(self._rows(K_STREAMS if streams else K_RESIDUAL, args, rows, self._per(rows)), label=label)
+        s = p.stage(self._rows(K_STREAMS if streams else K_RESIDUAL, args, rows, self._per_streamed(rows)), label=label)
         if prev is not None:
             for stage in prev if isinstance(prev, list) else [prev]:
                 p.after(stage, s)
