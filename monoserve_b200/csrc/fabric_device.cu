@@ -38,6 +38,7 @@
 #include "operands.h"
 #include "ptx.cuh"
 #include "rowwise.cuh"
+#include "wide_tile.cuh"
 
 namespace mf {
 namespace fab {
@@ -188,9 +189,9 @@ namespace fab {
 
 __device__ void tile_router(const TileDesc& t, int tid);
 __device__ void tile_norm(const TileDesc& t, int tid, bool add);
-__device__ void tile_router_logits(const TileDesc& t, int tid);
+__device__ bool tile_router_projection(const TileDesc& t, int tid, const LayerCtx& ctx);
 __device__ void tile_permute(const TileDesc& t, int tid);
-__device__ void tile_combine(const TileDesc& t, int tid);
+__device__ bool tile_combine(const TileDesc& t, int tid, uint8_t* ring, volatile int* abort_flag);
 __device__ void tile_asym_reduce(const TileDesc& t, int tid);
 __device__ void tile_norm_logits(const TileDesc& t, int tid);
 __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState& S, int tid);
@@ -249,8 +250,7 @@ __device__ bool run_core_tile(DeviceState& S, const WorkSlot& w, int tid, uint32
       tile_router(t, tid);
       return true;
     case kTileRouterLogits:
-      tile_router_logits(t, tid);
-      return true;
+      return tile_router_projection(t, tid, LayerCtx{s_exec_scratch, ring, tmem_base, abort_flag});
     case kTilePermute:
       tile_permute(t, tid);
       return true;
@@ -346,96 +346,85 @@ __device__ void tile_router(const TileDesc& t, int tid) {
 // Router projection tile (kind 48; not in the reference, whose router GEMM sums
 // K-split partials with atomics): logits[t][e] for rows [i0, i0 + i1) and experts
 // [i2, i2 + i3) (i3 = 0: all), lane l summing h = 256 j + 8 l + i in order with fmaf, then
-// the xor butterfly: the same bits as the stream kernel and the oracle.  A warp keeps one
-// expert's weight row in registers and walks the tile's rows, so the weights are read
-// once per tile and the activation rows come from L1.
-template <int J>
-__device__ __forceinline__ void router_logits_rows(const __nv_bfloat16* x, const __nv_bfloat16* wr, float* logits, int H,
-                                                   int E, int r0, int rows, int e_lo, int e_hi, int warp, int lane) {
-  if constexpr (J > 0) {
-    // two experts' weight rows in registers, two activation rows at a time: four independent
-    // fmaf chains per lane, each in the defined order
-    for (int e = e_lo + 2 * warp; e < e_hi; e += 2 * (kExecThreads / 32)) {
-      const bool two_e = e + 1 < e_hi;
-      const uint4* wa = reinterpret_cast<const uint4*>(wr + static_cast<size_t>(e) * H);
-      const uint4* wb = reinterpret_cast<const uint4*>(wr + static_cast<size_t>(two_e ? e + 1 : e) * H);
-      uint4 wva[J > 0 ? J : 1], wvb[J > 0 ? J : 1];
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        wva[j] = __ldg(wa + 32 * j + lane);
-        wvb[j] = __ldg(wb + 32 * j + lane);
-      }
-      for (int r = r0; r < r0 + rows; r += 2) {
-        const bool two_r = r + 1 < r0 + rows;
-        const uint4* xa = reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * H);
-        const uint4* xb = reinterpret_cast<const uint4*>(x + static_cast<size_t>(two_r ? r + 1 : r) * H);
-        float a00 = 0.f, a01 = 0.f, a10 = 0.f, a11 = 0.f;   // a[row][expert]
-#pragma unroll
-        for (int j = 0; j < J; ++j) {
-          float x0[8], x1[8], w0[8], w1[8];
-          unpack8(xa[32 * j + lane], x0);
-          unpack8(xb[32 * j + lane], x1);
-          unpack8(wva[j], w0);
-          unpack8(wvb[j], w1);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            a00 = __fmaf_rn(x0[i], w0[i], a00);
-            a01 = __fmaf_rn(x0[i], w1[i], a01);
-            a10 = __fmaf_rn(x1[i], w0[i], a10);
-            a11 = __fmaf_rn(x1[i], w1[i], a11);
-          }
-        }
-        a00 = warp_sum_xor(a00);
-        a01 = warp_sum_xor(a01);
-        a10 = warp_sum_xor(a10);
-        a11 = warp_sum_xor(a11);
-        if (lane == (e & 31)) {
-          logits[static_cast<size_t>(r) * E + e] = a00;
-          if (two_r) logits[static_cast<size_t>(r + 1) * E + e] = a10;
-        }
-        if (two_e && lane == ((e + 1) & 31)) {
-          logits[static_cast<size_t>(r) * E + e + 1] = a01;
-          if (two_r) logits[static_cast<size_t>(r + 1) * E + e + 1] = a11;
-        }
-      }
-    }
-  } else {
-    const int nj = H / 256;
-    for (int e = e_lo + warp; e < e_hi; e += kExecThreads / 32) {
-      const uint4* w4 = reinterpret_cast<const uint4*>(wr + static_cast<size_t>(e) * H);
-      for (int r = r0; r < r0 + rows; ++r) {
-        const uint4* x4 = reinterpret_cast<const uint4*>(x + static_cast<size_t>(r) * H);
-        float acc = 0.f;
-        for (int j = 0; j < nj; ++j) {
-          float xf[8], wf[8];
-          unpack8(x4[32 * j + lane], xf);
-          unpack8(__ldg(w4 + 32 * j + lane), wf);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) acc = __fmaf_rn(xf[i], wf[i], acc);
-        }
-        acc = warp_sum_xor(acc);
-        if (lane == (e & 31)) logits[static_cast<size_t>(r) * E + e] = acc;
-      }
-    }
+// the xor butterfly: the same bits as the stream kernel and the oracle.  A warp takes four experts and up to eight rows at a
+// time (router_block).
+//
+// Many rows against all experts (router_logits_bulk): 4 R rows stay in the ring, a quarter to each warp, and the weights come
+// past them four experts at a time.  From global memory every block of eight rows and four experts reads both again, which
+// the L2 bounds (the L1 beside the ring holds neither): 4096 rows x 128 experts, H = 2048, 171 -> 120 us (264 with a
+// row's loads and conversions for every two products).
+template <int R>
+__device__ __noinline__ bool router_logits_bulk(const TileDesc& t, int tid, const LayerCtx& ctx) {
+  __builtin_assume(__isShared(ctx.ring));
+  LogitsArgs A;
+  load_block(A, t.a[0]);
+  const int H = static_cast<int>(A.H), E = static_cast<int>(A.E), rows = static_cast<int>(t.i1), warp = tid >> 5;
+  const int groups = (E + 3) / 4;
+  const __nv_bfloat16* const wr = reinterpret_cast<const __nv_bfloat16*>(A.wr);
+  RowStages pipe(ctx, 8u * H, groups, tid, 8u * R * H);
+  auto fetch = [&](int k, int s) {
+    const uint32_t bytes = 2u * H * min(4, E - 4 * k);
+    mbar_arrive_expect_tx(pipe.bar + s, bytes);
+    bulk_in(pipe.stage(s), wr + static_cast<size_t>(4 * k) * H, bytes, pipe.bar + s);
+  };
+  if (tid == 0) {
+    mbar_expect_tx(pipe.bar, 2u * H * rows);   // with the first weights
+    bulk_in(ctx.ring, reinterpret_cast<const __nv_bfloat16*>(A.x) + static_cast<size_t>(t.i0) * H, 2u * H * rows, pipe.bar);
+    for (int k = 0; k < pipe.depth; ++k) fetch(k, k);
   }
+  const __nv_bfloat16* const x = reinterpret_cast<const __nv_bfloat16*>(ctx.ring);
+  float* const out = reinterpret_cast<float*>(A.logits) + static_cast<size_t>(t.i0) * E;
+  int k = 0;
+  bool ok = true;
+  for (; k < groups; ++k) {
+    ok = pipe.wait();
+    ok = __all_sync(0xffffffffu, ok);
+    if (ok && R * warp < rows)
+      router_block<R, 4, false, true>(x, reinterpret_cast<const __nv_bfloat16*>(pipe.stage(pipe.at)), out + 4 * k, H, E, R * warp,
+                                      min(rows, R * warp + R), 0, min(4, E - 4 * k));
+    ok = exec_and(ok);
+    if (!ok) break;
+    if (tid == 0 && k + pipe.depth < groups) {
+      fence_proxy_async_smem();
+      fetch(k + pipe.depth, pipe.at);
+    }
+    pipe.next();
+  }
+  pipe.close(tid, ok ? 0 : min(groups - k, pipe.depth));
+  return ok;
 }
 
-__device__ void tile_router_logits(const TileDesc& t, int tid) {
+__device__ __noinline__ void tile_router_logits(const TileDesc& t, int tid) {
   LogitsArgs A;   // a copy in registers: the block lives in global memory
   load_block(A, t.a[0]);
-  const int warp = tid >> 5, lane = tid & 31;
+  const int warp = tid >> 5;
   const int H = static_cast<int>(A.H), E = static_cast<int>(A.E);
   const __nv_bfloat16* x = reinterpret_cast<const __nv_bfloat16*>(A.x);
   const __nv_bfloat16* wr = reinterpret_cast<const __nv_bfloat16*>(A.wr);
   float* logits = reinterpret_cast<float*>(A.logits);
   const int e_lo = static_cast<int>(t.i2), e_hi = t.i3 ? min(E, e_lo + static_cast<int>(t.i3)) : E;
   const int r0 = static_cast<int>(t.i0), rows = static_cast<int>(t.i1);
-  switch (H / 256) {
-    case 2: router_logits_rows<2>(x, wr, logits, H, E, r0, rows, e_lo, e_hi, warp, lane); break;
-    case 4: router_logits_rows<4>(x, wr, logits, H, E, r0, rows, e_lo, e_hi, warp, lane); break;
-    case 8: router_logits_rows<8>(x, wr, logits, H, E, r0, rows, e_lo, e_hi, warp, lane); break;
-    default: router_logits_rows<0>(x, wr, logits, H, E, r0, rows, e_lo, e_hi, warp, lane); break;
+  for (int e = e_lo + 4 * warp; e < e_hi; e += 4 * (kExecThreads / 32)) {
+    const int e_end = min(e_hi, e + 4);
+    for (int r = r0; r < r0 + rows; r += 8) {
+      const int r_end = min(r0 + rows, r + 8);
+      if (r_end - r > 4) router_block<8, 4, true>(x, wr, logits, H, E, r, r_end, e, e_end);
+      else if (r_end - r > 1) router_block<4, 4, true>(x, wr, logits, H, E, r, r_end, e, e_end);
+      else router_block<1, 4, true>(x, wr, logits, H, E, r, r_end, e, e_end);
+    }
   }
+}
+
+__device__ bool tile_router_projection(const TileDesc& t, int tid, const LayerCtx& ctx) {
+  const LogitsArgs* p = reinterpret_cast<const LogitsArgs*>(t.a[0]);
+  const uint32_t H = __ldcg(&p->H);
+  if (t.i1 >= kLogitsRows && t.i2 == 0 && t.i3 == 0 && ((__ldcg(&p->x) | __ldcg(&p->wr)) & 15) == 0) {
+    // a quarter of the rows per warp in registers; in the ring all of them and two groups of weights
+    if (t.i1 <= 16 && (32 + 16) * H <= kWideRingBytes) return router_logits_bulk<4>(t, tid, ctx);
+    if (t.i1 <= 32 && (64 + 16) * H <= kWideRingBytes) return router_logits_bulk<8>(t, tid, ctx);
+  }
+  tile_router_logits(t, tid);
+  return true;
 }
 
 // Permute tile (kind 40, csrc/fabric/tiles/aux.cuh:648-684, PermuteArgs) for rows

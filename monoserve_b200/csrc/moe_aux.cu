@@ -23,61 +23,75 @@
 #include "detmath.cuh"
 #include "kernels.h"
 #include "peer_sync.cuh"
+#include "ptx.cuh"
 #include "rowwise.cuh"
 
 namespace mf {
 
 // ------------------------------------------------------------ router logits
-// One warp computes the logits of one token against kExpertsPerWarp experts.
-// Lane l owns elements h = 256 j + 8 l + i (j outer, i = 0..7 inner) and
-// accumulates them in that order with fused multiply-adds into one fp32
-// partial; the 32 partials are summed by the xor butterfly 16, 8, 4, 2, 1.
-constexpr int kExpertsPerWarp = 16;
-
-template <int J>
-__global__ void __launch_bounds__(256) router_logits_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wr,
+// A warp per R tokens x C experts (rowwise.cuh), four expert groups side by side in a block.  The tile is the largest that
+// still gives most schedulers a warp: its products per load grow with it, but a decode batch has few of them.
+template <int R, int C>
+__global__ void __launch_bounds__(128) router_logits_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wr,
                                                             float* __restrict__ logits, int T, int H, int E) {
   chain_release();
   chain_wait();
-  const int lane = threadIdx.x & 31;
-  const int groups = (E + kExpertsPerWarp - 1) / kExpertsPerWarp;
-  const long long unit = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (unit >= static_cast<long long>(T) * groups) return;
-  const int t = static_cast<int>(unit / groups), eg = static_cast<int>(unit % groups);
-  const int nj = J > 0 ? J : H / 256;
-  const uint4* x4 = reinterpret_cast<const uint4*>(x + static_cast<size_t>(t) * H);
-  float xr[J > 0 ? J : 1][8];
-  if (J > 0) {
+  const int warp = threadIdx.x >> 5, quads = (E + 4 * C - 1) / (4 * C);
+  const int t0 = static_cast<int>(blockIdx.x) / quads * R, e0 = (static_cast<int>(blockIdx.x) % quads * 4 + warp) * C;
+  if (t0 < T && e0 < E) router_block<R, C, false>(x, wr, logits, H, E, t0, min(T, t0 + R), e0, min(E, e0 + C));
+}
+
+// Many tokens: 16 warps of 4 tokens x 8 experts share 16 tokens x 32 experts, whose columns come 256 at a time through four
+// stages of shared memory (each warp loading its own: bound by the latency of those loads, 8192 x 128 x 2048 in 180 us against 145).
+constexpr int kStagedTokens = 16, kStagedExperts = 32, kStagedRows = kStagedTokens + kStagedExperts, kStagedDepth = 4;
+constexpr int kStagedBytes = kStagedDepth * kStagedRows * 512;
+
+__global__ void __launch_bounds__(512) router_logits_staged_kernel(const bf16* __restrict__ x, const bf16* __restrict__ wr,
+                                                                   float* __restrict__ out, int T, int H, int E) {
+  extern __shared__ __align__(16) uint8_t staged[];
+  chain_release();
+  chain_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nj = H / 256, blocks_e = (E + kStagedExperts - 1) / kStagedExperts;
+  const int t0 = static_cast<int>(blockIdx.x) / blocks_e * kStagedTokens, e0 = static_cast<int>(blockIdx.x) % blocks_e * kStagedExperts;
+  constexpr int kCopies = kStagedRows * 32 / 512;   // 16-byte pieces of a stage per thread: a row per warp and round
+  const bf16* from[kCopies];
 #pragma unroll
-    for (int j = 0; j < J; ++j) unpack8(x4[32 * j + lane], xr[j]);
+  for (int i = 0; i < kCopies; ++i) {
+    const int row = warp + 16 * i;                   // tokens, then experts; those past the end repeat the last
+    from[i] = (row < kStagedTokens ? x + static_cast<size_t>(min(t0 + row, T - 1)) * H
+                                   : wr + static_cast<size_t>(min(e0 + row - kStagedTokens, E - 1)) * H) + 8 * lane;
   }
-  const int e_hi = min(E, (eg + 1) * kExpertsPerWarp);
-  for (int e = eg * kExpertsPerWarp; e < e_hi; ++e) {
-    const uint4* w4 = reinterpret_cast<const uint4*>(wr + static_cast<size_t>(e) * H);
-    float acc = 0.f;
-    if (J > 0) {
-      uint4 wv[J > 0 ? J : 1];
+  auto stage = [&](int j) {
+    if (j < nj) {
 #pragma unroll
-      for (int j = 0; j < J; ++j) wv[j] = __ldg(w4 + 32 * j + lane);
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        float wf[8];
-        unpack8(wv[j], wf);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc = __fmaf_rn(xr[j][i], wf[i], acc);
-      }
-    } else {
-      for (int j = 0; j < nj; ++j) {
-        float xf[8], wf[8];
-        unpack8(x4[32 * j + lane], xf);
-        unpack8(__ldg(w4 + 32 * j + lane), wf);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) acc = __fmaf_rn(xf[i], wf[i], acc);
+      for (int i = 0; i < kCopies; ++i) {
+        const uint8_t* const to = staged + ((j % kStagedDepth) * kStagedRows + warp + 16 * i) * 512 + lane * 16;
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(to)), "l"(from[i] + 256 * j) : "memory");
       }
     }
-    acc = warp_sum_xor(acc);
-    if (lane == (e & 31)) logits[static_cast<size_t>(t) * E + e] = acc;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  for (int j = 0; j < kStagedDepth - 1; ++j) stage(j);
+  logits::Sums<4, 8> sums;
+  for (int j = 0; j < nj; ++j) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kStagedDepth - 2) : "memory");
+    __syncthreads();   // stage j is there, and stage j - 1 has been read by all
+    stage(j + kStagedDepth - 1);
+    const uint4* const in = reinterpret_cast<const uint4*>(staged + (j % kStagedDepth) * kStagedRows * 512) + lane;
+    logits::Columns<4, 8> k;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) k.x[r] = in[((warp >> 2) * 4 + r) * 32];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) k.w[c] = in[(kStagedTokens + (warp & 3) * 8 + c) * 32];
+    sums.multiply(k);
   }
+  sums.store(out, E, t0 + (warp >> 2) * 4, T, e0 + (warp & 3) * 8, E);
+}
+
+template <int R, int C>
+static cudaError_t launch_router_tiles(const bf16* x, const bf16* wr, float* logits, int T, int H, int E, cudaStream_t stream) {
+  const int blocks = (T + R - 1) / R * ((E + 4 * C - 1) / (4 * C));
+  return launch_chained(router_logits_kernel<R, C>, blocks, 128, 0, stream, x, wr, logits, T, H, E);
 }
 
 // -------------------------------------------------------------- router top-k
@@ -426,18 +440,22 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineParams A) {
 cudaError_t launch_router_logits(const void* x, const void* wr, float* logits, int T, int H, int E,
                                  cudaStream_t stream) {
   if (T == 0) return cudaSuccess;
-  const int groups = (E + kExpertsPerWarp - 1) / kExpertsPerWarp;
-  const long long units = static_cast<long long>(T) * groups;
-  const int blocks = static_cast<int>((units + 7) / 8);
   const bf16* xb = static_cast<const bf16*>(x);
   const bf16* wb = static_cast<const bf16*>(wr);
-  switch (H / 256) {
-    case 2: return launch_chained(router_logits_kernel<2>, blocks, 256, 0, stream, xb, wb, logits, T, H, E);
-    case 4: return launch_chained(router_logits_kernel<4>, blocks, 256, 0, stream, xb, wb, logits, T, H, E);
-    case 8: return launch_chained(router_logits_kernel<8>, blocks, 256, 0, stream, xb, wb, logits, T, H, E);
-    case 16: return launch_chained(router_logits_kernel<16>, blocks, 256, 0, stream, xb, wb, logits, T, H, E);
-    default: return launch_chained(router_logits_kernel<0>, blocks, 256, 0, stream, xb, wb, logits, T, H, E);
+  constexpr long long kWarps = 4 * 148;
+  const long long n = static_cast<long long>(T) * E;
+  if (n >= 32 * 4 * kWarps) {   // a block of 16 warps for every SM
+    static PerDeviceOnce once;
+    const cudaError_t err = once.run([] {
+      return cudaFuncSetAttribute(router_logits_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagedBytes);
+    });
+    if (err != cudaSuccess) return err;
+    const int blocks = (T + kStagedTokens - 1) / kStagedTokens * ((E + kStagedExperts - 1) / kStagedExperts);
+    return launch_chained(router_logits_staged_kernel, blocks, 512, kStagedBytes, stream, xb, wb, logits, T, H, E);
   }
+  if (n >= 32 * kWarps) return launch_router_tiles<4, 8>(xb, wb, logits, T, H, E, stream);
+  if (n >= 8 * kWarps) return launch_router_tiles<2, 4>(xb, wb, logits, T, H, E, stream);
+  return launch_router_tiles<1, 1>(xb, wb, logits, T, H, E, stream);
 }
 
 cudaError_t launch_router_topk(const RouterParams& A, cudaStream_t stream) {

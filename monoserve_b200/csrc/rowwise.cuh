@@ -27,6 +27,142 @@ __device__ __forceinline__ uint4 pack8(const float f[8]) {
   return u;
 }
 
+// Router projection of R tokens x C experts by one warp: logits[t][e] = sum_h x[t][h] wr[e][h] in the order that defines its
+// bits: lane l sums h = 256 j + 8 l + i (j outer, i = 0..7 inner) in one fmaf chain, the 32 sums are added by the xor
+// butterfly 16, 8, 4, 2, 1 (a sum of two lanes is the same in both, so each lane may keep half of its values at a step and
+// the R C sums take R C + log steps, not five each).  Bound by the fp32 units; at one expert a token row (C = 1) it was
+// bound by the loads and conversions of the weights, one per product.  The products of two experts go as packed pairs, each
+// half rounded like the scalar instruction, which leaves issue slots to the conversions.  kAhead: the next 256 columns'
+// loads are issued before this one's products (a lone warp per scheduler has nothing else to hide them behind).  kShared: x
+// and wr are in shared memory.
+// 8192 tokens x 128 experts, H = 2048: 326 -> 145 us; one token 16 -> 6.5.
+namespace logits {
+
+using Pair = unsigned long long;
+__device__ __forceinline__ Pair pair(uint32_t a, uint32_t b) {
+  Pair r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b));
+  return r;
+}
+__device__ __forceinline__ Pair fma_pair(Pair a, Pair b, Pair c) {
+  Pair r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// N values per lane, N a power of two: lane l ends with the sum over the warp of value l / (32 / N) (N <= 32).
+template <int N>
+__device__ __forceinline__ float sum_each(float (&v)[N], int lane) {
+#pragma unroll
+  for (int half = N / 2, bit = 16; half >= 1; half >>= 1, bit >>= 1) {
+    const bool hi = lane & bit;
+#pragma unroll
+    for (int c = 0; c < half; ++c) {
+      const float give = hi ? v[c] : v[c + half], have = hi ? v[c + half] : v[c];
+      v[c] = __fadd_rn(have, __shfl_xor_sync(0xffffffffu, give, bit));
+    }
+  }
+#pragma unroll
+  for (int bit = 16 / N; bit >= 1; bit >>= 1) v[0] = __fadd_rn(v[0], __shfl_xor_sync(0xffffffffu, v[0], bit));
+  return v[0];
+}
+
+template <int R, int C>
+struct Columns {   // 8 columns a lane of R token rows and C weight rows
+  uint4 x[R], w[C];
+};
+
+template <int R, int C>
+struct Sums {
+  static_assert(R * C <= 32 && (C == 1 || C % 2 == 0), "a sum per lane, experts in pairs");
+  static constexpr int P = C > 1 ? C / 2 : 1;
+  Pair acc[R][P];   // C = 1: the upper halves stay zero
+  __device__ __forceinline__ Sums() {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int p = 0; p < P; ++p) acc[r][p] = 0ull;
+  }
+  __device__ __forceinline__ void multiply(const Columns<R, C>& k) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {   // a word: columns 2 q and 2 q + 1
+      auto word = [&](const uint4& v) { return q == 0 ? v.x : q == 1 ? v.y : q == 2 ? v.z : v.w; };
+      Pair lo[P], hi[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const uint32_t a = word(k.w[p * 2]), b = C > 1 ? word(k.w[C > 1 ? p * 2 + 1 : 0]) : 0u;
+        lo[p] = pair(a << 16, b << 16);
+        hi[p] = pair(a & 0xffff0000u, b & 0xffff0000u);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t v = word(k.x[r]);
+        const Pair x_lo = pair(v << 16, v << 16), x_hi = pair(v & 0xffff0000u, v & 0xffff0000u);
+#pragma unroll
+        for (int p = 0; p < P; ++p) acc[r][p] = fma_pair(x_lo, lo[p], acc[r][p]);
+#pragma unroll
+        for (int p = 0; p < P; ++p) acc[r][p] = fma_pair(x_hi, hi[p], acc[r][p]);
+      }
+    }
+  }
+  // Tokens [t0, t_end) (at most R), experts [e0, e_end) (at most C).
+  __device__ __forceinline__ void store(float* out, int E, int t0, int t_end, int e0, int e_end) {
+    const int lane = threadIdx.x & 31;
+    float v[R * C];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        v[r * C + 2 * p] = __uint_as_float(static_cast<uint32_t>(acc[r][p]));
+        if constexpr (C > 1) v[r * C + 2 * p + 1] = __uint_as_float(static_cast<uint32_t>(acc[r][p] >> 32));
+      }
+    const float sum = sum_each<R * C>(v, lane);
+    constexpr int kPer = 32 / (R * C);
+    const int n = lane / kPer, t = t0 + n / C, e = e0 + n % C;
+    if (lane % kPer == 0 && t < t_end && e < e_end) out[static_cast<size_t>(t) * E + e] = sum;
+  }
+};
+
+}  // namespace logits
+
+// Tokens [t0, t_end) (at most R of them; the last is repeated for those missing), experts [e0, e_end) (at most C).
+template <int R, int C, bool kAhead, bool kShared = false>
+__device__ __forceinline__ void router_block(const __nv_bfloat16* x, const __nv_bfloat16* wr, float* out, int H, int E, int t0,
+                                             int t_end, int e0, int e_end) {
+  using namespace logits;
+  const int lane = threadIdx.x & 31, nj = H / 256;
+  const uint4 *xp[R], *wp[C];
+#pragma unroll
+  for (int r = 0; r < R; ++r) xp[r] = reinterpret_cast<const uint4*>(x + static_cast<size_t>(min(t0 + r, t_end - 1)) * H) + lane;
+#pragma unroll
+  for (int c = 0; c < C; ++c) wp[c] = reinterpret_cast<const uint4*>(wr + static_cast<size_t>(min(e0 + c, e_end - 1)) * H) + lane;
+  auto load = [&](int j, Columns<R, C>& k) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) k.x[r] = xp[r][32 * j];
+#pragma unroll
+    for (int c = 0; c < C; ++c) k.w[c] = kShared ? wp[c][32 * j] : __ldg(wp[c] + 32 * j);
+  };
+  Sums<R, C> sums;
+  if constexpr (kAhead) {
+    Columns<R, C> k, next;
+    load(0, next);
+#pragma unroll 1
+    for (int j = 0; j < nj; ++j) {
+      k = next;
+      load(min(j + 1, nj - 1), next);
+      sums.multiply(k);
+    }
+  } else {
+#pragma unroll(R * C >= 16 ? 1 : 8 / R)
+    for (int j = 0; j < nj; ++j) {
+      Columns<R, C> k;
+      load(j, k);
+      sums.multiply(k);
+    }
+  }
+  sums.store(out, E, t0, t_end, e0, e_end);
+}
+
 // Routing of one token by one warp: what the reference's router tile computes
 // (csrc/fabric/tiles/aux.cuh:326-417): scores = softmax of the E <= 256 logits, or their sigmoid with
 // an optional selection bias; K <= 16 picks, each the best remaining selection score with the lowest

@@ -20,10 +20,10 @@ import torch
 
 from monoserve_b200 import _C
 from monoserve_b200.attention import SCALE_LOG2, fabric_maps, fabric_tiles, plan_items
-from monoserve_b200.fabric import Program, Tile
+from monoserve_b200.fabric import Program, Tile, tile_array
 from monoserve_b200.fabric.args import pack
 from monoserve_b200.lane import SUB, logits_tiles
-from monoserve_b200.lane_base import (EPI_F32, EPI_ROWS_F32, EPI_SILU_MUL, EPI_STORE, HEIGHTS, K_SAMPLE, SPLIT_PARTS,  # noqa: F401
+from monoserve_b200.lane_base import (EPI_F32, EPI_ROWS_F32, EPI_SILU_MUL, EPI_STORE, HEIGHTS, K_SAMPLE, SPLIT_PARTS, up,  # noqa: F401
                                       SPLIT_ROWS, LaneBase, Mat, _Arena, _Blob, _block, _retarget, _u64, rope_table)
 
 K_ATTN_PREFILL, K_ATTN_DECODE, K_ATTN_MERGE, K_RMSNORM, K_QKROPE = 33, 34, 35, 36, 37
@@ -307,7 +307,13 @@ class ModelLane(LaneBase):
         key = ("logits", T, E)
         tmpl = self._templates.get(key)
         if tmpl is None:
-            tmpl = self._templates[key] = logits_tiles(0, T, E, rows=self._logit_rows(T, E))
+            nw = self.fab.num_workers
+            if T >= 8 * nw:   # rows of one tile against all experts (up to 16 or 32, in registers by quarters): even rounds of tiles
+                most = 32 if T >= 24 * nw else 16
+                tmpl = tile_array(K_LOGITS, i0=(r0 := np.arange(0, T, per := -(-T // (nw * -(-T // (most * nw)))))), i1=np.minimum(per, T - r0))
+            else:
+                tmpl = logits_tiles(0, T, E, rows=self._logit_rows(T, E))
+            self._templates[key] = tmpl
         return _retarget(tmpl, a0=args.data_ptr())
 
     def _moe(self, p, l, T, prev, norm_w, expands, fuse_norm=None):

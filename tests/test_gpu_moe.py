@@ -63,6 +63,13 @@ def test_router_logits_bit_exact(T, H, E):
     assert np.array_equal(out.cpu().numpy().view(np.int32), want.view(np.int32))
 
 
+# a warp's tile grows with tokens x experts: its steps, and tokens and experts that do not fill the last one
+@pytest.mark.parametrize("T,H,E", [(1, 256, 5), (36, 512, 128), (37, 512, 128), (39, 256, 127), (147, 512, 128), (148, 512, 128),
+                                   (151, 768, 131), (592, 256, 128), (601, 512, 129), (2500, 256, 33)])
+def test_router_logits_of_every_tile(T, H, E):
+    test_router_logits_bit_exact(T, H, E)
+
+
 @pytest.mark.parametrize("T,E,K,scoring", [(64, 128, 8, 0), (33, 16, 4, 0), (5, 256, 16, 0), (1, 8, 1, 0),
                                            (100, 160, 6, 1), (70, 128, 8, 1)])
 def test_router_topk_bit_exact(T, E, K, scoring):
