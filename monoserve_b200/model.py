@@ -431,7 +431,9 @@ class ModelLane(LaneBase):
                         cos_sin=self.cos_sin, ld_qkv=self.qkv_dim, hq=hq, hkv=hkv, rot_dim=cfg.rotary_dim,
                         theta=cfg.rope_theta, eps=cfg.rms_eps, max_pos=self.max_pos)
             # a small batch: few items per tile, so that every worker has one (an item is a chain of exposed loads)
-            rope_items = min(ROPE_ITEMS, max(4, -(-(T * heads) // (4 * self.fab.num_workers)) * 4))
+            # many items: two rounds of tiles, whose warps take eight items at a time
+            items, nw = T * heads, self.fab.num_workers
+            rope_items = up(-(-items // (2 * nw)), 32) if items > 2 * ROPE_ITEMS * nw else min(ROPE_ITEMS, max(4, -(-items // (4 * nw)) * 4))
             s_rope = p.stage(self._rows(K_QKROPE, qk, T * heads, rope_items), mark=(l << 8) | 1, label=("rope", l))
             p.after(s_qkv, s_rope)
             s_attn = attention(p, l, s_rope)
