@@ -255,8 +255,7 @@ __device__ bool run_core_tile(DeviceState& S, const WorkSlot& w, int tid, uint32
       tile_permute(t, tid);
       return true;
     case kTileCombine:
-      tile_combine(t, tid);
-      return true;
+      return tile_combine(t, tid, ring, abort_flag);
     case kTileAsymReduce:
       tile_asym_reduce(t, tid);
       return true;
@@ -477,14 +476,146 @@ __device__ void tile_permute(const TileDesc& t, int tid) {
   }
 }
 
+// The rows of a combine tile through the operand ring, in `parts` pieces of their columns when two whole rows do not fit: the
+// K expert rows, x2 and the shared expert's row by bulk copies, the four warps on one row.  (Their own loads drew 1.3 TB/s;
+// pieces of 512 columns per warp were bound by the rate of bulk copies: 129 us.)  4096 rows of 8 x 2048: 232 -> 134 us.
+// The arithmetic and its order are the other form's: the warps keep the rounded row in shared memory, and each forms the
+// sum of squares in the order of a warp that has the whole row.
+template <int NG>   // groups of eight columns of a piece per thread
+__device__ __noinline__ bool combine_bulk(const TileDesc& t, int tid, const LayerCtx& ctx, int parts) {
+  __builtin_assume(__isShared(ctx.ring));
+  CombineArgs A;
+  load_block(A, t.a[0]);
+  const int lane = tid & 31, K = static_cast<int>(A.K), H = static_cast<int>(A.H), cols = H / parts;
+  const uint32_t y_bytes = 4u * cols, x2_at = K * y_bytes, shared_at = x2_at + 2u * cols;
+  const uint32_t row_bytes = 2u * H;
+  const int n_rows = static_cast<int>(t.i1), total = n_rows * parts;
+  // in front of the stages: the norm's weights, and two rows of results in turn
+  RowStages pipe(ctx, shared_at + (A.shared ? y_bytes : 0), total, tid, 3 * row_bytes);
+  const uint4* const w4 = reinterpret_cast<const uint4*>(ctx.ring);
+  const uint32_t tx = K * y_bytes + (A.x2 ? 2u * cols : 0) + (A.shared ? y_bytes : 0);
+  // warp 0 fetches: a lane per copy
+  auto fetch = [&](int k, int s) {
+    const int part = k % parts, col = part * cols;
+    const size_t row = static_cast<size_t>(t.i0) + k / parts;
+    const int pos = lane < K ? reinterpret_cast<const int*>(A.pair_pos)[row * K + lane] : 0;
+    uint8_t* const to = pipe.stage(s);
+    if (lane == 0) mbar_arrive_expect_tx(pipe.bar + s, tx);
+    __syncwarp();
+    if (lane < K) bulk_in(to + lane * y_bytes, f32p(A.y) + static_cast<size_t>(pos) * H + col, y_bytes, pipe.bar + s);
+    else if (lane == 16 && A.x2)
+      bulk_in(to + x2_at, reinterpret_cast<const __nv_bfloat16*>(A.x2) + row * H + col, 2u * cols, pipe.bar + s);
+    else if (lane == 17 && A.shared)
+      bulk_in(to + shared_at, f32p(A.shared) + row * H + col, y_bytes, pipe.bar + s);
+  };
+  if (tid < 32) {
+    if (tid == 0 && A.w) {
+      mbar_expect_tx(pipe.bar, row_bytes);   // with the first piece
+      bulk_in(ctx.ring, reinterpret_cast<const __nv_bfloat16*>(A.w), row_bytes, pipe.bar);
+    }
+    __syncwarp();
+    for (int k = 0; k < pipe.depth; ++k) fetch(k, k);
+  }
+  auto weight_of = [&](int row) {
+    return lane < K ? reinterpret_cast<const float*>(A.topk_w)[(static_cast<size_t>(t.i0) + min(row, n_rows - 1)) * K + lane] : 0.f;
+  };
+  int k = 0;
+  bool ok = true;
+  float w = weight_of(0), w_next = 0.f;
+  for (; k < total; ++k) {
+    const int part = k % parts, at_row = k / parts;
+    uint4* const f_row = reinterpret_cast<uint4*>(ctx.ring + row_bytes + (at_row & 1) * row_bytes);
+    if (part == 0) w_next = weight_of(at_row + 1);
+    ok = __all_sync(0xffffffffu, pipe.wait());
+    const uint8_t* const in = pipe.stage(pipe.at);
+#pragma unroll
+    for (int i = 0; i < NG; ++i) {
+      const int g = tid + i * kExecThreads;   // the piece's group of eight columns (whole warps are in or out: H is a multiple of 256)
+      if (8 * g >= cols || !ok) continue;
+      float acc[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) acc[j] = 0.f;
+#pragma unroll 4
+      for (int q = 0; q < K; ++q) {
+        const float wk = __shfl_sync(0xffffffffu, w, q);
+        const float4* yr = reinterpret_cast<const float4*>(in + q * y_bytes) + 2 * g;
+        const float4 a = yr[0], b = yr[1];
+        const float yv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = __fmaf_rn(wk, yv[j], acc[j]);
+      }
+      if (A.shared) {
+        const float4* sr = reinterpret_cast<const float4*>(in + shared_at) + 2 * g;
+        const float4 a = sr[0], b = sr[1];
+        const float sv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[j] = __fadd_rn(acc[j], sv[j]);
+      }
+      float f[8] = {};
+      if (A.x2) unpack8(reinterpret_cast<const uint4*>(in + x2_at)[g], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = round_bf16(__fadd_rn(f[j], acc[j]));
+      f_row[part * (cols / 8) + g] = pack8(f);
+    }
+    ok = exec_and(ok);   // with the stage's release and the row's results
+    if (!ok) break;
+    if (tid < 32 && k + pipe.depth < total) {
+      fence_proxy_async_smem();
+      fetch(k + pipe.depth, pipe.at);
+    }
+    pipe.next();
+    if (part + 1 < parts) continue;
+    w = w_next;
+    const size_t row = static_cast<size_t>(t.i0) + at_row;
+    uint4* const xo = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(A.x) + row * H);
+    uint4* const out = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(A.out) + row * H);
+    float inv = 0.f;
+    if (A.w) {
+      float ss = 0.f;
+#pragma unroll 4
+      for (int c = lane; c < H / 8; c += 32) {
+        float f[8];
+        unpack8(f_row[c], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss = __fmaf_rn(f[j], f[j], ss);
+      }
+      inv = det_rsqrtf(__fadd_rn(__fdiv_rn(warp_sum_xor(ss), static_cast<float>(H)), A.eps));
+    }
+    for (int c = tid; c < H / 8; c += kExecThreads) {
+      const uint4 v = f_row[c];
+      xo[c] = v;
+      if (A.w) {
+        float f[8], g[8];
+        unpack8(v, f);
+        unpack8(w4[c], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = __fmul_rn(round_bf16(__fmul_rn(f[j], inv)), g[j]);
+        out[c] = pack8(f);
+      }
+    }
+  }
+  pipe.close(tid, ok ? 0 : min(total - k, pipe.depth));
+  return ok;
+}
+
 // Combine tile (kind 47; not in the reference, which adds with fp32 atomics in the
 // w2 epilogue and finishes in AddNorm): x[t] = bf16(x2[t] + sum_k w[t][k] * y[pos(t,k)])
 // with the sum in pick order (plus, when `shared` is set, the fp32 row shared[t] of a shared
 // expert: the GLM-style layer, tests/test_fabric_model_glm.py:57-67), then optionally
 // out = rmsnorm(x) * w.
-__device__ void tile_combine(const TileDesc& t, int tid) {
+__device__ bool tile_combine(const TileDesc& t, int tid, uint8_t* ring, volatile int* abort_flag) {
   CombineArgs A;   // a copy in registers: the block lives in global memory
   load_block(A, t.a[0]);
+  if (t.i1 >= kCombineRows && A.K <= 16 && A.H % 256 == 0 && ((A.y | A.x2 | A.shared | A.w) & 15) == 0) {
+    // the fewest pieces of a row of which the ring holds two; whole warps' groups of columns
+    for (int parts = 1; parts <= 4; parts *= 2) {
+      const uint32_t cols = A.H / parts;
+      if (cols % 256 || cols > 4096) continue;
+      if (6 * A.H + 2 * cols * (4 * A.K + 2 + (A.shared ? 4 : 0)) > kWideRingBytes) continue;
+      const LayerCtx ctx{s_exec_scratch, ring, 0, abort_flag};
+      return cols <= 2048 ? combine_bulk<2>(t, tid, ctx, parts) : combine_bulk<4>(t, tid, ctx, parts);
+    }
+  }
   const int warp = tid >> 5, lane = tid & 31;
   const int K = static_cast<int>(A.K), H = static_cast<int>(A.H), n16 = H / 8;
   const float* y = reinterpret_cast<const float*>(A.y);
@@ -541,6 +672,7 @@ __device__ void tile_combine(const TileDesc& t, int tid) {
       norm_store_row(xo, ss, reinterpret_cast<const __nv_bfloat16*>(A.w),
                      reinterpret_cast<__nv_bfloat16*>(A.out) + static_cast<size_t>(r) * H, nullptr, H, A.eps);
   }
+  return true;
 }
 
 // Expand tile (kind 39, csrc/fabric/tiles/aux.cuh:453-616, ExpandArgs), one per lane

@@ -330,7 +330,6 @@ class ModelLane(LaneBase):
                        w=norm_w if norm_w is not None else 0, out=self.xn, K=cfg.top_k, H=H, eps=cfg.rms_eps,
                        shared=self.y_shared if shared else 0)
         ex = self.arena.put(bytes(_C.struct_layouts()["ExpandArgs"][0]))   # filled once the dynamic region is laid out
-        per = self._per(T)
         if fuse_norm is not None:
             kind, nrm = fuse_norm
             key = ("norm_logits", T, E)
@@ -358,7 +357,7 @@ class ModelLane(LaneBase):
             p.after(s_ex, s_pm)
         w13_0 = p.stages(E, label=("w13", l))
         w2_0 = p.stages(E, label=("w2", l))
-        s_cb = p.stage(self._rows(K_COMBINE, cb, T, per), mark=(l << 8) | 3, label=("combine", l))
+        s_cb = p.stage(self._rows(K_COMBINE, cb, T, self._per_streamed(T)), mark=(l << 8) | 3, label=("combine", l))
         fetch_0 = p.stages(E, label=("fetch", l)) if self.staging[l] is not None else None
         p.fan_out(s_pm, w13_0, E)
         if fetch_0 is not None:   # the copy into the staging stack starts as soon as the expert's row count is known
