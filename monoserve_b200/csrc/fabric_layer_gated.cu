@@ -53,27 +53,6 @@ __device__ __forceinline__ void ld_pairs(const float* p, Pair& a, Pair& b) {
   b = q.y;
 }
 
-// NV values per lane summed over groups of LB lanes: lane l of a group ends with values [l NV / LB, ..), max(1, NV / LB) of
-// them, at the front of v.
-template <int N, int BIT, int NV>
-__device__ __forceinline__ void group_sum_from(float (&v)[NV], int lane) {
-  if constexpr (BIT >= 1) {
-    if constexpr (N > 1) {
-      const bool hi = lane & BIT;
-#pragma unroll
-      for (int c = 0; c < N / 2; ++c) {
-        const float give = hi ? v[c] : v[c + N / 2], have = hi ? v[c + N / 2] : v[c];
-        v[c] = have + __shfl_xor_sync(0xffffffffu, give, BIT);
-      }
-    } else {
-      v[0] += __shfl_xor_sync(0xffffffffu, v[0], BIT);
-    }
-    group_sum_from<(N > 1 ? N / 2 : 1), BIT / 2>(v, lane);
-  }
-}
-template <int NV, int LB>
-__device__ __forceinline__ void group_sum(float (&v)[NV], int lane) { group_sum_from<NV, LB / 2>(v, lane); }
-
 constexpr float kUnitFloor = 1e-6f;
 
 // ------------------------------------------------------------------ a request's rows

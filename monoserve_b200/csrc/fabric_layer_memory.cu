@@ -252,6 +252,270 @@ __device__ __noinline__ void memory_rows(const TileDesc& t, int tid, uint8_t* ri
   if (tid == 0) *m_state = m0;
 }
 
+// Kind 57 with a[1] columns to a block (i2 = head | column block << 16): four tokens are one step.  With M_b the running maximum
+// in front of the step, rel and M as in memory_rows, k and q as they come and v = 1 in the normaliser's column,
+//   o_i = e^(M_b - M_i) S q_i + sum_{j <= i} e^(rel_j - M_i) (q_i k_j) v_j
+//   S  <- e^(M_b - M_3) S + sum_j e^(rel_j - M_3) v_j k_j
+// so the state is read and written once per step, a step's decay is one factor of a head, and the dot products are numbers of
+// the step that one warp works out.  Sixteen lanes share C columns of the state, R rows each in groups of four,
+// 4 (l + 16 i) .. + 3, in registers for the whole portion: 8 C columns in a tile.  Bound by the fp32 pipe, nine packed products
+// per pair of state elements and step against twelve and a conversion of k and q for every eight columns, one token at a
+// time.  4 x 1024 tokens, 4 heads of 256 x 512: 786 -> 545 us.
+template <int R, int C>
+__device__ __noinline__ void memory_steps(const TileDesc& t, int tid, uint8_t* ring) {
+  using T = __nv_bfloat16;
+  constexpr int G = 16, DP = G * R, CB = 8 * C, kTokens = 32, kSteps = kTokens / 4, I4 = R / 4;
+  constexpr int kPer = G / (2 * C) > 1 ? G / (2 * C) : 1;   // lanes per sum of two tokens x C columns
+  static_assert(2 * C <= G && CB % kMemColumns == 0, "a sum per lane, copies of the running maximum of its own");
+  struct Raw {
+    T k[kTokens][DP], q[kTokens][DP], v[kTokens][CB];
+  };
+  struct Shared {
+    Raw in[2];
+    float mix[kSteps][16], read[kSteps][4], write[kSteps][4], keep[kSteps], low[kTokens];
+  };
+  static_assert(sizeof(Shared) <= kWideRingBytes, "the operand ring");
+  __builtin_assume(__isShared(ring));
+  Shared& sh = *reinterpret_cast<Shared*>(ring);
+  MemoryArgs A;
+  load_block(A, t.a[0]);
+  const int row0 = static_cast<int>(t.i0), rows = static_cast<int>(t.i1), slot = static_cast<int>(t.i3);
+  const int head = static_cast<int>(t.i2 & 0xffffu), col0 = static_cast<int>(t.i2 >> 16) * CB;
+  const int H = static_cast<int>(A.heads), d = static_cast<int>(A.d), e = static_cast<int>(A.e);
+  const int dp = (d + 3) & ~3, oe = (e + 4) & ~3, warp = tid >> 5, lane = tid & 31, l = lane & (G - 1);
+  const bool fresh = reinterpret_cast<const int*>(A.tok_pos)[row0] == 0;
+  const int n_v = max(0, min(CB, e - col0));                 // columns of v in this block
+  const int c_lo = (warp * 2 + lane / G) * C;                // this lane's first column of the block
+  float* const state = reinterpret_cast<float*>(A.state) + ((static_cast<size_t>(slot) * H + head) * (e + 1) + col0 + c_lo) * dp;
+  unsigned long long S[C][I4][2];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < I4; ++i) {
+      const int at = 4 * (l + G * i);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (!fresh && at < dp && col0 + c_lo + c <= e) v = *reinterpret_cast<const float4*>(state + static_cast<size_t>(c) * dp + at);
+      S[c][i][0] = pk2(v.x, v.y);
+      S[c][i][1] = pk2(v.z, v.w);
+    }
+  // a copy of the running maximum per kMemColumns columns: this tile reads its first and writes all of its own
+  const int copies = (e + kMemColumns) / kMemColumns, first_copy = col0 / kMemColumns;
+  float* const m_state = reinterpret_cast<float*>(A.m) + (static_cast<size_t>(slot) * H + head) * copies;
+  float m0 = fresh ? 0.f : m_state[first_copy];
+  const float *gates = f32p(A.gates), bi = f32p(A.gate_bias)[head], bf = f32p(A.gate_bias)[H + head];
+  const T *gk = reinterpret_cast<const T*>(A.k) + head * d, *gq = reinterpret_cast<const T*>(A.q) + head * d;
+  const T* gv = reinterpret_cast<const T*>(A.v) + static_cast<size_t>(head) * e + col0;
+  const bool kq16 = d % 8 == 0 && ((A.k | A.q) & 15) == 0, v16 = e % 8 == 0 && n_v % 8 == 0 && (A.v & 15) == 0;
+  for (int i = tid; i < static_cast<int>(sizeof(sh.in) / 16); i += kExecThreads)   // padding stays zero
+    reinterpret_cast<uint4*>(sh.in)[i] = make_uint4(0, 0, 0, 0);
+  exec_sync();
+  // a chunk's rows; those behind it that belong to its last step become zero
+  auto copy_row = [&](T* dst, const T* src, int n, bool pieces, bool zero) {
+    if (zero) {
+      for (int p = lane; p < n; p += 32) dst[p] = __ushort_as_bfloat16(0);
+    } else if (pieces) {
+      for (int p = lane; p < n / 8; p += 32) cp16(dst + p * 8, src + p * 8);
+    } else {
+      for (int p = lane; p < n; p += 32) dst[p] = src[p];
+    }
+  };
+  auto stage = [&](int base, Raw& in) {
+    const int nt = min(kTokens, rows - base), end = (nt + 3) & ~3;
+    for (int tok = warp; tok < end; tok += kExecThreads / 32) {
+      const size_t at = static_cast<size_t>(row0 + base + min(tok, nt - 1)) * A.ld_qkv;
+      copy_row(in.k[tok], gk + at, d, kq16, tok >= nt);
+      copy_row(in.q[tok], gq + at, d, kq16, tok >= nt);
+      copy_row(in.v[tok], gv + at, n_v, v16, tok >= nt);
+    }
+    cp_commit();
+  };
+  auto load_gates = [&](int base, float& gi, float& gf) {   // one token per lane
+    const int nt = min(kTokens, rows - base);
+    const size_t at = static_cast<size_t>(row0 + base + min(lane, nt - 1)) * A.ld_gates + head;
+    gi = lane < nt ? capped(raw_gate(A, gates + at) + bi, A.cap) : -INFINITY;
+    gf = lane < nt ? log_sigmoid(capped(raw_gate(A, gates + at + H) + bf, A.cap)) : 0.f;
+  };
+  auto four = [](const T* p, unsigned long long (&v)[2]) {
+    const uint2 u = *reinterpret_cast<const uint2*>(p);
+    v[0] = pk2(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u));
+    v[1] = pk2(__uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+  };
+  const int n_own = l / kPer, own_c = n_own / 2, own_t = n_own & 1, own_col = c_lo + own_c;   // the sum this lane ends with
+  const bool owner = l % kPer == 0 && col0 + own_col <= e, normaliser = col0 + own_col == e;
+  const size_t ld_out = static_cast<size_t>(H) * oe;
+  float* const out = reinterpret_cast<float*>(A.out) + static_cast<size_t>(row0) * ld_out + static_cast<size_t>(head) * oe + col0 + own_col;
+  stage(0, sh.in[0]);
+  float gi, gf;
+  load_gates(0, gi, gf);
+  for (int base = 0, b = 0; base < rows; base += kTokens, b ^= 1) {
+    const int nt = min(kTokens, rows - base), steps = (nt + 3) / 4;
+    cp_wait<0>();
+    exec_sync();   // the chunk is there, and the one before it has been read
+    float gi_next = 0.f, gf_next = 0.f;
+    if (base + kTokens < rows) {
+      stage(base + kTokens, sh.in[b ^ 1]);
+      load_gates(base + kTokens, gi_next, gf_next);
+    }
+    const Raw& in = sh.in[b];
+    float F = gf;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, F, o);
+      if (lane >= o) F += v;
+    }
+    const float rel = gi - F;
+    float M = rel;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float v = __shfl_up_sync(0xffffffffu, M, o);
+      if (lane >= o) M = fmaxf(M, v);
+    }
+    M = fmaxf(m0, M);
+    const float m = F + M, before = __shfl_sync(0xffffffffu, M, max((lane & ~3) - 1, 0));
+    const float keep = expf((lane < 4 ? m0 : before) - M);
+    float add[4];   // of the step's tokens j, for this lane's
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float x = __shfl_sync(0xffffffffu, rel, (lane & ~3) + j);
+      add[j] = j <= (lane & 3) ? expf(x - M) : 0.f;
+    }
+    if (warp == 0) sh.low[lane] = expf(-m);
+    m0 = __shfl_sync(0xffffffffu, m, nt - 1);
+    // ---- the numbers of the steps, a warp to a step
+    for (int s = warp; s < steps; s += kExecThreads / 32) {
+      float dot[16];
+      {
+        unsigned long long acc[10];
+#pragma unroll
+        for (int i = 0; i < 10; ++i) acc[i] = 0ull;
+#pragma unroll 1
+        for (int at = 4 * lane; at < DP; at += 128) {
+          unsigned long long kk[4][2], qq[4][2];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            four(&in.k[4 * s + i][at], kk[i]);
+            four(&in.q[4 * s + i][at], qq[i]);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j)
+#pragma unroll
+              for (int x = 0; x < 2; ++x) acc[i * (i + 1) / 2 + j] = fma2(qq[i][x], kk[j][x], acc[i * (i + 1) / 2 + j]);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 f = unpk2(j <= i ? acc[i * (i + 1) / 2 + j] : 0ull);
+            dot[4 * i + j] = f.x + f.y;
+          }
+      }
+      group_sum<16, 32>(dot, lane);   // lane x ends with sum x / 2
+      const int x = lane >> 1, from = 4 * s + (x >> 2);
+      float w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[j] = __shfl_sync(0xffffffffu, add[j], from);
+      const float weight = (x & 3) == 0 ? w[0] : (x & 3) == 1 ? w[1] : (x & 3) == 2 ? w[2] : w[3];
+      if ((lane & 1) == 0) sh.mix[s][x] = weight * dot[0] * A.q_scale;   // the weight of j > i is zero
+      const float k_all = __shfl_sync(0xffffffffu, keep, from);
+      if ((lane & 7) == 0) sh.read[s][x >> 2] = k_all * A.q_scale;
+      if (lane == 31) sh.keep[s] = k_all;
+      if (lane >= 24 && (lane & 1) == 0) sh.write[s][x & 3] = weight;
+    }
+    exec_sync();
+    // ---- the steps
+#pragma unroll 1
+    for (int s = 0; s < steps; ++s) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {   // read by two tokens at a time
+        unsigned long long acc[2][C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) acc[0][c] = acc[1][c] = 0ull;
+#pragma unroll
+        for (int i = 0; i < I4; ++i) {
+          unsigned long long x[2][2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) four(&in.q[4 * s + 2 * h + u][4 * (l + G * i)], x[u]);
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int u = 0; u < 2; ++u)
+#pragma unroll
+              for (int c = 0; c < C; ++c) acc[u][c] = fma2(S[c][i][p], x[u][p], acc[u][c]);
+        }
+        float o[2 * C];
+#pragma unroll
+        for (int c = 0; c < C; ++c)
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const float2 f = unpk2(acc[u][c]);
+            o[2 * c + u] = f.x + f.y;
+          }
+        group_sum<2 * C, G>(o, lane);
+        const int i = 2 * h + own_t;
+        float mix[4];
+        ld_vec<4>(sh.mix[s] + 4 * i, mix);
+        float y = sh.read[s][i] * o[0];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          y = fmaf(mix[j], normaliser ? 1.f : __bfloat162float(in.v[4 * s + j][own_col]), y);
+        const int tok = 4 * s + i;
+        if (owner && tok < nt)
+          out[static_cast<size_t>(base + tok) * ld_out] = normaliser ? fmaxf(fabsf(y), sh.low[tok]) + 1e-6f : y;
+      }
+      const unsigned long long kp = pk2(sh.keep[s], sh.keep[s]);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {   // written by two tokens at a time
+        unsigned long long U[2][C];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const float w = sh.write[s][2 * h + u];
+#pragma unroll
+          for (int c4 = 0; c4 < C; c4 += 4) {
+            unsigned long long two[2];
+            four(&in.v[4 * s + 2 * h + u][c_lo + c4], two);
+            const float2 a = unpk2(two[0]), z = unpk2(two[1]);
+            const float v[4] = {a.x, a.y, z.x, z.y};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              const float x = w * (col0 + c_lo + c4 + c == e ? 1.f : v[c]);
+              U[u][c4 + c] = pk2(x, x);
+            }
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < I4; ++i) {
+          unsigned long long x[2][2];
+#pragma unroll
+          for (int u = 0; u < 2; ++u) four(&in.k[4 * s + 2 * h + u][4 * (l + G * i)], x[u]);
+#pragma unroll
+          for (int p = 0; p < 2; ++p)
+#pragma unroll
+            for (int c = 0; c < C; ++c) {
+              if (h == 0) S[c][i][p] = mul2(kp, S[c][i][p]);
+              S[c][i][p] = fma2(U[0][c], x[0][p], S[c][i][p]);
+              S[c][i][p] = fma2(U[1][c], x[1][p], S[c][i][p]);
+            }
+        }
+      }
+    }
+    gi = gi_next;
+    gf = gf_next;
+  }
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+#pragma unroll
+    for (int i = 0; i < I4; ++i) {
+      const int at = 4 * (l + G * i);
+      if (at < dp && col0 + c_lo + c <= e) {
+        const float2 a = unpk2(S[c][i][0]), z = unpk2(S[c][i][1]);
+        *reinterpret_cast<float4*>(state + static_cast<size_t>(c) * dp + at) = make_float4(a.x, a.y, z.x, z.y);
+      }
+    }
+  if (tid < CB / kMemColumns && first_copy + tid < copies) m_state[first_copy + tid] = m0;
+}
+
 // Kind 56, MemoryArgs: one token.  Row i0, i2 = head | first column block << 16, i1 column blocks, slot i3.  The state
 // streams through registers, the next block's loads issued before this one's arithmetic.
 template <int ND, bool F32>
@@ -363,6 +627,19 @@ __device__ bool tile_memory(const TileDesc& t, int tid, uint8_t* ring) {
   const MemoryArgs* p = reinterpret_cast<const MemoryArgs*>(t.a[0]);
   const uint32_t d = __ldcg(&p->d);
   const bool f32 = __ldcg(&p->f32) != 0;
+  if (t.a[1]) {
+#define MF_STEPS(R, C)                             \
+  if (d <= 16 * R && t.a[1] == 8 * C && !f32) {    \
+    memory_steps<R, C>(t, tid, ring);              \
+    return true;                                   \
+  }
+    MF_STEPS(8, 8)
+    MF_STEPS(8, 4)
+    MF_STEPS(16, 8)
+    MF_STEPS(16, 4)
+#undef MF_STEPS
+    return false;
+  }
 #define MF_MEMORY(N)                             \
   if (d <= 128 * N) {                            \
     if (f32) memory_rows<N, true>(t, tid, ring); \

@@ -285,7 +285,7 @@ class MatrixMemory:
         mem = lane._dev("MemoryArgs", q=at, k=at + es * H * d, v=at + es * 2 * H * d, gates=raw.addr,
                         gate_parts=parts, gate_rows=lane.slab_rows(T), gate_bias=w.gate_b, state=st["S"], m=st["m"], out=lane.raw.addr, tok_pos=lane.tok_pos,
                         ld_qkv=lane.proj.ld, ld_gates=ld, heads=H, d=d, e=e, f32=f32, q_scale=d ** -0.5, cap=m.gate_cap)
-        s_m = p.stage(_retarget(b.memory_tiles(H, e), a0=mem.data_ptr()), label=("memory", run))
+        s_m = p.stage(_retarget(b.memory_tiles(H, e, d), a0=mem.data_ptr()), label=("memory", run))
         p.after(s, s_m)
         p.after(s_g, s_m)
         nrm = lane._dev("HeadNormArgs", o=lane.raw.addr, g=at + es * H * (2 * d + e), w=w.norm, out=lane.mix.addr, heads=H,
@@ -444,6 +444,15 @@ class _Buf:
         return self._maps[k]
 
 
+def memory_columns(portions, d, e, workers, f32):
+    """Columns of a portion's matrix memory tile (tile 57's a[1]): 32 or 64 of four-token steps, the width whose rounds of tiles
+    over the workers cost less (a tile of 64 is about 1.7 times one of 32); 0: one token at a time, for 32-bit activations and keys past 256 columns, whose
+    states the steps' registers do not hold."""
+    if f32 or d > 256:
+        return 0
+    return min((32, 64), key=lambda w: -(-portions * -(-(e + 1) // w) // workers) * (1.7 if w == 64 else 1))
+
+
 class _Batch:
     """The rows of one program: requests [(first row, rows, slot)], and the tile lists that depend on them only (made
     once per program and re-addressed per layer).  pos0: the requests' first positions, None for a decode step."""
@@ -510,13 +519,15 @@ class _Batch:
             return np.concatenate(out)
         return self._once(("scan", channels), make)
 
-    def memory_tiles(self, heads, e):
-        """Portions: a tile per head and block of columns; single tokens: as many column blocks in a tile as leave every
-        worker one."""
+    def memory_tiles(self, heads, e, d=None):
+        """Portions: a tile per head and block of columns (d: the keys' columns, for tiles of four-token steps where they are
+        taken); single tokens: as many column blocks in a tile as leave every worker one."""
         def make():
             blocks = -(-(e + 1) // MEMORY_COLUMNS)
-            h, c = np.meshgrid(np.arange(heads), np.arange(blocks), indexing="ij")
-            out = [tile_array(K_MEMORY, i0=row0, i1=n, i2=h | (c << 16), i3=slot)
+            portions = sum(1 for _, n, _ in self.requests if n > 1) * heads
+            width = 0 if d is None else memory_columns(portions, d, e, self.lane.fab.num_workers, self.lane.cfg.f32)
+            h, c = np.meshgrid(np.arange(heads), np.arange(-(-(e + 1) // (width or MEMORY_COLUMNS))), indexing="ij")
+            out = [tile_array(K_MEMORY, i0=row0, i1=n, i2=h | (c << 16), i3=slot, a1=width)
                    for row0, n, slot in sorted(self.requests, key=lambda q: -q[1]) if n > 1]
             ones = [(row0, slot) for row0, n, slot in self.requests if n == 1]
             if ones:
@@ -525,7 +536,7 @@ class _Batch:
                 h, c = np.arange(heads)[None, :, None], np.arange(0, blocks, per)[None, None, :]
                 out.append(tile_array(K_MEMORY_STEP, i0=row, i1=np.minimum(per, blocks - c), i2=h | (c << 16), i3=slot))
             return np.concatenate(out)
-        return self._once(("memory", heads, e), make)
+        return self._once(("memory", heads, e, d), make)
 
     def attn_tiles(self, heads, parts, kind=K_LATENT_ATTN):
         """One tile per row, group of heads and part, the rows that see most keys first."""

@@ -89,6 +89,24 @@ def test_attention_tile_shapes_fit_the_worker():
 REQUESTS, POS0 = [(0, 70, 4), (70, 1, 1), (71, 33, 2), (104, 2, 7), (106, 1, 0)], [0, 9, 0, 64, 0]
 
 
+def test_memory_tiles_of_four_token_steps_cover_columns_once():
+    from monoserve_b200.layer_list import K_MEMORY, _Batch, memory_columns
+    for d, e, heads, f32 in ((256, 512, 4, 0), (128, 63, 40, 0), (16, 64, 2, 0), (257, 512, 4, 0), (256, 512, 4, 1)):
+        plain = lane()
+        plain.cfg = types.SimpleNamespace(f32=f32)
+        b = _Batch(plain, REQUESTS, POS0)
+        t = fields(b.memory_tiles(heads, e, d))
+        width = memory_columns(3 * heads, d, e, plain.fab.num_workers, f32)   # three requests bring more than one token
+        assert (width == 0) == (f32 or d > 256) and width in (0, 32, 64)
+        seen = np.zeros((5, heads, e + 1), int)
+        for k, row, what, slot, w in zip(t["kind"], t["i0"], t["i2"], t["i3"], t["a1"]):
+            if k == K_MEMORY:
+                at = (what >> 16) * (width or 32)
+                assert w == width and at <= e
+                seen[[r for r, _, s in REQUESTS].index(row), what & 0xFFFF, at:at + (width or 32)] += 1
+        assert (seen[[n > 1 for _, n, _ in REQUESTS]] == 1).all()
+
+
 def test_tile_lists_cover_rows_channels_columns_and_heads_once():
     from monoserve_b200.layer_list import K_CONV, K_MEMORY, K_MEMORY_STEP, K_SCAN, K_SCAN_STEP, _Batch
     b = _Batch(lane(), REQUESTS, POS0)
