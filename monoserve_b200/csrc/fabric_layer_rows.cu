@@ -282,9 +282,11 @@ __device__ __noinline__ void streams_rows(const TileDesc& t, int tid, int* scrat
   }
 }
 
-// Rows of at most 512 NU columns and four streams: the row's streams and slabs (kEmbed: its token's row) come through RowStages,
-// the four warps on one row.  Bound by memory (a row of four streams of 2048: 40 KB in, 36 KB out).  4096 such rows: 285 -> 90 us, the embedding 230 -> 77.
-template <int NU, bool kEmbed>
+// At most four streams: the row's streams and slabs (kEmbed: its token's row) come through RowStages,
+// the four warps on one row.  Bound by memory (a row of four streams of 2048: 40 KB in, 36 KB out).  4096 such rows: 285 -> 71 us (90 with the loops unrolled).
+// The loops over a thread's columns stay rolled, the next sublayer's input between them in shared memory: unrolled, with one warp
+// per scheduler, the row was bound by the instructions' fetch (5700 cycles, 3300 of them in the first loop).
+template <bool kEmbed>
 __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const LayerCtx& ctx) {
   __builtin_assume(__isShared(ctx.ring));
   __builtin_assume(__isShared(ctx.scratch));
@@ -297,7 +299,10 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
   int* const tokens = ctx.scratch + 128;
   if constexpr (kEmbed)
     for (int k = tid; k < rows; k += kExecThreads) tokens[k] = reinterpret_cast<const int*>(A.tokens)[row0 + k];
-  RowStages pipe(ctx, kEmbed ? piece / 2 : static_cast<uint32_t>(ns + parts) * piece, rows, tid);
+  // in front of the stages: the norm's weights, and the input of the row at hand
+  RowStages pipe(ctx, kEmbed ? piece / 2 : static_cast<uint32_t>(ns + parts) * piece, rows, tid, 2 * piece);
+  const float* const w = reinterpret_cast<const float*>(ctx.ring);
+  float* const u_row = reinterpret_cast<float*>(ctx.ring + piece);
   auto fetch = [&](int k, int s) {
     const size_t r = static_cast<size_t>(row0 + k);
     uint8_t* const to = pipe.stage(s);
@@ -310,9 +315,12 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
     for (int q = 0; q < parts; ++q)
       bulk_in(to + (ns + q) * piece, f32p(A.y) + (static_cast<size_t>(q) * A.y_rows + r) * W, piece, pipe.bar + s);
   };
-  if (tid == 0)
+  if (tid == 0) {
+    mbar_expect_tx(pipe.bar, piece);   // with the first row
+    bulk_in(ctx.ring, f32p(A.w), piece, pipe.bar);
     for (int k = 0; k < pipe.depth; ++k) fetch(k, k);
-  float w_in[4], w_out[4], mix[16], w[NU][4];
+  }
+  float w_in[4], w_out[4], mix[16];
 #pragma unroll
   for (int s = 0; s < 4; ++s) {
     w_in[s] = s < ns ? f32p(A.hc_in)[s] : 0.f;
@@ -320,9 +328,6 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
 #pragma unroll
     for (int to = 0; to < 4; ++to) mix[s * 4 + to] = !kEmbed && s < ns && to < ns ? f32p(A.hc_mix)[s * ns + to] : 0.f;
   }
-#pragma unroll
-  for (int i = 0; i < NU; ++i)
-    if ((tid + i * kExecThreads) * 4 < W) ld_vec<4>(f32p(A.w) + (tid + i * kExecThreads) * 4, w[i]);
   int k = 0;
   bool ok = true;
   for (; k < rows; ++k) {
@@ -332,12 +337,10 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
     float* const sum_out = A.sum_out ? reinterpret_cast<float*>(A.sum_out) + r * W : nullptr;
     ok = pipe.wait();
     const float* const in = reinterpret_cast<const float*>(pipe.stage(pipe.at));
-    float u[NU][4], ss = 0.f;
-#pragma unroll
-    for (int i = 0; i < NU; ++i) {
-      const int c = (tid + i * kExecThreads) * 4;
-      if (c >= W || !ok) continue;
-      float x[4][4], y[4], nx[4][4], sum[4];
+    float ss = 0.f;
+#pragma unroll 1
+    for (int c = tid * 4; c < W && ok; c += kExecThreads * 4) {
+      float x[4][4], y[4], nx[4][4], sum[4], u[4];
       if constexpr (kEmbed) {
         const __nv_bfloat16* const e = reinterpret_cast<const __nv_bfloat16*>(in) + c;
 #pragma unroll
@@ -373,18 +376,19 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
             nx[to][j] = v;
           }
         }
-        u[i][j] = sum[j] = 0.f;
+        u[j] = sum[j] = 0.f;
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-          u[i][j] = fmaf(w_in[s], nx[s][j], u[i][j]);
+          u[j] = fmaf(w_in[s], nx[s][j], u[j]);
           if (s < ns) sum[j] += nx[s][j];
         }
-        ss = fmaf(u[i][j], u[i][j], ss);
+        ss = fmaf(u[j], u[j], ss);
       }
 #pragma unroll
       for (int s = 0; s < 4; ++s)
         if (s < ns) st_vec<4>(xs + s * W + c, nx[s]);
       if (sum_out) st_vec<4>(sum_out + c, sum);
+      st_vec<4>(u_row + c, u);   // read by this thread only
     }
     // one barrier a row: it carries the decision to go on, the sums (two sets in turn) and the stage's release
     ss = warp_sum(ss);
@@ -398,13 +402,13 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
     pipe.next();
     const float* const sums = red + (k & 1) * 4;
     const float inv = 1.f / sqrtf((sums[0] + sums[1] + sums[2] + sums[3]) / static_cast<float>(W) + A.eps);
+#pragma unroll 1
+    for (int c = tid * 4; c < W; c += kExecThreads * 4) {
+      float h[4], u[4], m[4];
+      ld_vec<4>(u_row + c, u);
+      ld_vec<4>(w + c, m);
 #pragma unroll
-    for (int i = 0; i < NU; ++i) {
-      const int c = (tid + i * kExecThreads) * 4;
-      if (c >= W) continue;
-      float h[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) h[j] = u[i][j] * inv * w[i][j];
+      for (int j = 0; j < 4; ++j) h[j] = u[j] * inv * m[j];
       auto st16 = [&](unsigned long long base, size_t at) {
         const __nv_bfloat162 q[2] = {__floats2bfloat162_rn(h[0], h[1]), __floats2bfloat162_rn(h[2], h[3])};
         *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(base) + at) = *reinterpret_cast<const uint2*>(q);
@@ -432,13 +436,13 @@ __device__ bool tile_streams(const TileDesc& t, int tid, const LayerCtx& ctx) {
   const StreamArgs* p = reinterpret_cast<const StreamArgs*>(t.a[0]);
   const uint32_t W = __ldcg(&p->W), ns = __ldcg(&p->streams), parts = __ldcg(&p->y_parts);
   const bool four = (W & 3) == 0 && ns <= 4;
-  if (t.i1 >= kBulkRows && four && W <= 4096) {
+  if (t.i1 >= kBulkRows && four) {
     // two rows in the ring at least, or nothing overlaps
-    if (__ldcg(&p->embed) == 0 && parts > 0 && 2 * (ns + parts) * W * 4 <= kWideRingBytes)
-      return W <= 2048 ? streams_bulk<4, false>(t, tid, ctx) : streams_bulk<8, false>(t, tid, ctx);
+    if (__ldcg(&p->embed) == 0 && parts > 0 && (2 * (ns + parts) + 2) * W * 4 <= kWideRingBytes) return streams_bulk<false>(t, tid, ctx);
     // (W % 8: whole 16-byte pieces of bf16 rows)
-    if (__ldcg(&p->embed) != 0 && parts == 0 && __ldcg(&p->step) == 0 && t.i1 <= 512 && (W & 7) == 0 && (__ldcg(&p->embed) & 15) == 0)
-      return W <= 2048 ? streams_bulk<4, true>(t, tid, ctx) : streams_bulk<8, true>(t, tid, ctx);
+    if (__ldcg(&p->embed) != 0 && parts == 0 && __ldcg(&p->step) == 0 && t.i1 <= 512 && (W & 7) == 0 && 3 * W * 4 <= kWideRingBytes &&
+        (__ldcg(&p->embed) & 15) == 0)
+      return streams_bulk<true>(t, tid, ctx);
   }
   if (four) streams_rows<4, 4>(t, tid, ctx.scratch);
   else streams_rows<1, kMaxStreams>(t, tid, ctx.scratch);
