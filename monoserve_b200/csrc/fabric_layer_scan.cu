@@ -165,8 +165,44 @@ __device__ __noinline__ void scan_rows(const TileDesc& t, int tid, uint8_t* ring
   for (int i = tid; i < 2 * kScanTokens * 2 * NP; i += kExecThreads)
     (&sh.in[i / (kScanTokens * 2 * NP)].bc[0][0])[i % (kScanTokens * 2 * NP)] = 0.f;
   exec_sync();
+  // Whole chunks of aligned rows: every thread keeps its place in the rows and copies a compile-time number of 16-byte pieces.
+  // (The general form below works out row and piece of each: 2500 cycles of a chunk's 7800.)
+  constexpr int kX = kScanChannels / kPer16, kXRows = kExecThreads / kX, kBc = 2 * NP / 4, kBcRows = kExecThreads / kBc > 0 ? kExecThreads / kBc : 1;
+  constexpr bool kEven = kExecThreads % kBc == 0 && kScanTokens % kBcRows == 0;
+  const bool even = kEven && z16 && bc16 && n == NP;
+  auto stage_whole = [&](int base, Chunk& k) {
+    const size_t r0 = static_cast<size_t>(row0 + base);
+    {
+      const int tok = tid >> 3, q = (tid & 7) * 4;
+      const float* from = f32p(A.dt) + (r0 + tok) * A.ld_dt + ch0 + q;
+#pragma unroll
+      for (int i = 0; i < kScanTokens / 16; ++i) cp16(&k.dt[tok + 16 * i][q], from + static_cast<size_t>(16 * i) * A.ld_dt);
+    }
+    {
+      const int tok = tid / kX, q = (tid % kX) * kPer16;
+      const T *x = reinterpret_cast<const T*>(A.x) + (r0 + tok) * A.ld_x + ch0 + q, *z = reinterpret_cast<const T*>(A.z) + (r0 + tok) * A.ld_z + ch0 + q;
+#pragma unroll
+      for (int i = 0; i < kScanTokens / kXRows; ++i) {
+        cp16(&k.x[tok + kXRows * i][q], x + static_cast<size_t>(kXRows * i) * A.ld_x);
+        cp16(&k.z[tok + kXRows * i][q], z + static_cast<size_t>(kXRows * i) * A.ld_z);
+      }
+    }
+    {
+      const int tok = tid / kBc, q = (tid % kBc) * 4;   // B, then C
+      const float* from = (q < NP ? f32p(A.b) + q : f32p(A.c) + q - NP) + (r0 + tok) * A.ld_bc;
+#pragma unroll
+      for (int i = 0; i < kScanTokens / kBcRows; ++i) cp16(&k.bc[tok + kBcRows * i][q], from + static_cast<size_t>(kBcRows * i) * A.ld_bc);
+    }
+    cp_commit();
+  };
   auto stage = [&](int base, Chunk& k) {
     const int nt = min(kScanTokens, rows - base);
+    if constexpr (kEven) {
+      if (even && nt == kScanTokens) {
+        stage_whole(base, k);
+        return;
+      }
+    }
     const T* x = reinterpret_cast<const T*>(A.x);
     const T* z = reinterpret_cast<const T*>(A.z);
     // rows of 32 channels: 8 pieces of dt, 32 / kPer16 of x and of z; rows are padded, so whole pieces may be read
@@ -231,39 +267,36 @@ __device__ __noinline__ void scan_rows(const TileDesc& t, int tid, uint8_t* ring
       k.dt[mine][my] = mine < nt ? dt : 0.f;
     }
     __syncwarp();
-#pragma unroll 1
-    for (int g = 0; g < nt; g += 4) {
-      const int mine = g + p;
-      const float x = value(k.x[mine][my]), z = value(k.z[mine][my]);
-      float part[4];
+    // A group's inputs are loaded while the group before it is computed, and its sums over the lanes, gate and store happen
+    // beside the group behind it: one group after the other waited for its loads, exponentials and exchanges in a row.
+    struct Group {
+      float dt[4], dx[4], B[4][NS], Cv[4][NS], x, z;
+    };
+    auto gather = [&](int g, Group& v) {
+      v.x = value(k.x[g + p][my]);
+      v.z = value(k.z[g + p][my]);
 #pragma unroll
       for (int i4 = 0; i4 < 4; ++i4) {
-        const float dk = k.dt[g + i4][my];
-        const float xk = g + i4 < nt ? dk * value(k.x[g + i4][my]) : 0.f;
-        float B[NS], Cv[NS];
+        v.dt[i4] = k.dt[g + i4][my];
+        v.dx[i4] = g + i4 < nt ? v.dt[i4] * value(k.x[g + i4][my]) : 0.f;
         const float *b = &k.bc[g + i4][s0], *cc = &k.bc[g + i4][NP + s0];
         if constexpr ((NS & 3) == 0) {
 #pragma unroll
           for (int i = 0; i < NS; i += 4) {
-            ld_vec<4>(b + i, *reinterpret_cast<float(*)[4]>(&B[i]));
-            ld_vec<4>(cc + i, *reinterpret_cast<float(*)[4]>(&Cv[i]));
+            ld_vec<4>(b + i, *reinterpret_cast<float(*)[4]>(&v.B[i4][i]));
+            ld_vec<4>(cc + i, *reinterpret_cast<float(*)[4]>(&v.Cv[i4][i]));
           }
         } else {
 #pragma unroll
           for (int i = 0; i < NS; ++i) {
-            B[i] = b[i];
-            Cv[i] = cc[i];
+            v.B[i4][i] = b[i];
+            v.Cv[i4][i] = cc[i];
           }
         }
-        float y = 0.f;
-#pragma unroll
-        for (int i = 0; i < NS; ++i) {
-          if constexpr (F32) S[i] += fmaf(S[i], expm1f(dk * a[i]), xk * B[i]);
-          else S[i] = fmaf(ex2(dk * a[i]), S[i], xk * B[i]);
-          y = fmaf(S[i], Cv[i], y);
-        }
-        part[i4] = y;
       }
+    };
+    auto finish = [&](int g, const float (&part)[4], float x, float z) {
+      const int mine = g + p;
       // the four lanes' sums, lane p ending with token p's
       const bool odd = p & 1, hi = p & 2;
       const float t0 = (odd ? part[1] : part[0]) + __shfl_xor_sync(0xffffffffu, odd ? part[0] : part[1], 1);
@@ -274,7 +307,38 @@ __device__ __noinline__ void scan_rows(const TileDesc& t, int tid, uint8_t* ring
         if constexpr (F32) sh.y[mine][my] = y;
         else sh.y[mine][my] = __float2bfloat16(y);
       }
+    };
+    constexpr bool kAhead = NS <= 6;   // more states a lane: their inputs do not fit the registers twice
+    Group cur, next;
+    if constexpr (kAhead) gather(0, next);
+    float held[4] = {}, held_x = 0.f, held_z = 0.f;
+#pragma unroll(kAhead ? 2 : 1)
+    for (int g = 0; g < nt; g += 4) {
+      if constexpr (kAhead) {
+        cur = next;
+        gather(min(g + 4, kScanTokens - 4), next);
+      } else {
+        gather(g, cur);
+      }
+      float part[4];
+#pragma unroll
+      for (int i4 = 0; i4 < 4; ++i4) {
+        float y = 0.f;
+#pragma unroll
+        for (int i = 0; i < NS; ++i) {
+          if constexpr (F32) S[i] += fmaf(S[i], expm1f(cur.dt[i4] * a[i]), cur.dx[i4] * cur.B[i4][i]);
+          else S[i] = fmaf(ex2(cur.dt[i4] * a[i]), S[i], cur.dx[i4] * cur.B[i4][i]);
+          y = fmaf(S[i], cur.Cv[i4][i], y);
+        }
+        part[i4] = y;
+      }
+      if (g > 0) finish(g - 4, held, held_x, held_z);
+#pragma unroll
+      for (int i4 = 0; i4 < 4; ++i4) held[i4] = part[i4];
+      held_x = cur.x;
+      held_z = cur.z;
     }
+    finish((nt - 1) & ~3, held, held_x, held_z);
     exec_sync();
     // rows of y are padded to whole pieces
     constexpr int kY = kScanChannels / kPer16;
