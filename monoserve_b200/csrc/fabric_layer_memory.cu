@@ -526,8 +526,7 @@ __device__ __noinline__ void memory_steps(const TileDesc& t, int tid, uint8_t* r
         }
       }
     }
-    gi = gi_next;
-    gf = gf_next;
+    if (base + kTokens < rows) to_gates(base + kTokens, zi, zf, gi, gf);
   }
 #pragma unroll
   for (int c = 0; c < C; ++c)
