@@ -433,7 +433,8 @@ __device__ bool tile_router_projection(const TileDesc& t, int tid, const LayerCt
 // (token ascending, pick ascending: the stable pack), the last term counted here from
 // the chunk's ids; otherwise the reference's arrival order through atomicAdd(fill[e]).
 // pair_pos (optional) receives the packed row of every pair.
-__device__ void tile_permute(const TileDesc& t, int tid) {
+// (Not inlined: its registers would be the fabric kernel's, whose GEMM and attention roles then spill.)
+__device__ __noinline__ void tile_permute(const TileDesc& t, int tid) {
   int* const s_ids = s_exec_scratch;   // ids of the chunk's rows up to the end of this tile
   PermuteArgs A;   // a copy in registers: the block lives in global memory
   load_block(A, t.a[0]);
@@ -449,7 +450,18 @@ __device__ void tile_permute(const TileDesc& t, int tid) {
     for (int p = tid; p < n; p += kExecThreads) s_ids[p] = ids[static_cast<size_t>(chunk0) * K + p];
     exec_sync();
   }
+  // a row's first 2048 columns are under way while its places are found (one 16-byte piece after the other: 79 us for 4096 rows
+  // x 8 x 2048, now 60)
+  constexpr int NR = 8;
+  uint4 v[NR];
+  auto load = [&](uint32_t r, int c0) {
+    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(A.src) + static_cast<size_t>(r) * H) + c0 + lane;
+#pragma unroll
+    for (int i = 0; i < NR; ++i)
+      if (c0 + 32 * i + lane < n16) v[i] = src[32 * i];
+  };
   for (uint32_t r = t.i0 + warp; r < t.i0 + t.i1; r += kExecThreads / 32) {
+    load(r, 0);
     int pos = 0;
     if (lane < K) {
       const int e = ids[static_cast<size_t>(r) * K + lane];
@@ -465,12 +477,14 @@ __device__ void tile_permute(const TileDesc& t, int tid) {
       reinterpret_cast<float*>(A.pair_weight)[pos] = tw[static_cast<size_t>(r) * K + lane];
       if (A.pair_pos) reinterpret_cast<int*>(A.pair_pos)[static_cast<size_t>(r) * K + lane] = pos;
     }
-    const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(A.src) + static_cast<size_t>(r) * H);
-    for (int c = lane; c < n16; c += 32) {
-      const uint4 v = src[c];
+    for (int c0 = 0; c0 < n16; c0 += 32 * NR) {
+      if (c0 > 0) load(r, c0);
       for (int k = 0; k < K; ++k) {
-        const int pk = __shfl_sync(0xffffffffu, pos, k);
-        reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(A.dst) + static_cast<size_t>(pk) * H)[c] = v;
+        uint4* const to = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(A.dst) +
+                                                   static_cast<size_t>(__shfl_sync(0xffffffffu, pos, k)) * H) + c0 + lane;
+#pragma unroll
+        for (int i = 0; i < NR; ++i)
+          if (c0 + 32 * i + lane < n16) to[32 * i] = v[i];
       }
     }
   }

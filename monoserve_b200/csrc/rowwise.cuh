@@ -190,13 +190,12 @@ __device__ __forceinline__ unsigned long long pick_key(float score, int expert) 
 }
 __device__ __forceinline__ int key_expert(unsigned long long key) { return static_cast<int>(0xffffffffu - static_cast<unsigned int>(key)); }
 
+// Two reductions of 32-bit words: the scores, then the experts of the lanes that hold the best one.  (Five exchanges of 64-bit
+// keys, each waiting for the one before, were most of a row's routing.)  Every lane's key is zero or has a nonzero lower word.
 __device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    const unsigned long long other = __shfl_xor_sync(0xffffffffu, k, o);
-    k = other > k ? other : k;
-  }
-  return k;
+  const uint32_t score = static_cast<uint32_t>(k >> 32), best = __reduce_max_sync(0xffffffffu, score);
+  const uint32_t expert = __reduce_max_sync(0xffffffffu, score == best ? static_cast<uint32_t>(k) : 0u);
+  return static_cast<unsigned long long>(best) << 32 | expert;
 }
 
 }  // namespace route

@@ -343,7 +343,8 @@ class ModelLane(LaneBase):
             s_lg = p.stage(tiles, label=("norm_logits", l))
         else:
             s_lg = p.stage(self._logits(lg, T, E), label=("router_logits", l))
-        s_rt = p.stage(self._rows(K_ROUTER, self.router_args[l], T, SUB), label=("router", l))
+        # a tile costs about as much before its first row as a few rows do: many rows go by whole chunks
+        s_rt = p.stage(self._rows(K_ROUTER, self.router_args[l], T, CHUNK if T >= 8 * nw else SUB), label=("router", l))
         p.after(prev, s_lg)
         p.after(s_lg, s_rt)
         xn_ready = s_lg if fuse_norm is not None else prev
