@@ -210,6 +210,7 @@ __device__ void tile_attn_plan(const TileDesc& t, const ProgramDesc* P, DeviceSt
 __device__ void tile_embed(const TileDesc& t, int tid) {
   NormArgs A;
   load_block(A, t.a[0]);
+  if (!A.step && t.i1 >= kAheadRows && A.H % 256 == 0 && A.H <= 2048) return norm_rows_ahead<true>(t, tid);
   const int warp = tid >> 5, lane = tid & 31;
   const int H = static_cast<int>(A.H), n16 = H / 8;
   StepArgs St{};

@@ -455,7 +455,7 @@ class ModelLane(LaneBase):
             if w.mlp_w13[l] is None and T <= FUSE_ROWS:
                 prev = self._moe(p, l, T, s_o, next_norm, expands, fuse_norm=(norm_kind, nrm))
                 continue
-            s_norm = p.stage(self._rows(norm_kind, nrm, T, self._per(T)),
+            s_norm = p.stage(self._rows(norm_kind, nrm, T, self._per_streamed(T)),
                              label=("norm", l))
             p.after(s_o, s_norm)
             next_norm = w.in_norm[l + 1] if l + 1 < L else None
@@ -470,7 +470,7 @@ class ModelLane(LaneBase):
                 prev = s_d2
                 if next_norm is not None:
                     nn = self._dev("NormArgs", x=self.x, w=next_norm, out=self.xn, H=H, ld=H, eps=cfg.rms_eps)
-                    prev = p.stage(self._rows(K_RMSNORM, nn, T, self._per(T)),
+                    prev = p.stage(self._rows(K_RMSNORM, nn, T, self._per_streamed(T)),
                                    label=("in_norm", l + 1))
                     p.after(s_d2, prev)
                 continue
@@ -479,7 +479,7 @@ class ModelLane(LaneBase):
         R = n_rows
         fin = self._dev("NormArgs", x=self.x, w=w.final_norm, out=self.xn, gather=self.gather, out2=self.xlast, H=H, ld=H,
                      eps=cfg.rms_eps)
-        s_fin = p.stage(self._rows(K_RMSNORM, fin, T, self._per(T)), label=("final_norm", L))
+        s_fin = p.stage(self._rows(K_RMSNORM, fin, T, self._per_streamed(T)), label=("final_norm", L))
         p.after(prev, s_fin)
         s_lm = self._gemm(p, self.m_lm, self.m_xlast, R, cfg.vocab, H, self.logits, cfg.vocab, EPI_F32, ("lm_head", L))
         p.after(s_fin, s_lm)
@@ -506,7 +506,7 @@ class ModelLane(LaneBase):
         p = Program()
         emb = self._dev("NormArgs", x=self.x, w=self.w.in_norm[0], out=self.xn, embed=self.w.embed, tokens=self.tokens,
                      H=cfg.hidden, ld=cfg.hidden, eps=cfg.rms_eps)
-        s_embed = p.stage(self._rows(K_EMBED, emb, T, CHUNK), label=("embed", 0))
+        s_embed = p.stage(self._rows(K_EMBED, emb, T, CHUNK if T <= 4 * self.fab.num_workers else self._per_streamed(T)), label=("embed", 0))
 
         item_tiles, merge_tiles = fabric_tiles(items, merge, 0, K_ATTN_PREFILL)   # the same work list in every layer
 

@@ -191,3 +191,56 @@ def test_router_projection(fab, H, rows, experts):  # noqa: F811
     run_program(fab, p, p.stage([Tile(48, i=(0, rows, 0, 0), a=(args.data_ptr(),))]))
     want = oracle.router_logits(oracle.bf16_bits(x), oracle.bf16_bits(wr))
     assert np.array_equal(out.cpu().numpy().view(np.int32), want.view(np.int32))
+
+
+@pytest.mark.parametrize("divide,silu", [(0, 1), (1, 0)])
+@pytest.mark.parametrize("e", [132, 256, 512, 516])
+def test_head_norm_ahead_or_not(fab, e, divide, silu):  # noqa: F811
+    """Tiles of more than four items load one item ahead (heads of 129 to 512 columns); tiles of four do not: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(e)
+    rows, heads = 13, 3
+    oe = (e + (4 if divide else 3)) & ~3
+    o, w = torch.randn(rows, heads, oe, generator=g, device="cuda"), torch.randn(heads, e, generator=g, device="cuda")
+    if divide:
+        o[:, :, e] = 0.5 + torch.rand(rows, heads, generator=g, device="cuda")
+    gate = torch.randn(rows, heads * e, generator=g, device="cuda").to(torch.bfloat16)
+    outs = []
+    for per in (4, 5, rows * heads):
+        out = torch.zeros(rows, heads * e, device="cuda", dtype=torch.bfloat16)
+        block = pack("HeadNormArgs", o=o, g=gate, w=w, out=out, heads=heads, e=e, ld_g=heads * e, ld_out=heads * e, eps=EPS, divide=divide, silu=silu,
+                     w_head=e)
+        torch.cuda.synchronize()
+        run_rows(fab, 58, block, rows * heads, per)
+        outs.append(out)
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    x = o[:, :, :e].double() / (o[:, :, e:e + 1].double() if divide else 1)
+    z = gate.double().view(rows, heads, e)
+    close(outs[0].view(rows, heads, e), over_rms(x) * w.double() * z.sigmoid() * (z if silu else 1), "out")
+
+
+@pytest.mark.parametrize("embedding", [False, True])
+@pytest.mark.parametrize("H", [256, 768, 2048, 2304])
+def test_norm_rows_ahead_or_not(fab, H, embedding):  # noqa: F811
+    """Tiles of eight rows and more load a row ahead (up to 2048 columns); tiles of four do not: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(H)
+    rows = 61
+    table, w = (torch.randn(n, H, generator=g, device="cuda").to(torch.bfloat16) for n in (40, 1))
+    tokens = torch.randint(0, 40, (rows,), generator=g, device="cuda", dtype=torch.int32)
+    gather = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    gather[rows - 1], gather[1] = 0, 1
+    outs = []
+    for per in (4, 9, 28):
+        x = torch.zeros(rows, H, device="cuda", dtype=torch.bfloat16) if embedding else table[tokens.long()]
+        out, out2 = (torch.zeros(n, H, device="cuda", dtype=torch.bfloat16) for n in (rows, 2))
+        more = dict(embed=table, tokens=tokens) if embedding else dict(gather=gather, out2=out2)
+        block = pack("NormArgs", x=x, w=w, out=out, H=H, ld=H, eps=EPS, **more)
+        torch.cuda.synchronize()
+        run_rows(fab, 42 if embedding else 36, block, rows, per)
+        outs.append((x, out, out2))
+    for other in outs[1:]:
+        for a, b in zip(outs[0], other):
+            assert torch.equal(a, b)
+    x, out, out2 = outs[0]
+    assert torch.equal(x, table[tokens.long()])
+    close(out, over_rms(x.double()) * w.double(), "out")
+    assert embedding or torch.equal(out2, out[[rows - 1, 1]])
