@@ -392,10 +392,15 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackParams A) {
 
 // ------------------------------------------------------------------- combine
 
-constexpr int kCombineSplit = 4;   // warps per token when no row reduction follows
+// Warps per token when no row reduction follows: four, and for batches that leave the schedulers idle (kFew) one per 256 columns.
+// There a warp's chain of loads is what it takes; where warps are many, four rows' loads in each cost registers and 1 % (8192
+// tokens).  64 tokens of 4096 columns: the layer 642 -> 620 us.
+constexpr int kFewTokens = 74;   // two blocks of four warps per token for an SM
+__host__ __device__ __forceinline__ int combine_split(int H, bool norm, bool few) { return norm ? 1 : few ? max(4, H / 256) : 4; }
 
+template <bool kFew>
 __global__ void __launch_bounds__(256) combine_kernel(const CombineParams A) {
-  // Without the fused RMSNorm a row needs no reduction, so kCombineSplit warps share a token's columns:
+  // Without the fused RMSNorm a row needs no reduction, so several warps share a token's columns:
   // a decode batch of a few hundred tokens otherwise leaves most of the machine idle.  Every column is
   // computed by the same instructions either way: the result does not depend on the split.
   const int lane = threadIdx.x & 31;
@@ -406,7 +411,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineParams A) {
       atomicOr(A.status, kErrWaitTimeout);
     __syncthreads();
   }
-  const int split = A.norm_w ? 1 : kCombineSplit;
+  const int split = combine_split(A.H, A.norm_w != nullptr, kFew);
   const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int t = unit / split, part = unit - t * split;
   if (t >= A.T) return;
@@ -429,20 +434,50 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineParams A) {
     float acc[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j] = 0.f;
-    for (int k = 0; k < K; ++k) {
-      const int pk = __shfl_sync(0xffffffffu, pos, k);
-      const float wk = __shfl_sync(0xffffffffu, w, k);
-      if (pk < 0 || (A.y_rows && pk >= A.y_rows)) continue;   // a dropped pair adds nothing
-      const float4* yr = reinterpret_cast<const float4*>(A.y + static_cast<size_t>(pk) * H) + 2 * c;
-      const float4 a = __ldcs(yr), b = __ldcs(yr + 1);
-      acc[0] = __fmaf_rn(wk, a.x, acc[0]);
-      acc[1] = __fmaf_rn(wk, a.y, acc[1]);
-      acc[2] = __fmaf_rn(wk, a.z, acc[2]);
-      acc[3] = __fmaf_rn(wk, a.w, acc[3]);
-      acc[4] = __fmaf_rn(wk, b.x, acc[4]);
-      acc[5] = __fmaf_rn(wk, b.y, acc[5]);
-      acc[6] = __fmaf_rn(wk, b.z, acc[6]);
-      acc[7] = __fmaf_rn(wk, b.w, acc[7]);
+    if constexpr (kFew) {   // four expert rows' loads are issued before the first is used
+      for (int k0 = 0; k0 < K; k0 += 4) {
+        float4 a[4], b[4];
+        bool there[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int pk = __shfl_sync(0xffffffffu, pos, min(k0 + i, K - 1));
+          there[i] = k0 + i < K && pk >= 0 && !(A.y_rows && pk >= A.y_rows);   // a dropped pair adds nothing
+          const float4* yr = reinterpret_cast<const float4*>(A.y + static_cast<size_t>(there[i] ? pk : 0) * H) + 2 * c;
+          if (there[i]) {
+            a[i] = __ldcs(yr);
+            b[i] = __ldcs(yr + 1);
+          }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float wk = __shfl_sync(0xffffffffu, w, min(k0 + i, K - 1));
+          if (!there[i]) continue;
+          acc[0] = __fmaf_rn(wk, a[i].x, acc[0]);
+          acc[1] = __fmaf_rn(wk, a[i].y, acc[1]);
+          acc[2] = __fmaf_rn(wk, a[i].z, acc[2]);
+          acc[3] = __fmaf_rn(wk, a[i].w, acc[3]);
+          acc[4] = __fmaf_rn(wk, b[i].x, acc[4]);
+          acc[5] = __fmaf_rn(wk, b[i].y, acc[5]);
+          acc[6] = __fmaf_rn(wk, b[i].z, acc[6]);
+          acc[7] = __fmaf_rn(wk, b[i].w, acc[7]);
+        }
+      }
+    } else {
+      for (int k = 0; k < K; ++k) {
+        const int pk = __shfl_sync(0xffffffffu, pos, k);
+        const float wk = __shfl_sync(0xffffffffu, w, k);
+        if (pk < 0 || (A.y_rows && pk >= A.y_rows)) continue;   // a dropped pair adds nothing
+        const float4* yr = reinterpret_cast<const float4*>(A.y + static_cast<size_t>(pk) * H) + 2 * c;
+        const float4 a = __ldcs(yr), b = __ldcs(yr + 1);
+        acc[0] = __fmaf_rn(wk, a.x, acc[0]);
+        acc[1] = __fmaf_rn(wk, a.y, acc[1]);
+        acc[2] = __fmaf_rn(wk, a.z, acc[2]);
+        acc[3] = __fmaf_rn(wk, a.w, acc[3]);
+        acc[4] = __fmaf_rn(wk, b.x, acc[4]);
+        acc[5] = __fmaf_rn(wk, b.y, acc[5]);
+        acc[6] = __fmaf_rn(wk, b.z, acc[6]);
+        acc[7] = __fmaf_rn(wk, b.w, acc[7]);
+      }
     }
     float f[8];
     if (x2) {
@@ -534,8 +569,9 @@ cudaError_t launch_pack_chain(const int* topk_ids, const float* topk_w, int T, i
 
 cudaError_t launch_combine(const CombineParams& A, cudaStream_t stream) {
   if (A.T == 0) return cudaSuccess;
-  const int units = A.T * (A.norm_w ? 1 : kCombineSplit);
-  return launch_chained(combine_kernel, (units + 7) / 8, 256, 0, stream, A);
+  const bool few = A.T <= kFewTokens;
+  const int units = A.T * combine_split(A.H, A.norm_w != nullptr, few);
+  return launch_chained(few ? combine_kernel<true> : combine_kernel<false>, (units + 7) / 8, 256, 0, stream, A);
 }
 
 }  // namespace mf
