@@ -42,13 +42,18 @@ __device__ bool run_layer_tile(const TileDesc& t, int tid, const LayerCtx& ctx);
 // Row tiles of at least this many rows bring them through the operand ring (RowStages): a step's few rows would wait for the
 // ring's earlier users and gain nothing.
 constexpr uint32_t kBulkRows = 4, kCombineRows = 16, kLogitsRows = 9;
-// Wide tiles: their exec warps use the operand ring as scratch memory, and TMEM.
+// Wide tiles: their exec warps use the operand ring as scratch memory, and TMEM.  The scheduler asks for every record, on the way of a
+// step's small stages: two bit tests by kind.
+constexpr unsigned long long kind_bit(uint32_t kind) { return 1ull << (kind - 32); }
 __device__ __forceinline__ bool tile_is_wide(const TileDesc& t) {
-  const uint32_t kind = t.kind, rows = t.i1;
-  if (kind == kTileStreams || kind == kTileResidual) return rows >= kBulkRows;
-  if (kind == kTileCombine) return rows >= kCombineRows;
-  if (kind == kTileRouterLogits) return rows >= kLogitsRows && t.i2 == 0 && t.i3 == 0;
-  return kind == kTileMemory || kind == kTileScan || kind == kTileGatedMemory || kind == kTileGatedStep || kind == kTileLatentMma || kind == kTileLatentDirect;
+  constexpr unsigned long long kAlways = kind_bit(kTileMemory) | kind_bit(kTileScan) | kind_bit(kTileGatedMemory) |
+                                         kind_bit(kTileGatedStep) | kind_bit(kTileLatentMma) | kind_bit(kTileLatentDirect);
+  constexpr unsigned long long kByRows = kind_bit(kTileStreams) | kind_bit(kTileResidual) | kind_bit(kTileCombine) | kind_bit(kTileRouterLogits);
+  const uint32_t kind = t.kind;
+  const unsigned long long bit = kind >= 32 && kind < 96 ? 1ull << (kind - 32) : 0ull;
+  if ((bit & kByRows) == 0) return (bit & kAlways) != 0;
+  if (kind == kTileRouterLogits) return t.i1 >= kLogitsRows && t.i2 == 0 && t.i3 == 0;
+  return t.i1 >= (kind == kTileCombine ? kCombineRows : kBulkRows);
 }
 
 __device__ bool tile_streams(const TileDesc& t, int tid, const LayerCtx& ctx);
