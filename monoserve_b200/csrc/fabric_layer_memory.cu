@@ -484,8 +484,10 @@ __device__ __noinline__ void memory_steps(const TileDesc& t, int tid, uint8_t* r
         ld_vec<4>(sh.mix[s] + 4 * i, mix);
         float y = sh.read[s][i] * o[0];
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          y = fmaf(mix[j], normaliser ? 1.f : __bfloat162float(in.v[4 * s + j][own_col]), y);
+        for (int j = 0; j <= 2 * h + 1; ++j) {   // the tokens up to this one: a weight of zero would carry a later one's infinity into it
+          const float x = normaliser ? 1.f : __bfloat162float(in.v[4 * s + j][own_col]);
+          y = fmaf(mix[j], j <= i ? x : 0.f, y);
+        }
         const int tok = 4 * s + i;
         if (owner && tok < nt)
           out[static_cast<size_t>(base + tok) * ld_out] = normaliser ? fmaxf(fabsf(y), sh.low[tok]) + 1e-6f : y;
