@@ -77,6 +77,11 @@ struct WorkSlot {
 // 64 gate rows at i0 and the 64 up rows at up_offset + i0, and a partial sum goes to column = weight row (the
 // layout the reduce tile, kind 46, reads).  The weights of the slice are re-read per row block (from L2 when
 // they are in HBM); the staged form is this library's own answer to reading a host-resident expert once.
+// Tiles of two weight slices: bf16 weights, and no epilogue that adds.
+__device__ __forceinline__ bool takes_two_slices(const GemmArgs& A) {
+  return A.w_fp8 == 0 && A.epi != kEpiAtomicF32 && A.epi != kEpiWeightedAdd;
+}
+
 __device__ bool make_gemm_work(const TileDesc& t, GemmWork& w, uint32_t block = 0) {
   GemmArgs A;
   const uint4* src = reinterpret_cast<const uint4*>(t.a[0]);
@@ -118,7 +123,7 @@ __device__ bool make_gemm_work(const TileDesc& t, GemmWork& w, uint32_t block = 
   w.w_fp8 = A.w_fp8 != 0;   // e4m3 weights: the exec warps expand every stage to bf16 before its MMAs
   w.fetch = 0;
   w.slices = 1 + static_cast<int32_t>((t.a[3] >> 32) & 1);
-  if (w.slices == 2 && (w.w_fp8 || A.epi == kEpiAtomicF32 || A.epi == kEpiWeightedAdd)) return false;
+  if (w.slices == 2 && !takes_two_slices(A)) return false;
   return w.k_tiles > 0 && A.epi <= kEpiDecay;
 }
 
@@ -782,7 +787,7 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
   int& s_active = s_exec_scratch[4 * (kMaxExperts + 1) + 1];
   int& s_skipped = s_exec_scratch[4 * (kMaxExperts + 1) + 2];
   int& s_overflow = s_exec_scratch[4 * (kMaxExperts + 1) + 3];
-  int& s_bf16 = s_exec_scratch[4 * (kMaxExperts + 1) + 4];
+  int& s_wide = s_exec_scratch[4 * (kMaxExperts + 1) + 4];
   int* const s_info = s_exec_scratch + 4 * (kMaxExperts + 1) + 16;   // [kMaxExperts]: slot << 12 | region << 4 | wide << 3 | height class
   // [28] u64: GemmArgs and activation maps per height class (w13, w2), weight maps per region (w13, w2)
   unsigned long long* const s_tab = reinterpret_cast<unsigned long long*>(s_exec_scratch + 5 * (kMaxExperts + 1) + 16 + 1);
@@ -846,9 +851,19 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
       if (e2 == ep) break;
       ep = e2;
     }
-    const unsigned long long a13 = reinterpret_cast<const unsigned long long*>(A.w13_args)[0];
-    s_bf16 = a13 != 0 && __ldcg(&reinterpret_cast<const GemmArgs*>(a13)->w_fp8) == 0;
     s_form = (f == 0 || f == 16 || f == 32 || f == 64 || f == 128) ? static_cast<int>(f) : 64;
+  } else if (tid == 32) {   // beside thread 0: whether both products can take 256-row blocks with tiles of two weight slices
+    auto tallest = [](unsigned long long table) { return reinterpret_cast<const unsigned long long*>(table)[4]; };
+    const unsigned long long a[2] = {tallest(A.w13_args), tallest(A.w2_args)};
+    bool ok = a[0] && a[1] && tallest(A.xp_maps) && tallest(A.h_maps);   // a program may leave the tallest class out
+    if (ok) {
+      GemmArgs g[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) load_block(g[i], a[i]);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ok = ok && g[i].bm == 256 && takes_two_slices(g[i]);
+    }
+    s_wide = ok;
   }
   exec_sync();
   stamp();
@@ -875,8 +890,8 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     if (link) return s_form ? s_form : 256;
     return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   };
-  // An expert in HBM with bf16 weights and more than 128 rows: blocks of 256 rows with tiles of two weight slices while
-  // more than 128 rows are left, then one block of up to 128 (its class is the one kept in s_info).  The two-slice tiles
+  // An expert in HBM with more than 128 rows, where both products take them (s_wide): blocks of 256 rows with tiles of two weight
+  // slices while more than 128 rows are left, then one block of up to 128 (its class is the one kept in s_info).  The two-slice tiles
   // read the L2 half as often per product: 4096 tokens over 128 experts, the layer's experts 590 -> 381 us.
   const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2;
   auto shape = [&](int M, int info, int& wide, int& narrow) {   // row blocks of either kind
@@ -892,7 +907,7 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     const int region = static_cast<int>(entry & 0xffffffffu), slot = static_cast<int>(entry >> 32);
     const bool link = region == static_cast<int>(A.host_region);
     const bool staged = link && can_stage && s_form == 0 && M > static_cast<int>(G.min_rows);
-    const bool wide = s_bf16 && M > 128 && (!link || staged);
+    const bool wide = s_wide && M > 128 && (!link || staged);
     const int left = M % 256;
     const int bm = wide ? block_rows(left > 128 ? 0 : left, false) : block_rows(M, link);
     int cls = 0;

@@ -80,7 +80,7 @@ struct GemmWork {
                               // partial sums go to column = weight row (kEpiSiluMul always reads two slabs)
   int32_t block;              // row block whose counter the epilogue bumps, or -1
   int32_t w_fp8;              // the weight tensor holds e4m3 bytes: W8A16 (exact e4m3 -> bf16 in shared memory)
-  int32_t slices;             // 1, or 2: two adjacent weight slices (bf16 weights, kEpiAtomicF32 excepted), each with an
+  int32_t slices;             // 1, or 2: two adjacent weight slices (bf16 weights, no epilogue that adds), each with an
                               // accumulator buffer of its own
   // A fetch record moves fetch_bytes from fetch_src (host-resident weights) to `out` (an HBM staging
   // buffer) through the operand ring, in stages of kFetchStageBytes: no MMA, no accumulator.

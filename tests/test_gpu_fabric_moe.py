@@ -84,6 +84,98 @@ def test_moe_layer_program(form, pack_hot):
         fab.close()
 
 
+def directed(counts, wr, seed):
+    """Activations that pick expert e counts[e] times (top-1), in a random order."""
+    g = torch.Generator().manual_seed(seed)
+    e = torch.repeat_interleave(torch.arange(len(counts)), torch.tensor(counts))
+    e = e[torch.randperm(len(e), generator=g)]
+    return (8 * wr[e].float() + 0.5 * torch.randn(len(e), wr.shape[1], generator=g)).to(torch.bfloat16), e
+
+
+EDGES = [1, 128, 129, 255, 256, 257, 0, 384, 385, 640, 700]   # row counts on the edges of 128- and 256-row blocks
+
+
+@pytest.mark.parametrize("hot,staged,form", [("all", False, 64), ("half", False, 64), ("half", True, 0), ("half", False, 0)])
+def test_row_blocks_at_their_edges(hot, staged, form):
+    """Experts whose row counts lie on the edges of row blocks, with an odd number of w13 slices, in HBM, read in place and
+    staged (more than 200 rows)."""
+    from monoserve_b200.fabric import Fabric
+    from monoserve_b200.lane import MoELane
+    H, I, E = 512, 192, len(EDGES)
+    wr, w13, w2 = weights(H, I, E, 11)
+    xn, _ = directed(EDGES, wr, 12)
+    T = len(xn)
+    x2 = acts(T, H, 13)[1]
+    fab = Fabric(pool_bytes=128 << 20)
+    fab.set_max_run(60)
+    try:
+        lane = MoELane(fab, 0, H, I, E, 1, T, wr, w13, w2, hot=list(range(0, E, 1 if hot == "all" else 2)), staged=staged,
+                       staged_min_rows=200)
+        lane.set_input(xn.cuda(), x2.cuda())
+        h = lane.build(T, iterations=1)
+        fab.start()
+        fab.publish(map=[0] * fab.num_workers, caps=[4], order=[0], programs=[h], forms=[form])
+        wait_iterations(fab, 0, 1)
+        fab.stop()
+        assert fab.progress()["error"] == 0
+        assert np.diff(lane.starts.cpu().numpy()).tolist() == EDGES
+        check_lane(lane, wr, w13, w2, xn, x2, 1)
+    finally:
+        fab.stop()
+        fab.close()
+
+
+@pytest.mark.parametrize("what", ["weighted_add", "no_tallest_class", "e4m3_w2"])
+def test_programs_whose_products_take_no_two_slice_tiles(what):
+    """Expand blocks with more than 128 rows an expert whose w2 adds with atomics, whose operand tables end at 128 rows, or
+    whose two products have weights of different types."""
+    from monoserve_b200 import _C
+    from monoserve_b200.fabric import Fabric
+    from monoserve_b200.lane import MoELane
+    from oracle import torch_path as tp
+    counts = [129, 300, 40, 256]
+    H, I, E = 512, 256, len(counts)
+    wr, w13, w2 = weights(H, I, E, 21)
+    xn, pick = directed(counts, wr, 22)
+    T = len(xn)
+    fab = Fabric(pool_bytes=128 << 20)
+    fab.set_max_run(60)
+    try:
+        lane = MoELane(fab, 0, H, I, E, 1, T, wr, w13, w2, hot=list(range(E)))
+        lane.set_input(xn.cuda())
+        acc = torch.zeros(T, H, device="cuda")
+        heights, fields = [16, 32, 64, 128, 256], dict(k_tiles=I // 64, n_limit=H, ld_out=H)
+        if what == "weighted_add":
+            fields.update(out=acc.data_ptr(), epi=2, pair_token=lane.pair_token.data_ptr(), pair_weight=lane.pair_weight.data_ptr())
+        elif what == "e4m3_w2":
+            q2, s2, w2 = tp.quantize_fp8(w2.float())
+            lane.hot_w2 = q2.cuda()
+            lane.w2_maps[1] = fab.tensor_map(lane.hot_w2.data_ptr(), [I, H, E], [I, H * I], [128, 64, 1], dtype=2, swizzle=0)
+            lane.scales = (torch.ones(E, 2 * I, device="cuda"), s2.float().cuda())
+            fields.update(out=lane.y.data_ptr(), epi=5, w_fp8=1)
+        if what == "no_tallest_class":
+            for t in (lane.w13_args, lane.w2_args, lane.xp_maps, lane.h_maps):
+                t[4] = 0
+        else:
+            blocks = [torch.frombuffer(bytearray(_C.gemm_args(bm=bm, **fields)), dtype=torch.uint8).cuda() for bm in heights]
+            lane.w2_args.copy_(torch.tensor([b.data_ptr() for b in blocks]))
+        h = lane.build(T, iterations=1)
+        fab.start()
+        fab.publish(map=[0] * fab.num_workers, caps=[4], order=[0], programs=[h], forms=[64])
+        wait_iterations(fab, 0, 1)
+        fab.stop()
+        assert fab.progress()["error"] == 0
+        y = torch.zeros(T, H)
+        for e in range(E):
+            y[pick == e] = tp.ffn(xn[pick == e].float(), w13[e].float(), w2[e].float())   # top-1: the routing weight is one
+        got = acc.cpu() if what == "weighted_add" else lane.x[:T].float().cpu()
+        rel = float((got - y).norm() / y.norm())
+        assert rel < 1e-2, rel   # h and x are bf16: 2^-9 of each value
+    finally:
+        fab.stop()
+        fab.close()
+
+
 @pytest.mark.parametrize("hot", ["none", "half"])
 def test_staged_form_reads_each_expert_once(hot):
     """Form 0 with a staging stack: host-resident experts with more rows than the threshold are
