@@ -268,7 +268,7 @@ __device__ __forceinline__ bool gemm_mma_two(const GemmWork& w, uint8_t* ring, G
     uint32_t vb, ve;
     const uint32_t phys = pipe.alloc(size, vb, ve);
     ok = ok && mbar_wait_bounded(&bar.full[pipe.slot], pipe.parity, abort_flag, kWaitBudgetNs);
-    __syncwarp();   // a lane two laps of the barrier ring behind the leader would wait for a phase that never comes
+    __syncwarp();   // as in gemm_mma
     tc_fence_after_sync();
     const uint64_t da = desc0 + ((ring_addr + phys) >> 4), db = da + (2 * kATileBytes >> 4);
     if (leader && ok) {
@@ -295,8 +295,8 @@ __device__ __forceinline__ bool gemm_mma_two(const GemmWork& w, uint8_t* ring, G
 }
 
 // MMA issue for one tile into accumulator g (buffer g & 1).
-// The whole MMA warp runs the K loop in step (every lane waits for the stage itself) and one elected
-// lane issues the four tcgen05.mma and the commit of a stage.  Because the loop is convergent code,
+// The whole MMA warp runs the K loop in step (every lane waits for the stage itself, and the warp meets behind the wait) and one
+// elected lane issues the four tcgen05.mma and the commit of a stage.  Because the loop is convergent code,
 // its descriptors and addresses are warp-uniform values; with the loop inside a single-lane branch
 // the MMA warp spent twice as long issuing (measured: 67 -> 32 us of a 150 us launch), which is
 // what bounds small-N tiles.
@@ -326,20 +326,19 @@ __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmB
     const int k_steps = w.k_tiles;
     const uint32_t fetch_bytes = kFetch ? w.fetch_bytes : 0;
     uint8_t* const fetch_out = static_cast<uint8_t*>(w.out);
-    for (int kt = 0; ok && kt < n_stages; ++kt) {
+    for (int kt = 0; kt < n_stages; ++kt) {
       uint32_t vb, ve;
       const uint32_t phys = pipe.alloc(size, vb, ve);
       const long long tw = wait_cycles ? clock64() : 0;
       const uint32_t ready_parity = fp8 ? (pipe.conv_bits >> pipe.slot) & 1u : pipe.parity;
-      if (!mbar_wait_bounded(&ready[pipe.slot], ready_parity, abort_flag, kWaitBudgetNs)) {
-        ok = 0;
-        break;
-      }
+      ok = ok && mbar_wait_bounded(&ready[pipe.slot], ready_parity, abort_flag, kWaitBudgetNs);
+      // a lane that has not seen the stage when the leader frees it would miss its phase once it is filled again, and wait for good
+      __syncwarp();
       if (fp8) pipe.conv_bits ^= 1u << pipe.slot;
       if (wait_cycles) wait_cycles[0] += clock64() - tw;
       if (fetch) {
         // the stage goes on to the staging buffer; its shared memory is free once the store has read it
-        if (leader) {
+        if (leader && ok) {
           const uint32_t at = kt * kFetchStageBytes;
           bulk_store(fetch_out + at, ring + phys, min(kFetchStageBytes, fetch_bytes - at));
           bulk_commit();
@@ -350,7 +349,7 @@ __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmB
         continue;
       }
       const long long ti = wait_cycles ? clock64() : 0;
-      if (!leader) {
+      if (!leader || !ok) {
       } else if (!fp8) {   // one K step: weight tile, activation tile
         const uint64_t da = desc0 + ((ring_addr + phys) >> 4);
         const uint64_t db = da + (kATileBytes >> 4);
@@ -369,7 +368,7 @@ __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmB
             umma_bf16(acc, da + (kATileBytes >> 4) + 2 * k, db + (b_bytes >> 4) + 2 * k, idesc, true);
         }
       }
-      if (leader) umma_commit(&bar.empty[pipe.slot]);
+      if (leader && ok) umma_commit(&bar.empty[pipe.slot]);
       if (wait_cycles) wait_cycles[1] += clock64() - ti;
       pipe.advance();
     }
