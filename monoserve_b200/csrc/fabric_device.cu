@@ -491,8 +491,8 @@ __device__ __noinline__ void tile_router_logits(const TileDesc& t, int tid) {
 
 __device__ bool tile_router_projection(const TileDesc& t, int tid, const LayerCtx& ctx) {
   const LogitsArgs* p = reinterpret_cast<const LogitsArgs*>(t.a[0]);
-  const uint32_t H = __ldcg(&p->H);
   if (t.i1 >= kLogitsRows && t.i2 == 0 && t.i3 == 0 && ((__ldcg(&p->x) | __ldcg(&p->wr)) & 15) == 0) {
+    const uint32_t H = __ldcg(&p->H);
     // a quarter of the rows per warp in registers; in the ring all of them and two groups of weights
     if (t.i1 <= 16 && (32 + 16) * H <= kWideRingBytes) return router_logits_bulk<4>(t, tid, ctx);
     if (t.i1 <= 32 && (64 + 16) * H <= kWideRingBytes) return router_logits_bulk<8>(t, tid, ctx);

@@ -434,9 +434,10 @@ __device__ __noinline__ bool streams_bulk(const TileDesc& t, int tid, const Laye
 // Kind 53, StreamArgs: rows [i0, i0 + i1).
 __device__ bool tile_streams(const TileDesc& t, int tid, const LayerCtx& ctx) {
   const StreamArgs* p = reinterpret_cast<const StreamArgs*>(t.a[0]);
-  const uint32_t W = __ldcg(&p->W), ns = __ldcg(&p->streams), parts = __ldcg(&p->y_parts);
+  const uint32_t W = __ldcg(&p->W), ns = __ldcg(&p->streams);
   const bool four = (W & 3) == 0 && ns <= 4;
   if (t.i1 >= kBulkRows && four) {
+    const uint32_t parts = __ldcg(&p->y_parts);
     // two rows in the ring at least, or nothing overlaps
     if (__ldcg(&p->embed) == 0 && parts > 0 && (2 * (ns + parts) + 2) * W * 4 <= kWideRingBytes) return streams_bulk<false>(t, tid, ctx);
     // (W % 8: whole 16-byte pieces of bf16 rows)

@@ -468,14 +468,14 @@ __device__ __forceinline__ float epi_value(uint32_t acc, float sc, float bias, f
 // with a branch per row (two activations, rows past the end) a chunk took 1.9 us and the epilogue, one warp per
 // scheduler, bounded the products: 128 rows of a SwiGLU tile 8.2 us, now 2.2.  The next chunk's TMEM load, and the
 // residual's values of the next chunk, are under way while this one is converted and stored.  (The residual loaded where
-// it was added, a 2-byte load behind each 2-byte store, took 0.6 us a row.)
-template <int E>
+// it was added, a 2-byte load behind each 2-byte store, took 0.6 us a row.)  kSixteen: a tile may have 16 rows only.
+template <int E, bool kSixteen = false>
 __device__ __forceinline__ void epilogue_chunks(const GemmWork& w, uint32_t tacc, int f, int wrow, bool f_ok, float sc,
                                                 float bias, float coef) {
   const int lane = threadIdx.x & 31;
   const int n = w.n, rows = w.rows, ld = w.ld_out, c_end = min(n, rows);
   const bool lo = lane < 16;
-  constexpr bool kGated = E == kEpiSiluMul || E == kEpiGeluMul, kHalf = kGated || E == kEpiStoreBf16;
+  constexpr bool kGated = E == kEpiSiluMul || E == kEpiGeluMul;
   const size_t first = static_cast<size_t>(w.b_row0) * ld + (E == kEpiAtomicF32 && (w.a_packed & 4) ? wrow : f);
   unsigned short* const out16 = reinterpret_cast<unsigned short*>(w.out) + first;
   float* const out32 = reinterpret_cast<float*>(w.out) + first;
@@ -492,7 +492,7 @@ __device__ __forceinline__ void epilogue_chunks(const GemmWork& w, uint32_t tacc
   };
   uint32_t next[32];
   load_res(0);
-  if (n >= 32) {
+  if (!kSixteen || n >= 32) {
     tmem_ld_32x32(tacc, next);
   } else {
     uint32_t r16[16];
@@ -601,6 +601,102 @@ __device__ __forceinline__ void epilogue_chunks(const GemmWork& w, uint32_t tacc
   }
 }
 
+// The fabric kernel calls them: seven of them inlined cost its other roles registers (252 bytes of spills against 48).
+template <int E>
+__device__ __noinline__ void epilogue_call(const GemmWork& w, uint32_t tacc, int f, int wrow, bool f_ok, float sc, float bias,
+                                           float coef) {
+  __builtin_assume(__isShared(&w));
+  epilogue_chunks<E>(w, tacc, f, wrow, f_ok, sc, bias, coef);
+}
+
+// The one chunk of a tile of at most 32 activation rows, in the fabric: each row's store behind its own condition.  A decode step
+// runs every epilogue once or twice per SM, so what it waits for is the fetch of the instructions, of which epilogue_chunks has
+// several times as many.  (One step of 32 sequences of Sinotar 983 -> 961 us, of eight of the decoder 1515 -> 1499; the expert
+// kernel has two epilogues, which stay in its instruction cache, and takes epilogue_chunks for any height: 256 tokens 189 -> 184.)
+__device__ __forceinline__ void epilogue_few(const GemmWork& w, uint32_t tacc, int f, int wrow, bool f_ok, float sc, float bias) {
+  const int lane = threadIdx.x & 31;
+  uint32_t r[32];
+  if (w.n >= 32) {
+    tmem_ld_32x32(tacc, r);
+  } else {
+    uint32_t r16[16];
+    tmem_ld_32x16(tacc, r16);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      r[j] = r16[j];
+      r[16 + j] = 0;
+    }
+  }
+  tmem_ld_wait();
+  if (epi_gated(w.epi)) {
+    // lanes < 16 own gate rows, lanes >= 16 the matching up rows; exchange halves
+    const bool lo = lane < 16, gelu = w.epi == kEpiGeluMul;
+    const int t0 = lo ? 0 : 16;
+    unsigned short* out = reinterpret_cast<unsigned short*>(w.out) + static_cast<size_t>(w.b_row0 + t0) * w.ld_out + f;
+    unsigned short hv[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float mine = __uint_as_float(lo ? r[j] : r[16 + j]) * sc;
+      const float other = __shfl_xor_sync(0xffffffffu, __uint_as_float(lo ? r[16 + j] : r[j]) * sc, 16);
+      const float gate = lo ? mine : other, up = lo ? other : mine;
+      hv[j] = __bfloat16_as_ushort(__float2bfloat16(gelu ? gelu_mul(gate, up) : silu_mul(gate, up)));
+    }
+    if (!f_ok) return;
+    const int m_hi = w.rows - t0;
+#pragma unroll
+    for (int j = 0; j < 16; ++j)
+      if (j < m_hi) out[static_cast<size_t>(j) * w.ld_out] = hv[j];
+    return;
+  }
+  if (!f_ok) return;
+  if (w.epi == kEpiStoreBf16) {
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(w.out) + static_cast<size_t>(w.b_row0) * w.ld_out + f;
+    const __nv_bfloat16* res = w.residual ? w.residual + static_cast<size_t>(w.b_row0) * w.ld_res + f : nullptr;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      if (j < w.rows) {
+        float v = __uint_as_float(r[j]) * sc + bias;
+        if (res) v += __bfloat162float(res[static_cast<size_t>(j) * w.ld_res]);
+        __stcs(reinterpret_cast<unsigned short*>(out + static_cast<size_t>(j) * w.ld_out),
+               __bfloat16_as_ushort(__float2bfloat16(v)));
+      }
+    }
+    return;
+  }
+  if (w.epi == kEpiWeightedAdd) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      if (j < w.rows) {
+        const int m = w.b_row0 + j;
+        atomicAdd(reinterpret_cast<float*>(w.out) + f + static_cast<size_t>(w.pair_token[m]) * w.ld_out,
+                  w.pair_weight[m] * (__uint_as_float(r[j]) * sc));
+      }
+    }
+    return;
+  }
+  // a two-slab tile (partial sums of a SwiGLU pair) adds into the column of its weight row
+  float* const out = reinterpret_cast<float*>(w.out) + static_cast<size_t>(w.b_row0) * w.ld_out +
+                     (w.epi == kEpiAtomicF32 && (w.a_packed & 4) ? wrow : f);
+  if (w.epi == kEpiAtomicF32) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < w.rows) atomicAdd(out + static_cast<size_t>(j) * w.ld_out, __uint_as_float(r[j]) * sc + bias);
+  } else if (w.epi == kEpiDecay) {
+    const float coef = w.pair_weight[f];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(epi_value<kEpiDecay>(r[j], sc, bias, coef));
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < w.rows) out[static_cast<size_t>(j) * w.ld_out] = __uint_as_float(r[j]);
+  } else {
+    // fp32 rows that are read once, later (per-pair expert outputs, logits): streaming stores
+#pragma unroll
+    for (int j = 0; j < 32; ++j)
+      if (j < w.rows) __stcs(out + static_cast<size_t>(j) * w.ld_out, __uint_as_float(r[j]) * sc + bias);
+  }
+}
+
 // Epilogue of one slice of a tile from accumulator buffer `buf` (the four epilogue warps
 // call): everything except handing the buffer back to the MMA warp.  kFetch = false: the expert kernel, which has two
 // epilogues and no fetch records.
@@ -631,21 +727,22 @@ __device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, int slice,
   const float sc = (w.scale && f_ok) ? w.scale[wrow] : 1.f;
   if constexpr (kFetch) {
     const float bias = (w.bias && f_ok && w.k0 == 0) ? __bfloat162float(w.bias[f]) : 0.f;
-    switch (w.epi) {
-      case kEpiStoreBf16: epilogue_chunks<kEpiStoreBf16>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
-      case kEpiSiluMul: epilogue_chunks<kEpiSiluMul>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
-      case kEpiGeluMul: epilogue_chunks<kEpiGeluMul>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
-      case kEpiWeightedAdd: epilogue_chunks<kEpiWeightedAdd>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
-      case kEpiAtomicF32: epilogue_chunks<kEpiAtomicF32>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+    if (w.n <= 32) epilogue_few(w, tacc, f, wrow, f_ok, sc, bias);
+    else switch (w.epi) {
+      case kEpiStoreBf16: epilogue_call<kEpiStoreBf16>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiSiluMul: epilogue_call<kEpiSiluMul>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiGeluMul: epilogue_call<kEpiGeluMul>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiWeightedAdd: epilogue_call<kEpiWeightedAdd>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      case kEpiAtomicF32: epilogue_call<kEpiAtomicF32>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
       case kEpiDecay:
-        epilogue_chunks<kEpiDecay>(w, tacc, f, wrow, f_ok, sc, bias, f_ok ? w.pair_weight[f] : 0.f);
+        epilogue_call<kEpiDecay>(w, tacc, f, wrow, f_ok, sc, bias, f_ok ? w.pair_weight[f] : 0.f);
         break;
-      default: epilogue_chunks<kEpiStoreF32>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
+      default: epilogue_call<kEpiStoreF32>(w, tacc, f, wrow, f_ok, sc, bias, 0.f); break;
     }
   } else if (w.epi == kEpiSiluMul) {
-    epilogue_chunks<kEpiSiluMul>(w, tacc, f, wrow, f_ok, sc, 0.f, 0.f);
+    epilogue_chunks<kEpiSiluMul, true>(w, tacc, f, wrow, f_ok, sc, 0.f, 0.f);
   } else {
-    epilogue_chunks<kEpiRowsF32>(w, tacc, f, wrow, f_ok, sc, 0.f, 0.f);
+    epilogue_chunks<kEpiRowsF32, true>(w, tacc, f, wrow, f_ok, sc, 0.f, 0.f);
   }
   tc_fence_before_sync();
   __syncwarp();

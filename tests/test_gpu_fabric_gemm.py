@@ -116,6 +116,53 @@ def test_two_slice_tiles_equal_one_slice_tiles(fab, rows, epi):
     assert float((outs[1].float() - ref).norm() / ref.norm()) < 1e-2
 
 
+EPI_ROWS, EPI_GELU_MUL, EPI_DECAY = 5, 6, 7
+
+
+@pytest.mark.parametrize("epi", [EPI_STORE, EPI_SILU_MUL, EPI_WADD, EPI_F32, EPI_ATOMIC, EPI_ROWS, EPI_GELU_MUL, EPI_DECAY])
+@pytest.mark.parametrize("bm", [16, 32, 64])
+def test_every_epilogue(fab, bm, epi):
+    """Tiles of at most 32 rows have an epilogue of their own: full and ragged row blocks, the last features left out."""
+    torch.manual_seed(4)
+    F = torch.nn.functional
+    K, n_out, limit = 320, 192, 168
+    gated, f32 = epi in (EPI_SILU_MUL, EPI_GELU_MUL), epi not in (EPI_STORE, EPI_SILU_MUL, EPI_GELU_MUL)
+    w = (torch.randn(1, n_out * (2 if gated else 1), K, device="cuda") * 0.05).to(torch.bfloat16)
+    xs = torch.randn(200, K, device="cuda").to(torch.bfloat16)
+    res, bias = (torch.randn(*n, device="cuda").to(torch.bfloat16) for n in ((200, n_out), (n_out,)))
+    coef, tw = 0.1 + torch.rand(n_out, device="cuda"), torch.rand(200, device="cuda")
+    wm = weight_map(fab, w.data_ptr(), w.shape)
+    for rows in (1, 15, 16, 17, 32, 33, 65):
+        x = xs[:rows]
+        tok = torch.randperm(rows, device="cuda").to(torch.int32)
+        out = torch.full((rows, n_out), 0.5, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+        more = {EPI_STORE: dict(residual=res.data_ptr(), ld_res=n_out, bias=bias.data_ptr()), EPI_F32: dict(bias=bias.data_ptr()),
+                EPI_DECAY: dict(bias=bias.data_ptr(), pair_weight=coef.data_ptr()),
+                EPI_WADD: dict(pair_token=tok.data_ptr(), pair_weight=tw.data_ptr())}.get(epi, {})
+        args = args_tensor(out=out.data_ptr(), ld_out=n_out, k_tiles=K // 64, epi=epi, bm=bm, n_limit=limit,
+                           up_offset=n_out if gated else 0, **more)
+        xm = act_map(fab, x, bm)
+        tiles = [Tile(KIND_GEMM, i=(n0, m0, min(bm, rows - m0), 0), a=(args.data_ptr(), wm, xm))
+                 for n0 in range(0, n_out, 64 if gated else 128) for m0 in range(0, rows, bm)]
+        p = Program()
+        run_program(fab, p, p.stage(tiles))
+        y = x.double() @ w[0].double().t()
+        if gated:
+            gate, up = y[:, :n_out], y[:, n_out:]
+            want = (F.silu(gate) if epi == EPI_SILU_MUL else F.gelu(gate, approximate="tanh")) * up
+        elif epi == EPI_STORE:
+            want = y + bias.double() + res[:rows].double()
+        elif epi == EPI_DECAY:
+            want = torch.expm1(-coef.double() * F.softplus(y + bias.double()))
+        elif epi == EPI_WADD:
+            want = 0.5 + torch.zeros_like(y).index_copy_(0, tok.long(), tw[:rows, None].double() * y)
+        else:
+            want = y + (bias.double() if epi == EPI_F32 else 0) + (0.5 if epi == EPI_ATOMIC else 0)
+        err = float((out[:, :limit].double() - want[:, :limit]).norm() / want[:, :limit].norm())
+        assert err < (1e-5 if f32 else 4e-3), (rows, err)   # fp32 sums of 320 exact products; bf16: 2^-9 of a value
+        assert bool((out[:, limit:] == 0.5).all()), rows
+
+
 @pytest.mark.parametrize("where", ["hbm", "cpu"])
 def test_expert_ffn(fab, where):
     """w13 tiles with the SiLU-and-multiply epilogue, then w2 tiles that add
