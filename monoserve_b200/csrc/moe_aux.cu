@@ -262,9 +262,12 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanParams A) 
   if (e == 0) A.starts[E] = total;
 
   if (!A.q) return;   // scan only: counts, starts and chunk prefixes
-  // Row blocks of an expert in HBM: of 256 rows while more than 128 are left ("wide": bf16 tiles of two weight
-  // slices, which read the L2 half as often per product as 128-row blocks of one slice do), then one of up to 128.
-  // 8192 tokens over 128 experts (hidden 2048, width 768): experts kernel 1084 -> 734 us.
+  // Row blocks of an expert in HBM: of 256 rows, the last of what is left.  With bf16 weights a block of more than 128 rows
+  // is "wide": tiles of two weight slices, which read the L2 half as often per product as 128-row blocks of one slice do
+  // (8192 tokens over 128 experts, hidden 2048, width 768: experts kernel 1084 -> 734 us).  e4m3 weights take tiles of one slice, which
+  // read and expand the slice once where two blocks of 128 rows do it twice, with two stages of 96 KB in the ring instead of three of
+  // 64 (4096 x 1408, blocks of 128 -> 256 rows: 2048 tokens 1284 -> 1271 us, with a Zipf-skewed choice of experts 1378 -> 1260;
+  // 1000 tokens 818 -> 821, the same).
   int tier = kTierHot, z = 0, bh = 256, nb = 0, nw = 0;
   const int expert = (e < E && A.seg_expert) ? A.seg_expert[e] : e;
   // A segment of an expert the table does not hold, a negative count or more rows than the packed-row
@@ -394,8 +397,8 @@ __global__ void __launch_bounds__(256) pack_kernel(const PackParams A) {
 
 // Warps per token when no row reduction follows: four, and for batches that leave the schedulers idle (kFew) one per 256 columns.
 // There a warp's chain of loads is what it takes; where warps are many, four rows' loads in each cost registers and 1 % (8192
-// tokens).  64 tokens of 4096 columns: the layer 642 -> 620 us.
-constexpr int kFewTokens = 74;   // two blocks of four warps per token for an SM
+// tokens).  64 tokens of 4096 columns, with the projection's smaller tiles: the layer 638 -> 626 us.
+constexpr int kFewTokens = 74;   // four warps a token leave every other scheduler (4 x 148) without one
 __host__ __device__ __forceinline__ int combine_split(int H, bool norm, bool few) { return norm ? 1 : few ? max(4, H / 256) : 4; }
 
 template <bool kFew>

@@ -422,6 +422,25 @@ def test_fp8_layer_against_dequantised_reference(hot, pack_hot, form):
     m.close()
 
 
+@pytest.mark.parametrize("I", [192, 256])
+def test_fp8_row_blocks_at_their_edges(I):
+    """e4m3 experts in HBM whose row counts lie on the edges of 128- and 256-row blocks (tiles of one slice, up to 256 rows)."""
+    rows = [1, 128, 129, 255, 256, 257, 384, 385, 512, 0, 640, 700]
+    E, H, P = len(rows), 512, sum(rows)
+    m, _, d13, d2 = make_fp8_layer(P, H, I, E, 1, list(range(E)), seed=25)
+    x = acts(P, H, 26)[0]
+    m.workspace("xp")[:P * H].copy_(x.flatten().cuda())
+    m.experts(torch.tensor(rows, dtype=torch.int32, device="cuda"))
+    torch.cuda.synchronize()
+    assert m.status() == 0
+    y, at = m.workspace("y")[:P * H].view(P, H).cpu(), 0
+    for e, n in enumerate(rows):
+        if n:
+            assert rel_l2(y[at:at + n], tp.ffn(x[at:at + n].float(), d13[e], d2[e])) < 2e-3, (e, n)   # the rounding of h: 2^-9 of each term
+        at += n
+    m.close()
+
+
 @pytest.mark.parametrize("I", [384, 320])
 def test_fp8_qwen_shape_prefill_rows(I):
     """GLM-like FP8 at a larger shape with long expert segments (prefill-sized rows); I = 320 gives the
