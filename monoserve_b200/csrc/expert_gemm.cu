@@ -7,7 +7,7 @@
 //             h = bf16(silu(g) * u)                       (kEpiSiluMul)
 //   w2 tile : 128 output rows x the same row block over h, epilogue stores the
 //             fp32 rows y[pos][n] of every routed pair     (kEpiRowsF32)
-// A row block of more than 128 rows takes tiles of two slices (128 features, 256 output rows).
+// A row block of more than 64 rows takes tiles of two slices (128 features, 256 output rows).
 // A w2 tile may start only when every w13 tile of its row block has stored h:
 // the epilogue warps of w13 tiles count into done[block] (release), and the
 // scheduler waits (bounded) for the count before it hands a w2 tile to the
@@ -146,6 +146,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
         w.w_fp8 = ph.w_fp8;
         w.fetch = 0;
         w.slices = tile.tier_phase >> 16;
+        w.by_rows = takes_rows(tile.n, ph.epi, ph.w_fp8, ph.scale != nullptr);
         w.bias = nullptr;
         w.residual = nullptr;
         w.pair_token = nullptr;
@@ -228,9 +229,9 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
       trace_ev(p, 2, it, 0);
       if (own && lane == 0 && it == 0) own[1] = globaltimer_ns();
       long long waited[3] = {0, 0, 0};
-      const uint32_t slices = sh.work[slot].slices;
+      const uint32_t accs = gemm_accs(sh.work[slot]);
       if (!gemm_mma<false>(sh.work[slot], ring, sh.bar, pipe, tmem_base, g, abort_flag, p.trace ? waited : nullptr)) break;
-      g += slices;
+      g += accs;
       trace_ev(p, 2, it, 1);
       if (own && lane == 0) {
         sum_wait += waited[0];
@@ -278,8 +279,8 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
       if (warp == 2) trace_ev(p, 3, it, 0);
       unsigned long long* seen =
           (p.trace && blockIdx.x == 0 && warp == 2 && it < 32) ? &p.trace[(3 * 32 + it) * 4 + 3] : nullptr;
-      if (!gemm_epilogue<false>(w, sh.bar, tmem_base, g, abort_flag, seen)) break;
-      g += w.slices;
+      if (!gemm_epilogue<false>(w, sh.bar, tmem_base, g, abort_flag, ring, seen)) break;
+      g += gemm_accs(w);
       if (warp == 2) trace_ev(p, 3, it, 1);
       if (w.block >= 0) {
         // publish this warp's part of h, then count it into the row block

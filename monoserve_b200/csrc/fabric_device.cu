@@ -124,6 +124,7 @@ __device__ bool make_gemm_work(const TileDesc& t, GemmWork& w, uint32_t block = 
   w.fetch = 0;
   w.slices = 1 + static_cast<int32_t>((t.a[3] >> 32) & 1);
   if (w.slices == 2 && !takes_two_slices(A)) return false;
+  w.by_rows = takes_rows(w.n, w.epi, w.w_fp8, w.scale != nullptr);
   return w.k_tiles > 0 && A.epi <= kEpiDecay;
 }
 
@@ -151,6 +152,7 @@ __device__ bool make_fetch_work(const TileDesc& t, GemmWork& w) {
   w.w_fp8 = 0;
   w.fetch = 1;
   w.slices = 1;
+  w.by_rows = 0;
   w.fetch_bytes = t.i0;
   w.fetch_src = reinterpret_cast<const uint8_t*>(t.a[0]);
   return t.i0 > 0 && ((t.i0 | t.a[0] | t.a[1]) & 15) == 0 && t.a[0] != 0 && t.a[1] != 0;
@@ -852,16 +854,16 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
       ep = e2;
     }
     s_form = (f == 0 || f == 16 || f == 32 || f == 64 || f == 128) ? static_cast<int>(f) : 64;
-  } else if (tid == 32) {   // beside thread 0: whether both products can take 256-row blocks with tiles of two weight slices
-    auto tallest = [](unsigned long long table) { return reinterpret_cast<const unsigned long long*>(table)[4]; };
-    const unsigned long long a[2] = {tallest(A.w13_args), tallest(A.w2_args)};
-    bool ok = a[0] && a[1] && tallest(A.xp_maps) && tallest(A.h_maps);   // a program may leave the tallest class out
+  } else if (tid == 32) {   // beside thread 0: whether both products can take 128-row blocks with tiles of two weight slices
+    auto class128 = [](unsigned long long table) { return reinterpret_cast<const unsigned long long*>(table)[3]; };
+    const unsigned long long a[2] = {class128(A.w13_args), class128(A.w2_args)};
+    bool ok = a[0] && a[1] && class128(A.xp_maps) && class128(A.h_maps);   // a program may leave a class out
     if (ok) {
       GemmArgs g[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) load_block(g[i], a[i]);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) ok = ok && g[i].bm == 256 && takes_two_slices(g[i]);
+      for (int i = 0; i < 2; ++i) ok = ok && g[i].bm == 128 && takes_two_slices(g[i]);
     }
     s_wide = ok;
   }
@@ -890,13 +892,12 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     if (link) return s_form ? s_form : 256;
     return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   };
-  // An expert in HBM with more than 128 rows, where both products take them (s_wide): blocks of 256 rows with tiles of two weight
-  // slices while more than 128 rows are left, then one block of up to 128 (its class is the one kept in s_info).  The two-slice tiles
-  // read the L2 half as often per product: 4096 tokens over 128 experts, the layer's experts 590 -> 381 us.
+  // An expert in HBM with more than 64 rows, where both products take them (s_wide): blocks of 128 rows with tiles of two weight
+  // slices while more than 64 rows are left, then one block of up to 64 (its class is the one kept in s_info).
   const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2;
   auto shape = [&](int M, int info, int& wide, int& narrow) {   // row blocks of either kind
-    wide = (info & 8) ? M / 256 + (M % 256 > 128) : 0;
-    const int bm = 16 << (info & 7), left = M - 256 * wide;
+    wide = (info & 8) ? M / 128 + (M % 128 > 64) : 0;
+    const int bm = 16 << (info & 7), left = M - 128 * wide;
     narrow = left > 0 ? (left + bm - 1) / bm : 0;
   };
   for (int e = tid; e < E; e += kExecThreads) {
@@ -907,9 +908,9 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     const int region = static_cast<int>(entry & 0xffffffffu), slot = static_cast<int>(entry >> 32);
     const bool link = region == static_cast<int>(A.host_region);
     const bool staged = link && can_stage && s_form == 0 && M > static_cast<int>(G.min_rows);
-    const bool wide = s_wide && M > 128 && (!link || staged);
-    const int left = M % 256;
-    const int bm = wide ? block_rows(left > 128 ? 0 : left, false) : block_rows(M, link);
+    const bool wide = s_wide && M > 64 && (!link || staged);
+    const int left = M % 128;
+    const int bm = wide ? block_rows(left > 64 ? 0 : left, false) : block_rows(M, link);
     int cls = 0;
     while ((16 << cls) < bm) ++cls;   // 16, 32, 64, 128, 256 -> 0..4
     if (wide) cls |= 8;
@@ -990,9 +991,9 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
           const int local = is13 ? g : g - n13, per = is13 ? f13 : f2, half = is13 ? h13 : h2;
           const bool wide = local < n_wide * half;
           const int past = local - n_wide * half;   // among the narrow blocks' tiles
-          const int blk = wide ? local / half : past / per, f = wide ? 2 * (local - blk * half) : past - blk * per;
-          const int cls = wide ? 4 : info & 7, bm = 16 << cls;
-          const int at = (wide ? 0 : 256 * n_wide) + blk * bm;   // the block's first row among the expert's
+          const int blk = wide ? local % n_wide : past / per, f = wide ? 2 * (local / n_wide) : past - blk * per;   // blocks of a slice: neighbours
+          const int cls = wide ? 3 : info & 7, bm = 16 << cls;
+          const int at = (wide ? 0 : 128 * n_wide) + blk * bm;   // the block's first row among the expert's
           const unsigned long long a0 = s_tab[(is13 ? 0 : 5) + cls], a1 = is13 ? wmap13 : wmap2;
           const unsigned long long a2 = s_tab[(is13 ? 10 : 15) + cls], a4 = is13 ? scale13 : scale2;
           v0.x = kTileGemm;                                          // kind | lane | flags; stage (unused)
@@ -1438,9 +1439,9 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
         attn_mma<1>(w.attn, c);
         attn_advance(c.n_tiles, aq, ab);
       } else if (w.is_gemm) {
-        const uint32_t slices = w.gemm.slices;
+        const uint32_t accs = gemm_accs(w.gemm);
         ok = gemm_mma(w.gemm, ring, sh.bar, pipe, tmem_base, g, abort_flag);
-        g += slices;
+        g += accs;
       }
       if (lane == 0) {
         *reinterpret_cast<volatile unsigned int*>(&sh.mma_done) = n + 1;
@@ -1489,10 +1490,10 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
             conv_pipe.advance();
           }
         }
-        const uint32_t slices = w.gemm.slices;
-        ok = ok && gemm_epilogue(w.gemm, sh.bar, tmem_base, g, abort_flag);
+        const uint32_t accs = gemm_accs(w.gemm);
+        ok = ok && gemm_epilogue(w.gemm, sh.bar, tmem_base, g, abort_flag, ring);
         if (!ok && tid == 0) raise_error(S, kFabErrTileWait);
-        g += slices;
+        g += accs;
       } else if (w.is_wide) {
         if (!run_core_tile(S, w, tid, worker, &sh.t0, ring, tmem_base, abort_flag) && tid == 0) raise_error(S, kFabErrBadTile);
         fence_proxy_async_smem();   // the exec warps' accesses of the ring before the next record's TMA writes

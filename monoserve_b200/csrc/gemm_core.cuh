@@ -5,23 +5,28 @@
 // One tile (the reference's GEMM tile, csrc/fabric/tiles/gemm.cuh:1-18,133-346,
 // csrc/fabric/model_types.h:37-49): 128 weight rows (output features) as the MMA
 // M operand times up to 256 activation rows as the N operand, over a range of
-// 64-element K steps; fp32 accumulation in TMEM.  A tile of two slices takes 256 weight rows:
-// both 128-row halves meet the same activation tile of a stage, each with an accumulator buffer.
-// What bounds a prompt's products is the SMs' reads of the L2 (about 10 TB/s in all, whatever the
-// tile): per 128 x 128 x 64 step a tile of n = 128 reads 32 KB, one of n = 256 24 KB, and one of
-// two slices and n = 256 16 KB.  Both operands are K-major with
-// the 128-byte swizzle.  The weight slice is fetched as eight TMA boxes of 16
-// rows, which lets a SwiGLU tile interleave 64 gate rows and 64 up rows in groups
+// 64-element K steps; fp32 accumulation in TMEM.  Tiles of at least 128 activation rows swap
+// the operands (takes_rows): rows on M, 128 or, of two slices, 256 weight rows on N.  Both operands are K-major with
+// the 128-byte swizzle.  A weight slice is one TMA box of 128 rows, or eight of 16
+// rows, which interleave the 64 gate rows and 64 up rows of a SwiGLU tile in groups
 // of 16: TMEM lane 32q+i (i < 16) then holds gate feature 16q+i and lane 32q+16+i
 // the matching up feature, so the epilogue pairs them with a warp shuffle instead
-// of a trip through shared memory.
+// of a trip through shared memory (with the rows on M they are columns of one lane).
 //
-// Roles: produce() runs in ONE thread (TMA issue), mma() in one warp (one lane
+// What bounds the products of prompts (cycles a K step and SM, loads from the L2): the MMAs are 512 of a 128 x 256
+// tile and 1024 of 256 x 256, and the SM can read twice what either needs.  In the way were, one after the other, the
+// producer's loop (770 a stage, now 550; a small tile's two K steps a stage, 650 a step, now 310), weights evicted
+// from the L2 before their other row blocks read them, and the epilogue, 13000 cycles of a 256 x 256 tile.  4096 x 12288 x
+// 2048: 221 -> 159 us a stage of the fabric; 8192 tokens over 128 experts, hidden 2048, width 768: 1180 -> 1108 us a layer.
+//
+// Roles: produce() runs in one warp (an elected lane issues TMA), mma() in one warp (one lane
 // issues tcgen05.mma / tcgen05.commit), epilogue() in the four warps whose
 // warp index modulo 4 covers the four TMEM lane quadrants.
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_fp8.h>
+
+#include <type_traits>
 
 #include "ptx.cuh"
 #include "types.h"
@@ -32,12 +37,12 @@ constexpr int kBlockK = 64;                      // elements per K step (128 byt
 constexpr int kATileBytes = 128 * kBlockK * 2;   // 16 KB
 constexpr int kGemmMaxN = 256;
 // Operand stages live in one byte ring: a stage takes 16 KB for the weight tile
-// plus n * 128 bytes for the activation tile, so small-n (decode) tiles keep up
-// to 12 stages in flight (about 200 KB per SM, which is what it takes to cover
-// the loaded HBM latency) and n = 256 tiles still get four.
-constexpr int kRingBytes = 216 * 1024;
+// plus n * 128 bytes for the activation tile: eleven stages of a decode tile, four of 128 x 256.  Behind
+// the ring, 4 KB for each epilogue warp, through which rows leave in whole lines (epilogue_rows).
+constexpr int kRingBytes = 200 * 1024;
+constexpr int kOutBytes = 4 * 4096;
 constexpr int kGemmStages = 12;                  // most stages in flight (barrier pairs)
-constexpr int kGemmSmemBytes = kRingBytes + 1024;
+constexpr int kGemmSmemBytes = kRingBytes + kOutBytes + 1024;
 constexpr int kTmemCols = 512;
 constexpr int kAccCols = 256;                    // TMEM columns per accumulator buffer (two buffers)
 constexpr unsigned long long kWaitBudgetNs = 4000000000ull;   // 4 s of device time per wait
@@ -80,8 +85,9 @@ struct GemmWork {
                               // partial sums go to column = weight row (kEpiSiluMul always reads two slabs)
   int32_t block;              // row block whose counter the epilogue bumps, or -1
   int32_t w_fp8;              // the weight tensor holds e4m3 bytes: W8A16 (exact e4m3 -> bf16 in shared memory)
-  int32_t slices;             // 1, or 2: two adjacent weight slices (bf16 weights, no epilogue that adds), each with an
-                              // accumulator buffer of its own
+  int32_t slices;             // 1, or 2: two adjacent weight slices (bf16 weights, no epilogue that adds)
+  int32_t by_rows;            // the activation rows are the MMA's M dimension: an accumulator holds 128 of them times the
+                              // weight rows (takes_rows); otherwise 128 weight rows times the n activation rows
   // A fetch record moves fetch_bytes from fetch_src (host-resident weights) to `out` (an HBM staging
   // buffer) through the operand ring, in stages of kFetchStageBytes: no MMA, no accumulator.
   int32_t fetch;
@@ -122,9 +128,10 @@ struct GemmPipe {   // a role's cursor over the stage ring; producer and MMA war
   }
 };
 
-// Producer-only bookkeeping of the stages in flight.
+// Producer-only bookkeeping of the stages in flight, the same in every lane but for vbegin.
 struct GemmInflight {
-  uint32_t vbegin[kGemmStages];
+  uint32_t vbegin = 0;        // lane i: where the stage of barrier pair i begins (an array indexed by the pair would live in local memory)
+  uint32_t tail_vbegin = 0;   // of the oldest
   uint32_t tail = 0;          // oldest stage not yet known to be consumed
   uint32_t tail_slot = 0;
   uint32_t tail_parity = 0;
@@ -132,16 +139,29 @@ struct GemmInflight {
 
 // Bytes of one stage: weight tile (bf16), activation tile, and for FP8 weights the
 // raw e4m3 tile the converter warps expand.
+// Which tiles put the activation rows on the MMA's M dimension (TMEM lanes): those of at least 128 rows whose epilogue stores,
+// of bf16 weights.  A lane then owns a row of the output and stores its 32 columns as whole 32-byte sectors, and gate and up of
+// a feature lie in one lane; with the weights on M a warp's store covers one feature of 32 lanes, 2 bytes each, and a
+// 256-column accumulator took 6500 to 8600 cycles to drain, more than half of it exposed behind the MMAs of a tile of two
+// accumulators (they fill TMEM).  Fewer than 128 rows would leave MMA rows empty, e4m3 weights bring a scale per column, and
+// the adding epilogues are for small tiles.
+__host__ __device__ __forceinline__ bool takes_rows(int n, int epi, bool w_fp8, bool scaled) {
+  return n >= 128 && !w_fp8 && !scaled && epi != kEpiWeightedAdd && epi != kEpiAtomicF32;
+}
+// Accumulators a tile uses, one after the other; rows past the end of the last block get none.
+__device__ __forceinline__ uint32_t gemm_accs(const GemmWork& w) { return w.by_rows ? (w.rows > 128 ? 2u : 1u) : w.slices; }
+
 // K steps (of kBlockK elements) one stage holds.  A stage of e4m3 weights holds two: a row of the raw
 // tile is then 128 bytes, which is what makes reads of host-resident weights over the link efficient
-// (64-byte reads reach 42 GB/s, 128-byte reads 51 GB/s).
+// (64-byte reads reach 42 GB/s, 128-byte reads 51 GB/s).  So does one of bf16 weights for up to 64 rows: their MMAs take 32 to 128
+// cycles a K step where the producer takes 540 a stage, which is what a worker with one or two tiles waits for.
 constexpr uint32_t kFetchStageBytes = 32 * 1024;
-__device__ __forceinline__ int gemm_ksteps(const GemmWork& w) { return w.w_fp8 ? 2 : 1; }
+__device__ __forceinline__ int gemm_ksteps(const GemmWork& w) { return w.w_fp8 || (w.n <= 64 && w.slices == 1) ? 2 : 1; }
 // kFetch = false (a kernel that never sees fetch records) compiles their handling away.
 template <bool kFetch = true>
 __device__ __forceinline__ int gemm_stage_count(const GemmWork& w) {
   if (kFetch && w.fetch) return static_cast<int>((w.fetch_bytes + kFetchStageBytes - 1) / kFetchStageBytes);
-  return w.w_fp8 ? (w.k_tiles + 1) >> 1 : w.k_tiles;
+  return gemm_ksteps(w) == 2 ? (w.k_tiles + 1) >> 1 : w.k_tiles;
 }
 // Bytes of one stage: per K step the bf16 weight tile and the activation tile; layout: weight tiles,
 // then activation tiles.  The raw e4m3 tile (128 rows of 128 bytes) lands in the second weight tile
@@ -173,10 +193,11 @@ __device__ __forceinline__ void gemm_barriers_init(GemmBarriers& b) {
   }
 }
 
-// TMA issue for one tile.  The WHOLE producer warp calls it: every lane keeps
-// the same bookkeeping, lane 0 arms the barrier, and the copies of one stage go
-// out as a single warp-wide instruction (lanes 0..7 the weight boxes, lane 8 the
-// activation box, lanes 16..23 the second slice's), which costs one issue slot instead of nine.
+// TMA issue for one tile.  The WHOLE producer warp calls it in step: every lane keeps the same bookkeeping, and one elected
+// lane arms the barrier and issues the copies of a stage (one or two weight boxes and the activation rows).  Weights that are
+// gathered from eight 16-row boxes go out as a single warp-wide instruction (lanes 0..7 the boxes, lane 8 the activation box,
+// lanes 16..23 the second slice's).  What a stage costs here bounds every tile whose MMAs take less: 770 cycles for 128 x 256
+// with an array of stages in flight and lanes in roles, now 548 (its MMAs are 512), 650 -> 520 for 16 rows.
 // Returns false when a wait was abandoned.
 template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,
@@ -197,11 +218,13 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
   // groups of 16 rows alternately, so its tile starts at row 2 * a_row_lo).
   const bool slab2 = epi_gated(w.epi) || (w.a_packed & 4);
   const bool gather = slab2 && !(w.a_packed & 1);
-  const int second = lane >> 4;   // lanes 16.. bring the second slice's boxes
-  const int a_row = gather ? ((lane & 1) ? w.a_row_hi : w.a_row_lo) + 16 * ((lane & 7) >> 1) + 64 * second
-                           : (slab2 ? 2 * w.a_row_lo : w.a_row_lo) + 128 * second;
-  const int n_a = gather ? 8 : 1;
-  const bool brings_a = (lane & 15) < n_a && second < slices;
+  const bool leader = elect_one();
+  const int a_row0 = slab2 ? 2 * w.a_row_lo : w.a_row_lo;
+  const bool wide_k = ks == 2 && !w.w_fp8;   // two weight tiles, one for each K step
+  const int second = lane >> 4;   // lanes 16.. bring the boxes of the second slice, or of the second K step
+  const int a_row = ((lane & 1) ? w.a_row_hi : w.a_row_lo) + 16 * ((lane & 7) >> 1) + (wide_k ? 0 : 64 * second);
+  const int a_x = wide_k ? kBlockK * second : 0;
+  const bool brings_a = (lane & 15) < 8 && second < (wide_k ? 2 : slices);
   const uint32_t a_at = a_off + second * kATileBytes + (lane & 7) * a_box;
   // read once: the record lives in shared memory and every copy below is a memory barrier to the compiler
   const bool fetch = kFetch && w.fetch != 0;
@@ -210,21 +233,28 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
   const CUtensorMap* const a_map = w.a_map;
   const CUtensorMap* const b_map = w.b_map;
   const int a_z = w.a_z, b_row0 = w.b_row0, k0 = w.k0;
-  const uint32_t tx_bytes = slices * kATileBytes + ks * b_bytes;
+  // A block of 128 rows or more is one of several that read the slice; evicted first, 8192 tokens over 128 experts read 3.1 GB
+  // from HBM where the weights and rows are 1.6.
+  const uint64_t pol_a = w.n >= 128 ? policy_evict_normal() : pol_w;
+  const uint32_t tx_bytes = (wide_k ? 2 : slices) * kATileBytes + ks * b_bytes;
   for (int st = 0; st < n_stages; ++st) {
     uint32_t vb, ve;
     const uint32_t phys = pipe.alloc(size, vb, ve);
     // room in the ring and a free barrier pair: retire the oldest stages as needed
-    while (pipe.i - fl.tail >= kGemmStages || (pipe.i != fl.tail && ve - fl.vbegin[fl.tail_slot] > kRingBytes)) {
+    while (pipe.i - fl.tail >= kGemmStages ||
+           (pipe.i != fl.tail && ve - fl.tail_vbegin > kRingBytes)) {
       if (!mbar_wait_bounded(&bar.empty[fl.tail_slot], fl.tail_parity, abort_flag, kWaitBudgetNs)) return false;
       ++fl.tail;
       if (++fl.tail_slot == kGemmStages) {
         fl.tail_slot = 0;
         fl.tail_parity ^= 1;
       }
+      // also where the warp meets behind the wait: a lane still in it when the stage is filled and freed again would miss the phase
+      fl.tail_vbegin = __shfl_sync(0xffffffffu, fl.vbegin, fl.tail_slot);
     }
     const uint32_t slot = pipe.slot;
-    fl.vbegin[slot] = vb;
+    if (lane == static_cast<int>(slot)) fl.vbegin = vb;
+    if (pipe.i == fl.tail) fl.tail_vbegin = vb;
     uint8_t* a = ring + phys;
     uint64_t* full = &bar.full[slot];
     if (fetch) {
@@ -239,11 +269,23 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
       continue;
     }
     // the second K step of an odd K range's last stage is loaded but not multiplied (gemm_mma)
+    const int x = (k0 + st * ks) * kBlockK;
+    if (!gather) {
+      if (leader) {
+        mbar_arrive_expect_tx(full, tx_bytes);
+        tma_load_3d(a + a_off, a_map, full, x, a_row0, a_z, pol_a);
+        if (slices == 2) tma_load_3d(a + kATileBytes, a_map, full, x, a_row0 + 128, a_z, pol_a);
+        if (wide_k) tma_load_3d(a + kATileBytes, a_map, full, x + kBlockK, a_row0, a_z, pol_a);
+        tma_load_2d(a + b_off, b_map, full, x, b_row0, pol_x);
+        if (ks == 2) tma_load_2d(a + b_off + b_bytes, b_map, full, x + kBlockK, b_row0, pol_x);
+      }
+      pipe.advance();
+      continue;
+    }
     if (lane == 0) mbar_arrive_expect_tx(full, tx_bytes);
     __syncwarp();
-    const int x = (k0 + st * ks) * kBlockK;
     if (brings_a) {
-      tma_load_3d(a + a_at, a_map, full, x, a_row, a_z, pol_w);
+      tma_load_3d(a + a_at, a_map, full, x + a_x, a_row, a_z, pol_a);
     } else if (lane >= 8 && lane < 8 + ks) {
       tma_load_2d(a + b_off + (lane - 8) * b_bytes, b_map, full, x + (lane - 8) * kBlockK, b_row0, pol_x);
     }
@@ -252,17 +294,18 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
   return true;
 }
 
-// MMA issue for a tile of two slices (bf16 weights): accumulators g and g + 1, eight MMAs a stage.  A loop of its own: the
-// one-slice loop bounds small tiles, and a branch on the slices inside it cost it 100 cycles a stage.
+// MMA issue for a tile of two accumulators (bf16 weights), g and g + 1, eight MMAs a stage: two weight slices against the
+// activation rows, or (by_rows) two blocks of 128 activation rows against the weight rows.  A loop of its own: the
+// one-accumulator loop bounds small tiles, and a branch on their number inside it cost it 100 cycles a stage.
 __device__ __forceinline__ bool gemm_mma_two(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,
                                              uint32_t tmem_base, uint32_t g, volatile int* abort_flag) {
   const bool leader = elect_one();
   const uint32_t b0 = g & 1, b1 = b0 ^ 1;
   int ok = mbar_wait_bounded(&bar.acc_empty[b0], ((g >> 1) & 1) ^ 1, abort_flag, kWaitBudgetNs);
-  const uint32_t idesc = umma_idesc_bf16(128, w.n);
+  const uint32_t idesc = umma_idesc_bf16(128, w.by_rows ? 128 * w.slices : w.n);
   const uint32_t acc0 = tmem_base + b0 * kAccCols, acc1 = tmem_base + b1 * kAccCols;
-  const uint32_t size = gemm_stage_bytes<false>(w), ring_addr = smem_u32(ring);
-  const uint64_t desc0 = umma_desc_sw128(0);
+  const uint32_t size = gemm_stage_bytes<false>(w), ring_addr = smem_u32(ring), w_bytes = w.slices * kATileBytes;
+  const uint64_t desc0 = umma_desc_sw128(0), m_off = (w.by_rows ? w_bytes : 0) >> 4, n_off = (w.by_rows ? 0 : w_bytes) >> 4;
   const int n_stages = w.k_tiles;
   for (int kt = 0; kt < n_stages; ++kt) {
     uint32_t vb, ve;
@@ -270,12 +313,12 @@ __device__ __forceinline__ bool gemm_mma_two(const GemmWork& w, uint8_t* ring, G
     ok = ok && mbar_wait_bounded(&bar.full[pipe.slot], pipe.parity, abort_flag, kWaitBudgetNs);
     __syncwarp();   // as in gemm_mma
     tc_fence_after_sync();
-    const uint64_t da = desc0 + ((ring_addr + phys) >> 4), db = da + (2 * kATileBytes >> 4);
+    const uint64_t stage = desc0 + ((ring_addr + phys) >> 4), da = stage + m_off, db = stage + n_off;
     if (leader && ok) {
 #pragma unroll
       for (int k = 0; k < kBlockK / 16; ++k) umma_bf16(acc0, da + 2 * k, db + 2 * k, idesc, (kt | k) != 0);
     }
-    if (kt == 0) {   // the first slice's MMAs run while the second's accumulator is still being drained
+    if (kt == 0) {   // the first accumulator's MMAs run while the second is still being drained
       ok = ok && mbar_wait_bounded(&bar.acc_empty[b1], (((g + 1) >> 1) & 1) ^ 1, abort_flag, kWaitBudgetNs);
       tc_fence_after_sync();
     }
@@ -304,7 +347,7 @@ template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,
                                          uint32_t tmem_base, uint32_t g, volatile int* abort_flag,
                                          long long* wait_cycles = nullptr) {
-  if (w.slices == 2) return gemm_mma_two(w, ring, bar, pipe, tmem_base, g, abort_flag);
+  if (gemm_accs(w) == 2) return gemm_mma_two(w, ring, bar, pipe, tmem_base, g, abort_flag);
   int ok = 1;
   const uint32_t buf = g & 1, acc_parity = (g >> 1) & 1;
   const bool leader = elect_one();
@@ -313,7 +356,7 @@ __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmB
     if (!mbar_wait_bounded(&bar.acc_empty[buf], acc_parity ^ 1, abort_flag, kWaitBudgetNs)) ok = 0;
     if (wait_cycles) wait_cycles[2] += clock64() - ta;
     tc_fence_after_sync();
-    const uint32_t idesc = umma_idesc_bf16(128, w.n);
+    const uint32_t idesc = umma_idesc_bf16(128, w.by_rows ? 128 * w.slices : w.n);
     const uint32_t acc = tmem_base + buf * kAccCols;
     const uint32_t size = gemm_stage_bytes<kFetch>(w);
     uint64_t* ready = w.w_fp8 ? bar.conv : bar.full;
@@ -321,8 +364,9 @@ __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmB
     const uint64_t desc0 = umma_desc_sw128(0);
     const int n_stages = gemm_stage_count<kFetch>(w);
     const uint32_t b_bytes = w.n * kBlockK * 2;
+    const uint64_t m_off = (w.by_rows ? w.slices * kATileBytes : 0) >> 4, n_off = (w.by_rows ? 0 : kATileBytes) >> 4;
     // read once: the record lives in shared memory and every wait below is a memory barrier to the compiler
-    const bool fp8 = w.w_fp8 != 0, fetch = kFetch && w.fetch != 0;
+    const bool fp8 = w.w_fp8 != 0, fetch = kFetch && w.fetch != 0, one_step = gemm_ksteps(w) == 1;
     const int k_steps = w.k_tiles;
     const uint32_t fetch_bytes = kFetch ? w.fetch_bytes : 0;
     uint8_t* const fetch_out = static_cast<uint8_t*>(w.out);
@@ -350,9 +394,8 @@ __device__ __forceinline__ bool gemm_mma(const GemmWork& w, uint8_t* ring, GemmB
       }
       const long long ti = wait_cycles ? clock64() : 0;
       if (!leader || !ok) {
-      } else if (!fp8) {   // one K step: weight tile, activation tile
-        const uint64_t da = desc0 + ((ring_addr + phys) >> 4);
-        const uint64_t db = da + (kATileBytes >> 4);
+      } else if (one_step) {   // weight tile, activation tile
+        const uint64_t stage = desc0 + ((ring_addr + phys) >> 4), da = stage + m_off, db = stage + n_off;
 #pragma unroll
         for (int k = 0; k < kBlockK / 16; ++k) umma_bf16(acc, da + 2 * k, db + 2 * k, idesc, (kt | k) != 0);
       } else {      // two K steps: weight tiles 0 and 1, then activation tiles 0 and 1
@@ -601,6 +644,180 @@ __device__ __forceinline__ void epilogue_chunks(const GemmWork& w, uint32_t tacc
   }
 }
 
+// 32 bytes to a 32-byte aligned address, one sector; kStream: read once, later.
+template <bool kStream>
+__device__ __forceinline__ void st_sector(void* p, const uint32_t (&v)[8]) {
+  if constexpr (kStream)
+    asm volatile("st.global.cs.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+  else
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(v[0]), "r"(v[1]), "r"(v[2]),
+                 "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// The rows [row0, row0 + 32) of a warp under a by_rows tile, one in each lane; columns of the accumulator are weight rows.
+// 32 columns at a time (16 features of a gated tile: 16 gate columns, then their up columns), the next 32 under way
+// meanwhile, as are the residual's.  A lane puts its values into the warp's 4 KB of shared memory (`buf`, 16-byte pieces swizzled
+// by the row), from where 128 bytes of a row leave as one line, four lanes a row.  (Each lane storing its own row, 32
+// bytes of 32 rows an instruction, held the SM to 17 bytes a cycle.)  Rows that are not on sector boundaries, and a last chunk that
+// the features do not fill, go element by element.
+template <int E>
+__device__ __forceinline__ void epilogue_rows(const GemmWork& w, uint32_t tacc, int row0, uint8_t* buf) {
+  const int lane = threadIdx.x & 31, row = row0 + lane;
+  constexpr bool kGated = E == kEpiSiluMul || E == kEpiGeluMul, kHalf = kGated || E == kEpiStoreBf16;
+  constexpr int NF = kGated ? 16 : 32;   // features of a chunk
+  const int first = w.a_row_lo, left = w.n_limit - first;   // features from here on
+  const int chunks = min(4 * w.slices, (left + NF - 1) / NF), rows = w.rows;
+  const bool row_ok = row < rows;
+  using Out = typename std::conditional<kHalf, unsigned short, float>::type;
+  const size_t ld = w.ld_out;
+  Out* const out = reinterpret_cast<Out*>(w.out) + static_cast<size_t>(w.b_row0 + row0) * ld + first;
+  const int whole = (reinterpret_cast<uintptr_t>(out) & 31) == 0 && ((ld * sizeof(Out)) & 31) == 0 ? min(chunks, left / NF) : 0;
+  constexpr int kBytes = NF * static_cast<int>(sizeof(Out)), kLine = 128 / kBytes;   // of a chunk's row; chunks of a line
+  uint4* const mine = reinterpret_cast<uint4*>(buf) + 8 * lane;
+  Out* const to = out + static_cast<size_t>(lane >> 2) * ld + (lane & 3) * (32 / sizeof(Out));
+  const __nv_bfloat16* const bias = !kGated && E != kEpiRowsF32 && w.bias && w.k0 == 0 ? w.bias + first : nullptr;
+  const float* const coef = E == kEpiDecay ? w.pair_weight + first : nullptr;
+  const unsigned short* const res = E == kEpiStoreBf16 && w.residual && row_ok
+      ? reinterpret_cast<const unsigned short*>(w.residual) + static_cast<size_t>(w.b_row0 + row) * w.ld_res + first : nullptr;
+  const bool res16 = (reinterpret_cast<uintptr_t>(res) & 15) == 0;
+  constexpr int kRes = E == kEpiStoreBf16 ? 4 : 1;
+  uint4 rn[kRes];   // the next chunk's residual
+  auto load_res = [&](int c) {
+    if (E != kEpiStoreBf16 || !res) return;
+    const unsigned short* p = res + c * NF;
+    if (res16 && (c + 1) * NF <= left) {
+#pragma unroll
+      for (int i = 0; i < kRes; ++i) rn[i] = reinterpret_cast<const uint4*>(p)[i];
+    } else {
+      uint32_t v[4 * kRes];
+#pragma unroll
+      for (int i = 0; i < 4 * kRes; ++i) {
+        const uint32_t a = c * NF + 2 * i < left ? p[2 * i] : 0, b = c * NF + 2 * i + 1 < left ? p[2 * i + 1] : 0;
+        v[i] = a | b << 16;
+      }
+#pragma unroll
+      for (int i = 0; i < kRes; ++i) rn[i] = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    }
+  };
+  uint32_t next[32];
+  load_res(0);
+  __syncwarp();
+  tmem_ld_32x32(tacc, next);
+  if (chunks <= 0) tmem_ld_wait();
+#pragma unroll 1
+  for (int c = 0; c < chunks; ++c) {
+    uint32_t r[32], rv[4 * kRes];
+    __syncwarp();
+    tmem_ld_wait_for(next);
+#pragma unroll
+    for (int j = 0; j < 32; ++j) r[j] = next[j];
+#pragma unroll
+    for (int i = 0; i < kRes; ++i) {
+      rv[4 * i] = rn[i].x;
+      rv[4 * i + 1] = rn[i].y;
+      rv[4 * i + 2] = rn[i].z;
+      rv[4 * i + 3] = rn[i].w;
+    }
+    if (c + 1 < chunks) {
+      tmem_ld_32x32(tacc + 32 * (c + 1), next);
+      load_res(c + 1);
+    }
+    const int f = c * NF, n = min(NF, left - f);   // features of this chunk that exist
+    uint32_t o[kHalf ? NF / 2 : NF];
+    if constexpr (kGated) {
+#pragma unroll
+      for (int j = 0; j < NF; j += 2) {
+        float h[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const float gate = __uint_as_float(r[j + i]), up = __uint_as_float(r[16 + j + i]);
+          h[i] = E == kEpiGeluMul ? gelu_mul(gate, up) : silu_mul(gate, up);
+        }
+        o[j / 2] = pack_bf16(h[0], h[1]);
+      }
+    } else {
+      float v[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
+      if (bias) {   // the same for every lane
+        if (n == NF && (reinterpret_cast<uintptr_t>(bias) & 15) == 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint4 b = reinterpret_cast<const uint4*>(bias + f)[i];
+            const uint32_t u[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+            for (int j = 0; j < 8; ++j) v[8 * i + j] += __uint_as_float(j & 1 ? u[j / 2] & 0xffff0000u : u[j / 2] << 16);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += j < n ? __bfloat162float(bias[f + j]) : 0.f;
+        }
+      }
+      if constexpr (E == kEpiDecay) {
+        if (n == NF && (reinterpret_cast<uintptr_t>(coef) & 15) == 0) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float4 k = reinterpret_cast<const float4*>(coef + f)[i];
+            v[4 * i] = decay_less_one(v[4 * i], k.x);
+            v[4 * i + 1] = decay_less_one(v[4 * i + 1], k.y);
+            v[4 * i + 2] = decay_less_one(v[4 * i + 2], k.z);
+            v[4 * i + 3] = decay_less_one(v[4 * i + 3], k.w);
+          }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] = decay_less_one(v[j], j < n ? coef[f + j] : 0.f);
+        }
+      }
+      if constexpr (E == kEpiStoreBf16) {
+        if (res) {
+#pragma unroll
+          for (int j = 0; j < 32; ++j) v[j] += __uint_as_float(j & 1 ? rv[j / 2] & 0xffff0000u : rv[j / 2] << 16);
+        }
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) o[j / 2] = pack_bf16(v[j], v[j + 1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) o[j] = __float_as_uint(v[j]);
+      }
+    }
+    if (c < whole) {
+      const int at = c % kLine;   // place in the line
+#pragma unroll
+      for (int i = 0; i < kBytes / 16; ++i)
+        mine[(at * (kBytes / 16) + i) ^ (lane & 7)] = make_uint4(o[4 * i], o[4 * i + 1], o[4 * i + 2], o[4 * i + 3]);
+      if (at != kLine - 1 && c + 1 != whole) continue;
+      __syncwarp();
+      const int p = lane & 3;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = 8 * i + (lane >> 2);
+        if (row0 + r < rows && p < (at + 1) * (kBytes / 32)) {
+          const uint4* from = reinterpret_cast<const uint4*>(buf) + 8 * r;
+          const uint4 a = from[(2 * p) ^ (r & 7)], b = from[(2 * p + 1) ^ (r & 7)];
+          const uint32_t q[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+          st_sector<!kHalf && E != kEpiDecay>(to + 8 * i * ld + (c - at) * NF, q);
+        }
+      }
+      __syncwarp();
+    } else if (row_ok) {
+      Out* const own = out + lane * ld + f;
+#pragma unroll
+      for (int j = 0; j < NF; ++j) {
+        if (j >= n) continue;
+        if constexpr (kHalf) own[j] = static_cast<unsigned short>(j & 1 ? o[j / 2] >> 16 : o[j / 2] & 0xffffu);
+        else own[j] = __uint_as_float(o[j]);
+      }
+    }
+  }
+}
+
 // The fabric kernel calls them: seven of them inlined cost its other roles registers (252 bytes of spills against 48).
 template <int E>
 __device__ __noinline__ void epilogue_call(const GemmWork& w, uint32_t tacc, int f, int wrow, bool f_ok, float sc, float bias,
@@ -697,12 +914,19 @@ __device__ __forceinline__ void epilogue_few(const GemmWork& w, uint32_t tacc, i
   }
 }
 
-// Epilogue of one slice of a tile from accumulator buffer `buf` (the four epilogue warps
+template <int E>
+__device__ __noinline__ void epilogue_rows_call(const GemmWork& w, uint32_t tacc, int row0, uint8_t* buf) {
+  __builtin_assume(__isShared(&w));
+  __builtin_assume(__isShared(buf));
+  epilogue_rows<E>(w, tacc, row0, buf);
+}
+
+// Epilogue of one accumulator of a tile from buffer `buf` (the four epilogue warps
 // call): everything except handing the buffer back to the MMA warp.  kFetch = false: the expert kernel, which has two
 // epilogues and no fetch records.
 template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, int slice, GemmBarriers& bar, uint32_t tmem_base,
-                                                   uint32_t buf, uint32_t acc_parity, volatile int* abort_flag,
+                                                   uint32_t buf, uint32_t acc_parity, volatile int* abort_flag, uint8_t* ring,
                                                    unsigned long long* acc_seen = nullptr) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3;
   if (!mbar_wait_bounded(&bar.acc_full[buf], acc_parity, abort_flag, kWaitBudgetNs)) return false;
@@ -713,6 +937,28 @@ __device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, int slice,
     return true;
   }
   const uint32_t tacc = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + buf * kAccCols;
+  if (w.by_rows) {
+    const int row0 = 128 * slice + 32 * quad;
+    uint8_t* const lines = ring + kRingBytes + 4096 * quad;
+    if (row0 >= w.rows) {   // no row of this warp exists
+    } else if constexpr (kFetch) {
+      switch (w.epi) {
+        case kEpiStoreBf16: epilogue_rows_call<kEpiStoreBf16>(w, tacc, row0, lines); break;
+        case kEpiSiluMul: epilogue_rows_call<kEpiSiluMul>(w, tacc, row0, lines); break;
+        case kEpiGeluMul: epilogue_rows_call<kEpiGeluMul>(w, tacc, row0, lines); break;
+        case kEpiDecay: epilogue_rows_call<kEpiDecay>(w, tacc, row0, lines); break;
+        default: epilogue_rows_call<kEpiStoreF32>(w, tacc, row0, lines); break;
+      }
+    } else if (w.epi == kEpiSiluMul) {
+      epilogue_rows<kEpiSiluMul>(w, tacc, row0, lines);
+    } else {
+      epilogue_rows<kEpiRowsF32>(w, tacc, row0, lines);
+    }
+    fence_proxy_async_smem();   // a wide tile may fill the lines' memory by copies next
+    tc_fence_before_sync();
+    __syncwarp();
+    return true;
+  }
   const bool slab2 = epi_gated(w.epi) || (w.a_packed & 4);
   // output feature of this lane, and the weight row its accumulator row came from
   int f, wrow;
@@ -749,14 +995,14 @@ __device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, int slice,
   return true;
 }
 
-// The four epilogue warps: every slice of a tile whose first accumulator is g.
+// The four epilogue warps: every accumulator of a tile whose first one is g.
 template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_epilogue(const GemmWork& w, GemmBarriers& bar, uint32_t tmem_base, uint32_t g,
-                                              volatile int* abort_flag, unsigned long long* acc_seen = nullptr) {
-  const int slices = w.slices;
+                                              volatile int* abort_flag, uint8_t* ring, unsigned long long* acc_seen = nullptr) {
+  const int accs = static_cast<int>(gemm_accs(w));
 #pragma unroll 1
-  for (int i = 0; i < slices; ++i, ++g) {
-    if (!gemm_epilogue_body<kFetch>(w, i, bar, tmem_base, g & 1, (g >> 1) & 1, abort_flag, acc_seen)) return false;
+  for (int i = 0; i < accs; ++i, ++g) {
+    if (!gemm_epilogue_body<kFetch>(w, i, bar, tmem_base, g & 1, (g >> 1) & 1, abort_flag, ring, acc_seen)) return false;
     if ((threadIdx.x & 31) == 0) mbar_arrive(&bar.acc_empty[g & 1]);
   }
   return true;

@@ -262,9 +262,8 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanParams A) 
   if (e == 0) A.starts[E] = total;
 
   if (!A.q) return;   // scan only: counts, starts and chunk prefixes
-  // Row blocks of an expert in HBM: of 256 rows, the last of what is left.  With bf16 weights a block of more than 128 rows
-  // is "wide": tiles of two weight slices, which read the L2 half as often per product as 128-row blocks of one slice do
-  // (8192 tokens over 128 experts, hidden 2048, width 768: experts kernel 1084 -> 734 us).  e4m3 weights take tiles of one slice, which
+  // Row blocks of an expert in HBM.  bf16 weights: of 128 rows, the last of what is left; a block of more than 64 rows is "wide",
+  // with tiles of two weight slices (gemm_core.cuh: 128 x 256, two accumulators).  e4m3 weights: of 256 rows and tiles of one slice, which
   // read and expand the slice once where two blocks of 128 rows do it twice, with two stages of 96 KB in the ring instead of three of
   // 64 (4096 x 1408, blocks of 128 -> 256 rows: 2048 tokens 1284 -> 1271 us, with a Zipf-skewed choice of experts 1378 -> 1260;
   // 1000 tokens 818 -> 821, the same).
@@ -278,7 +277,10 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanParams A) 
     tier = A.table[2 * expert] == 0 ? kTierHost : kTierHot;
     z = A.table[2 * expert + 1];
     if (tier == kTierHost) bh = A.form ? A.form : 256;
-    else nw = A.slices > 1 ? cnt / 256 + (cnt % 256 > 128) : 0;
+    else if (A.slices > 1) {
+      bh = 128;
+      nw = cnt / 128 + (cnt % 128 > 64);
+    }
     nb = (cnt + bh - 1) / bh;
   }
   const int f13 = (A.I + 63) / 64, f2 = (A.H + 127) / 128;
@@ -333,8 +335,9 @@ __global__ void __launch_bounds__(kPlanThreads) plan_kernel(const PlanParams A) 
       const bool up = j >= n13;   // a w2 tile
       const int jj = up ? j - n13 : j, per = up ? f2 : f13, half = up ? h2 : h13;
       const bool wide = jj < x_nw * half;
-      const int b = wide ? jj / half : x_nw + (jj - x_nw * half) / per;
-      const int f = wide ? 2 * (jj - b * half) : (jj - x_nw * half) - (b - x_nw) * per;   // first slice
+      // the row blocks of a weight slice are neighbours in the list: they read it at about the same time
+      const int b = wide ? jj % x_nw : x_nw + (jj - x_nw * half) / per;
+      const int f = wide ? 2 * (jj / x_nw) : (jj - x_nw * half) - (b - x_nw) * per;   // first slice
       const int rows = min(x_bh, x_cnt - b * x_bh);
       int n = 16;
       while (n < rows) n <<= 1;

@@ -81,14 +81,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   volatile int* abort_flag,
                                                   unsigned long long budget_ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const unsigned long long t0 = globaltimer_ns();
-  uint32_t spins = 0;
-  while (true) {
+  unsigned long long t0 = 0;   // the first reading of the timer, which is slow: most waits end before it
+  for (uint32_t spins = 1;; ++spins) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((++spins & 63u) == 0) {
+    if ((spins & 63u) == 0) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > budget_ns) {
+      const unsigned long long now = globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > budget_ns) {
         *abort_flag = 1;
         return false;
       }
@@ -101,11 +101,16 @@ __device__ __forceinline__ void prefetch_tensormap(const void* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
 }
 
-// L2 eviction-priority policies for the streaming weight operand (read once)
-// and the re-read activation operand.
+// L2 eviction-priority policies for weights that are read once, weights that several row
+// blocks read, and the re-read activation operand.
 __device__ __forceinline__ uint64_t policy_evict_first() {
   uint64_t p;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t policy_evict_normal() {
+  uint64_t p;
+  asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
   return p;
 }
 __device__ __forceinline__ uint64_t policy_evict_last() {

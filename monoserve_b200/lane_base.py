@@ -15,6 +15,7 @@ SPLIT_ROWS, SPLIT_PARTS = 64, 8   # a dense GEMM of at most SPLIT_ROWS rows may 
 EPI_STORE, EPI_SILU_MUL, EPI_F32, EPI_ROWS_F32, EPI_GELU_MUL, EPI_DECAY = 0, 1, 3, 5, 6, 7
 GATED = (EPI_SILU_MUL, EPI_GELU_MUL)
 HEIGHTS = [16, 32, 64, 128, 256]
+TILE_SHAPES = [(256, 2, 1420, 11000), (128, 2, 900, 8000), (128, 1, 700, 4000), (64, 1, 600, 3000), (32, 1, 560, 2000)]   # LaneBase._shape
 TWO_SLICES = 32   # bit of a GEMM tile's a[3]: 256 weight rows
 
 
@@ -248,35 +249,41 @@ class LaneBase:
         return p.stage(tiles, mark=mark, label=label)
 
     def _gemm(self, p, wmap, amaps, rows, n_out, k, out, ld_out, epi, label, residual=None, ld_res=0, mark=None,
-              mat=None, bias=None, up_offset=0, bm=None, coef=None):
+              mat=None, bias=None, up_offset=0, coef=None):
         """A dense GEMM stage: out[rows][n_out] = act[rows][k] x weight[n_out (x2 for SiLU-mul)][k]^T.
-        mat: the weight's Mat (e4m3 weights carry their scales into the tiles); bm: the row-block height, when not the
-        largest; coef: fp32 per output of the decay epilogue."""
-        bm = bm or _bm(rows)
+        mat: the weight's Mat (e4m3 weights carry their scales into the tiles); coef: fp32 per output of the decay epilogue."""
         fp8 = mat is not None and mat.fp8
+        step = 64 if epi in GATED else 128
+        bm, slices = (_bm(rows), 1) if fp8 else self._shape(rows, n_out, k, step)
         args = self.arena.put(_C.gemm_args(
             out=out.data_ptr(), ld_out=ld_out, k_tiles=-(-k // 64), epi=epi, bm=bm, n_limit=n_out,
             residual=residual.data_ptr() if residual is not None else 0, ld_res=ld_res,
             bias=bias.data_ptr() if bias is not None else 0, up_offset=up_offset, w_fp8=int(fp8),
             pair_weight=coef.data_ptr() if coef is not None else 0))
         xm = amaps[HEIGHTS.index(bm)]
-        step = 64 if epi in GATED else 128
-        two = not fp8 and bm == HEIGHTS[-1] and self._two_slices(-(-rows // bm), n_out, step)
-        key = ("gemm", rows, bm, n_out, step, two)
+        key = ("gemm", rows, bm, n_out, step, slices)
         tmpl = self._templates.get(key)
         if tmpl is None:
-            m0, n0 = np.meshgrid(np.arange(0, rows, bm), np.arange(0, n_out, step * (1 + two)), indexing="ij")
+            # the row blocks of a weight slice are neighbours: a round of tiles reads all rows and a few slices, once from HBM
+            n0, m0 = np.meshgrid(np.arange(0, n_out, step * slices), np.arange(0, rows, bm), indexing="ij")
             tmpl = self._templates[key] = tile_array(K_GEMM, i0=n0, i1=m0, i2=np.minimum(bm, rows - m0),
-                                                     a3=(two & (n0 + step < n_out)).astype(np.int64) << TWO_SLICES)
+                                                     a3=((slices == 2) & (n0 + step < n_out)).astype(np.int64) << TWO_SLICES)
         tiles = _retarget(tmpl, a0=args.data_ptr(), a1=wmap, a2=xm, a4=mat.scale.data_ptr() if fp8 else 0)
         return p.stage(tiles, mark=mark, label=label)
 
-    def _two_slices(self, blocks, n_out, step):
-        """Whether a product of `blocks` full row blocks takes tiles of two weight slices: a K step of theirs reads 64 KB,
-        of one slice 48 KB, and the SMs' reads of the L2 are what bounds these products, so the rounds of tiles over the
-        workers decide.  (Rows x outputs x K: 4096 x 12288 x 2048 270 -> 219 us, 4096 x 2048 x 6144 111 -> 85 us, with the epilogues as they are now.)"""
-        one, two = (-(-(blocks * -(-n_out // (s * step))) // self.fab.num_workers) for s in (1, 2))
-        return 4 * two < 3 * one
+    def _shape(self, rows, n_out, k, step):
+        """(row-block height, weight slices) of a bf16 product's tiles: the shape whose rounds of tiles over the workers take
+        least.  Cycles of a K step and of an epilogue, as prompts of 3706 rows run them: 256 rows x 256 weights fill TMEM, so
+        their epilogue is not hidden; under the others it is, unless it is the longer."""
+        if rows <= 64:
+            return _bm(rows), 1
+
+        def cycles(shape):
+            height, slices, per_step, epilogue = shape
+            rounds = -(-(-(-rows // height) * -(-n_out // (slices * step))) // self.fab.num_workers)
+            steps = -(-k // 64) * per_step
+            return rounds * (steps + epilogue if (height, slices) == (256, 2) else max(steps, epilogue))
+        return min((s for s in TILE_SHAPES if s[0] <= _bm(rows)), key=cycles)[:2]
 
     def _rows(self, kind, args, rows, per):
         key = ("rows", kind, rows, per)

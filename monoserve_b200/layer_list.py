@@ -123,7 +123,10 @@ class Weights:
             MIXERS[layer.kind].place(self, w, layer.m, lambda name: g("mix." + name))
             if layer.ff:
                 w.norm2, w.hc2 = norm("norm2"), after(2)
-                w.gate_up = self.mat(torch.cat([g("mlp.gate"), g("mlp.up")]))
+                # groups of 16 gate and 16 up rows, so that a tile's weights are one box (32-bit products read the plain order)
+                w.packed = not cfg.f32 and layer.ff % 16 == 0
+                halves = [g("mlp.gate"), g("mlp.up")]
+                w.gate_up = self.mat(torch.stack([h.unflatten(0, (-1, 16)) for h in halves], 1).flatten(0, 2) if w.packed else torch.cat(halves))
                 w.down = self.mat(g("mlp.down"))
             self.layers.append(w)
 
@@ -643,7 +646,7 @@ class LayerListLane(LaneBase):
         self.xlast.maps(cfg.hidden)
         for layer, lw in zip(cfg.layers, w.layers):
             if layer.ff:
-                wm(lw.gate_up), wm(lw.down), self.hd.maps(layer.ff)
+                wm(lw.gate_up, lw.packed), wm(lw.down), self.hd.maps(layer.ff)
         for l, state in zip(cfg.order, self.kv.runs):
             layer, lw = cfg.layers[l], w.layers[l]
             MIXERS[layer.kind].prepare(self, layer, lw, state)
@@ -657,9 +660,9 @@ class LayerListLane(LaneBase):
         return self._cos_sin[base, r]
 
     # ------------------------------------------------------------------ products
-    def weight_map(self, t):
+    def weight_map(self, t, packed=False):
         if t.data_ptr() not in self._wmaps:
-            self._wmaps[t.data_ptr()] = self._wmap(t)
+            self._wmaps[t.data_ptr()] = self._wmap(t, packed=packed)
         return self._wmaps[t.data_ptr()]
 
     def head_maps(self, addr, ld, k, heads):
@@ -692,18 +695,10 @@ class LayerListLane(LaneBase):
         else:
             s = self._gemm(p, self.weight_map(w), x.maps(k), rows, n, k, out.t, ld,
                            epi if epi is not None else (EPI_STORE if out16 else EPI_F32), label, up_offset=up_offset,
-                           bm=self.row_block(rows, n), bias=bias, coef=coef)
+                           bias=bias, coef=coef)
         for stage in prev if isinstance(prev, list) else [prev]:
             p.after(stage, s)
         return s
-
-    def row_block(self, rows, n):
-        """Row-block height of a GEMM: the largest that still gives most workers a tile (a narrow product over many rows
-        takes lower blocks), at least 32 rows."""
-        for bm in reversed(HEIGHTS):
-            if bm <= _bm(rows) and -(-rows // bm) * -(-n // 128) * 4 >= 3 * self.fab.num_workers:
-                return bm
-        return min(32, _bm(rows))
 
     def _product_tiles(self, rows, n, row0=0):
         key = ("product", rows, n, row0)
@@ -729,12 +724,13 @@ class LayerListLane(LaneBase):
             s = p.stage(tiles, label=label)
         else:
             tiles = []
-            for bm in sorted({_bm(rows) for _, rows in spans}):
+            height = {rows: min(_bm(rows), 128) for _, rows in spans}
+            for bm in sorted(set(height.values())):
                 # the tile's activation rows are h * T + m and its output row is counted from there: the base makes up for it
                 args = [self.arena.put(_C.gemm_args(out=(out_addr + 2 * (h * head_stride - h * self.T * ld_out)) % (1 << 64),
                                                     ld_out=ld_out, k_tiles=-(-k // 64), epi=EPI_STORE, bm=bm, n_limit=n)).data_ptr()
                         for h in range(heads)]
-                m0, count = (np.array(v) for v in zip(*[(row0 + i, min(bm, rows - i)) for row0, rows in spans if _bm(rows) == bm
+                m0, count = (np.array(v) for v in zip(*[(row0 + i, min(bm, rows - i)) for row0, rows in spans if height[rows] == bm
                                                         for i in range(0, rows, bm)]))
                 h, m, n0 = np.meshgrid(np.arange(heads), np.arange(len(m0)), np.arange(0, n, 128), indexing="ij")
                 tiles.append(tile_array(K_GEMM, i0=n0, i1=h * self.T + m0[m], i2=count[m], i3=h,

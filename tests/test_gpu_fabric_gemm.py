@@ -163,6 +163,54 @@ def test_every_epilogue(fab, bm, epi):
         assert bool((out[:, limit:] == 0.5).all()), rows
 
 
+@pytest.mark.parametrize("epi", [EPI_STORE, EPI_SILU_MUL, EPI_F32, EPI_ROWS, EPI_GELU_MUL, EPI_DECAY])
+@pytest.mark.parametrize("bm, two, odd", [(128, 0, 0), (128, 1, 0), (128, 1, 1), (256, 0, 1), (256, 1, 0)])
+def test_tall_tiles(fab, bm, two, odd, epi):
+    """Tiles of at least 128 rows put the rows on the TMEM lanes: ragged rows (whole warps, one of two accumulators, a block of a
+    single row without rows), a last chunk that the features do not fill, rows of the output that are not on sector
+    boundaries (odd), which go element by element."""
+    torch.manual_seed(5)
+    F = torch.nn.functional
+    K, n_out, limit = 320, 320, 296 - odd
+    ld, gated, f32 = n_out + odd, epi in (EPI_SILU_MUL, EPI_GELU_MUL), epi not in (EPI_STORE, EPI_SILU_MUL, EPI_GELU_MUL)
+    w = (torch.randn(1, n_out * (2 if gated else 1), K, device="cuda") * 0.05).to(torch.bfloat16)
+    xs = torch.randn(512, K, device="cuda").to(torch.bfloat16)
+    res, bias = (torch.randn(*n, device="cuda").to(torch.bfloat16) for n in ((300, ld), (n_out,)))
+    coef = 0.1 + torch.rand(n_out, device="cuda")
+    wm, step = weight_map(fab, w.data_ptr(), w.shape), 64 if gated else 128
+    for rows in (1, 31, 127, 128, 129, 257, 300):
+        x = xs[:rows]
+        out = torch.full((rows, ld), 0.5, device="cuda", dtype=torch.float32 if f32 else torch.bfloat16)
+        more = {EPI_STORE: dict(residual=res.data_ptr(), ld_res=ld, bias=bias.data_ptr()), EPI_F32: dict(bias=bias.data_ptr()),
+                EPI_DECAY: dict(bias=bias.data_ptr(), pair_weight=coef.data_ptr())}.get(epi, {})
+        args = args_tensor(out=out.data_ptr(), ld_out=ld, k_tiles=K // 64, epi=epi, bm=bm, n_limit=limit,
+                           up_offset=n_out if gated else 0, **more)
+        xm = act_map(fab, x, bm)
+        tiles = [Tile(KIND_GEMM, i=(n0, m0, min(bm, rows - m0), 0), a=(args.data_ptr(), wm, xm, (two and n0 + step < n_out) << 32))
+                 for n0 in range(0, n_out, step << two) for m0 in range(0, rows, bm)]
+        p = Program()
+        first, done = p.stage(tiles), fab.iterations(0)   # counted over the programs of a fabric
+        h = p.upload(fab, first=first)
+        fab.start()
+        fab.publish(map=[0] * fab.num_workers, caps=[0], order=[0], programs=[h])
+        fab.iteration_times(0, done, 1)
+        fab.stop()
+        assert fab.progress()["error"] == 0
+        y = x.double() @ w[0].double().t()
+        if gated:
+            gate, up = y[:, :n_out], y[:, n_out:]
+            want = (F.silu(gate) if epi == EPI_SILU_MUL else F.gelu(gate, approximate="tanh")) * up
+        elif epi == EPI_STORE:
+            want = y + bias.double() + res[:rows, :n_out].double()
+        elif epi == EPI_DECAY:
+            want = torch.expm1(-coef.double() * F.softplus(y + bias.double()))
+        else:
+            want = y + (bias.double() if epi == EPI_F32 else 0)
+        err = float((out[:, :limit].double() - want[:, :limit]).norm() / want[:, :limit].norm())
+        assert err < (1e-5 if f32 else 4e-3), (rows, err)   # as above
+        assert bool((out[:, limit:] == 0.5).all()), rows
+
+
 @pytest.mark.parametrize("where", ["hbm", "cpu"])
 def test_expert_ffn(fab, where):
     """w13 tiles with the SiLU-and-multiply epilogue, then w2 tiles that add
