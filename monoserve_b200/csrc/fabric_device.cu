@@ -56,7 +56,7 @@ struct WorkSlot {
   TileDesc tile;
   GemmWork gemm;          // filled by the scheduler for GEMM tiles
   AttnWork attn;          // filled by the scheduler for attention work items
-  const ProgramDesc* prog;
+  ProgTables prog;
   uint32_t stage, tile_lane, link, index, cmd, worker_lane, is_gemm, is_attn;
   uint32_t counts, is_wide;   // counts: this record completes its tile (0 for all but the last row block of a kind-45 tile);
                             // is_wide: the exec warps use the operand ring as scratch memory
@@ -318,8 +318,8 @@ __device__ bool run_core_tile(DeviceState& S, const WorkSlot& w, int tid, uint32
     case kTileZeroRuntime:
       for (uint32_t s = t.i0 + tid; s < t.i1; s += kExecThreads) {
         if (s == t.i2) continue;
-        w.prog->runtime[s].done = 0;
-        w.prog->runtime[s].deps = w.prog->stages[s].deps_init;
+        w.prog.runtime[s].done = 0;
+        w.prog.runtime[s].deps = w.prog.stages[s].deps_init;
       }
       __threadfence();
       return true;
@@ -340,7 +340,7 @@ __device__ bool run_core_tile(DeviceState& S, const WorkSlot& w, int tid, uint32
       tile_norm_logits(t, tid);
       return true;
     case kTileExpand:
-      tile_expand(t, w.prog, S, tid);
+      tile_expand(t, w.prog.prog, S, tid);
       return true;
     case kTileRmsNorm:
       tile_norm(t, tid, false);
@@ -361,7 +361,7 @@ __device__ bool run_core_tile(DeviceState& S, const WorkSlot& w, int tid, uint32
       tile_sample(t, tid);
       return true;
     case kTileAttnPlan:
-      tile_attn_plan(t, w.prog, S, tid);
+      tile_attn_plan(t, w.prog.prog, S, tid);
       return true;
     default:
       return run_layer_tile(t, tid, LayerCtx{s_exec_scratch, ring, tmem_base, abort_flag});
@@ -1272,6 +1272,8 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
     sh.ws.n_lanes = 0;
     sh.ws.left = 0;
     sh.ws.row_block = 0;
+    sh.ws.idle = sh.ws.polls = 0;
+    sh.ws.view.prog = nullptr;
     fence_barrier_init();
   }
   if (warp == 6) {
@@ -1288,7 +1290,8 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
     // ------------------------------------------------------------ scheduler
     // The whole warp schedules (fabric_sched.cuh); lane 0 owns the worker state and the work records.
     WorkerState& ws = sh.ws;
-    unsigned long long t_start = 0;
+    const unsigned long long* const polled = polled_word(S, lane);
+    unsigned long long seen = 0, t_start = 0;
     if (lane == 0) t_start = globaltimer_ns();
     // Lane 0: has the host asked the fabric to stop, or has the run-time limit passed?
     auto must_leave = [&](bool check_shutdown) {
@@ -1305,10 +1308,10 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
       uint32_t cmd = kCmdRun;
       if (ws.left == 0) {
         for (;;) {
-          cmd = schedule(S, ws, sh.sched_wl);
+          cmd = schedule(S, ws, sh.sched_wl, polled, seen);
           if (cmd != kCmdIdle) break;
           int leave = 0;
-          if (lane == 0 && must_leave(false)) {
+          if (lane == 0 && (ws.polls & 15) == 0 && must_leave(false)) {
             give_slot_back(S, ws);
             leave = 1;
           }
@@ -1328,7 +1331,7 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
       }
       WorkSlot& w = sh.slot[s];
       if (cmd == kCmdRun && lane < 4)   // the 64-byte descriptor, one 16-byte piece per lane
-        reinterpret_cast<uint4*>(&w.tile)[lane] = __ldcg(reinterpret_cast<const uint4*>(&ws.prog->tiles[ws.next_index]) + lane);
+        reinterpret_cast<uint4*>(&w.tile)[lane] = __ldcg(reinterpret_cast<const uint4*>(&ws.tiles[ws.next_index]) + lane);
       __syncwarp();
       if (lane == 0) {
         w.cmd = cmd;

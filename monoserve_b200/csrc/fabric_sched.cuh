@@ -15,7 +15,15 @@
 // probes up to 32 ring entries at once, drops a run of exhausted head entries with a
 // single compare-and-swap, walks a visiting order computed once per epoch, and sizes
 // claims for a 148-SM machine; completion releases a stage's successors 32 at a time.
+//
+// A stage that does next to nothing is a chain of round trips to the L2 (0.7 us each): from the count that completes it
+// to its successor's published word, and from there through a worker's reading of the rings, its claim, the tile and its
+// operands.  The polling of an idle worker is one load of all words it depends on, and what a step of the chain does not need from
+// the one before it goes out beside it: a one-token step of 39 stages (Teganex, 32 sequences) 893 -> 735 us, of 57 stages (a
+// mixture-of-experts decoder, 32 sequences) 2371 -> 2179.
 #pragma once
+#include <cstddef>
+
 #include "fabric_types.h"
 #include "ptx.cuh"
 
@@ -102,84 +110,137 @@ using Worklist = WorklistOf<kWorklistCap>;
 using SmallWorklist = WorklistOf<16>;   // the scheduler's: it only ever releases the empty stages at a program's start
 
 // ---------------------------------------------------------------------- rings
-// Producer side, any one thread: reserve m places, fill them, and move the published tail over
-// them once every earlier reservation has been published.  The wait for earlier producers is
+// Producer side, any one thread: move the published tail over the m places at `at`, which are filled, once every
+// earlier reservation has been published (next: that is known already).  The wait for earlier producers is
 // bounded; if it runs out the entries stay unpublished and the host sees kFabErrRingWait.
-__device__ __forceinline__ void ring_publish(DeviceState& S, Ring& R, const uint32_t* words, int m) {
-  if (m <= 0) return;
-  const unsigned long long at = atomicAdd(&R.reserve, static_cast<unsigned long long>(m));
-  for (int i = 0; i < m; ++i) R.ids[(at + i) & (kRingCap - 1)] = words[i];
-  const unsigned long long give_up = globaltimer_ns() + kRingWaitBudgetNs;
-  for (unsigned int pause = 32; ld_acq(&R.tail) != at; pause = pause < 512 ? pause * 2 : pause) {
-    __nanosleep(pause);
-    if (globaltimer_ns() > give_up) {
-      raise_error(S, kFabErrRingWait);
-      return;
+__device__ __forceinline__ void ring_announce(DeviceState& S, Ring& R, unsigned long long at, int m, bool next) {
+  if (!next) {
+    const unsigned long long give_up = globaltimer_ns() + kRingWaitBudgetNs;
+    for (unsigned int pause = 32; ld_acq(&R.tail) != at; pause = pause < 512 ? pause * 2 : pause) {
+      __nanosleep(pause);
+      if (globaltimer_ns() > give_up) {
+        raise_error(S, kFabErrRingWait);
+        return;
+      }
     }
   }
   st_rel(&R.tail, at + m);
 }
+// One word.
+__device__ __forceinline__ void ring_publish(DeviceState& S, Ring& R, uint32_t word) {
+  const unsigned long long at = atomicAdd(&R.reserve, 1ull);
+  R.ids[at & (kRingCap - 1)] = word;
+  ring_announce(S, R, at, 1, false);
+}
 
 // ---------------------------------------------------------------------- claims
+// The tables of a program as a worker keeps them: the descriptor itself does not change while a lane runs it.
+struct ProgView {
+  const ProgramDesc* prog;
+  StageStatic* stages;
+  StageRuntime* runtime;
+  const TileDesc* tiles;
+  const uint32_t* succ;
+  uint32_t n_stages, gen;
+};
+// The WHOLE warp.  gen: of the lane, which is new for every program it is given (an address may come back).
+__device__ __forceinline__ void view_program(ProgView& v, const ProgramDesc* P, uint32_t gen) {
+  if (v.prog == P && v.gen == gen) return;
+  __syncwarp();
+  if ((threadIdx.x & 31) == 0) {
+    v.stages = ld_volatile(&P->stages);
+    v.runtime = ld_volatile(&P->runtime);
+    v.tiles = ld_volatile(&P->tiles);
+    v.succ = ld_volatile(&P->succ);
+    v.n_stages = ld_volatile(&P->n_stages);
+    v.prog = P;
+    v.gen = gen;
+  }
+  __syncwarp();
+}
+
+// What a work record keeps of it.
+struct ProgTables {
+  const ProgramDesc* prog;
+  StageStatic* stages;
+  StageRuntime* runtime;
+  const uint32_t* succ;
+};
+
 struct Claim {
   uint32_t stage, first_tile, n;
 };
+// What a probe of a ring entry found; left = 0: its stage has moved on to another activation or has been handed out.
+struct Probe {
+  uint32_t left, first, count;
+};
 
-// Tiles a ring entry can still give: 0 if its stage has moved on to another activation or
-// has been handed out completely.  A read-only probe; the claim itself re-checks.
-__device__ __forceinline__ uint32_t tiles_left(const ProgramDesc* P, uint32_t word) {
+__device__ __forceinline__ uint2 stage_tiles(const StageStatic* st) {   // (first, count) by one load
+  const unsigned long long v = ld_volatile(reinterpret_cast<const unsigned long long*>(st));
+  return make_uint2(static_cast<uint32_t>(v), static_cast<uint32_t>(v >> 32));
+}
+
+// A read-only probe; the claim itself re-checks.  The two loads may be answered in either order: a stage's tiles change only
+// while it is closed (tag 0), which the claim sees.
+__device__ __forceinline__ Probe probe_entry(const ProgView& V, uint32_t word) {
+  Probe p{0, 0, 0};
   const uint32_t s = word & kStageMask;
-  if (s >= P->n_stages) return 0;
-  const StageWord w(ld_acq(&P->runtime[s].tag_next));
-  const uint32_t count = ld_volatile(&P->stages[s].count);
-  return (w.tag == (word >> kStageBits) && w.next < count) ? count - w.next : 0;
+  if (s >= V.n_stages) return p;
+  const unsigned long long tn = ld_volatile(&V.runtime[s].tag_next);
+  const uint2 t = stage_tiles(V.stages + s);
+  const StageWord w(tn);
+  p.first = t.x;
+  p.count = t.y;
+  if (w.tag == (word >> kStageBits) && w.next < p.count) p.left = p.count - w.next;
+  return p;
 }
 
 // The fetch-and-add.  `left` is the probe's answer and only sizes the claim.
-__device__ __forceinline__ bool claim_tiles(const ProgramDesc* P, uint32_t word, uint32_t left, Claim& c) {
+__device__ __forceinline__ bool claim_tiles(const ProgView& V, uint32_t word, Probe p, Claim& c) {
   const uint32_t s = word & kStageMask;
-  uint32_t want = left >> kClaimShareLog2;
+  uint32_t want = p.left >> kClaimShareLog2;
   want = want < 1 ? 1 : (want > kClaimMax ? kClaimMax : want);
-  const StageWord before(atomicAdd(&P->runtime[s].tag_next, static_cast<unsigned long long>(want)));
+  const StageWord before(atomicAdd(&V.runtime[s].tag_next, static_cast<unsigned long long>(want)));
   // The add may land on a later activation of the stage (or on a stage that was closed, tag 0).
   // On a later activation it hands out that activation's tiles, which is as good; on a closed
   // stage, or past the end, it hands out nothing and the overshoot is harmless: `next` is only
   // ever compared with the count.
   if (before.tag == 0) return false;
-  if (before.tag != (word >> kStageBits)) __threadfence();   // a later activation: its stage record may be newer than the probe saw
-  const uint32_t count = ld_volatile(&P->stages[s].count);
-  if (before.next >= count) return false;
+  if (before.tag != (word >> kStageBits)) {   // a later activation: its stage record may be newer than the probe saw
+    __threadfence();
+    const uint2 t = stage_tiles(V.stages + s);
+    p.first = t.x;
+    p.count = t.y;
+  }
+  if (before.next >= p.count) return false;
   c.stage = s;
-  c.first_tile = ld_volatile(&P->stages[s].first) + before.next;
-  c.n = min(want, count - before.next);
+  c.first_tile = p.first + before.next;
+  c.n = min(want, p.count - before.next);
   return true;
 }
 
 // Consumer side, the WHOLE warp: lane i probes entry head + i; a run of exhausted entries at the
 // head is dropped with one compare-and-swap; the first entry that still has tiles is claimed.
-__device__ __forceinline__ bool ring_take(Ring& R, const ProgramDesc* P, Claim& c) {
+// head and tail come from one reading of both: a pair out of step only looks empty, or begins at
+// entries that are exhausted and fail the compare-and-swap.
+__device__ __forceinline__ bool ring_take(Ring& R, unsigned long long head, unsigned long long tail, const ProgView& V, Claim& c) {
   const int lane = threadIdx.x & 31;
-  // head and tail by two lanes at once (one round trip): a pair read out of step only looks empty, or
-  // begins at entries that are exhausted and fail the compare-and-swap below
-  unsigned long long word01 = 0;
-  if (lane == 0) word01 = ld_acq(&R.head);
-  else if (lane == 1) word01 = ld_acq(&R.tail);
-  const unsigned long long head = __shfl_sync(kWarp, word01, 0), tail = __shfl_sync(kWarp, word01, 1);
   if (tail <= head) return false;
   const int n = static_cast<int>(min(tail - head, 32ull));
-  uint32_t word = 0, left = 0;
+  uint32_t word = 0;
+  Probe p{0, 0, 0};
   if (lane < n) {
     word = ld_volatile(&R.ids[(head + lane) & (kRingCap - 1)]);
-    left = tiles_left(P, word);
+    p = probe_entry(V, word);
   }
-  unsigned live = __ballot_sync(kWarp, left != 0);
+  unsigned live = __ballot_sync(kWarp, p.left != 0);
   const int spent = live ? __ffs(live) - 1 : n;   // exhausted entries in front of the first live one
   if (spent > 0 && lane == 0) atomicCAS(&R.head, head, head + spent);   // losing the race is fine: someone else dropped them
   while (live) {
     const int src = __ffs(live) - 1;
     live &= live - 1;
     int ok = 0;
-    if (lane == src) ok = claim_tiles(P, word, left, c);
+    if (lane == src) ok = claim_tiles(V, word, p, c);
     ok = __shfl_sync(kWarp, ok, src);
     if (ok) {
       c.stage = __shfl_sync(kWarp, c.stage, src);
@@ -236,8 +297,7 @@ __device__ __forceinline__ void open_wave(DeviceState& S, uint32_t lane, const P
   st_rel(&L.tag, tag);
   const uint32_t s = P->first_stage;
   if (arm_stage(S, lane, P, s, tag, wl)) {
-    const uint32_t word = ring_word(s, tag);
-    ring_publish(S, L.ring[(ld_volatile(&P->stages[s].flags) & kStageLink) ? 1 : 0], &word, 1);
+    ring_publish(S, L.ring[(ld_volatile(&P->stages[s].flags) & kStageLink) ? 1 : 0], ring_word(s, tag));
   }
 }
 
@@ -270,10 +330,57 @@ __device__ __forceinline__ const ProgramDesc* close_iteration(DeviceState& S, ui
   return P;
 }
 
+// The WHOLE warp.  Counts down and arms the successors succ[first ..) of a completed stage, the 32 lanes side by side, and
+// publishes their ring words in two publications (ungated, link), so a stage with 128 successors releases them in a few
+// microseconds.  Each step is a round trip to the L2 that every stage of a program waits for, so what does not depend
+// on one another goes out together.
+template <class WL>
+__device__ __forceinline__ void release_stage(DeviceState& S, uint32_t lane_id, StageStatic* stages, StageRuntime* runtime,
+                                              const uint32_t* succs, uint32_t first, uint32_t count, uint32_t tag, bool tracing, WL& wl) {
+  const int lane = threadIdx.x & 31;
+  LaneState& L = S.lane[lane_id];
+  for (uint32_t base = 0; base < count; base += 32) {
+    enum { kNone, kUngated, kLink, kEmpty };
+    int fate = kNone;
+    uint32_t word = 0, succ = 0;
+    if (base + lane < count) {
+      succ = ld_volatile(succs + first + base + lane);
+      // a skipped stage is never armed, so that its count has no meaning
+      const unsigned int before = atomicSub(&runtime[succ].deps, 1u);
+      const uint32_t flags = ld_volatile(&stages[succ].flags), tiles = ld_volatile(&stages[succ].count);
+      if (before == 1u && !(flags & kStageSkip)) {
+        if (tracing) trace_stage(S, lane_id, succ, 0, tag);
+        if (tiles == 0) {
+          fate = kEmpty;
+        } else {
+          atomicExch(&runtime[succ].tag_next, armed_word(tag));
+          word = ring_word(succ, tag);
+          fate = (flags & kStageLink) ? kLink : kUngated;
+        }
+      }
+    }
+#pragma unroll
+    for (int want = kUngated; want <= kLink; ++want) {
+      const unsigned mask = __ballot_sync(kWarp, fate == want);
+      if (mask == 0) continue;
+      Ring& R = L.ring[want == kLink ? 1 : 0];
+      unsigned long long got = 0;
+      if (lane == 0) got = atomicAdd(&R.reserve, static_cast<unsigned long long>(__popc(mask)));
+      else if (lane == 1) got = ld_volatile(&R.tail);
+      const unsigned long long at = __shfl_sync(kWarp, got, 0), tail = __shfl_sync(kWarp, got, 1);
+      if (fate == want) R.ids[(at + __popc(mask & ((1u << lane) - 1))) & (kRingCap - 1)] = word;
+      __syncwarp();   // the stages' tags and words, by all lanes, are in front of lane 0's release
+      if (lane == 0) ring_announce(S, R, at, __popc(mask), tail == at);
+    }
+    for (unsigned mask = __ballot_sync(kWarp, fate == kEmpty); mask; mask &= mask - 1) {
+      const uint32_t v = __shfl_sync(kWarp, succ, __ffs(mask) - 1);
+      if (lane == 0) wl.push(v);
+    }
+  }
+}
+
 // The WHOLE warp.  Processes the worklist: for every completed stage, lane 0 reports marks and
-// handles the iteration boundary; the stage's successors are counted down and armed by the 32
-// lanes side by side, and their ring words go out in two publications (ungated, link), so a
-// stage with 128 successors releases them in a few microseconds.
+// handles the iteration boundary; then its successors are released.
 template <class WL>
 __device__ __forceinline__ void release_successors(DeviceState& S, uint32_t lane_id, const ProgramDesc* P, WL& wl) {
   const int lane = threadIdx.x & 31;
@@ -303,57 +410,41 @@ __device__ __forceinline__ void release_successors(DeviceState& S, uint32_t lane
     count = __shfl_sync(kWarp, count, 0);
     tag = __shfl_sync(kWarp, tag, 0);
     const ProgramDesc* Pw = reinterpret_cast<const ProgramDesc*>(__shfl_sync(kWarp, reinterpret_cast<unsigned long long>(P), 0));
-    for (uint32_t base = 0; base < count; base += 32) {
-      enum { kNone, kUngated, kLink, kEmpty };
-      int fate = kNone;
-      uint32_t word = 0, succ = 0;
-      if (base + lane < count) {
-        succ = Pw->succ[first + base + lane];
-        const uint32_t flags = ld_volatile(&Pw->stages[succ].flags);
-        if (!(flags & kStageSkip) && atomicSub(&Pw->runtime[succ].deps, 1u) == 1u) {
-          trace_stage(S, lane_id, succ, 0, tag);
-          if (ld_volatile(&Pw->stages[succ].count) == 0) {
-            fate = kEmpty;
-          } else {
-            atomicExch(&Pw->runtime[succ].tag_next, armed_word(tag));
-            __threadfence();   // armed before lane 0 publishes the word
-            word = ring_word(succ, tag);
-            fate = (flags & kStageLink) ? kLink : kUngated;
-          }
-        }
-      }
-      for (int want = kUngated; want <= kEmpty; ++want) {
-        unsigned mask = __ballot_sync(kWarp, fate == want);
-        uint32_t batch[32];
-        int n = 0;
-        for (; mask; mask &= mask - 1) {
-          const uint32_t v = __shfl_sync(kWarp, want == kEmpty ? succ : word, __ffs(mask) - 1);
-          if (lane == 0) {
-            if (want == kEmpty) wl.push(v);
-            else batch[n++] = v;
-          }
-        }
-        if (lane == 0 && want != kEmpty) ring_publish(S, L.ring[want == kLink ? 1 : 0], batch, n);
-      }
-    }
+    release_stage(S, lane_id, Pw->stages, Pw->runtime, Pw->succ, first, count, tag, true, wl);
   }
   if (lane == 0 && wl.overflow) raise_error(S, kFabErrWorklist);
 }
 
 // The WHOLE warp.  n tiles of stage s are done; the warp whose tiles complete the stage releases
-// its successors.
-__device__ __forceinline__ void tiles_completed(DeviceState& S, uint32_t lane_id, const ProgramDesc* P, uint32_t s, uint32_t n,
-                                                Worklist& wl) {
+// its successors.  What that takes of the stage's record is loaded beside the count.
+__device__ __forceinline__ void tiles_completed(DeviceState& S, uint32_t lane_id, const ProgTables& V, uint32_t s, uint32_t n, Worklist& wl) {
   int last = 0;
-  if ((threadIdx.x & 31) == 0) last = atomicAdd(&P->runtime[s].done, n) + n == ld_volatile(&P->stages[s].count);
+  uint32_t count = 0, first = 0, n_succ = 0, flags = 0, tag = 0, tracing = 0;
+  if ((threadIdx.x & 31) == 0) {
+    const unsigned int done = atomicAdd(&V.runtime[s].done, n) + n;
+    const StageStatic* st = V.stages + s;
+    count = ld_volatile(&st->count);
+    first = ld_volatile(&st->succ_first);
+    n_succ = ld_volatile(&st->succ_count);
+    flags = ld_volatile(&st->flags);
+    tag = ld_volatile(&S.lane[lane_id].tag);
+    tracing = ld_volatile(&S.trace_cap);
+    last = done == count;
+  }
   if (!__shfl_sync(kWarp, last, 0)) return;
   __threadfence();   // the other workers' tiles of the stage are visible before its successors start
+  const bool plain = !(__shfl_sync(kWarp, flags, 0) & (kStageMark | kStageReset));
   if ((threadIdx.x & 31) == 0) {
     wl.clear();
-    wl.push(s);
+    if (!plain) wl.push(s);
+    else if (tracing) trace_stage(S, lane_id, s, 1, tag);
   }
   __syncwarp();
-  release_successors(S, lane_id, P, wl);
+  if (plain)
+    release_stage(S, lane_id, V.stages, V.runtime, V.succ, __shfl_sync(kWarp, first, 0), __shfl_sync(kWarp, n_succ, 0),
+                  __shfl_sync(kWarp, tag, 0) & kTagMask, __shfl_sync(kWarp, tracing, 0) != 0, wl);
+  __syncwarp();
+  release_successors(S, lane_id, V.prog, wl);
 }
 
 // ------------------------------------------------------------------ the worker
@@ -366,8 +457,11 @@ struct WorkerState {
   ProgramDesc* prog_snap[kMaxLanes];
   uint32_t visit[kMaxLanes];   // lanes in the order this worker looks for work: its own, then the borrowing order
   uint32_t n_visit;
+  ProgView view;               // of the program looked at last
+  uint32_t idle, polls;        // the last round found nothing; polls since work was last found
   // the current claim
-  const ProgramDesc* prog;
+  ProgTables prog;
+  const TileDesc* tiles;
   uint32_t stage, tile_lane, link, next_index, left;
   uint32_t row_block;   // a kind-45 tile runs as one record per row block: the block of its next record
   // The link slot this worker holds (kNoLane = none).  The worker runs its records through a pipeline
@@ -460,26 +554,56 @@ __device__ __forceinline__ void start_waiting_lanes(DeviceState& S, WorkerState&
   }
 }
 
+// The words a round of scheduling depends on, one for each lane of the scheduler warp: lanes 7 l .. 7 l + 6 read lane l's
+// published tails (ungated, link), held link slots, running flag, generation, ungated head and program; lane 30 the
+// published epoch, lane 31 the shutdown flag (low half) and the idle cap.  One load instead of a chain of them: an idle
+// worker sees a new stage a round trip after it is published, and has its ring's ends and program in hand.
+constexpr int kWordsPerLane = 7, kEpochLane = 30, kStopLane = 31;
+static_assert(kWordsPerLane * kMaxLanes <= kEpochLane, "one word for each lane of a warp");
+static_assert(offsetof(LaneState, slots) % 8 == 0 && offsetof(LaneState, inflight_max) % 8 == 0 && offsetof(LaneState, gen) % 8 == 0 &&
+              offsetof(LaneState, running) == offsetof(LaneState, inflight_max) + 4 && offsetof(DeviceState, shutdown) % 8 == 0 &&
+              offsetof(DeviceState, idle_cap) == offsetof(DeviceState, shutdown) + 4, "pairs read as one word");
+enum { kWTail, kWLinkTail, kWSlots, kWRunning, kWGen, kWHead, kWProg };
+__device__ __forceinline__ const unsigned long long* polled_word(DeviceState& S, int lane) {
+  if (lane == kEpochLane) return &S.published;
+  if (lane == kStopLane) return reinterpret_cast<const unsigned long long*>(&S.shutdown);
+  if (lane >= kWordsPerLane * kMaxLanes) return nullptr;
+  LaneState& L = S.lane[lane / kWordsPerLane];
+  switch (lane % kWordsPerLane) {
+    case kWTail: return &L.ring[0].tail;
+    case kWLinkTail: return &L.ring[1].tail;
+    case kWSlots: return reinterpret_cast<const unsigned long long*>(&L.slots);
+    case kWRunning: return reinterpret_cast<const unsigned long long*>(&L.inflight_max);
+    case kWGen: return reinterpret_cast<const unsigned long long*>(&L.gen);
+    case kWHead: return &L.ring[0].head;
+    default: return &L.prog;
+  }
+}
+
 // The WHOLE scheduler warp.  Look for tiles in lane l: link stages first, under a slot; then the
 // ungated ring.  On success the claim is in ws (written by lane 0).
-__device__ __forceinline__ bool look_in_lane(DeviceState& S, WorkerState& ws, uint32_t l) {
+__device__ __forceinline__ bool look_in_lane(DeviceState& S, WorkerState& ws, uint32_t l, unsigned long long words) {
   const int lane = threadIdx.x & 31;
   LaneState& L = S.lane[l];
-  // `running` and the link ring's ends by three lanes at once, then the program (which is read after
-  // `running`, as before): two round trips instead of four
-  unsigned long long v = 0;
-  if (lane == 0) v = ld_acq(&L.running);
-  else if (lane == 1) v = ld_acq(&L.ring[1].tail);
-  else if (lane == 2) v = ld_volatile(&L.ring[1].head);
-  const bool running = __shfl_sync(kWarp, v, 0) != 0;
-  if (!running) return false;
-  const bool link_waiting = __shfl_sync(kWarp, v, 1) > __shfl_sync(kWarp, v, 2);
-  unsigned long long prog = 0;
-  if (lane == 0) prog = ld_acq(&L.prog);
-  const ProgramDesc* P = reinterpret_cast<const ProgramDesc*>(__shfl_sync(kWarp, prog, 0));
-  if (P == nullptr) return false;
+  auto word = [&](int which) { return __shfl_sync(kWarp, words, l * kWordsPerLane + which); };
+  const unsigned long long running = word(kWRunning), tail = word(kWTail), link_tail = word(kWLinkTail), gen = word(kWGen),
+                           head = word(kWHead), prog = word(kWProg);
+  if (!running || !prog) return false;
+  unsigned long long link_head = 0;
+  if (link_tail) {
+    if (lane == 0) link_head = ld_volatile(&L.ring[1].head);
+    link_head = __shfl_sync(kWarp, link_head, 0);
+  }
+  if (tail <= head && link_tail <= link_head) return false;
+  ProgView& V = ws.view;
+  view_program(V, reinterpret_cast<const ProgramDesc*>(prog), static_cast<uint32_t>(gen));
+  auto took = [&](const Claim& c, uint32_t link) {
+    if (lane == 0) {
+      ws.prog = ProgTables{V.prog, V.stages, V.runtime, V.succ}; ws.tiles = V.tiles; ws.stage = c.stage; ws.tile_lane = l; ws.link = link; ws.next_index = c.first_tile; ws.left = c.n;
+    }
+  };
   Claim c;
-  if (link_waiting) {
+  if (link_tail > link_head) {
     int held = 0;
     if (lane == 0) {
       held = ws.slot_lane == l;
@@ -496,52 +620,85 @@ __device__ __forceinline__ bool look_in_lane(DeviceState& S, WorkerState& ws, ui
       }
     }
     if (__shfl_sync(kWarp, held, 0)) {
-      if (ring_take(L.ring[1], P, c)) {
-        if (lane == 0) {
-          ws.prog = P; ws.stage = c.stage; ws.tile_lane = l; ws.link = 1; ws.next_index = c.first_tile; ws.left = c.n;
-        }
+      if (ring_take(L.ring[1], link_head, link_tail, V, c)) {
+        took(c, 1);
         return true;
       }
       if (lane == 0) give_slot_back(S, ws);
     }
   }
-  if (!ring_take(L.ring[0], P, c)) return false;
-  if (lane == 0) {
-    give_slot_back(S, ws);
-    ws.prog = P; ws.stage = c.stage; ws.tile_lane = l; ws.link = 0; ws.next_index = c.first_tile; ws.left = c.n;
-  }
+  if (!ring_take(L.ring[0], head, tail, V, c)) return false;
+  if (lane == 0) give_slot_back(S, ws);
+  took(c, 0);
   return true;
 }
 
 // The WHOLE scheduler warp.  One scheduling round: kCmdRun with a claim in ws, kCmdExit when the
-// host asked the fabric to stop, or kCmdIdle after a back-off that grows to the plan's idle cap.
-__device__ __forceinline__ uint32_t schedule(DeviceState& S, WorkerState& ws, SmallWorklist& wl) {
-  const int lane = threadIdx.x & 31;
-  adopt_epoch(S, ws);
-  int stop = 0;
-  if (lane == 0) stop = ld_acq(&S.shutdown) != 0;
-  if (__shfl_sync(kWarp, stop, 0)) {
+// host asked the fabric to stop, or kCmdIdle.  `at` is this lane's polled word, `seen` what it was in the last round: a round in
+// which no word has changed since one that found nothing is only the reading of the words.  While a lane
+// runs, the reading is repeated at once (a stage is over in microseconds); otherwise the back-off grows to the idle cap.
+__device__ __forceinline__ uint32_t schedule(DeviceState& S, WorkerState& ws, SmallWorklist& wl, const unsigned long long* at,
+                                             unsigned long long& seen) {
+  const int lane = threadIdx.x & 31, which = lane % kWordsPerLane;
+  const bool of_lane = lane < kWordsPerLane * kMaxLanes;
+  const uint32_t n_lanes = ws.n_lanes;
+  unsigned long long words = 0;
+  if (lane >= kEpochLane || (of_lane && lane / kWordsPerLane < n_lanes)) words = ld_acq(at);
+  __syncwarp();
+  if (of_lane && (which == kWSlots || which == kWGen)) words &= 0xffffffffull;
+  if (of_lane && which == kWRunning) words >>= 32;
+  const bool changed = __any_sync(kWarp, words != seen && !(of_lane && which >= kWHead));
+  auto idle = [&](bool found_nothing, bool more = false) {
+    const bool busy = __any_sync(kWarp, of_lane && which == kWRunning && words != 0);
+    const uint32_t cap = max(64u, static_cast<uint32_t>(__shfl_sync(kWarp, words, kStopLane) >> 32));
+    if (lane == 0) {
+      ws.idle = found_nothing && !more;
+      ++ws.polls;
+      if (found_nothing) {
+        __nanosleep(busy ? 32 : ws.idle_ns);
+        ws.idle_ns = busy ? 64 : min(ws.idle_ns * 2, cap);
+      }
+    }
+    __syncwarp();
+    return kCmdIdle;
+  };
+  if (ws.idle && !changed) return idle(true);
+  seen = words;
+  if (static_cast<uint32_t>(__shfl_sync(kWarp, words, kStopLane)) != 0) {
     if (lane == 0) give_slot_back(S, ws);
     return kCmdExit;
   }
-  start_waiting_lanes(S, ws, wl);
-  __syncwarp();
+  if (__shfl_sync(kWarp, words, kEpochLane) != ws.epoch) {
+    adopt_epoch(S, ws);
+    return idle(false);   // the words of the plan's lanes are read next
+  }
+  const unsigned long long running = __shfl_up_sync(kWarp, words, kWGen - kWRunning);
+  const uint32_t l = lane / kWordsPerLane;
+  const bool starts = of_lane && which == kWGen && l < n_lanes && running == 0 && ws.prog_snap[l] != nullptr &&
+                      ws.prog_gen[l] != static_cast<uint32_t>(words);
+  if (__any_sync(kWarp, starts)) {
+    start_waiting_lanes(S, ws, wl);
+    __syncwarp();
+    return idle(false);
+  }
   const uint32_t n_visit = ws.n_visit;
   for (uint32_t i = 0; i < n_visit; ++i) {
-    if (look_in_lane(S, ws, ws.visit[i])) {
-      if (lane == 0) ws.idle_ns = 64;
+    if (ws.visit[i] >= n_lanes) continue;
+    if (look_in_lane(S, ws, ws.visit[i], words)) {
+      if (lane == 0) {
+        ws.idle_ns = 64;
+        ws.idle = 0;
+        ws.polls = 0;
+      }
       __syncwarp();
       return kCmdRun;
     }
   }
-  if (lane == 0) {
-    give_slot_back(S, ws);
-    __nanosleep(ws.idle_ns);
-    const uint32_t cap = max(64u, ld_volatile(&S.idle_cap));
-    ws.idle_ns = min(ws.idle_ns * 2, cap);
-  }
-  __syncwarp();
-  return kCmdIdle;
+  if (lane == 0) give_slot_back(S, ws);
+  // Entries past the 32 that were probed, and link stages (whose ring's head and slots are read apart), are looked at again.
+  const unsigned long long head = __shfl_down_sync(kWarp, words, kWHead - kWTail);
+  const bool more = of_lane && ((which == kWTail && words > head + 32) || (which == kWLinkTail && words != 0));
+  return idle(true, __any_sync(kWarp, more));
 }
 
 }  // namespace fab

@@ -259,3 +259,32 @@ def test_upload_rejects_malformed_programs(fab):
         fab.upload(tiles.to(torch.int32), stages, succ, 0, 0, 1)
     with pytest.raises(RuntimeError, match="lanes"):
         fab.publish(map=[0], caps=[0] * 5, order=[0] * 5, programs=[0] * 5)
+
+
+@pytest.mark.parametrize("link", [False, True])
+def test_many_ring_entries_after_a_long_idle(fab, link):
+    """More stages at once than a worker probes in one look, some of them empty, gated ones under fewer slots than there are
+    workers, after an idle stretch in which every worker has settled on "nothing has changed"; three iterations, twice."""
+    trace = trace_buffer(512)
+    p = Program()
+    root, idx, stages = p.stage([spin(2_000, trace, 0)]), 1, []
+    for i in range(150):
+        n = i % 3
+        stages.append(p.stage([spin(3_000, trace, idx + k) for k in range(n)], link=link and i % 2 == 1))
+        idx += n
+    join = p.stage([spin(2_000, trace, idx)])
+    for s in stages:
+        p.after(root, s)
+        p.after(s, join)
+    handles = [p.upload(fab, first=root, iterations=3) for _ in range(2)]
+    fab.start()
+    for turn, h in enumerate(handles):
+        time.sleep(0.05)
+        done = fab.iterations(0)
+        fab.publish(map=[0] * fab.num_workers, caps=[3], order=[0], programs=[h])
+        fab.iteration_times(0, done, 3)
+    fab.stop()
+    assert fab.progress()["error"] == 0
+    tr = decode_trace(trace)
+    assert (tr["count"][:idx + 1] == 6).all()
+    assert tr["start"][idx] >= tr["end"][:idx].max()
