@@ -81,14 +81,14 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity,
                                                   volatile int* abort_flag,
                                                   unsigned long long budget_ns) {
-  unsigned long long t0 = 0;   // the first reading of the timer, which is slow: most waits end before it
-  for (uint32_t spins = 1;; ++spins) {
+  if (mbar_try_wait(bar, parity)) return true;
+  const unsigned long long t0 = globaltimer_ns();
+  uint32_t spins = 0;
+  while (true) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((spins & 63u) == 0) {
+    if ((++spins & 63u) == 0) {
       if (*abort_flag) return false;
-      const unsigned long long now = globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > budget_ns) {
+      if (globaltimer_ns() - t0 > budget_ns) {
         *abort_flag = 1;
         return false;
       }
