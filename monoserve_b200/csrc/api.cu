@@ -163,8 +163,6 @@ int forward_locked(monofab_moe* m, const void* xn, const void* x2, void* out, in
   MF_CUDA(mark());
   RouterParams rp{m->logits, m->router_bias, m->topk_ids, m->topk_w, nullptr, m->chunk_counts, m->pair_rank,
                   T, E, K, c.scoring, c.renorm, c.routed_scale, 0};
-  MF_CUDA(launch_router_topk(rp, st));
-  MF_CUDA(mark());
   PlanParams pp{};
   pp.chunk_counts = m->chunk_counts;
   pp.counts = m->counts;
@@ -186,12 +184,19 @@ int forward_locked(monofab_moe* m, const void* xn, const void* x2, void* out, in
   pp.tile_cap = m->tile_cap;
   pp.n_experts = E;
   pp.rows_cap = static_cast<int>(m->pairs_cap) - 256;
-  MF_CUDA(launch_plan(pp, st));
-  MF_CUDA(mark());
   PackParams kp{m->topk_ids, m->topk_w, m->pair_rank, m->chunk_counts, m->starts, static_cast<const bf16*>(xn),
                 static_cast<bf16*>(m->xp), m->pair_token,
                 m->pair_weight, m->pair_pos, T, E, K, H, m->status};
-  MF_CUDA(launch_pack(kp, st));
+  if (route_in_one(T)) {
+    MF_CUDA(launch_route(rp, pp, kp, st));
+    MF_CUDA(mark());   // the plan is part of the launch that chooses the experts
+  } else {
+    MF_CUDA(launch_router_topk(rp, st));
+    MF_CUDA(mark());
+    MF_CUDA(launch_plan(pp, st));
+  }
+  MF_CUDA(mark());
+  if (!route_packs(T)) MF_CUDA(launch_pack(kp, st));
   MF_CUDA(mark());
   m->gp.cap = m->credits;
   m->gp.trace = m->trace_on ? m->trace : nullptr;

@@ -146,6 +146,11 @@ cudaError_t launch_chunk_rank(const int* topk_ids, int* pair_rank, int* chunk_co
                               int* status, cudaStream_t stream);
 cudaError_t launch_plan(const PlanParams& A, cudaStream_t stream);
 cudaError_t launch_pack(const PackParams& A, cudaStream_t stream);
+// launch_router_topk (chunk counts and ranks set), launch_plan (of these chunks, with tiles) and, where route_packs(T), launch_pack;
+// for the T of route_in_one.
+cudaError_t launch_route(const RouterParams& R, const PlanParams& P, const PackParams& K, cudaStream_t stream);
+bool route_in_one(int T);
+bool route_packs(int T);
 cudaError_t launch_combine(const CombineParams& A, cudaStream_t stream);
 cudaError_t launch_expert_gemm(const GemmParams& p, int ctas, cudaStream_t stream);
 cudaError_t launch_pack_w13(const void* src, void* dst, int n, int I, int H, int elt_bytes, cudaStream_t stream);

@@ -39,7 +39,8 @@ struct GemmQueues {
   int32_t slots;           // link slots in use
   int32_t n_blocks;        // row blocks (entries of the done[] array in use)
   int32_t need;            // epilogue-warp arrivals that complete a row block's w13
-  int32_t pad[9];
+  uint32_t routed;         // blocks of a routing launch that have counted their chunk (back at 0 when the launch ends)
+  int32_t pad[8];
 };
 static_assert(sizeof(GemmQueues) == 64, "GemmQueues is 64 bytes");
 

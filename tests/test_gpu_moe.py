@@ -149,6 +149,16 @@ def test_layer_small_all_intermediates(T, H, I, E, K):
     m.close()
 
 
+def test_routing_launch_at_its_edges():
+    """One launch chooses the experts, makes the plan in the block that counts its chunk last and packs up to four tokens: batches
+    around a chunk of 32 tokens and around that number, one after the other on one layer."""
+    H, I, E, K = 256, 64, 16, 8
+    m, wr, w13, w2 = make_layer(300, H, I, E, K, hot=list(range(0, E, 2)), seed=3)
+    for T in (1, 300, 4, 5, 31, 32, 33, 4, 64, 65, 3, 97):
+        check_layer_against_c_oracle(m, wr, w13, w2, *acts(T, H, T), K)
+    m.close()
+
+
 def test_layer_empty_batch_and_bounds():
     m, wr, w13, w2 = make_layer(16, 256, 128, 8, 2, hot=[0, 1])
     xn, _ = acts(4, 256, 1)
