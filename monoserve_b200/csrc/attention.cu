@@ -194,7 +194,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attention_kernel(const 
       }
       w.item = p.items[i];
       attn_derive(w, c);
-      attn_produce<true>(w, c);
+      attn_produce(w, c);
       attn_advance(c.n_tiles, c.q_phase, c.base);
       if (*abort_flag) break;
     }
@@ -217,12 +217,12 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attention_kernel(const 
       w.trace = (p.pad && blockIdx.x == 0 && it == 0) ? g_attn_trace : nullptr;
       attn_derive(w, c);
       if (warp == 1) {
-        if (c.rep) attn_mma<2, true>(w, c);
-        else attn_mma_alt<true>(w, c);
+        if (c.rep) attn_mma<2>(w, c);
+        else attn_mma_alt(w, c);
       } else if (c.rep) {
         softmax_role<true, 2, kAttnGroups, true, true>(w, c, (warp - 2) >> 2);
       } else {
-        softmax_alt<true>(w, c, (warp - 2) >> 2, xbuf);
+        softmax_alt(w, c, (warp - 2) >> 2, xbuf);
       }
       attn_advance(c.n_tiles, c.q_phase, c.base);
       if (warp == 1 && *abort_flag) break;   // the softmax threads decide at the top of the loop

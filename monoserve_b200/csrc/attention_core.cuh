@@ -71,7 +71,7 @@ struct AttnCtx {
   uint32_t base[2];       // every per-tile barrier [s]: tiles of parity s so far
   volatile unsigned int* note;   // this role's wait note (tile << 8 | site), or NULL
   float* xbuf;            // several softmax groups: float [groups][128] for the exchange between the parts of a row
-  uint64_t* q_empty;      // chained items only: completes once per item, when its last S MMA has read Q
+  uint64_t* q_empty;      // completes once per item, when its last S MMA has read Q
   uint64_t* s_free;       // alternating softmax groups only: [2], S[s] of a tile has been read into registers
 };
 
@@ -159,6 +159,107 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
+// Scores of keys past the visible ones, the first `lim`, are as low as can be: they are no maximum and their exponential is zero.
+template <int NC>
+__device__ __forceinline__ void mask_scores(uint32_t (&v)[NC], int lim) {
+  if (lim >= NC) return;
+#pragma unroll
+  for (int i = 0; i < NC; ++i) v[i] = i < lim ? v[i] : 0xff800000u;
+}
+template <int NC>
+__device__ __forceinline__ float max_scores(const uint32_t (&v)[NC], float mx) {   // four chains
+  float m[4] = {mx, mx, mx, mx};
+#pragma unroll
+  for (int i = 0; i < NC; ++i) m[i & 3] = fmaxf(m[i & 3], __uint_as_float(v[i]));
+  return fmaxf(fmaxf(m[0], m[1]), fmaxf(m[2], m[3]));
+}
+// 64 columns of a row, at TMEM address `at`, by the whole warp.
+__device__ __forceinline__ void load_columns(uint32_t at, uint32_t (&v)[64]) {
+  __syncwarp();
+  tmem_ld_32x32(at, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+  tmem_ld_32x32(at + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
+  tmem_ld_wait();
+}
+// P of 32 scores: exp2(s * scale + neg_mx) as bf16 at chunks [chunk, chunk + 4) of a row of 128 bytes (128-byte swizzle, `swz`:
+// the row's number modulo eight), and the sums of the rounded values.
+__device__ __forceinline__ void store_weights(const uint32_t* v, float scale, float neg_mx, uint8_t* row, int chunk, int swz, float& sum0,
+                                              float& sum1) {
+  uint32_t packed[16];
+#pragma unroll
+  for (int i = 0; i < 32; i += 2) {
+    const float p0 = fast_exp2(fmaf(__uint_as_float(v[i]), scale, neg_mx));
+    const float p1 = fast_exp2(fmaf(__uint_as_float(v[i + 1]), scale, neg_mx));
+    const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
+    const uint32_t u = *reinterpret_cast<const uint32_t*>(&b);
+    sum0 += __uint_as_float(u << 16);
+    sum1 += __uint_as_float(u & 0xffff0000u);
+    packed[i >> 1] = u;
+  }
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    *reinterpret_cast<uint4*>(row + (((chunk + q) ^ swz) << 4)) =
+        make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
+}
+// The two halves of a tile's row, one after the other through the same code: a warp that has a scheduler to itself is bound by
+// the fetch of straight-line code (128 keys in line: 2600 cycles a tile, where the
+// special-function unit needs 1024, and 4000 in the first item of a stage).
+__device__ __forceinline__ float row_max(uint32_t tmem_s, int lim) {
+  float mx = -1e30f;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    uint32_t v[64];
+    load_columns(tmem_s + 64 * h, v);
+    mask_scores(v, lim - 64 * h);
+    mx = max_scores(v, mx);
+  }
+  return mx;
+}
+// Weights of a row into P, the row's halves kHalfBytes apart; the sum of the rounded weights.  `read`: called once S has been read.
+template <class Read>
+__device__ __forceinline__ float row_weights(uint32_t tmem_s, int lim, float scale, float neg_mx, uint8_t* row, int swz, Read read) {
+  float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    uint32_t v[64];
+    load_columns(tmem_s + 64 * h, v);
+    if (h == 1) read();
+    const int lh = lim - 64 * h;
+    if (lh > 0) {
+      mask_scores(v, lh);
+      store_weights(&v[0], scale, neg_mx, row, 0, swz, sum0, sum1);
+      store_weights(&v[32], scale, neg_mx, row, 4, swz, sum0, sum1);
+    } else {   // every key of the half is masked
+#pragma unroll
+      for (int q = 0; q < 8; ++q) *reinterpret_cast<uint4*>(row + 16 * q) = make_uint4(0, 0, 0, 0);
+    }
+    row += kHalfBytes;
+  }
+  return sum0 + sum1;
+}
+
+// 64 columns of the output rows of a warp's lanes: through its own rows of P's memory (`rows`: of lane 0, 128 bytes each, 16-byte
+// pieces swizzled by the row), from where a row's 128 bytes leave side by side.  (16 bytes of 32 rows an instruction: 4200 cycles for
+// 128 columns of 128 rows.)  to: lane's row of the output, NULL for none.
+__device__ __forceinline__ void store_rows(const float (&f)[64], uint8_t* rows, __nv_bfloat16* to) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    __nv_bfloat162 h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(f[8 * q + 2 * i], f[8 * q + 2 * i + 1]);
+    *reinterpret_cast<uint4*>(rows + lane * 128 + ((q ^ (lane & 7)) << 4)) = *reinterpret_cast<const uint4*>(h);
+  }
+  __syncwarp();
+  const int piece = lane & 7;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = 4 * i + (lane >> 3);
+    uint4* const dst = reinterpret_cast<uint4*>(__shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(to), r));
+    const uint4 v = *reinterpret_cast<const uint4*>(rows + r * 128 + ((piece ^ (r & 7)) << 4));
+    if (dst) dst[piece] = v;
+  }
+}
+
 __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
@@ -213,11 +314,10 @@ __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volati
 }
 
 // The TMA producer role: the whole warp calls it.
-// kChain: the CTA works through a list of items with no barrier between them and the producer runs ahead of
-// the other roles into the next item.  The first uses of a ring stage by an item then wait for the stage's
+// A CTA works through a list of items with no barrier between them and the producer runs ahead of
+// the other roles into the next item.  The first uses of a ring stage by an item wait for the stage's
 // last use by the item before (the barriers count uses across items: AttnCtx::base), and Q waits until the
 // MMAs of the item before have read it.
-template <bool kChain = false>
 __device__ __forceinline__ void attn_produce(const AttnWork& p, const AttnCtx& c) {
   AttnShared& sh = *c.sh;
   volatile int* abort_flag = c.abort_flag;
@@ -228,7 +328,7 @@ __device__ __forceinline__ void attn_produce(const AttnWork& p, const AttnCtx& c
   uint8_t* const sQ = c.smem;
   uint8_t* const sK = c.smem + kTileBytes;
   uint8_t* const sV = c.smem + 3 * kTileBytes;
-  if (kChain && c.q_phase > 0 && !warp_wait(c.q_empty, (c.q_phase - 1) & 1u, abort_flag, kAttnWaitNs)) {
+  if (c.q_phase > 0 && !warp_wait(c.q_empty, (c.q_phase - 1) & 1u, abort_flag, kAttnWaitNs)) {
     attn_gave_up(sh, kAttnSiteProdQ);
     return;
   }
@@ -256,7 +356,7 @@ __device__ __forceinline__ void attn_produce(const AttnWork& p, const AttnCtx& c
   // have been on its way.  One tile ahead where the tile loop is bound by the loads (a quad-replicated item,
   // and inside the fabric worker), two under the alternating softmax groups, whose S of tile j + 2 goes out
   // before P V of tile j.
-  const int lead = (kChain && !rep) ? 2 : 1;
+  const int lead = (c.s_free && !rep) ? 2 : 1;
   auto page_of = [&](int j) {
     // pages past the visible range repeat the last visible page; their keys are masked
     const int pg = min((tile0 + j) * pages_per_tile + lane, last_page);
@@ -266,7 +366,7 @@ __device__ __forceinline__ void attn_produce(const AttnWork& p, const AttnCtx& c
     if (step < n_tiles) {
       const int j = step, s = j & 1;
       const uint32_t uses = c.base[s] + (j >> 1);        // earlier uses of this stage, by this item and those before
-      const bool reuse = kChain ? uses > 0 : j >= 2;
+      const bool reuse = uses > 0;
       const uint32_t prev = (uses - 1) & 1u;             // the stage's previous use (tile j - 2 of this item, if j >= 2)
       if (lane == 0) attn_note(c, j, kAttnSiteProdK);
       if (reuse && !warp_wait(&sh.k_empty[s], prev, abort_flag, kAttnWaitNs)) { attn_gave_up(sh, kAttnSiteProdK); break; }
@@ -278,7 +378,7 @@ __device__ __forceinline__ void attn_produce(const AttnWork& p, const AttnCtx& c
     if (step >= lead) {
       const int j = step - lead, s = j & 1;
       const uint32_t uses = c.base[s] + (j >> 1);
-      const bool reuse = kChain ? uses > 0 : j >= 2;
+      const bool reuse = uses > 0;
       const uint32_t prev = (uses - 1) & 1u;
       if (lane == 0) attn_note(c, j, kAttnSiteProdV);
       if (reuse && !warp_wait(&sh.v_empty[s], prev, abort_flag, kAttnWaitNs)) { attn_gave_up(sh, kAttnSiteProdV); break; }
@@ -295,7 +395,7 @@ __device__ __forceinline__ void attn_produce(const AttnWork& p, const AttnCtx& c
 // descriptors are warp-uniform values (in a single-lane branch the issue path was about twice as slow).
 // PB = P buffers in shared memory (2: the stand-alone kernel; 1: inside the fabric
 // worker, whose operand ring holds six 32 KB tiles).
-template <int PB, bool kChain = false>
+template <int PB>
 __device__ __forceinline__ void attn_mma(const AttnWork& p, const AttnCtx& c) {
   AttnShared& sh = *c.sh;
   volatile int* abort_flag = c.abort_flag;
@@ -317,10 +417,9 @@ __device__ __forceinline__ void attn_mma(const AttnWork& p, const AttnCtx& c) {
     if (leader) attn_note(c, j, kAttnSiteMmaK);
     if (!mbar_wait_bounded(&sh.k_full[s], attn_parity(c, j), abort_flag, kAttnWaitNs)) return attn_gave_up(sh, kAttnSiteMmaK);
     if (leader) attn_note(c, j, kAttnSiteMmaSFree);
-    // S[s] is free once the softmax threads have turned its previous tile (j - 2, or, in a chain of items,
-    // the last one of the item before) into P
+    // S[s] is free once the softmax threads have turned its previous tile (j - 2, or the last one of the item before) into P
     const uint32_t uses = c.base[s] + (j >> 1);
-    if ((kChain ? uses > 0 : j >= 2) && !mbar_wait_bounded(&sh.p_full[s], (uses - 1) & 1u, abort_flag, kAttnWaitNs))
+    if (uses > 0 && !mbar_wait_bounded(&sh.p_full[s], (uses - 1) & 1u, abort_flag, kAttnWaitNs))
       return attn_gave_up(sh, kAttnSiteMmaSFree);
     tc_fence_after_sync();
     const uint32_t k_addr = smem_u32(sK + s * kTileBytes);
@@ -330,11 +429,11 @@ __device__ __forceinline__ void attn_mma(const AttnWork& p, const AttnCtx& c) {
         umma_bf16(tmem_base + s * 128, desc_kmajor(q_addr, i), desc_k_tile(k_addr, i), idesc_s, i != 0);
       umma_commit(&sh.s_full[s]);
       umma_commit(&sh.k_empty[s]);
-      if (kChain && j == n_tiles - 1) umma_commit(c.q_empty);   // Q has been read for the last time
+      if (j == n_tiles - 1) umma_commit(c.q_empty);   // Q has been read for the last time
     }
     return true;
   };
-  if (kChain && ok && n_tiles == 0 && leader) mbar_arrive(c.q_empty);
+  if (ok && n_tiles == 0 && leader) mbar_arrive(c.q_empty);
   if (ok && n_tiles > 0) ok = mma_s(0);
   if (ok && n_tiles > 1) ok = mma_s(1);
   for (int j = 0; ok && j < n_tiles; ++j) {
@@ -375,15 +474,8 @@ __device__ __forceinline__ void named_barrier_n(int id, int threads) {
 // The softmax / output role.  WG = softmax warp groups of four warps (1 inside the fabric
 // worker, kAttnGroups in the stand-alone kernel); `wg` is the caller's group.  A thread's row is
 // its TMEM lane.  kRep (quad-replicated item, at most 32 rows): the thread's row is `lane`, its
-// columns are quarter `quad` of the tile, and only group 0 works.  Otherwise the thread owns one
-// of 128 query rows and, with WG groups, 1 / WG of the tile's key columns and of the row's output:
-// the WG threads of a row agree on the row maximum through shared memory (`c.xbuf`) and a
-// barrier per lane quadrant, which all warps of the quadrant pass exactly twice per tile
-// whatever else happens, so that none can be left waiting.  (Two groups: with four, 576 threads
-// leave 96 registers each and the spills cost more than the extra warps hide: decode 517 us
-// against 226, prefill 301 us against 253 on the benchmark shapes.  The stand-alone kernel no longer splits
-// columns between its groups: its items with more than 32 rows run softmax_alt below, 634 TFLOP/s against 542
-// on the prefill benchmark.)
+// columns are quarter `quad` of the tile, and only group 0 works.  Otherwise (the fabric's worker) the thread owns one
+// of 128 query rows.
 // kChain (a chain of items, see attn_produce): the K / V stages already receive the next item while this one
 // ends, so the merge of a quad-replicated item uses the two P buffers (64 KB, rows XOR-swizzled by 16-byte
 // chunk instead of padded) and `c.xbuf` for the (max, sum) pairs, and every softmax thread of the CTA, working
@@ -399,8 +491,8 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     named_barrier_n(6, 128 * WG);
     return;
   }
-  constexpr int NC = kRep ? 32 : kKeysPerTile / WG;   // key columns of a tile this thread handles
-  constexpr int ND = kRep ? kHeadDim : kHeadDim / WG; // output columns of its row it rescales and stores
+  static_assert(kRep || WG == 1, "a row of an item that is not replicated has one thread");
+  constexpr int NC = kRep ? 32 : kKeysPerTile;   // key columns of a tile this thread handles
   AttnShared& sh = *c.sh;
   volatile int* abort_flag = c.abort_flag;
   const AttnItem& item = p.item;
@@ -415,14 +507,12 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
   const int lr = kRep ? lane : r;                 // row of the item
   const bool row_ok = lr < c.rows;
   const bool works = kRep ? wg == 0 : quad * 32 < c.rows;   // warp-uniform: false = keep the barrier protocol only
-  const bool pair = !kRep && WG > 1 && works;               // exchanges with the other warps of its quadrant
   const int group = p.group;
   const int token = lr / group, head = item.kv_head * group + lr % group;
   const int qpos = item.pos0 + token;
-  const int c_lo = kRep ? quad * 32 : wg * NC;
-  const int d_lo = kRep ? 0 : wg * ND;
+  const int c_lo = kRep ? quad * 32 : 0;
   const uint32_t lane_off = static_cast<uint32_t>(quad * 32) << 16;
-  const uint32_t tmem_o = c.tmem_base + 256 + lane_off + d_lo;
+  const uint32_t tmem_o = c.tmem_base + 256 + lane_off;
   const int n_tiles = c.n_tiles;
   float m = -1e30f, l = 0.f;
   bool ok = true;
@@ -461,36 +551,20 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     const int key0 = item.key_begin + j * kKeysPerTile + c_lo;
     // keys this thread may use among its NC columns: [0, lim)
     const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, NC) : 0;
-    if (!ok) {   // after a wait gave up: only what the partner warp may still be waiting for
-      if (pair) {
-        named_barrier_n(2 + quad, 32 * WG);
-        named_barrier_n(2 + quad, 32 * WG);
-      }
-      continue;
-    }
-    uint32_t v[NC];
-    __syncwarp();
-#pragma unroll
-    for (int c0 = 0; c0 < NC; c0 += 32) tmem_ld_32x32(tmem_s + c0, *reinterpret_cast<uint32_t(*)[32]>(&v[c0]));
-    tmem_ld_wait();
+    if (!ok) continue;   // a wait gave up
+    uint32_t v[32];   // of a quad-replicated item: the thread's quarter of the row
     // the scale is positive: the maximum of the scaled scores is the scaled maximum
-    float mx = -1e30f;
-    if (lim >= NC) {
-#pragma unroll
-      for (int i = 0; i < NC; ++i) mx = fmaxf(mx, __uint_as_float(v[i]));
+    float mx;
+    if constexpr (kRep) {
+      __syncwarp();
+      tmem_ld_32x32(tmem_s, v);
+      tmem_ld_wait();
+      mask_scores(v, lim);
+      mx = max_scores(v, -1e30f);
     } else {
-#pragma unroll
-      for (int i = 0; i < NC; ++i)
-        if (i < lim) mx = fmaxf(mx, __uint_as_float(v[i]));
+      mx = row_max(tmem_s, lim);
     }
     mx = mx > -1e30f ? mx * p.scale_log2 : -1e30f;
-    if (pair) {   // the row maximum over all parts of the tile
-      c.xbuf[wg * 128 + r] = mx;
-      named_barrier_n(2 + quad, 32 * WG);
-#pragma unroll
-      for (int g = 0; g < WG; ++g) mx = fmaxf(mx, c.xbuf[g * 128 + r]);
-      named_barrier_n(2 + quad, 32 * WG);
-    }
     mx = fmaxf(mx, m);
     lap(1);
     // The reference point of a row's exponentials moves only when the row's maximum has grown past
@@ -507,7 +581,7 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
       tc_fence_after_sync();
       const float alpha = fast_exp2(m - mx);
 #pragma unroll
-      for (int c0 = 0; c0 < ND; c0 += 32) {
+      for (int c0 = 0; c0 < kHeadDim; c0 += 32) {
         uint32_t o[32];
         __syncwarp();
         tmem_ld_32x32(tmem_o + c0, o);
@@ -529,45 +603,14 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     }
     const float neg_mx = -mx;
     // P = exp2(s - max) as bf16 into shared memory (K-major, 128-byte swizzle); row sum of the rounded P
-    float sum0 = 0.f, sum1 = 0.f;
-    uint8_t* p_tile = sP + (j % PB) * kTileBytes;
-#pragma unroll
-    for (int c0 = 0; c0 < NC; c0 += 32) {
-      uint32_t packed[16];
-      if (c0 + 32 <= lim) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(v[c0 + i]), p.scale_log2, neg_mx));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(v[c0 + i + 1]), p.scale_log2, neg_mx));
-          const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
-          const uint32_t u = *reinterpret_cast<const uint32_t*>(&b);
-          sum0 += __uint_as_float(u << 16);
-          sum1 += __uint_as_float(u & 0xffff0000u);
-          packed[i >> 1] = u;
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = c0 + i < lim ? fast_exp2(fmaf(__uint_as_float(v[c0 + i]), p.scale_log2, neg_mx)) : 0.f;
-          const float p1 = c0 + i + 1 < lim ? fast_exp2(fmaf(__uint_as_float(v[c0 + i + 1]), p.scale_log2, neg_mx)) : 0.f;
-          const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
-          const uint32_t u = *reinterpret_cast<const uint32_t*>(&b);
-          sum0 += __uint_as_float(u << 16);
-          sum1 += __uint_as_float(u & 0xffff0000u);
-          packed[i >> 1] = u;
-        }
-      }
-      // 32 keys = four 16-byte chunks of this row in key half col / 64
-      const int col = c_lo + c0;
-      uint8_t* row_base = p_tile + (col >> 6) * kHalfBytes + r * 128;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int chunk = ((col & 63) >> 3) + q;
-        *reinterpret_cast<uint4*>(row_base + ((chunk ^ (r & 7)) << 4)) =
-            make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-      }
+    uint8_t* const p_row = sP + (j % PB) * kTileBytes + r * 128;
+    if constexpr (kRep) {
+      float sum0 = 0.f, sum1 = 0.f;
+      store_weights(v, p.scale_log2, neg_mx, p_row + (c_lo >> 6) * kHalfBytes, (c_lo & 63) >> 3, r & 7, sum0, sum1);
+      l += sum0 + sum1;
+    } else {
+      l += row_weights(tmem_s, lim, p.scale_log2, neg_mx, p_row, r & 7, [] {});
     }
-    l += sum0 + sum1;
     tc_fence_before_sync();
     fence_proxy_async_smem();
     mbar_arrive(&sh.p_full[s]);
@@ -587,51 +630,37 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
   }
   const bool split = item.ws_row0 >= 0;
   if (!kRep) {
-    if (pair) {   // the row sum over all parts, added in group order
-      c.xbuf[wg * 128 + r] = l;
-      named_barrier_n(2 + quad, 32 * WG);
-      l = 0.f;
-#pragma unroll
-      for (int g = 0; g < WG; ++g) l += c.xbuf[g * 128 + r];
-      if (kChain) named_barrier_n(2 + quad, 32 * WG);   // the next item's first exchange reuses the slots
-    }
     // The TMEM loads are warp-wide (.sync.aligned): they sit in code every lane of the warp
     // runs, apart from anything that depends on the lane's row, and a warp barrier separates
     // them from the per-row stores so that the two cannot be merged into one divergent region.
     if (ok && works) {
-      uint32_t o[ND];
-      if (n_tiles > 0) {
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      __nv_bfloat16* const dst = p.out + (static_cast<size_t>(item.q_row0 + token) * p.hq + head) * kHeadDim;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        uint32_t o[64];
+        if (n_tiles > 0) {
+          load_columns(tmem_o + 64 * h, o);
+        } else {
 #pragma unroll
-        for (int c0 = 0; c0 < ND; c0 += 32) tmem_ld_32x32(tmem_o + c0, *reinterpret_cast<uint32_t(*)[32]>(&o[c0]));
-        tmem_ld_wait();
-      } else {
+          for (int i = 0; i < 64; ++i) o[i] = 0;
+        }
+        __syncwarp();
+        if (!split) {
+          float f[64];
 #pragma unroll
-        for (int i = 0; i < ND; ++i) o[i] = 0;
-      }
-      __syncwarp();
-      if (row_ok) {
-        if (split) {
-          float4* wdst = reinterpret_cast<float4*>(p.ws_o + static_cast<size_t>(item.ws_row0 + lr) * kHeadDim + d_lo);
-          if (wg == 0) p.ws_ml[item.ws_row0 + lr] = make_float2(m, l);
+          for (int i = 0; i < 64; ++i) f[i] = __uint_as_float(o[i]) * inv;
+          store_rows(f, sP + quad * 4096, row_ok ? dst + 64 * h : nullptr);
+        } else if (row_ok) {
+          float4* wdst = reinterpret_cast<float4*>(p.ws_o + static_cast<size_t>(item.ws_row0 + lr) * kHeadDim + 64 * h);
+          if (h == 0) p.ws_ml[item.ws_row0 + lr] = make_float2(m, l);
 #pragma unroll
-          for (int i = 0; i < ND / 4; ++i)
+          for (int i = 0; i < 16; ++i)
             wdst[i] = make_float4(__uint_as_float(o[4 * i]), __uint_as_float(o[4 * i + 1]), __uint_as_float(o[4 * i + 2]),
                                   __uint_as_float(o[4 * i + 3]));
-        } else {
-          const float inv = l > 0.f ? 1.f / l : 0.f;
-          uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(item.q_row0 + token) * p.hq + head) * kHeadDim +
-                                                d_lo);
-#pragma unroll
-          for (int q = 0; q < ND / 8; ++q) {
-            __nv_bfloat162 h[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              h[i] = __floats2bfloat162_rn(__uint_as_float(o[8 * q + 2 * i]) * inv, __uint_as_float(o[8 * q + 2 * i + 1]) * inv);
-            dst[q] = *reinterpret_cast<const uint4*>(h);
-          }
         }
+        __syncwarp();
       }
-      __syncwarp();
     }
     return;
   }
@@ -722,7 +751,6 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
 
 // The MMA role of such an item (the whole warp, one elected lane issues).  S of tile j + 2 is issued before
 // P V of tile j: it needs the S buffer (s_free), not P.
-template <bool kChain>
 __device__ __forceinline__ void attn_mma_alt(const AttnWork& p, const AttnCtx& c) {
   AttnShared& sh = *c.sh;
   volatile int* abort_flag = c.abort_flag;
@@ -744,7 +772,7 @@ __device__ __forceinline__ void attn_mma_alt(const AttnWork& p, const AttnCtx& c
     if (!mbar_wait_bounded(&sh.k_full[s], attn_parity(c, j), abort_flag, kAttnWaitNs)) return attn_gave_up(sh, kAttnSiteMmaK);
     if (leader) attn_note(c, j, kAttnSiteMmaSFree);
     const uint32_t uses = c.base[s] + (j >> 1);   // the buffer's previous tile has been read into registers
-    if ((kChain ? uses > 0 : j >= 2) && !mbar_wait_bounded(&c.s_free[s], (uses - 1) & 1u, abort_flag, kAttnWaitNs))
+    if (uses > 0 && !mbar_wait_bounded(&c.s_free[s], (uses - 1) & 1u, abort_flag, kAttnWaitNs))
       return attn_gave_up(sh, kAttnSiteMmaSFree);
     tc_fence_after_sync();
     const uint32_t k_addr = smem_u32(sK + s * kTileBytes);
@@ -754,11 +782,11 @@ __device__ __forceinline__ void attn_mma_alt(const AttnWork& p, const AttnCtx& c
         umma_bf16(tmem_base + s * 128, desc_kmajor(q_addr, i), desc_k_tile(k_addr, i), idesc_s, i != 0);
       umma_commit(&sh.s_full[s]);
       umma_commit(&sh.k_empty[s]);
-      if (kChain && j == n_tiles - 1) umma_commit(c.q_empty);
+      if (j == n_tiles - 1) umma_commit(c.q_empty);
     }
     return true;
   };
-  if (kChain && ok && n_tiles == 0 && leader) mbar_arrive(c.q_empty);
+  if (ok && n_tiles == 0 && leader) mbar_arrive(c.q_empty);
   if (ok && n_tiles > 0) ok = mma_s(0);
   if (ok && n_tiles > 1) ok = mma_s(1);
   for (int j = 0; ok && j < n_tiles; ++j) {
@@ -791,7 +819,6 @@ __device__ __forceinline__ void attn_mma_alt(const AttnWork& p, const AttnCtx& c
 // The softmax / output role of such an item: group `wg` of two.  `ml`: float2 [2][128] for the (max, sum) exchange.
 // Every thread passes the quadrant barrier once and the barrier of all softmax threads once per item, whatever
 // else happens.
-template <bool kChain>
 __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c, int wg, float2* ml) {
   AttnShared& sh = *c.sh;
   volatile int* abort_flag = c.abort_flag;
@@ -845,35 +872,8 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
     }
     const int key0 = item.key_begin + j * kKeysPerTile;
     const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, kKeysPerTile) : 0;   // keys [0, lim) of the tile count
-    uint32_t v[64];
-    // pass 1: the row maximum (the scale is positive: the maximum of the scaled scores is the scaled maximum)
-    float mx0 = -1e30f, mx1 = -1e30f, mx2 = -1e30f, mx3 = -1e30f;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      __syncwarp();
-      tmem_ld_32x32(tmem_s + 64 * h, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-      tmem_ld_32x32(tmem_s + 64 * h + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
-      tmem_ld_wait();
-      const int lh = lim - 64 * h;
-      if (lh >= 64) {
-#pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          mx0 = fmaxf(mx0, __uint_as_float(v[i]));
-          mx1 = fmaxf(mx1, __uint_as_float(v[i + 1]));
-          mx2 = fmaxf(mx2, __uint_as_float(v[i + 2]));
-          mx3 = fmaxf(mx3, __uint_as_float(v[i + 3]));
-        }
-      } else if (lh > 0) {
-#pragma unroll
-        for (int i = 0; i < 64; i += 4) {
-          mx0 = fmaxf(mx0, i < lh ? __uint_as_float(v[i]) : -1e30f);
-          mx1 = fmaxf(mx1, i + 1 < lh ? __uint_as_float(v[i + 1]) : -1e30f);
-          mx2 = fmaxf(mx2, i + 2 < lh ? __uint_as_float(v[i + 2]) : -1e30f);
-          mx3 = fmaxf(mx3, i + 3 < lh ? __uint_as_float(v[i + 3]) : -1e30f);
-        }
-      }
-    }
-    float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3));
+    // the row maximum (the scale is positive: the maximum of the scaled scores is the scaled maximum)
+    float mx = row_max(tmem_s, lim);
     mx = mx > -1e30f ? mx * p.scale_log2 : -1e30f;
     mx = fmaxf(mx, m);
     lap(1);
@@ -909,59 +909,11 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
       ok = attn_gave_up(sh, kAttnSiteSmaxPFree);
       break;
     }
-    const float neg_mx = -mx;
-    float sum0 = 0.f, sum1 = 0.f;
-    // pass 2: P = exp2(s - max) as bf16 into shared memory (K-major, 128-byte swizzle); row sum of the rounded P
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      __syncwarp();
-      tmem_ld_32x32(tmem_s + 64 * h, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
-      tmem_ld_32x32(tmem_s + 64 * h + 32, *reinterpret_cast<uint32_t(*)[32]>(&v[32]));
-      tmem_ld_wait();
-      if (h == 1) {   // S has been read for the last time: the MMA warp may overwrite it
-        tc_fence_before_sync();
-        mbar_arrive(&c.s_free[s]);
-      }
-      const int lh = lim - 64 * h;
-      uint8_t* row_base = p_tile + h * kHalfBytes + r * 128;
-#pragma unroll
-      for (int c0 = 0; c0 < 64; c0 += 32) {
-        uint32_t packed[16];
-        if (c0 + 32 <= lh) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float p0 = fast_exp2(fmaf(__uint_as_float(v[c0 + i]), p.scale_log2, neg_mx));
-            const float p1 = fast_exp2(fmaf(__uint_as_float(v[c0 + i + 1]), p.scale_log2, neg_mx));
-            const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
-            const uint32_t u = *reinterpret_cast<const uint32_t*>(&b);
-            sum0 += __uint_as_float(u << 16);
-            sum1 += __uint_as_float(u & 0xffff0000u);
-            packed[i >> 1] = u;
-          }
-        } else if (lh <= c0) {   // every key of the chunk is masked (half of a diagonal tile, on average)
-#pragma unroll
-          for (int i = 0; i < 16; ++i) packed[i] = 0;
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const float p0 = c0 + i < lh ? fast_exp2(fmaf(__uint_as_float(v[c0 + i]), p.scale_log2, neg_mx)) : 0.f;
-            const float p1 = c0 + i + 1 < lh ? fast_exp2(fmaf(__uint_as_float(v[c0 + i + 1]), p.scale_log2, neg_mx)) : 0.f;
-            const __nv_bfloat162 b = __floats2bfloat162_rn(p0, p1);
-            const uint32_t u = *reinterpret_cast<const uint32_t*>(&b);
-            sum0 += __uint_as_float(u << 16);
-            sum1 += __uint_as_float(u & 0xffff0000u);
-            packed[i >> 1] = u;
-          }
-        }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int chunk = (c0 >> 3) + q;
-          *reinterpret_cast<uint4*>(row_base + ((chunk ^ (r & 7)) << 4)) =
-              make_uint4(packed[4 * q], packed[4 * q + 1], packed[4 * q + 2], packed[4 * q + 3]);
-        }
-      }
-    }
-    l += sum0 + sum1;
+    // P = exp2(s - max) as bf16 into shared memory (K-major, 128-byte swizzle); row sum of the rounded P
+    l += row_weights(tmem_s, lim, p.scale_log2, -mx, p_tile + r * 128, r & 7, [&] {
+      tc_fence_before_sync();
+      mbar_arrive(&c.s_free[s]);   // S has been read for the last time: the MMA warp may overwrite it
+    });
     tc_fence_before_sync();
     fence_proxy_async_smem();
     mbar_arrive(&sh.p_full[s]);
@@ -1006,9 +958,9 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
   // nobody goes on to the next item (whose MMAs overwrite the accumulators, and whose exchange reuses `ml`)
   // before every thread has read both
   named_barrier_n(6, 256);
-  if (ok && row_ok) {
-    const bool split = item.ws_row0 >= 0;
-    if (split) {
+  if (!ok || !works) return;
+  if (item.ws_row0 >= 0) {   // one part of a split
+    if (row_ok) {
       float4* wdst = reinterpret_cast<float4*>(p.ws_o + static_cast<size_t>(item.ws_row0 + r) * kHeadDim + d_lo);
       if (wg == 0) p.ws_ml[item.ws_row0 + r] = make_float2(M, L);
 #pragma unroll
@@ -1017,21 +969,15 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
                               __uint_as_float(oa[4 * i + 1]) * wa + __uint_as_float(ob[4 * i + 1]) * wb,
                               __uint_as_float(oa[4 * i + 2]) * wa + __uint_as_float(ob[4 * i + 2]) * wb,
                               __uint_as_float(oa[4 * i + 3]) * wa + __uint_as_float(ob[4 * i + 3]) * wb);
-    } else {
-      const float inv = L > 0.f ? 1.f / L : 0.f;
-      const float fa = wa * inv, fb = wb * inv;
-      uint4* dst = reinterpret_cast<uint4*>(p.out + (static_cast<size_t>(item.q_row0 + token) * p.hq + head) * kHeadDim + d_lo);
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        __nv_bfloat162 h[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          h[i] = __floats2bfloat162_rn(
-              __uint_as_float(oa[8 * q + 2 * i]) * fa + __uint_as_float(ob[8 * q + 2 * i]) * fb,
-              __uint_as_float(oa[8 * q + 2 * i + 1]) * fa + __uint_as_float(ob[8 * q + 2 * i + 1]) * fb);
-        dst[q] = *reinterpret_cast<const uint4*>(h);
-      }
     }
+  } else {
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    const float fa = wa * inv, fb = wb * inv;
+    float f[64];
+#pragma unroll
+    for (int i = 0; i < 64; ++i) f[i] = __uint_as_float(oa[i]) * fa + __uint_as_float(ob[i]) * fb;
+    store_rows(f, p_tile + quad * 4096,
+               row_ok ? p.out + (static_cast<size_t>(item.q_row0 + token) * p.hq + head) * kHeadDim + d_lo : nullptr);
   }
 }
 

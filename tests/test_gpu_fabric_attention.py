@@ -75,6 +75,47 @@ def test_attention_items_in_fabric(fab, hq, hkv, page, part_tiles):
         row += n
 
 
+@pytest.mark.parametrize("hq,hkv,page,part_tiles", [(32, 4, 16, 1 << 30), (16, 2, 8, 1 << 30), (16, 8, 64, 4)])
+def test_items_behind_one_another(fab, hq, hkv, page, part_tiles):
+    """Several items for every worker in an order without order: prompts, whose items follow one another without a wait, quad-replicated
+    items of a few rows and parts of split ones between them, key tiles from one to ten, last blocks of a few rows."""
+    lens = [900, 130, 1237, 65, 700, 1100, 1, 640, 333, 1300]
+    rows = [900, 130, 700, 2, 650, 1, 1, 515, 3, 1200]
+    kc, vc, bt, _ = make_cache(lens, hkv, page, seed=hq + page)
+    q = torch.randn(sum(rows), hq, 128, generator=torch.Generator().manual_seed(7)).to(torch.bfloat16).cuda()
+    req_info, row = [], 0
+    for n, L in zip(rows, lens):
+        req_info.append((row, L - n, n, L))
+        row += n
+    kcd, vcd, btd = kc.cuda(), vc.cuda(), bt.cuda()
+    out = torch.zeros_like(q)
+    items, merge, ws_rows = plan_items(req_info, hq, hkv, part_tiles=part_tiles)
+    items = items[torch.randperm(items.shape[0], generator=torch.Generator().manual_seed(1))]
+    ws = torch.zeros(max(ws_rows, 1) * 130, dtype=torch.float32, device="cuda")
+    q_map, q_small, k_map, v_map = fabric_maps(fab, q, kcd, vcd)
+    args = torch.frombuffer(bytearray(pack(
+        "AttnArgs", q_map=q_map, k_map=k_map, v_map=v_map, out=out, ws_o=ws, ws_m=ws.data_ptr() + ws_rows * 512,
+        block_table=btd, scale_log2=SCALE_LOG2, bt_stride=btd.shape[1], hq=hq, hkv=hkv, group=hq // hkv,
+        page_size=page, q_map_small=q_small)), dtype=torch.uint8).cuda()
+    tiles, merges = fabric_tiles(items, merge, args.data_ptr())
+    p = Program()
+    s_attn = p.stage(tiles)
+    s_merge = p.stage(merges)
+    p.after(s_attn, s_merge)
+    run(fab, p, s_attn)
+    alone = paged_attention(q, kcd, vcd, btd, req_info, part_tiles=part_tiles).float()
+    assert (out.float() - alone).abs().max().item() < 4e-3   # as above
+    row = 0
+    for i, (n, L) in enumerate(zip(rows, lens)):   # a request against torch in 64 bits: P in 16 bits is 2^-9 of each weight
+        pages = btd[i, :-(-L // page)].long()
+        k, v = (t[pages].flatten(0, 1)[:L].double().repeat_interleave(hq // hkv, 1) for t in (kcd, vcd))
+        s = torch.einsum("nhd,mhd->hnm", q[row:row + n].double(), k) * 128 ** -0.5
+        later = torch.arange(L, device="cuda")[None] > L - n + torch.arange(n, device="cuda")[:, None]
+        want = torch.einsum("hnm,mhd->nhd", s.masked_fill(later, -float("inf")).softmax(-1), v)
+        assert float((out[row:row + n].double() - want).norm() / want.norm()) < 8e-3, i   # and the result's own 2^-9
+        row += n
+
+
 @pytest.mark.parametrize("hq,hkv,chunk_keys", [(32, 4, 0), (32, 4, 1024), (96, 8, 0)])
 def test_decode_plan_tile(fab, hq, hkv, chunk_keys):
     """The per-step plan of the decode attention (kind 44): from req_info = {row, position, 1, keys}
