@@ -1485,6 +1485,7 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
         if (tid == 0) sh.wait_ctx[2] = role_ctx(n, aq, ab);
         if (c.rep) softmax_role<true, 1, 1>(w.attn, c, 0);
         else softmax_role<false, 1, 1>(w.attn, c, 0);
+        fence_proxy_async_smem();   // output rows and merges go through the ring's memory: before the next record's TMA writes
         attn_advance(c.n_tiles, aq, ab);
       } else if (w.is_gemm) {
         // The exec warps follow the operand ring like the producer and the MMA warp do: for e4m3
