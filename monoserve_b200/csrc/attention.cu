@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attention_kernel(const 
       attn_derive(w, c);
       attn_produce(w, c);
       attn_advance(c.n_tiles, c.q_phase, c.base);
-      if (*abort_flag) break;
+      if (__any_sync(0xffffffffu, *abort_flag != 0)) break;   // the warp goes on, or leaves, as one
     }
     // a CTA that gives up still makes its failing claim, so that the counter ends at 0 for the slot's next launch
     if (!list_ended && lane == 0)
@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attention_kernel(const 
         softmax_alt(w, c, (warp - 2) >> 2, xbuf);
       }
       attn_advance(c.n_tiles, c.q_phase, c.base);
-      if (warp == 1 && *abort_flag) break;   // the softmax threads decide at the top of the loop
+      if (warp == 1 && __any_sync(0xffffffffu, *abort_flag != 0)) break;   // the softmax threads decide at the top of the loop
     }
   }
 

@@ -311,7 +311,7 @@ __device__ __forceinline__ void tma_load_3d_plain(void* smem, const void* map, u
 // warp-wide TMEM instructions that follow are never reached by a part of a warp.
 __device__ __forceinline__ bool warp_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           unsigned long long budget_ns) {
-  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, budget_ns));
+  return mbar_wait_warp(bar, parity, abort_flag, budget_ns);
 }
 
 // The TMA producer role: the whole warp calls it.

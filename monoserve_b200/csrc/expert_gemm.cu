@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
     GemmInflight inflight;
     for (int it = 0;; ++it) {
       const int slot = it % kWorkSlots;
-      if (!mbar_wait_bounded(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
+      if (!mbar_wait_warp(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
       if (!sh.work[slot].valid) break;
       trace_ev(p, 1, it, 0);
       if (!gemm_produce<false>(sh.work[slot], ring, sh.bar, pipe, inflight, abort_flag, pol_w, pol_x)) break;
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
     for (int it = 0;; ++it) {
       const int slot = it % kWorkSlots;
       const long long tw = own ? clock64() : 0;
-      if (!mbar_wait_bounded(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
+      if (!mbar_wait_warp(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
       if (own) sum_work += clock64() - tw;
       if (!sh.work[slot].valid) break;
       trace_ev(p, 2, it, 0);
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
     const int row = threadIdx.x - 7 * 32;
     for (int it = 0;; ++it) {
       const int slot = it % kWorkSlots;
-      if (!mbar_wait_bounded(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
+      if (!mbar_wait_warp(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
       if (!sh.work[slot].valid) break;
       if (!gemm_convert(sh.work[slot], ring, sh.bar, pipe, row, abort_flag)) break;
       __syncwarp();
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(FP8 ? kGemmThreadsFp8 : kGemmThreads, 1)
     uint32_t g = 0;
     for (int it = 0;; ++it) {
       const int slot = it % kWorkSlots;
-      if (!mbar_wait_bounded(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
+      if (!mbar_wait_warp(&sh.work_full[slot], (it / kWorkSlots) & 1, abort_flag, kWaitBudgetNs)) break;
       if (!sh.work[slot].valid) break;
       const GemmWork w = sh.work[slot];
       __syncwarp();

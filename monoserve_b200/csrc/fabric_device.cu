@@ -1397,7 +1397,7 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
     uint32_t aq = 0, ab[2] = {0, 0};   // phases the attention barriers have completed
     for (uint32_t n = 0;; ++n) {
       const int s = n % kSlots;
-      if (!mbar_wait_bounded(&sh.slot_full[s], (n / kSlots) & 1, abort_flag, kForever)) break;
+      if (!mbar_wait_warp(&sh.slot_full[s], (n / kSlots) & 1, abort_flag, kForever)) break;
       const WorkSlot& w = sh.slot[s];
       if (w.cmd == kCmdExit) break;
       bool ok = true;
@@ -1439,7 +1439,7 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
     uint32_t aq = 0, ab[2] = {0, 0};
     for (uint32_t n = 0;; ++n) {
       const int s = n % kSlots;
-      if (!mbar_wait_bounded(&sh.slot_full[s], (n / kSlots) & 1, abort_flag, kForever)) break;
+      if (!mbar_wait_warp(&sh.slot_full[s], (n / kSlots) & 1, abort_flag, kForever)) break;
       const WorkSlot& w = sh.slot[s];
       if (w.cmd == kCmdExit) break;
       bool ok = true;
@@ -1469,7 +1469,7 @@ __global__ void __launch_bounds__(kWorkerThreads, 1) fabric_kernel(DeviceState* 
     GemmPipe conv_pipe;
     for (uint32_t n = 0;; ++n) {
       const int s = n % kSlots;
-      if (!mbar_wait_bounded(&sh.slot_full[s], (n / kSlots) & 1, abort_flag, kForever)) break;
+      if (!mbar_wait_warp(&sh.slot_full[s], (n / kSlots) & 1, abort_flag, kForever)) break;
       const WorkSlot& w = sh.slot[s];
       if (w.cmd == kCmdExit) break;
       if (tid == 0) {

@@ -243,13 +243,12 @@ __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, G
     // room in the ring and a free barrier pair: retire the oldest stages as needed
     while (pipe.i - fl.tail >= kGemmStages ||
            (pipe.i != fl.tail && ve - fl.tail_vbegin > kRingBytes)) {
-      if (!mbar_wait_bounded(&bar.empty[fl.tail_slot], fl.tail_parity, abort_flag, kWaitBudgetNs)) return false;
+      if (!mbar_wait_warp(&bar.empty[fl.tail_slot], fl.tail_parity, abort_flag, kWaitBudgetNs)) return false;
       ++fl.tail;
       if (++fl.tail_slot == kGemmStages) {
         fl.tail_slot = 0;
         fl.tail_parity ^= 1;
       }
-      // also where the warp meets behind the wait: a lane still in it when the stage is filled and freed again would miss the phase
       fl.tail_vbegin = __shfl_sync(0xffffffffu, fl.vbegin, fl.tail_slot);
     }
     const uint32_t slot = pipe.slot;
@@ -444,7 +443,7 @@ __device__ __forceinline__ bool gemm_convert(const GemmWork& w, uint8_t* ring, G
   for (int kt = 0; kt < n_stages; ++kt) {
     uint32_t vb, ve;
     const uint32_t phys = pipe.alloc(size, vb, ve);
-    if (!mbar_wait_bounded(&bar.full[pipe.slot], pipe.parity, abort_flag, kWaitBudgetNs)) return false;
+    if (!mbar_wait_warp(&bar.full[pipe.slot], pipe.parity, abort_flag, kWaitBudgetNs)) return false;
     // The row's raw bytes [64 h, 64 h + 64) are K step h.  The thread reads its whole row before it
     // writes (the second K step's output overwrites the raw row), starting at 16-byte chunk t & 7 so
     // that the eight threads of a shared-memory phase read eight different bank groups.
@@ -929,7 +928,7 @@ __device__ __forceinline__ bool gemm_epilogue_body(const GemmWork& w, int slice,
                                                    uint32_t buf, uint32_t acc_parity, volatile int* abort_flag, uint8_t* ring,
                                                    unsigned long long* acc_seen = nullptr) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, quad = warp & 3;
-  if (!mbar_wait_bounded(&bar.acc_full[buf], acc_parity, abort_flag, kWaitBudgetNs)) return false;
+  if (!mbar_wait_warp(&bar.acc_full[buf], acc_parity, abort_flag, kWaitBudgetNs)) return false;
   tc_fence_after_sync();
   if (acc_seen && lane == 0) *acc_seen = globaltimer_ns();
   if (kFetch && w.fetch) {   // nothing to drain: the MMA warp has already moved the bytes

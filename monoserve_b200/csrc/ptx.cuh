@@ -96,6 +96,12 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
 }
 
+// The same by the whole warp, which goes on or gives up as one: left to each lane, one may see the phase and another the abort flag, and
+// a lane that leaves alone is missed by the next operation that names all 32.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned long long budget_ns) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, budget_ns));
+}
+
 // --------------------------------------------------------------------- TMA
 __device__ __forceinline__ void prefetch_tensormap(const void* map) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");

@@ -1,9 +1,14 @@
 """A host model of the operand ring's barriers as the MMA warp of the GEMM tiles sees them (gemm_mma in
 monoserve_b200/csrc/gemm_core.cuh): the producer fills stages, every lane of the warp waits for a stage by the parity of its use, and one
-lane frees it.  The lanes may run apart between the points where the warp meets; the model lets them, at random."""
+lane frees it.  The lanes may run apart between the points where the warp meets; the model lets them, at random.  A second model has
+a warp whose waits are given up: the abort flag goes up at any moment, and every lane has to get out of its loop."""
+import os
 import random
+import re
 
 import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "monoserve_b200", "csrc")
 
 STAGES, LANES = 12, 4
 
@@ -64,13 +69,73 @@ def test_a_lane_that_does_not_meet_the_others_may_miss_a_phase():
 
 
 def test_the_loops_of_the_mma_warp_meet_behind_each_wait():
-    import os
-    import re
-    path = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "monoserve_b200", "csrc", "gemm_core.cuh")
-    text = open(path).read()
+    text = open(os.path.join(CSRC, "gemm_core.cuh")).read()
     for name in ("gemm_mma_two", "gemm_mma"):
         body = text[re.search(rf"__device__ __forceinline__ bool {name}\(", text).start():]
         body = body[:body.index("\n}\n")]
         loop = body[body.index("for (int kt = 0;"):]
         assert re.search(r"mbar_wait_bounded\(&\w+(\.full)?\[pipe\.slot\][^;]*;\s*(//[^\n]*\s*)*__syncwarp\(\);", loop), name
         assert "break" not in loop, name   # a lane that leaves alone would leave the others waiting at the meeting
+
+
+def give_up(seed, combined):
+    """Lanes that wait for stages, each trying the barrier and then looking at the abort flag, and meet behind each wait.  True: all have
+    left the loop.  `combined`: a lane's answer counts once all lanes have one, and all take the same."""
+    rnd = random.Random(seed)
+    n_stages, aborted = 12, rnd.randrange(400)
+    step, filled = [0], [0]
+    answers = [[None] * LANES for _ in range(n_stages)]
+    met, left = [0] * LANES, []
+
+    def lane(who):
+        for i in range(n_stages):
+            while True:
+                if filled[0] > i:
+                    got = True
+                    break
+                yield None                       # the try and the look at the flag are two steps
+                if step[0] >= aborted:
+                    got = False
+                    break
+                yield None
+            answers[i][who] = got
+            if combined:
+                yield lambda: None not in answers[i]
+                got = all(answers[i])
+            if not got:
+                break
+            met[who] = i + 1                     # an operation that names all 32 lanes
+            yield lambda: min(met) > i
+        left.append(who)
+
+    roles = [lane(k) for k in range(LANES)]
+    want = {k: None for k in range(LANES)}
+    for step[0] in range(4000):
+        if step[0] < aborted and rnd.random() < 0.05:
+            filled[0] += 1
+        ready = [k for k, w in want.items() if w is None or w()]
+        if not ready:
+            continue
+        k = rnd.choice(ready)
+        try:
+            want[k] = next(roles[k])
+        except StopIteration:
+            del want[k]
+    return len(left) == LANES
+
+
+def test_a_warp_gives_up_as_one():
+    assert all(give_up(seed, combined=True) for seed in range(200))
+    assert not all(give_up(seed, combined=False) for seed in range(200))
+
+
+def test_no_lane_leaves_a_wait_of_its_warp_alone():
+    """A return or a break right behind a wait that each lane decides for itself, anywhere but in code of one lane (the schedulers) and
+    in roles that only set a flag and go on (attention's MMA warps, which meet at their end)."""
+    alone = re.compile(r"if \([^;{}]*!mbar_wait_bounded\([^;{}]*\)\)\s*(return false|break);")
+    for name in ("gemm_core.cuh", "expert_gemm.cu", "fabric_device.cu", "attention.cu"):
+        text = open(os.path.join(CSRC, name)).read()
+        found = [m.group(0) for m in alone.finditer(text)]
+        assert [f for f in found if "work_empty" not in f] == [], name
+    attention = open(os.path.join(CSRC, "attention.cu")).read()
+    assert not re.search(r"\(\*abort_flag\) break|&& \*abort_flag\) break", attention)
