@@ -159,13 +159,17 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Scores of keys past the visible ones, the first `lim`, are as low as can be: they are no maximum and their exponential is zero.
+// Scores of keys past the visible ones, the first `lim`, become `masked`: as low as can be for a maximum, and for the weights the
+// infinity that the scale takes to minus infinity, whose exponential is zero.
+constexpr uint32_t kNegInf = 0xff800000u, kPosInf = 0x7f800000u;
 template <int NC>
-__device__ __forceinline__ void mask_scores(uint32_t (&v)[NC], int lim) {
+__device__ __forceinline__ void mask_scores(uint32_t (&v)[NC], int lim, uint32_t masked) {
   if (lim >= NC) return;
 #pragma unroll
-  for (int i = 0; i < NC; ++i) v[i] = i < lim ? v[i] : 0xff800000u;
+  for (int i = 0; i < NC; ++i) v[i] = i < lim ? v[i] : masked;
 }
+// A scale of zero as the least normal number, with which finite scores weigh the same: zero times an infinite score would be no number.
+__device__ __forceinline__ float attn_scale(float scale) { return scale == 0.f ? 1.17549435e-38f : scale; }
 template <int NC>
 __device__ __forceinline__ float max_scores(const uint32_t (&v)[NC], float mx) {   // four chains
   float m[4] = {mx, mx, mx, mx};
@@ -209,7 +213,7 @@ __device__ __forceinline__ float row_max(uint32_t tmem_s, int lim) {
   for (int h = 0; h < 2; ++h) {
     uint32_t v[64];
     load_columns(tmem_s + 64 * h, v);
-    mask_scores(v, lim - 64 * h);
+    mask_scores(v, lim - 64 * h, kNegInf);
     mx = max_scores(v, mx);
   }
   return mx;
@@ -218,6 +222,7 @@ __device__ __forceinline__ float row_max(uint32_t tmem_s, int lim) {
 template <class Read>
 __device__ __forceinline__ float row_weights(uint32_t tmem_s, int lim, float scale, float neg_mx, uint8_t* row, int swz, Read read) {
   float sum0 = 0.f, sum1 = 0.f;
+  const uint32_t masked = scale < 0.f ? kPosInf : kNegInf;
 #pragma unroll 1
   for (int c0 = 0; c0 < kKeysPerTile; c0 += 32) {
     uint32_t v[32];
@@ -228,7 +233,7 @@ __device__ __forceinline__ float row_weights(uint32_t tmem_s, int lim, float sca
     uint8_t* const to = row + (c0 >> 6) * kHalfBytes;
     const int piece = (c0 & 32) >> 3;
     if (lim > c0) {
-      mask_scores(v, lim - c0);
+      mask_scores(v, lim - c0, masked);
       store_weights(v, scale, neg_mx, to, piece, swz, sum0, sum1);
     } else {   // every key is masked
 #pragma unroll
@@ -554,13 +559,14 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, NC) : 0;
     if (!ok) continue;   // a wait gave up
     uint32_t v[32];   // of a quad-replicated item: the thread's quarter of the row
-    // the scale is positive: the maximum of the scaled scores is the scaled maximum
+    // with a positive scale the maximum of the scaled scores is the scaled maximum; with a negative one it is a reference point as good
+    // as any while the exponentials are finite
     float mx;
     if constexpr (kRep) {
       __syncwarp();
       tmem_ld_32x32(tmem_s, v);
       tmem_ld_wait();
-      mask_scores(v, lim);
+      mask_scores(v, lim, kNegInf);
       mx = max_scores(v, -1e30f);
     } else {
       mx = row_max(tmem_s, lim);
@@ -607,6 +613,7 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     uint8_t* const p_row = sP + (j % PB) * kTileBytes + r * 128;
     if constexpr (kRep) {
       float sum0 = 0.f, sum1 = 0.f;
+      if (p.scale_log2 < 0.f) mask_scores(v, lim, kPosInf);
       store_weights(v, p.scale_log2, neg_mx, p_row + (c_lo >> 6) * kHalfBytes, (c_lo & 63) >> 3, r & 7, sum0, sum1);
       l += sum0 + sum1;
     } else {
@@ -873,7 +880,7 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
     }
     const int key0 = item.key_begin + j * kKeysPerTile;
     const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, kKeysPerTile) : 0;   // keys [0, lim) of the tile count
-    // the row maximum (the scale is positive: the maximum of the scaled scores is the scaled maximum)
+    // the row maximum (as in softmax_role)
     float mx = row_max(tmem_s, lim);
     mx = mx > -1e30f ? mx * p.scale_log2 : -1e30f;
     mx = fmaxf(mx, m);

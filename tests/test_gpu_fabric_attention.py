@@ -116,6 +116,49 @@ def test_items_behind_one_another(fab, hq, hkv, page, part_tiles):
         row += n
 
 
+@pytest.mark.parametrize("scale", [0.0, -0.03, 1e-30, 0.2])
+@pytest.mark.parametrize("hq,hkv,part_tiles", [(32, 4, 4), (16, 8, 1 << 30)])
+def test_any_scale(fab, monkeypatch, hq, hkv, part_tiles, scale):
+    """Masked keys have no weight whatever the scale's sign, in tiles with none, some and all of their keys masked, whole and split items,
+    prompts and quad-replicated rows, on the fabric and alone; a scale of zero weighs all visible keys alike."""
+    from monoserve_b200 import attention
+    page, lens, rows = 16, [300, 777, 1000, 1025], [300, 700, 1, 3]
+    kc, vc, bt, _ = make_cache(lens, hkv, page, seed=hq)
+    q = torch.randn(sum(rows), hq, 128, generator=torch.Generator().manual_seed(3)).to(torch.bfloat16).cuda()
+    req_info, row = [], 0
+    for n, L in zip(rows, lens):
+        req_info.append((row, L - n, n, L))
+        row += n
+    kcd, vcd, btd = kc.cuda(), vc.cuda(), bt.cuda()
+    scale_log2 = scale * 1.4426950408889634
+    monkeypatch.setattr(attention, "SCALE_LOG2", scale_log2)
+    alone = paged_attention(q, kcd, vcd, btd, req_info, part_tiles=part_tiles)
+    out = torch.zeros_like(q)
+    items, merge, ws_rows = plan_items(req_info, hq, hkv, part_tiles=part_tiles)
+    ws = torch.zeros(max(ws_rows, 1) * 130, dtype=torch.float32, device="cuda")
+    q_map, q_small, k_map, v_map = fabric_maps(fab, q, kcd, vcd)
+    args = torch.frombuffer(bytearray(pack(
+        "AttnArgs", q_map=q_map, k_map=k_map, v_map=v_map, out=out, ws_o=ws, ws_m=ws.data_ptr() + ws_rows * 512,
+        block_table=btd, scale_log2=scale_log2, bt_stride=btd.shape[1], hq=hq, hkv=hkv, group=hq // hkv,
+        page_size=page, q_map_small=q_small)), dtype=torch.uint8).cuda()
+    tiles, merges = fabric_tiles(items, merge, args.data_ptr())
+    p = Program()
+    s_attn = p.stage(tiles)
+    s_merge = p.stage(merges)
+    p.after(s_attn, s_merge)
+    run(fab, p, s_attn)
+    row = 0
+    for i, (n, L) in enumerate(zip(rows, lens)):
+        pages = btd[i, :-(-L // page)].long()
+        k, v = (t[pages].flatten(0, 1)[:L].double().repeat_interleave(hq // hkv, 1) for t in (kcd, vcd))
+        s = torch.einsum("nhd,mhd->hnm", q[row:row + n].double(), k) * scale
+        later = torch.arange(L, device="cuda")[None] > L - n + torch.arange(n, device="cuda")[:, None]
+        want = torch.einsum("hnm,mhd->nhd", s.masked_fill(later, -float("inf")).softmax(-1), v)
+        for got in (out, alone):   # P in 16 bits is 2^-9 of each weight, and the result's own 2^-9
+            assert float((got[row:row + n].double() - want).norm() / want.norm()) < 8e-3, i
+        row += n
+
+
 @pytest.mark.parametrize("hq,hkv,chunk_keys", [(32, 4, 0), (32, 4, 1024), (96, 8, 0)])
 def test_decode_plan_tile(fab, hq, hkv, chunk_keys):
     """The per-step plan of the decode attention (kind 44): from req_info = {row, position, 1, keys}
