@@ -366,7 +366,7 @@ __device__ __forceinline__ void release_stage(DeviceState& S, uint32_t lane_id, 
       Ring& R = L.ring[want == kLink ? 1 : 0];
       unsigned long long got = 0;
       if (lane == 0) got = atomicAdd(&R.reserve, static_cast<unsigned long long>(__popc(mask)));
-      else if (lane == 1) got = ld_volatile(&R.tail);
+      else if (lane == 1) got = ld_acq(&R.tail);   // the earlier publishers' entries go on with the release behind it
       const unsigned long long at = __shfl_sync(kWarp, got, 0), tail = __shfl_sync(kWarp, got, 1);
       if (fate == want) R.ids[(at + __popc(mask & ((1u << lane) - 1))) & (kRingCap - 1)] = word;
       __syncwarp();   // the stages' tags and words, by all lanes, are in front of lane 0's release

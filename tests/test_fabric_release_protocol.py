@@ -1,0 +1,117 @@
+"""Host models of what the fabric's scheduler (monoserve_b200/csrc/fabric_sched.cuh) orders with its loads, stores and atomics when a stage
+completes, on a memory in which a plain load may return any value a location has had since the last one its thread is bound to have
+seen: an acquire load takes over what the release store it reads was bound to, an atomic reads the newest value, a fence makes
+atomics before it acquire and atomics after it release.  Each rule of the device code is shown by leaving it out."""
+import os
+import random
+import re
+
+import pytest
+
+SCHED = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "monoserve_b200", "csrc", "fabric_sched.cuh")).read()
+
+
+def body_of(name):
+    text = SCHED[re.search(rf"\b{name}\(", SCHED).start():]
+    return text[:text.index("\n}\n")]
+
+
+class Memory:
+    def __init__(self, **init):
+        self.at = {k: [(v, {})] for k, v in init.items()}
+
+
+class Thread:
+    """Views are {location: index of the oldest value that may still be read}."""
+
+    def __init__(self, mem, rnd):
+        self.mem, self.rnd = mem, rnd
+        self.view, self.pending, self.released = {}, {}, {}
+
+    @staticmethod
+    def _join(a, b):
+        for k, i in b.items():
+            a[k] = max(a.get(k, 0), i)
+
+    def load(self, loc, acquire=False):
+        past = self.mem.at[loc]
+        i = self.rnd.randrange(self.view.get(loc, 0), len(past))
+        self.view[loc] = i
+        value, view = past[i]
+        self._join(self.view if acquire else self.pending, view)
+        return value
+
+    def _write(self, loc, value, view):
+        past = self.mem.at[loc]
+        self.view[loc] = len(past)
+        past.append((value, dict(view, **{loc: len(past)})))
+
+    def store(self, loc, value, release=False):
+        self._write(loc, value, self.view if release else self.released)
+
+    def atomic(self, loc, f, acquire=False):
+        value, view = self.mem.at[loc][-1]
+        self._join(self.view if acquire else self.pending, view)
+        merged = dict(self.released)
+        self._join(merged, view)   # an atomic goes on what it reads
+        self._write(loc, f(value), merged)
+        return value
+
+    def fence(self):
+        self._join(self.view, self.pending)
+        self.released = dict(self.view)
+
+
+def interleave(rnd, roles, limit=2000):
+    """Runs the generators at random until all are done; False: somebody is still waiting at the limit."""
+    roles = list(roles)
+    for _ in range(limit):
+        if not roles:
+            return True
+        r = rnd.choice(roles)
+        try:
+            next(r)
+        except StopIteration:
+            roles.remove(r)
+    return False
+
+
+# ------------------------------------------------------------------------------------------ the published tail of a ring
+def publish(th, entry, acquire):
+    at = th.atomic("reserve", lambda v: v + 1)
+    yield
+    tail = th.load("tail", acquire)     # beside the reservation
+    yield
+    th.store(f"id{at}", entry)
+    yield
+    while tail != at:                   # an earlier reservation is not published yet
+        tail = th.load("tail", acquire=True)
+        yield
+    th.store("tail", at + 1, release=True)
+
+
+def two_publishers(seed, acquire):
+    rnd = random.Random(seed)
+    mem = Memory(reserve=0, tail=0, id0=None, id1=None)
+    got = []
+
+    def worker():
+        th = Thread(mem, rnd)
+        tail = 0
+        while tail < 2:
+            tail = th.load("tail", acquire=True)
+            yield
+        got.extend(th.load(f"id{i}") for i in range(2))
+
+    assert interleave(rnd, [publish(Thread(mem, rnd), "a", acquire), publish(Thread(mem, rnd), "b", acquire), worker()])
+    return sorted(map(str, got)) == ["a", "b"]
+
+
+def test_a_later_publication_carries_the_earlier_one():
+    assert all(two_publishers(seed, acquire=True) for seed in range(500))
+    assert not all(two_publishers(seed, acquire=False) for seed in range(500))
+
+
+def test_every_load_of_a_published_tail_acquires():
+    assert re.search(r"ld_acq\(&R\.tail\)", body_of("release_stage"))
+    assert not re.search(r"ld_volatile\(&R\.tail\)", SCHED)
