@@ -362,6 +362,12 @@ int monofab_fabric_upload(monofab_fabric* f, const int64_t* tiles, int n_tiles, 
   uint8_t* base = f->pool;
   std::vector<StageRuntime> rt(n_stages);
   for (int s = 0; s < n_stages; ++s) rt[s] = StageRuntime{0ull, 0u, static_cast<unsigned int>(stages[8 * s + 4])};
+  std::vector<uint32_t> marked(n_succ);
+  for (int k = 0; k < n_succ; ++k) {
+    const int32_t* r = stages + 8 * succ[k];
+    const bool late = r[1] == 0 || (static_cast<uint32_t>(r[5]) & kStageSkip);
+    marked[k] = static_cast<uint32_t>(succ[k]) | (late ? kSuccLate : 0u) | (r[4] > 1 ? kSuccJoin : 0u);
+  }
   ProgramDesc d{};
   d.tiles = reinterpret_cast<TileDesc*>(base + rec.blocks[0]);
   d.stages = reinterpret_cast<StageStatic*>(base + rec.blocks[1]);
@@ -382,7 +388,7 @@ int monofab_fabric_upload(monofab_fabric* f, const int64_t* tiles, int n_tiles, 
   if (n_tiles) r = to_device(f, d.tiles, tiles, size_t(n_tiles) * 64);
   if (!r) r = to_device(f, d.stages, stages, size_t(n_stages) * 32);
   if (!r) r = to_device(f, d.runtime, rt.data(), size_t(n_stages) * 16);
-  if (!r) r = to_device(f, d.succ, succ, size_t(n_succ) * 4);
+  if (!r) r = to_device(f, d.succ, marked.data(), size_t(n_succ) * 4);
   if (!r) r = to_device(f, base + rec.blocks[4], &d, sizeof d);
   if (r) {
     for (int i = 0; i < 5; ++i) pool_free(f, rec.blocks[i], rec.sizes[i]);

@@ -48,6 +48,12 @@ template <class T>
 __device__ __forceinline__ T ld_volatile(const T* p) { return *reinterpret_cast<const volatile T*>(p); }
 __device__ __forceinline__ unsigned int ld_acq(const unsigned int* p) { return ld_acquire_gpu(p); }
 __device__ __forceinline__ unsigned long long ld_acq(const unsigned long long* p) { return ld_acquire_gpu64(p); }
+// The count before one is taken off; what the threads that took the others off had written, or knew of, is known here behind it.
+__device__ __forceinline__ unsigned int take_one_acq(unsigned int* p) {
+  unsigned int before;
+  asm volatile("atom.acquire.gpu.global.add.u32 %0, [%1], %2;" : "=r"(before) : "l"(p), "r"(0xffffffffu) : "memory");
+  return before;
+}
 __device__ __forceinline__ void st_rel(unsigned int* p, unsigned int v) { st_release_gpu(p, v); }
 __device__ __forceinline__ void st_rel(unsigned long long* p, unsigned long long v) {
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
@@ -333,7 +339,8 @@ __device__ __forceinline__ const ProgramDesc* close_iteration(DeviceState& S, ui
 // The WHOLE warp.  Counts down and arms the successors succ[first ..) of a completed stage, the 32 lanes side by side, and
 // publishes their ring words in two publications (ungated, link), so a stage with 128 successors releases them in a few
 // microseconds.  Each step is a round trip to the L2 that every stage of a program waits for, so what does not depend
-// on one another goes out together.
+// on one another goes out together: the record of a successor beside its count, unless a tile of the program writes that record
+// (kSuccLate) and may do so ahead of another predecessor than this one (kSuccJoin); then it is read behind the count.
 template <class WL>
 __device__ __forceinline__ void release_stage(DeviceState& S, uint32_t lane_id, StageStatic* stages, StageRuntime* runtime,
                                               const uint32_t* succs, uint32_t first, uint32_t count, uint32_t tag, bool tracing, WL& wl) {
@@ -344,10 +351,15 @@ __device__ __forceinline__ void release_stage(DeviceState& S, uint32_t lane_id, 
     int fate = kNone;
     uint32_t word = 0, succ = 0;
     if (base + lane < count) {
-      succ = ld_volatile(succs + first + base + lane);
+      const uint32_t entry = ld_volatile(succs + first + base + lane);
+      succ = entry & kStageMask;
+      uint32_t flags = ld_volatile(&stages[succ].flags), tiles = ld_volatile(&stages[succ].count);
       // a skipped stage is never armed, so that its count has no meaning
-      const unsigned int before = atomicSub(&runtime[succ].deps, 1u);
-      const uint32_t flags = ld_volatile(&stages[succ].flags), tiles = ld_volatile(&stages[succ].count);
+      const unsigned int before = take_one_acq(&runtime[succ].deps);
+      if (before == 1u && (entry & kSuccLate) && (entry & kSuccJoin)) {
+        flags = ld_volatile(&stages[succ].flags);
+        tiles = ld_volatile(&stages[succ].count);
+      }
       if (before == 1u && !(flags & kStageSkip)) {
         if (tracing) trace_stage(S, lane_id, succ, 0, tag);
         if (tiles == 0) {
@@ -372,7 +384,9 @@ __device__ __forceinline__ void release_stage(DeviceState& S, uint32_t lane_id, 
       __syncwarp();   // the stages' tags and words, by all lanes, are in front of lane 0's release
       if (lane == 0) ring_announce(S, R, at, __popc(mask), tail == at);
     }
-    for (unsigned mask = __ballot_sync(kWarp, fate == kEmpty); mask; mask &= mask - 1) {
+    const unsigned empty = __ballot_sync(kWarp, fate == kEmpty);
+    if (empty) __threadfence();   // what was acquired above goes on with the counts that these stages' completion takes from
+    for (unsigned mask = empty; mask; mask &= mask - 1) {
       const uint32_t v = __shfl_sync(kWarp, succ, __ffs(mask) - 1);
       if (lane == 0) wl.push(v);
     }

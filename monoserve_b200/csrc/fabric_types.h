@@ -79,6 +79,10 @@ enum StageFlags : uint32_t {
   kStageSkip = 1u << 3,   // out of this iteration
 };
 
+// Marks that an upload puts on the entries of a successor list (stage ids have 20 bits).
+constexpr uint32_t kSuccLate = 1u << 31;   // the stage was uploaded without tiles, or as skipped: a tile of the program may write its record
+constexpr uint32_t kSuccJoin = 1u << 30;   // it has several predecessors
+
 struct alignas(64) TileDesc {
   uint16_t kind;
   uint8_t lane;

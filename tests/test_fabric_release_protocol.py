@@ -115,3 +115,63 @@ def test_a_later_publication_carries_the_earlier_one():
 def test_every_load_of_a_published_tail_acquires():
     assert re.search(r"ld_acq\(&R\.tail\)", body_of("release_stage"))
     assert not re.search(r"ld_volatile\(&R\.tail\)", SCHED)
+
+
+# ------------------------------------------------------------------------------------------ a record written ahead of one predecessor
+def joined(seed, acquire, behind):
+    """A stage with two predecessors: a plan, which writes its tile count, and another stage; whoever completes last publishes it, with the
+    count read beside its own decrement or behind it.  True: every tile ran, with the operands that both have left."""
+    rnd = random.Random(seed)
+    mem = Memory(count=0, deps=2, tail=0, id0=None, from_plan=0, from_other=0)
+    ran = []
+
+    def complete(th):
+        th.fence()
+        tiles = th.load("count")
+        yield
+        before = th.atomic("deps", lambda v: v - 1, acquire)
+        yield
+        if before != 1:
+            return
+        if behind:
+            tiles = th.load("count")
+            yield
+        th.store("id0", tiles)
+        th.store("tail", 1, release=True)
+
+    def plan():
+        th = Thread(mem, rnd)
+        th.store("count", 3)
+        th.store("from_plan", 1)
+        yield
+        yield from complete(th)
+
+    def other():
+        th = Thread(mem, rnd)
+        th.store("from_other", 1)
+        yield
+        yield from complete(th)
+
+    def worker():
+        th = Thread(mem, rnd)
+        while not th.load("tail", acquire=True):
+            yield
+        ran.append((th.load("id0"), th.load("count"), th.load("from_plan"), th.load("from_other")))
+
+    assert interleave(rnd, [plan(), other(), worker()])
+    return ran == [(3, 3, 1, 1)]
+
+
+def test_the_last_decrement_sees_what_the_others_wrote():
+    assert all(joined(seed, acquire=True, behind=True) for seed in range(500))
+    assert not all(joined(seed, acquire=True, behind=False) for seed in range(500))
+    assert not all(joined(seed, acquire=False, behind=True) for seed in range(500))
+
+
+def test_the_release_of_a_stage_acquires_and_reads_late_records_behind():
+    text = body_of("release_stage")
+    assert "take_one_acq(&runtime[succ].deps)" in text and "atomicSub" not in text
+    assert "atom.acquire.gpu" in body_of("take_one_acq")
+    behind = text[text.index("take_one_acq"):]
+    assert re.search(r"kSuccLate\) && \(entry & kSuccJoin\)\) \{\s*flags = ld_volatile\(&stages\[succ\]\.flags\);\s*tiles = ld_volatile", behind)
+    assert re.search(r"if \(empty\) __threadfence\(\);", behind)   # stages that are complete at once pass on what was acquired
