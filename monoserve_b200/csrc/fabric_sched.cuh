@@ -353,9 +353,11 @@ __device__ __forceinline__ void release_stage(DeviceState& S, uint32_t lane_id, 
     if (base + lane < count) {
       const uint32_t entry = ld_volatile(succs + first + base + lane);
       succ = entry & kStageMask;
+      // a skipped stage keeps its count: one taken off late would be missed by the next iteration, whose end does not wait for it
+      uint32_t skip = 0;
+      if (entry & kSuccLate) skip = ld_volatile(&stages[succ].flags) & kStageSkip;
       uint32_t flags = ld_volatile(&stages[succ].flags), tiles = ld_volatile(&stages[succ].count);
-      // a skipped stage is never armed, so that its count has no meaning
-      const unsigned int before = take_one_acq(&runtime[succ].deps);
+      const unsigned int before = skip ? 0u : take_one_acq(&runtime[succ].deps);
       if (before == 1u && (entry & kSuccLate) && (entry & kSuccJoin)) {
         flags = ld_volatile(&stages[succ].flags);
         tiles = ld_volatile(&stages[succ].count);

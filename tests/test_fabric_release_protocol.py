@@ -175,3 +175,41 @@ def test_the_release_of_a_stage_acquires_and_reads_late_records_behind():
     behind = text[text.index("take_one_acq"):]
     assert re.search(r"kSuccLate\) && \(entry & kSuccJoin\)\) \{\s*flags = ld_volatile\(&stages\[succ\]\.flags\);\s*tiles = ld_volatile", behind)
     assert re.search(r"if \(empty\) __threadfence\(\);", behind)   # stages that are complete at once pass on what was acquired
+
+
+# ------------------------------------------------------------------------------------------ successors that are skipped
+def skipped(seed, asks_first):
+    """A stage releases two batches of successors, one that the iteration waits for and one that is skipped in it; the reset behind the
+    first rewrites the second's count.  True: the next iteration finds the count whole."""
+    rnd = random.Random(seed)
+    mem = Memory(flags=1, deps=1, tail=0)
+
+    def release():
+        th = Thread(mem, rnd)
+        th.store("tail", 1, release=True)       # the first batch
+        yield
+        if not (asks_first and th.load("flags")):
+            th.atomic("deps", lambda v: v - 1)
+        yield
+
+    def rest():
+        th = Thread(mem, rnd)
+        while not th.load("tail", acquire=True):
+            yield
+        th.store("deps", 1)                     # the reset tile
+        yield
+
+    assert interleave(rnd, [release(), rest()])
+    return mem.at["deps"][-1][0] == 1
+
+
+def test_a_skipped_stage_keeps_its_count():
+    assert all(skipped(seed, asks_first=True) for seed in range(200))
+    assert not all(skipped(seed, asks_first=False) for seed in range(200))
+
+
+def test_the_release_of_a_stage_asks_before_it_takes():
+    text = body_of("release_stage")
+    asks = re.search(r"if \(entry & kSuccLate\) skip = ld_volatile\(&stages\[succ\]\.flags\) & kStageSkip;", text)
+    takes = re.search(r"skip \? 0u : take_one_acq", text)
+    assert asks and takes and asks.start() < takes.start()
