@@ -228,20 +228,28 @@ __device__ __forceinline__ bool claim_tiles(const ProgView& V, uint32_t word, Pr
 // Consumer side, the WHOLE warp: lane i probes entry head + i; a run of exhausted entries at the
 // head is dropped with one compare-and-swap; the first entry that still has tiles is claimed.
 // head and tail come from one reading of both: a pair out of step only looks empty, or begins at
-// entries that are exhausted and fail the compare-and-swap.
-__device__ __forceinline__ bool ring_take(Ring& R, unsigned long long head, unsigned long long tail, const ProgView& V, Claim& c) {
+// entries that are exhausted and fail the compare-and-swap.  V comes from the same reading, whose words are not ordered among
+// themselves: against the tables of a program that the lane ran before, entries of the one it runs now would pass for exhausted.
+// Entries are dropped only where the lane's program, read behind the tail, is still V's.
+__device__ __forceinline__ bool ring_take(const LaneState& L, Ring& R, unsigned long long head, unsigned long long tail, const ProgView& V, Claim& c) {
   const int lane = threadIdx.x & 31;
   if (tail <= head) return false;
   const int n = static_cast<int>(min(tail - head, 32ull));
   uint32_t word = 0;
   Probe p{0, 0, 0};
+  unsigned long long prog = 0;
+  uint32_t gen = 0;
+  if (lane == 0) {   // beside the entries
+    prog = ld_volatile(&L.prog);
+    gen = ld_volatile(&L.gen);
+  }
   if (lane < n) {
     word = ld_volatile(&R.ids[(head + lane) & (kRingCap - 1)]);
     p = probe_entry(V, word);
   }
   unsigned live = __ballot_sync(kWarp, p.left != 0);
   const int spent = live ? __ffs(live) - 1 : n;   // exhausted entries in front of the first live one
-  if (spent > 0 && lane == 0) atomicCAS(&R.head, head, head + spent);   // losing the race is fine: someone else dropped them
+  if (spent > 0 && lane == 0 && prog == reinterpret_cast<unsigned long long>(V.prog) && gen == V.gen) atomicCAS(&R.head, head, head + spent);   // losing the race is fine: someone else dropped them
   while (live) {
     const int src = __ffs(live) - 1;
     live &= live - 1;
@@ -636,14 +644,14 @@ __device__ __forceinline__ bool look_in_lane(DeviceState& S, WorkerState& ws, ui
       }
     }
     if (__shfl_sync(kWarp, held, 0)) {
-      if (ring_take(L.ring[1], link_head, link_tail, V, c)) {
+      if (ring_take(L, L.ring[1], link_head, link_tail, V, c)) {
         took(c, 1);
         return true;
       }
       if (lane == 0) give_slot_back(S, ws);
     }
   }
-  if (!ring_take(L.ring[0], head, tail, V, c)) return false;
+  if (!ring_take(L, L.ring[0], head, tail, V, c)) return false;
   if (lane == 0) give_slot_back(S, ws);
   took(c, 0);
   return true;

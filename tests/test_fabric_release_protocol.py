@@ -213,3 +213,52 @@ def test_the_release_of_a_stage_asks_before_it_takes():
     asks = re.search(r"if \(entry & kSuccLate\) skip = ld_volatile\(&stages\[succ\]\.flags\) & kStageSkip;", text)
     takes = re.search(r"skip \? 0u : take_one_acq", text)
     assert asks and takes and asks.start() < takes.start()
+
+
+# ------------------------------------------------------------------------------------------ a lane that goes on to another program
+def switched(seed, asks_again):
+    """A worker reads the lane's words in any order while the lane goes on from program 1 to program 2 and publishes an entry of it;
+    entries that are not of the program it looks at pass for exhausted and are dropped.  True: the entry is still in the ring."""
+    rnd = random.Random(seed)
+    mem = Memory(prog=1, gen=1, head=4, tail=4)
+
+    def lane():
+        th = Thread(mem, rnd)
+        th.atomic("head", lambda v: 4)
+        yield
+        th.store("prog", 2, release=True)
+        yield
+        th.store("gen", 2, release=True)
+        yield
+        th.store("tail", 5, release=True)
+
+    def worker():
+        th = Thread(mem, rnd)
+        for _ in range(6):
+            words = ["prog", "gen", "head", "tail"]
+            rnd.shuffle(words)
+            seen = {}
+            for w in words:
+                seen[w] = th.load(w, acquire=True)
+                yield
+            if seen["tail"] <= seen["head"]:
+                continue
+            now = th.load("prog"), th.load("gen")
+            yield
+            if seen["prog"] != 2 and (not asks_again or now == (seen["prog"], seen["gen"])):
+                th.atomic("head", lambda v: seen["tail"] if v == seen["head"] else v)
+
+    assert interleave(rnd, [lane(), worker()])
+    return mem.at["head"][-1][0] == 4
+
+
+def test_entries_of_the_program_that_runs_now_are_not_dropped():
+    assert all(switched(seed, asks_again=True) for seed in range(500))
+    assert not all(switched(seed, asks_again=False) for seed in range(500))
+
+
+def test_the_drop_of_exhausted_entries_asks_for_the_program_again():
+    text = body_of("bool ring_take")
+    again = text.index("ld_volatile(&L.prog)"), text.index("ld_volatile(&L.gen)")
+    drop = re.search(r"if \([^;]*prog == reinterpret_cast<unsigned long long>\(V\.prog\) && gen == V\.gen\) atomicCAS\(&R\.head", text)
+    assert drop and max(again) < drop.start()
