@@ -482,7 +482,7 @@ struct WorkerState {
   uint32_t visit[kMaxLanes];   // lanes in the order this worker looks for work: its own, then the borrowing order
   uint32_t n_visit;
   ProgView view;               // of the program looked at last
-  uint32_t idle, polls;        // the last round found nothing; polls since work was last found
+  uint32_t idle, polls;        // the last round found nothing; rounds that found nothing, ever
   // the current claim
   ProgTables prog;
   const TileDesc* tiles;
@@ -712,7 +712,6 @@ __device__ __forceinline__ uint32_t schedule(DeviceState& S, WorkerState& ws, Sm
       if (lane == 0) {
         ws.idle_ns = 64;
         ws.idle = 0;
-        ws.polls = 0;
       }
       __syncwarp();
       return kCmdRun;

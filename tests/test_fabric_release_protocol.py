@@ -262,3 +262,24 @@ def test_the_drop_of_exhausted_entries_asks_for_the_program_again():
     again = text.index("ld_volatile(&L.prog)"), text.index("ld_volatile(&L.gen)")
     drop = re.search(r"if \([^;]*prog == reinterpret_cast<unsigned long long>\(V\.prog\) && gen == V\.gen\) atomicCAS\(&R\.head", text)
     assert drop and max(again) < drop.start()
+
+
+# ------------------------------------------------------------------------------------------ the run-time limit
+def test_the_run_time_limit_is_looked_at_whatever_lies_between_claims():
+    """Every 16th round that finds nothing looks at the limit.  Counted anew behind each claim, rounds of a worker that finds work every
+    time before the 16th would never get there."""
+    def looks(gaps, anew):
+        polls = n = 0
+        for gap in gaps:
+            for _ in range(gap):
+                polls += 1
+                n += polls % 16 == 0
+            if anew:
+                polls = 0
+        return n
+    rnd = random.Random(1)
+    gaps = [rnd.randrange(16) for _ in range(1000)]
+    assert looks(gaps, anew=True) == 0 and looks(gaps, anew=False) == sum(gaps) // 16
+    device = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "monoserve_b200", "csrc", "fabric_device.cu")).read()
+    assert "(ws.polls & 15) == 0 && must_leave(false)" in device
+    assert not re.search(r"ws\.polls = 0", SCHED)   # set where the worker starts, and only there

@@ -288,3 +288,24 @@ def test_many_ring_entries_after_a_long_idle(fab, link):
     tr = decode_trace(trace)
     assert (tr["count"][:idx + 1] == 6).all()
     assert tr["start"][idx] >= tr["end"][:idx].max()
+
+
+def test_run_time_limit_between_short_claims(fab):
+    """Stages of three short tiles for each worker, over and over: a worker never looks for work for long, and still sees that its
+    time is over."""
+    trace = trace_buffer(64)
+    p = Program()
+    stages = [p.stage([spin(1_000, trace, i)] * 3 * fab.num_workers) for i in range(20)]
+    for a, b in zip(stages, stages[1:]):
+        p.after(a, b)
+    h = p.upload(fab, first=stages[0], iterations=0)   # until it is replaced
+    fab.set_max_run(0.3)
+    fab.start()
+    fab.publish(map=[0] * fab.num_workers, caps=[0], order=[0], programs=[h])
+    wait_until(lambda: fab.progress()["lanes"][0]["iterations"] > 10, what="iterations")
+    time.sleep(0.8)
+    done = fab.iterations(0)
+    time.sleep(0.2)
+    assert fab.iterations(0) == done, "workers past their time go on"
+    assert fab.progress()["error"] == 4   # the run-time limit, and nothing else
+    fab.stop()
