@@ -313,7 +313,8 @@ int monofab_fabric_stop(monofab_fabric* f);
  * such launch. */
 int monofab_fabric_start_on(monofab_fabric* f, uint64_t stream, uint64_t context, int workers, int first_worker);
 
-/* Longest idle back-off of a worker (Fabric.set_idle_cap, csrc/host/fabric.h:50), and
+/* Longest idle back-off of a worker while no lane runs; while one does, 1/128 of it, at least 32 ns
+ * (Fabric.set_idle_cap, csrc/host/fabric.h:50; 4096 ns unless set, 0 = as it is), and
  * the run-time limit after which the kernel leaves on its own with
  * MONOFAB_FABRIC_ERR_DEADLINE (default 120 s, 0 = no limit; no counterpart in the
  * reference, whose kernel can only be stopped by the host). */

@@ -659,8 +659,9 @@ __device__ __forceinline__ bool look_in_lane(DeviceState& S, WorkerState& ws, ui
 
 // The WHOLE scheduler warp.  One scheduling round: kCmdRun with a claim in ws, kCmdExit when the
 // host asked the fabric to stop, or kCmdIdle.  `at` is this lane's polled word, `seen` what it was in the last round: a round in
-// which no word has changed since one that found nothing is only the reading of the words.  While a lane
-// runs, the reading is repeated at once (a stage is over in microseconds); otherwise the back-off grows to the idle cap.
+// which no word has changed since one that found nothing is only the reading of the words.  The back-off grows to the idle cap, and
+// while a lane runs, to 1/128 of it, which by default is none to speak of (a stage is over in microseconds).
+constexpr uint32_t kBusyCapLog2 = 7;
 __device__ __forceinline__ uint32_t schedule(DeviceState& S, WorkerState& ws, SmallWorklist& wl, const unsigned long long* at,
                                              unsigned long long& seen) {
   const int lane = threadIdx.x & 31, which = lane % kWordsPerLane;
@@ -674,13 +675,13 @@ __device__ __forceinline__ uint32_t schedule(DeviceState& S, WorkerState& ws, Sm
   const bool changed = __any_sync(kWarp, words != seen && !(of_lane && which >= kWHead));
   auto idle = [&](bool found_nothing, bool more = false) {
     const bool busy = __any_sync(kWarp, of_lane && which == kWRunning && words != 0);
-    const uint32_t cap = max(64u, static_cast<uint32_t>(__shfl_sync(kWarp, words, kStopLane) >> 32));
+    const uint32_t cap = max(64u, static_cast<uint32_t>(__shfl_sync(kWarp, words, kStopLane) >> 32)), most = busy ? max(32u, cap >> kBusyCapLog2) : cap;
     if (lane == 0) {
       ws.idle = found_nothing && !more;
       ++ws.polls;
       if (found_nothing) {
-        __nanosleep(busy ? 32 : ws.idle_ns);
-        ws.idle_ns = busy ? 64 : min(ws.idle_ns * 2, cap);
+        __nanosleep(min(ws.idle_ns, most));
+        ws.idle_ns = min(ws.idle_ns * 2, most);
       }
     }
     __syncwarp();

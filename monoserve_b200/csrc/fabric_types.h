@@ -177,7 +177,7 @@ struct alignas(128) DeviceState {
   Snapshot snap[2];
   unsigned long long published;   // current epoch; the host writes it last
   unsigned int shutdown;
-  unsigned int idle_cap;          // longest idle back-off, ns
+  unsigned int idle_cap;          // longest idle back-off, ns (fabric_sched.cuh, schedule)
   unsigned int trace_cap, trace_n;
   unsigned long long trace_ptr;   // u64 [trace_cap][2] stage events
   unsigned long long max_run_ns;  // the kernel leaves on its own after this long (0 = no limit)

@@ -52,6 +52,7 @@ class Fabric:
             self._C.check(self._lib.monofab_fabric_stop(self._h))
 
     def set_idle_cap(self, ns):
+        """Longest back-off of a worker that finds nothing to do, 4096 ns unless set; 1/128 of it while a lane runs."""
         self._C.check(self._lib.monofab_fabric_set_limits(self._h, int(ns), 120 * 10 ** 9))
 
     def set_max_run(self, seconds):

@@ -309,3 +309,27 @@ def test_run_time_limit_between_short_claims(fab):
     assert fab.iterations(0) == done, "workers past their time go on"
     assert fab.progress()["error"] == 4   # the run-time limit, and nothing else
     fab.stop()
+
+
+def test_idle_cap_bounds_the_back_off_while_a_lane_runs(fab):
+    """How long behind a stage of 20 ms the next one starts: at once by default, within the back-off that a larger cap allows otherwise
+    (1/128 of it, and a sleep may take twice what it is asked for)."""
+    trace = trace_buffer(256)
+    p = Program()
+    a = p.stage([spin(20_000_000, trace, 200)])
+    b = p.stage([spin(5_000, trace, i) for i in range(150)])
+    p.after(a, b)
+    waits = {}
+    for cap in (4096, 1 << 24):
+        fab.set_idle_cap(cap)
+        waits[cap] = []
+        for _ in range(3):
+            h, done = p.upload(fab, first=a), fab.iterations(0)
+            fab.start()
+            fab.publish(map=[0] * fab.num_workers, caps=[0], order=[0], programs=[h])
+            fab.iteration_times(0, done, 1)
+            fab.stop()
+            tr = decode_trace(trace)
+            waits[cap].append(int(tr["start"][:150].min() - tr["end"][200]))
+    assert fab.progress()["error"] == 0
+    assert max(waits[4096]) < 60_000 < max(waits[1 << 24]) < 600_000, waits
