@@ -37,6 +37,7 @@
 #include "gemm_core.cuh"
 #include "operands.h"
 #include "ptx.cuh"
+#include "row_blocks.h"
 #include "rowwise.cuh"
 #include "wide_tile.cuh"
 
@@ -790,6 +791,7 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
   int& s_skipped = s_exec_scratch[4 * (kMaxExperts + 1) + 2];
   int& s_overflow = s_exec_scratch[4 * (kMaxExperts + 1) + 3];
   int& s_wide = s_exec_scratch[4 * (kMaxExperts + 1) + 4];
+  int& s_tall = s_exec_scratch[4 * (kMaxExperts + 1) + 5];
   int* const s_info = s_exec_scratch + 4 * (kMaxExperts + 1) + 16;   // [kMaxExperts]: slot << 12 | region << 4 | wide << 3 | height class
   // [28] u64: GemmArgs and activation maps per height class (w13, w2), weight maps per region (w13, w2)
   unsigned long long* const s_tab = reinterpret_cast<unsigned long long*>(s_exec_scratch + 5 * (kMaxExperts + 1) + 16 + 1);
@@ -854,18 +856,19 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
       ep = e2;
     }
     s_form = (f == 0 || f == 16 || f == 32 || f == 64 || f == 128) ? static_cast<int>(f) : 64;
-  } else if (tid == 32) {   // beside thread 0: whether both products can take 128-row blocks with tiles of two weight slices
-    auto class128 = [](unsigned long long table) { return reinterpret_cast<const unsigned long long*>(table)[3]; };
-    const unsigned long long a[2] = {class128(A.w13_args), class128(A.w2_args)};
-    bool ok = a[0] && a[1] && class128(A.xp_maps) && class128(A.h_maps);   // a program may leave a class out
+  } else if (tid == 32 || tid == 64) {   // beside thread 0: whether both products can take blocks of 128, 256 rows with tiles of two slices
+    const int cls = tid == 32 ? 3 : 4;
+    auto of_class = [cls](unsigned long long table) { return reinterpret_cast<const unsigned long long*>(table)[cls]; };
+    const unsigned long long a[2] = {of_class(A.w13_args), of_class(A.w2_args)};
+    bool ok = a[0] && a[1] && of_class(A.xp_maps) && of_class(A.h_maps);   // a program may leave a class out
     if (ok) {
       GemmArgs g[2];
 #pragma unroll
       for (int i = 0; i < 2; ++i) load_block(g[i], a[i]);
 #pragma unroll
-      for (int i = 0; i < 2; ++i) ok = ok && g[i].bm == 128 && takes_two_slices(g[i]);
+      for (int i = 0; i < 2; ++i) ok = ok && g[i].bm == 16u << cls && takes_two_slices(g[i]);
     }
-    s_wide = ok;
+    (cls == 3 ? s_wide : s_tall) = ok;
   }
   exec_sync();
   stamp();
@@ -892,12 +895,13 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     if (link) return s_form ? s_form : 256;
     return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   };
-  // An expert in HBM with more than 64 rows, where both products take them (s_wide): blocks of 128 rows with tiles of two weight
-  // slices while more than 64 rows are left, then one block of up to 64 (its class is the one kept in s_info).
-  const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2;
-  auto shape = [&](int M, int info, int& wide, int& narrow) {   // row blocks of either kind
-    wide = (info & 8) ? M / 128 + (M % 128 > 64) : 0;
-    const int bm = 16 << (info & 7), left = M - 128 * wide;
+  // An expert in HBM with more than 64 rows, where both products take them: blocks with tiles of two weight slices (row_blocks.h).  Where
+  // blocks of 256 rows are left out (s_tall): of 128 while more than 64 rows are left, then one of up to 64, whose class is kept in s_info.
+  const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2, rows_total = s_start[E];
+  const bool tall = s_tall != 0;
+  auto shape = [&](int M, int info, RowBlocks& wide, int& narrow) {   // row blocks of either kind
+    wide = !(info & 8) ? RowBlocks{0, 0} : tall ? row_blocks(M, rows_total) : RowBlocks{M / 128 + (M % 128 > 64), 0};
+    const int bm = 16 << (info & 7), left = wide.n && tall ? 0 : M - 128 * wide.n;
     narrow = left > 0 ? (left + bm - 1) / bm : 0;
   };
   for (int e = tid; e < E; e += kExecThreads) {
@@ -908,15 +912,16 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     const int region = static_cast<int>(entry & 0xffffffffu), slot = static_cast<int>(entry >> 32);
     const bool link = region == static_cast<int>(A.host_region);
     const bool staged = link && can_stage && s_form == 0 && M > static_cast<int>(G.min_rows);
-    const bool wide = s_wide && M > 64 && (!link || staged);
+    const bool wide = s_wide && M > kNarrowRows && (!link || staged);
     const int left = M % 128;
     const int bm = wide ? block_rows(left > 64 ? 0 : left, false) : block_rows(M, link);
     int cls = 0;
     while ((16 << cls) < bm) ++cls;   // 16, 32, 64, 128, 256 -> 0..4
     if (wide) cls |= 8;
-    int n_wide, n_narrow;
-    shape(M, cls, n_wide, n_narrow);
-    s_n[e] = n_wide * (h13 + h2) + n_narrow * (f13 + f2) + (staged ? nf13 + nf2 : 0);
+    RowBlocks wides;
+    int n_narrow;
+    shape(M, cls, wides, n_narrow);
+    s_n[e] = wides.n * (h13 + h2) + n_narrow * (f13 + f2) + (staged ? nf13 + nf2 : 0);
     // a staged expert's GEMM tiles read region 3 (the lane's staging stack), slot = expert id
     s_info[e] = staged ? (e << 12) | (1 << 11) | (3 << 4) | cls : (slot << 12) | ((region & 0x7f) << 4) | cls;
   }
@@ -961,8 +966,10 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
       const int info = s_info[e];
       const int slot = info >> 12, region = (info >> 4) & 0x7f;
       const int nf = ((info >> 11) & 1) ? nf13 + nf2 : 0;
-      int n_wide, n_narrow;
-      shape(M, info, n_wide, n_narrow);
+      RowBlocks wides;
+      int n_narrow;
+      shape(M, info, wides, n_narrow);
+      const int n_wide = wides.n;
       const int n13 = n_wide * h13 + n_narrow * f13, total = nf + n13 + n_wide * h2 + n_narrow * f2;
       // One lane builds one whole 64-byte descriptor and stores it as four 16-byte pieces back to back.
       TileDesc* const out = p_tiles + A.dyn_first + s_off[e];
@@ -992,14 +999,15 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
           const bool wide = local < n_wide * half;
           const int past = local - n_wide * half;   // among the narrow blocks' tiles
           const int blk = wide ? local % n_wide : past / per, f = wide ? 2 * (local / n_wide) : past - blk * per;   // blocks of a slice: neighbours
-          const int cls = wide ? 3 : info & 7, bm = 16 << cls;
-          const int at = (wide ? 0 : 128 * n_wide) + blk * bm;   // the block's first row among the expert's
+          const int at = wide ? row_block_first(wides, blk) : 128 * n_wide + blk * (16 << (info & 7));   // the block's first row among the expert's
+          const int rows = !wide ? min(16 << (info & 7), M - at) : tall ? row_block_rows(wides, blk, M) : min(128, M - at);
+          const int cls = !wide ? info & 7 : rows > 128 ? 4 : 3;
           const unsigned long long a0 = s_tab[(is13 ? 0 : 5) + cls], a1 = is13 ? wmap13 : wmap2;
           const unsigned long long a2 = s_tab[(is13 ? 10 : 15) + cls], a4 = is13 ? scale13 : scale2;
           v0.x = kTileGemm;                                          // kind | lane | flags; stage (unused)
           v0.z = static_cast<uint32_t>(is13 ? f * 64 : f * 128);     // i0 first weight row
           v0.w = static_cast<uint32_t>(row0 + at);                   // i1 first activation row
-          v1.x = static_cast<uint32_t>(min(bm, M - at));             // i2 rows
+          v1.x = static_cast<uint32_t>(rows);                        // i2 rows
           v1.y = static_cast<uint32_t>(slot);                        // i3 weight slot
           v1.z = static_cast<uint32_t>(a0);                          // a[0] GemmArgs
           v1.w = static_cast<uint32_t>(a0 >> 32);
@@ -1023,9 +1031,10 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     const uint32_t base = A.dyn_first + s_off[e];
     StageStatic& s13 = p_stages[A.w13_stage0 + e];
     StageStatic& s2 = p_stages[A.w2_stage0 + e];
-    int n_wide, n_narrow;
-    shape(M, s_info[e], n_wide, n_narrow);
-    const int n13 = n_wide * h13 + n_narrow * f13, n2 = n_wide * h2 + n_narrow * f2;
+    RowBlocks wides;
+    int n_narrow;
+    shape(M, s_info[e], wides, n_narrow);
+    const int n_wide = wides.n, n13 = n_wide * h13 + n_narrow * f13, n2 = n_wide * h2 + n_narrow * f2;
     const bool staged = M > 0 && ((s_info[e] >> 11) & 1);
     const int nf = staged ? nf13 + nf2 : 0;
     const uint32_t gemm_flags = link ? kStageLink : 0u;   // staged (region 3): only the fetch tiles use the link

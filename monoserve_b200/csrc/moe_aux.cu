@@ -24,6 +24,7 @@
 #include "kernels.h"
 #include "peer_sync.cuh"
 #include "ptx.cuh"
+#include "row_blocks.h"
 #include "rowwise.cuh"
 
 namespace mf {
@@ -260,12 +261,12 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
   if (e == 0) A.starts[E] = total;
 
   if (!A.q) return;   // scan only: counts, starts and chunk prefixes
-  // Row blocks of an expert in HBM.  bf16 weights: of 128 rows, the last of what is left; a block of more than 64 rows is "wide",
-  // with tiles of two weight slices (gemm_core.cuh: 128 x 256, two accumulators).  e4m3 weights: of 256 rows and tiles of one slice, which
+  // Row blocks of an expert in HBM.  bf16 weights: one of up to 64 rows, or "wide" ones with tiles of two weight slices (row_blocks.h).  e4m3 weights: of 256 rows and tiles of one slice, which
   // read and expand the slice once where two blocks of 128 rows do it twice, with two stages of 96 KB in the ring instead of three of
   // 64 (4096 x 1408, blocks of 128 -> 256 rows: 2048 tokens 1284 -> 1271 us, with a Zipf-skewed choice of experts 1378 -> 1260;
   // 1000 tokens 818 -> 821, the same).
-  int tier = kTierHot, z = 0, bh = 256, nb = 0, nw = 0;
+  int tier = kTierHot, z = 0, bh = 256, nb = 0;
+  RowBlocks wide_blocks{0, 0};
   const int expert = (e < E && A.seg_expert) ? A.seg_expert[e] : e;
   // A segment of an expert the table does not hold, a negative count or more rows than the packed-row
   // buffers take: no tile is emitted and the layer reports a plan overflow.
@@ -275,12 +276,10 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
     tier = A.table[2 * expert] == 0 ? kTierHost : kTierHot;
     z = A.table[2 * expert + 1];
     if (tier == kTierHost) bh = A.form ? A.form : 256;
-    else if (A.slices > 1) {
-      bh = 128;
-      nw = cnt / 128 + (cnt % 128 > 64);
-    }
-    nb = (cnt + bh - 1) / bh;
+    else if (A.slices > 1 && cnt > kNarrowRows) wide_blocks = row_blocks(cnt, total);
+    nb = wide_blocks.n ? wide_blocks.n : (cnt + bh - 1) / bh;
   }
+  const int nw = wide_blocks.n;   // all of an expert's blocks, or none
   const int f13 = (A.I + 63) / 64, f2 = (A.H + 127) / 128;
   const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2;   // tiles of a wide block
   // per tier: [w13 tiles of every expert][w2 tiles of every expert]; row blocks numbered over all experts
@@ -307,7 +306,8 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
   // Every expert's tile list is written by a warp, a tile per lane (an expert at decode batch sizes has
   // 28 tiles; written from one thread per expert they were the longest serial stretch of the layer).
   __shared__ int s_job[kMaxExperts][8];   // nb, bh, rows, first row, slot, tier, first w13 tile, first w2 tile (+ block0 below)
-  __shared__ int s_block0[kMaxExperts], s_expert[kMaxExperts], s_wide[kMaxExperts];
+  __shared__ int s_block0[kMaxExperts], s_expert[kMaxExperts];
+  __shared__ RowBlocks s_wide[kMaxExperts];
   if (e < E) {
     s_job[e][0] = overflow ? 0 : nb;
     s_job[e][1] = bh;
@@ -319,29 +319,30 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
     s_job[e][7] = total13[tier] + first2[tier];
     s_block0[e] = block0;
     s_expert[e] = expert;
-    s_wide[e] = nw;
+    s_wide[e] = wide_blocks;
   }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int x = warp; x < E; x += static_cast<int>(blockDim.x >> 5)) {
     const int x_nb = s_job[x][0];
     if (x_nb == 0) continue;
-    const int x_bh = s_job[x][1], x_cnt = s_job[x][2], x_start = s_job[x][3], x_tier = s_job[x][5], x_nw = s_wide[x];
+    const int x_bh = s_job[x][1], x_cnt = s_job[x][2], x_start = s_job[x][3], x_tier = s_job[x][5];
+    const RowBlocks x_wide = s_wide[x];
     GemmTile* const list = A.tiles[x_tier];
-    const int n13 = x_nw * h13 + (x_nb - x_nw) * f13, n2 = x_nw * h2 + (x_nb - x_nw) * f2;
+    const bool wide = x_wide.n > 0;
+    const int n13 = x_nb * (wide ? h13 : f13), n2 = x_nb * (wide ? h2 : f2);
     for (int j = lane; j < n13 + n2; j += 32) {
       const bool up = j >= n13;   // a w2 tile
-      const int jj = up ? j - n13 : j, per = up ? f2 : f13, half = up ? h2 : h13;
-      const bool wide = jj < x_nw * half;
-      // the row blocks of a weight slice are neighbours in the list: they read it at about the same time
-      const int b = wide ? jj % x_nw : x_nw + (jj - x_nw * half) / per;
-      const int f = wide ? 2 * (jj / x_nw) : (jj - x_nw * half) - (b - x_nw) * per;   // first slice
-      const int rows = min(x_bh, x_cnt - b * x_bh);
+      const int jj = up ? j - n13 : j, per = up ? f2 : f13;
+      // wide blocks: those of a weight slice are neighbours in the list, so that they read it at about the same time
+      const int b = wide ? jj % x_nb : jj / per, f = wide ? 2 * (jj / x_nb) : jj % per;   // f: first slice
+      const int first = wide ? row_block_first(x_wide, b) : b * x_bh;
+      const int rows = wide ? row_block_rows(x_wide, b, x_cnt) : min(x_bh, x_cnt - first);
       int n = 16;
       while (n < rows) n <<= 1;
       GemmTile t;
       t.w_row0 = up ? f * 128 : f * 64;
-      t.act_row0 = x_start + b * x_bh;
+      t.act_row0 = x_start + first;
       t.rows = rows;
       t.n = n;
       t.z = s_job[x][4];

@@ -357,3 +357,27 @@ def test_glm_style_layer_program(pack_hot):
     finally:
         fab.stop()
         fab.close()
+
+
+def test_row_blocks_of_many_rows():
+    """A pass of at least 32768 rows: experts are cut into blocks of 256 rows, the last of 65 to 256."""
+    from monoserve_b200.fabric import Fabric
+    from monoserve_b200.lane import MoELane
+    T, H, I, E, K = 4160, 256, 192, 16, 8
+    wr, w13, w2 = weights(H, I, E, 31)
+    xn, x2 = acts(T, H, 32)
+    fab = Fabric(pool_bytes=128 << 20)
+    fab.set_max_run(60)
+    try:
+        lane = MoELane(fab, 0, H, I, E, K, T, wr, w13, w2, hot=list(range(E)))
+        lane.set_input(xn.cuda(), x2.cuda())
+        h = lane.build(T, iterations=1)
+        fab.start()
+        fab.publish(map=[0] * fab.num_workers, caps=[4], order=[0], programs=[h])
+        wait_iterations(fab, 0, 1)
+        fab.stop()
+        assert fab.progress()["error"] == 0
+        check_lane(lane, wr, w13, w2, xn, x2, K)
+    finally:
+        fab.stop()
+        fab.close()

@@ -466,3 +466,11 @@ def test_fp8_qwen_shape_prefill_rows(I):
     ref, _, _ = tp.moe_layer(xn.float(), x2.float(), wr, d13, d2, K, routing=(w, ids))
     assert rel_l2(out.float().cpu(), ref) < TOL_FP8
     m.close()
+
+
+def test_row_blocks_of_many_rows():
+    """Experts above 256 rows in a pass of at least 32768 rows: blocks of 256 rows, the last of 65 to 256; an odd number of w13 slices."""
+    H, I, E, K = 256, 192, 16, 8
+    m, wr, w13, w2 = make_layer(4160, H, I, E, K, hot=list(range(E)), seed=4)
+    check_layer_against_c_oracle(m, wr, w13, w2, *acts(4160, H, 6), K)
+    m.close()

@@ -1,0 +1,34 @@
+"""The row blocks of an expert (monoserve_b200/csrc/row_blocks.h), compiled for the host, over every number of rows: they cover the rows in
+order, of 65 to 256 rows each, whichever way the pass cuts its experts."""
+import os
+import subprocess
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "monoserve_b200", "csrc")
+CHECK = r"""
+#include "row_blocks.h"
+#include <cstdio>
+using namespace mf;
+int main() {
+  const int totals[] = {0, kManyRows - 1, kManyRows, 1 << 20};
+  for (int total : totals)
+    for (int rows = kNarrowRows + 1; rows < 70000; ++rows) {
+      const RowBlocks b = row_blocks(rows, total);
+      int at = 0;
+      for (int i = 0; i < b.n; ++i) {
+        const int n = row_block_rows(b, i, rows);
+        if (row_block_first(b, i) != at || n <= kNarrowRows || n > 256) return printf("rows %d of %d, block %d\n", rows, total, i), 1;
+        if (total < kManyRows && rows > 256 && i < b.n - 1 && n != 128) return printf("rows %d: block %d of %d rows\n", rows, i, n), 1;
+        at += n;
+      }
+      if (at != rows || b.n > (rows + 127) / 128 || b.tall >= b.n + (b.tall == 0)) return printf("rows %d of %d: %d\n", rows, total, at), 1;
+    }
+  return 0;
+}
+"""
+
+
+def test_blocks_cover_the_rows(tmp_path):
+    (tmp_path / "check.cpp").write_text(CHECK)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", CSRC, str(tmp_path / "check.cpp"), "-o", str(tmp_path / "check")], check=True)
+    r = subprocess.run([str(tmp_path / "check")], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout
