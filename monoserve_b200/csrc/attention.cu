@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(kAttnThreads, 1) paged_attention_kernel(const 
   w.ws_o = p.ws_o;
   w.ws_ml = p.ws_ml;
   w.trace = nullptr;
-  w.scale_log2 = attn_scale(p.scale_log2);
+  set_scale(w, p.scale_log2);
   w.bt_stride = p.bt_stride;
   w.hq = p.hq;
   w.group = p.group;

@@ -52,7 +52,8 @@ struct AttnWork {
   float* ws_o;                      // split items: unnormalised O rows, fp32 [rows][128]
   float2* ws_ml;                    // and their (max, sum)
   unsigned long long* trace;        // phase trace of this item's first softmax lane, or NULL
-  float scale_log2;
+  float scale_log2;                 // positive (set_scale)
+  int32_t negate;                   // the scores' sign is changed
   int32_t bt_stride, hq, group, page, q_box_rows, rep_ok;
   AttnItem item;
 };
@@ -159,17 +160,21 @@ __device__ __forceinline__ float fast_exp2(float x) {
   return y;
 }
 
-// Scores of keys past the visible ones, the first `lim`, become `masked`: as low as can be for a maximum, and for the weights the
-// infinity that the scale takes to minus infinity, whose exponential is zero.
-constexpr uint32_t kNegInf = 0xff800000u, kPosInf = 0x7f800000u;
+// Scores of keys past the visible ones, the first `lim`, are as low as can be: they are no maximum and their exponential is zero.
 template <int NC>
-__device__ __forceinline__ void mask_scores(uint32_t (&v)[NC], int lim, uint32_t masked) {
+__device__ __forceinline__ void mask_scores(uint32_t (&v)[NC], int lim) {
   if (lim >= NC) return;
 #pragma unroll
-  for (int i = 0; i < NC; ++i) v[i] = i < lim ? v[i] : masked;
+  for (int i = 0; i < NC; ++i) v[i] = i < lim ? v[i] : 0xff800000u;
 }
-// A scale of zero as the least normal number, with which finite scores weigh the same: zero times an infinite score would be no number.
-__device__ __forceinline__ float attn_scale(float scale) { return scale == 0.f ? 1.17549435e-38f : scale; }
+// The scale that the scores are taken with.  The masks above want it positive: a negative one's sign goes into the product (the MMA
+// negates Q), and one of zero, with which all visible keys weigh the same, is the least normal number.
+__device__ __forceinline__ void set_scale(AttnWork& w, float scale) {
+  const float size = fabsf(scale), least = 1.17549435e-38f;
+  w.scale_log2 = size < least ? least : size;
+  w.negate = scale < 0.f;
+}
+__device__ __forceinline__ uint32_t scores_idesc(const AttnWork& w) { return umma_idesc_bf16(128, 128) | (w.negate ? kUmmaNegateA : 0u); }
 template <int NC>
 __device__ __forceinline__ float max_scores(const uint32_t (&v)[NC], float mx) {   // four chains
   float m[4] = {mx, mx, mx, mx};
@@ -213,7 +218,7 @@ __device__ __forceinline__ float row_max(uint32_t tmem_s, int lim) {
   for (int h = 0; h < 2; ++h) {
     uint32_t v[64];
     load_columns(tmem_s + 64 * h, v);
-    mask_scores(v, lim - 64 * h, kNegInf);
+    mask_scores(v, lim - 64 * h);
     mx = max_scores(v, mx);
   }
   return mx;
@@ -222,7 +227,6 @@ __device__ __forceinline__ float row_max(uint32_t tmem_s, int lim) {
 template <class Read>
 __device__ __forceinline__ float row_weights(uint32_t tmem_s, int lim, float scale, float neg_mx, uint8_t* row, int swz, Read read) {
   float sum0 = 0.f, sum1 = 0.f;
-  const uint32_t masked = scale < 0.f ? kPosInf : kNegInf;
 #pragma unroll 1
   for (int c0 = 0; c0 < kKeysPerTile; c0 += 32) {
     uint32_t v[32];
@@ -233,7 +237,7 @@ __device__ __forceinline__ float row_weights(uint32_t tmem_s, int lim, float sca
     uint8_t* const to = row + (c0 >> 6) * kHalfBytes;
     const int piece = (c0 & 32) >> 3;
     if (lim > c0) {
-      mask_scores(v, lim - c0, masked);
+      mask_scores(v, lim - c0);
       store_weights(v, scale, neg_mx, to, piece, swz, sum0, sum1);
     } else {   // every key is masked
 #pragma unroll
@@ -413,7 +417,7 @@ __device__ __forceinline__ void attn_mma(const AttnWork& p, const AttnCtx& c) {
   uint8_t* const sV = c.smem + 3 * kTileBytes;
   uint8_t* const sP = c.smem + 5 * kTileBytes;
   // S = Q K^T: both K-major; O += P V: A K-major, B (V) MN-major
-  const uint32_t idesc_s = umma_idesc_bf16(128, 128);
+  const uint32_t idesc_s = scores_idesc(p);
   const uint32_t idesc_o = umma_idesc_bf16(128, 128) | (1u << 16);
   const uint32_t q_addr = smem_u32(sQ);
   if (leader) attn_note(c, 0, kAttnSiteMmaQ);
@@ -559,14 +563,13 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, NC) : 0;
     if (!ok) continue;   // a wait gave up
     uint32_t v[32];   // of a quad-replicated item: the thread's quarter of the row
-    // with a positive scale the maximum of the scaled scores is the scaled maximum; with a negative one it is a reference point as good
-    // as any while the exponentials are finite
+    // the scale is positive: the maximum of the scaled scores is the scaled maximum
     float mx;
     if constexpr (kRep) {
       __syncwarp();
       tmem_ld_32x32(tmem_s, v);
       tmem_ld_wait();
-      mask_scores(v, lim, kNegInf);
+      mask_scores(v, lim);
       mx = max_scores(v, -1e30f);
     } else {
       mx = row_max(tmem_s, lim);
@@ -613,7 +616,6 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     uint8_t* const p_row = sP + (j % PB) * kTileBytes + r * 128;
     if constexpr (kRep) {
       float sum0 = 0.f, sum1 = 0.f;
-      if (p.scale_log2 < 0.f) mask_scores(v, lim, kPosInf);
       store_weights(v, p.scale_log2, neg_mx, p_row + (c_lo >> 6) * kHalfBytes, (c_lo & 63) >> 3, r & 7, sum0, sum1);
       l += sum0 + sum1;
     } else {
@@ -769,7 +771,7 @@ __device__ __forceinline__ void attn_mma_alt(const AttnWork& p, const AttnCtx& c
   uint8_t* const sK = c.smem + kTileBytes;
   uint8_t* const sV = c.smem + 3 * kTileBytes;
   uint8_t* const sP = c.smem + 5 * kTileBytes;
-  const uint32_t idesc_s = umma_idesc_bf16(128, 128);
+  const uint32_t idesc_s = scores_idesc(p);
   const uint32_t idesc_o = umma_idesc_bf16(128, 128) | (1u << 16);
   const uint32_t q_addr = smem_u32(sQ);
   if (leader) attn_note(c, 0, kAttnSiteMmaQ);
@@ -880,7 +882,7 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
     }
     const int key0 = item.key_begin + j * kKeysPerTile;
     const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, kKeysPerTile) : 0;   // keys [0, lim) of the tile count
-    // the row maximum (as in softmax_role)
+    // the row maximum (the scale is positive: the maximum of the scaled scores is the scaled maximum)
     float mx = row_max(tmem_s, lim);
     mx = mx > -1e30f ? mx * p.scale_log2 : -1e30f;
     mx = fmaxf(mx, m);

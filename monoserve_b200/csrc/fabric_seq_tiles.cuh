@@ -35,7 +35,7 @@ __device__ bool make_attn_work(const TileDesc& t, AttnWork& w) {
   w.ws_o = reinterpret_cast<float*>(A.ws_o);
   w.ws_ml = reinterpret_cast<float2*>(A.ws_m);
   w.trace = nullptr;
-  w.scale_log2 = attn_scale(A.scale_log2);
+  set_scale(w, A.scale_log2);
   w.bt_stride = static_cast<int32_t>(A.bt_stride);
   w.hq = static_cast<int32_t>(A.hq);
   w.group = group;

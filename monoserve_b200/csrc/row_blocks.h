@@ -9,7 +9,7 @@
 // microseconds with blocks of 128 rows and one of up to 64 for the rest, and with this rule:
 //   uniform choice   2304 tokens 481 -> 407, 2560 511 -> 434, 3072 514 -> 463, 3840 535 -> 514, 6600 898 -> 835, 8192 1025 -> 995
 //   Zipf-skewed 1.1  2304 tokens 402 -> 411, 2560 434 -> 439, 4096 580 -> 580, 6600 866 -> 851, 8192 1022 -> 1006
-// and as lane programs, the experts of a layer: 2535 tokens of prompts 395 -> 334, 3706 tokens 412 -> 381.
+// and as lane programs, the experts of a layer: 2533 tokens of prompts 395 -> 334, 3706 tokens 412 -> 381.
 #pragma once
 
 #ifndef __CUDACC__
