@@ -559,8 +559,10 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     }
     const uint32_t tmem_s = c.tmem_base + s * 128 + lane_off + c_lo;
     const int key0 = item.key_begin + j * kKeysPerTile + c_lo;
-    // keys this thread may use among its NC columns: [0, lim)
-    const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, NC) : 0;
+    // keys this thread may use among its NC columns: [0, lim).  All, where it has no row of a long tile: its results go nowhere, and a
+    // warp with few rows would mask in every tile for the others (32 decode steps of 12 rows an item: attention stage 121 us, now 100;
+    // quad-replicated items, with a quarter of the columns: 223 us without masks, 227 with, so they keep zeros).
+    const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, NC) : kRep ? 0 : NC;
     if (!ok) continue;   // a wait gave up
     uint32_t v[32];   // of a quad-replicated item: the thread's quarter of the row
     // the scale is positive: the maximum of the scaled scores is the scaled maximum
@@ -582,7 +584,7 @@ __device__ __forceinline__ void softmax_role(const AttnWork& p, const AttnCtx& c
     // sums and within bf16's range, the result is the same quotient, and the rescale of the row's
     // part of O in TMEM (which waits for the previous P V) becomes rare instead of per tile.
     if (j > 0 && mx <= m + kMaxSlack) mx = m;
-    if (j > 0 && __any_sync(0xffffffffu, mx > m)) {
+    if (j > 0 && __any_sync(0xffffffffu, mx > m && (kRep || row_ok))) {
       if (lane == 0) attn_note(c, j, kAttnSiteSmaxRescale);
       if (!warp_wait(&sh.o_full[s ^ 1], attn_parity(c, j - 1), abort_flag, kAttnWaitNs)) {
         ok = attn_gave_up(sh, kAttnSiteSmaxRescale);
@@ -881,7 +883,7 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
       continue;
     }
     const int key0 = item.key_begin + j * kKeysPerTile;
-    const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, kKeysPerTile) : 0;   // keys [0, lim) of the tile count
+    const int lim = row_ok ? min(min(c.kv_end, qpos + 1) - key0, kKeysPerTile) : kKeysPerTile;   // keys [0, lim) of the tile count (as in softmax_role)
     // the row maximum (the scale is positive: the maximum of the scaled scores is the scaled maximum)
     float mx = row_max(tmem_s, lim);
     mx = mx > -1e30f ? mx * p.scale_log2 : -1e30f;
@@ -890,7 +892,7 @@ __device__ __forceinline__ void softmax_alt(const AttnWork& p, const AttnCtx& c,
     // the reference point of the row's exponentials moves only when the maximum has grown past it by more than
     // kMaxSlack (see softmax_role); the group's accumulator is rescaled then, after its previous P V
     if (j >= 2 && mx <= m + kMaxSlack) mx = m;
-    if (j >= 2 && __any_sync(0xffffffffu, mx > m)) {
+    if (j >= 2 && __any_sync(0xffffffffu, mx > m && row_ok)) {
       if (lane == 0) attn_note(c, j, kAttnSiteSmaxRescale);
       if (!warp_wait(&sh.o_full[s], attn_parity(c, j - 2), abort_flag, kAttnWaitNs)) {
         ok = attn_gave_up(sh, kAttnSiteSmaxRescale);

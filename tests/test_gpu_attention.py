@@ -190,3 +190,25 @@ def test_many_items_per_cta_mixed_kinds():
         err = (out[row:row + n] - ref).abs().max().item()
         assert err < TOL, (r, err)
         row += n
+
+
+@pytest.mark.parametrize("hq,hkv", [(96, 8), (32, 4)])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_rows_that_an_item_does_not_have_reach_no_other(hq, hkv, bad):
+    """An item's box of queries holds rows of the next requests; whatever they are, its own rows come out the same."""
+    from monoserve_b200.attention import paged_attention
+    lens, rows = [700, 300, 260], [1, 5, 130]
+    kc, vc, bt, _ = make_cache(lens, hkv, 16, seed=2)
+    kc, vc, bt = kc.cuda(), vc.cuda(), bt.cuda()
+    q = torch.randn(sum(rows) + 40, hq, 128, generator=torch.Generator().manual_seed(2)).to(torch.bfloat16).cuda()
+    req_info, row = [], 0
+    for n, L in zip(rows, lens):
+        req_info.append((row, L - n, n, L))
+        row += n
+    want = paged_attention(q, kc, vc, bt, req_info)
+    for i in range(len(rows)):
+        first, _, n, _ = req_info[i]
+        other = torch.full_like(q, bad)
+        other[first:first + n] = q[first:first + n]
+        got = paged_attention(other, kc, vc, bt, req_info)
+        assert torch.equal(got[first:first + n], want[first:first + n]), i
