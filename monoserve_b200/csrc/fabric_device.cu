@@ -895,14 +895,14 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
     if (link) return s_form ? s_form : 256;
     return M <= 16 ? 16 : M <= 32 ? 32 : M <= 64 ? 64 : 128;
   };
-  // An expert in HBM with more than 64 rows, where both products take them: blocks with tiles of two weight slices (row_blocks.h).  Where
-  // blocks of 256 rows are left out (s_tall): of 128 while more than 64 rows are left, then one of up to 64, whose class is kept in s_info.
+  // An expert in HBM with more than 64 rows, where both products take them: blocks with tiles of two weight slices, and behind them
+  // possibly one of up to 64 rows, whose class is kept in s_info (row_blocks.h).
   const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2, rows_total = s_start[E];
   const bool tall = s_tall != 0;
   auto shape = [&](int M, int info, RowBlocks& wide, int& narrow) {   // row blocks of either kind
-    wide = !(info & 8) ? RowBlocks{0, 0} : tall ? row_blocks(M, rows_total) : RowBlocks{M / 128 + (M % 128 > 64), 0};
-    const int bm = 16 << (info & 7), left = wide.n && tall ? 0 : M - 128 * wide.n;
-    narrow = left > 0 ? (left + bm - 1) / bm : 0;
+    wide = (info & 8) ? row_blocks(M, rows_total, tall) : RowBlocks{0, 0, M};
+    const int bm = 16 << (info & 7);
+    narrow = (wide.rest + bm - 1) / bm;
   };
   for (int e = tid; e < E; e += kExecThreads) {
     const int M = s_cnt[e];
@@ -999,8 +999,8 @@ __device__ void tile_expand(const TileDesc& t, const ProgramDesc* P, DeviceState
           const bool wide = local < n_wide * half;
           const int past = local - n_wide * half;   // among the narrow blocks' tiles
           const int blk = wide ? local % n_wide : past / per, f = wide ? 2 * (local / n_wide) : past - blk * per;   // blocks of a slice: neighbours
-          const int at = wide ? row_block_first(wides, blk) : 128 * n_wide + blk * (16 << (info & 7));   // the block's first row among the expert's
-          const int rows = !wide ? min(16 << (info & 7), M - at) : tall ? row_block_rows(wides, blk, M) : min(128, M - at);
+          const int at = wide ? row_block_first(wides, blk) : M - wides.rest + blk * (16 << (info & 7));   // the block's first row among the expert's
+          const int rows = wide ? row_block_rows(wides, blk, M) : min(16 << (info & 7), M - at);
           const int cls = !wide ? info & 7 : rows > 128 ? 4 : 3;
           const unsigned long long a0 = s_tab[(is13 ? 0 : 5) + cls], a1 = is13 ? wmap13 : wmap2;
           const unsigned long long a2 = s_tab[(is13 ? 10 : 15) + cls], a4 = is13 ? scale13 : scale2;

@@ -266,7 +266,7 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
   // 64 (4096 x 1408, blocks of 128 -> 256 rows: 2048 tokens 1284 -> 1271 us, with a Zipf-skewed choice of experts 1378 -> 1260;
   // 1000 tokens 818 -> 821, the same).
   int tier = kTierHot, z = 0, bh = 256, nb = 0;
-  RowBlocks wide_blocks{0, 0};
+  RowBlocks wide_blocks{0, 0, 0};
   const int expert = (e < E && A.seg_expert) ? A.seg_expert[e] : e;
   // A segment of an expert the table does not hold, a negative count or more rows than the packed-row
   // buffers take: no tile is emitted and the layer reports a plan overflow.
@@ -277,9 +277,9 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
     z = A.table[2 * expert + 1];
     if (tier == kTierHost) bh = A.form ? A.form : 256;
     else if (A.slices > 1 && cnt > kNarrowRows) wide_blocks = row_blocks(cnt, total);
-    nb = wide_blocks.n ? wide_blocks.n : (cnt + bh - 1) / bh;
+    nb = wide_blocks.n ? wide_blocks.n + (wide_blocks.rest > 0) : (cnt + bh - 1) / bh;
   }
-  const int nw = wide_blocks.n;   // all of an expert's blocks, or none
+  const int nw = wide_blocks.n;
   const int f13 = (A.I + 63) / 64, f2 = (A.H + 127) / 128;
   const int h13 = (f13 + 1) / 2, h2 = (f2 + 1) / 2;   // tiles of a wide block
   // per tier: [w13 tiles of every expert][w2 tiles of every expert]; row blocks numbered over all experts
@@ -329,15 +329,16 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
     const int x_bh = s_job[x][1], x_cnt = s_job[x][2], x_start = s_job[x][3], x_tier = s_job[x][5];
     const RowBlocks x_wide = s_wide[x];
     GemmTile* const list = A.tiles[x_tier];
-    const bool wide = x_wide.n > 0;
-    const int n13 = x_nb * (wide ? h13 : f13), n2 = x_nb * (wide ? h2 : f2);
+    const int x_nw = x_wide.n, n13 = x_nw * h13 + (x_nb - x_nw) * f13, n2 = x_nw * h2 + (x_nb - x_nw) * f2;
     for (int j = lane; j < n13 + n2; j += 32) {
       const bool up = j >= n13;   // a w2 tile
-      const int jj = up ? j - n13 : j, per = up ? f2 : f13;
+      const int jj = up ? j - n13 : j, per = up ? f2 : f13, half = up ? h2 : h13;
+      const bool wide = jj < x_nw * half;
+      const int past = jj - x_nw * half;   // among the tiles of one slice
       // wide blocks: those of a weight slice are neighbours in the list, so that they read it at about the same time
-      const int b = wide ? jj % x_nb : jj / per, f = wide ? 2 * (jj / x_nb) : jj % per;   // f: first slice
-      const int first = wide ? row_block_first(x_wide, b) : b * x_bh;
-      const int rows = wide ? row_block_rows(x_wide, b, x_cnt) : min(x_bh, x_cnt - first);
+      const int b = wide ? jj % x_nw : x_nw + past / per, f = wide ? 2 * (jj / x_nw) : past % per;   // f: first slice
+      const int first = x_nw ? row_block_first(x_wide, b) : b * x_bh;
+      const int rows = x_nw ? row_block_rows(x_wide, b, x_cnt) : min(x_bh, x_cnt - first);
       int n = 16;
       while (n < rows) n <<= 1;
       GemmTile t;

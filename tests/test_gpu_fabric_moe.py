@@ -359,17 +359,23 @@ def test_glm_style_layer_program(pack_hot):
         fab.close()
 
 
-def test_row_blocks_of_many_rows():
-    """A pass of at least 32768 rows: experts are cut into blocks of 256 rows, the last of 65 to 256."""
+BLOCK_EDGES = [1, 64, 65, 128, 129, 192, 193, 255, 256, 257, 320, 321, 0, 384, 385, 512, 513]
+
+
+@pytest.mark.parametrize("more", [1, 6200, 30000])
+def test_row_blocks_in_passes_of_some_and_many_rows(more):
+    """The edges of row blocks in a pass of few rows, of some and of many, which cut their experts differently."""
     from monoserve_b200.fabric import Fabric
     from monoserve_b200.lane import MoELane
-    T, H, I, E, K = 4160, 256, 192, 16, 8
+    counts = BLOCK_EDGES + [more]
+    H, I, E, T = 256, 192, len(counts), sum(counts)
     wr, w13, w2 = weights(H, I, E, 31)
-    xn, x2 = acts(T, H, 32)
+    xn, _ = directed(counts, wr, 32)
+    x2 = acts(T, H, 33)[1]
     fab = Fabric(pool_bytes=128 << 20)
     fab.set_max_run(60)
     try:
-        lane = MoELane(fab, 0, H, I, E, K, T, wr, w13, w2, hot=list(range(E)))
+        lane = MoELane(fab, 0, H, I, E, 1, T, wr, w13, w2, hot=list(range(E)))
         lane.set_input(xn.cuda(), x2.cuda())
         h = lane.build(T, iterations=1)
         fab.start()
@@ -377,7 +383,8 @@ def test_row_blocks_of_many_rows():
         wait_iterations(fab, 0, 1)
         fab.stop()
         assert fab.progress()["error"] == 0
-        check_lane(lane, wr, w13, w2, xn, x2, K)
+        assert np.diff(lane.starts.cpu().numpy()).tolist() == counts
+        check_lane(lane, wr, w13, w2, xn, x2, 1)
     finally:
         fab.stop()
         fab.close()

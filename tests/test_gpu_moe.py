@@ -468,9 +468,16 @@ def test_fp8_qwen_shape_prefill_rows(I):
     m.close()
 
 
-def test_row_blocks_of_many_rows():
-    """Experts above 256 rows in a pass of at least 32768 rows: blocks of 256 rows, the last of 65 to 256; an odd number of w13 slices."""
-    H, I, E, K = 256, 192, 16, 8
-    m, wr, w13, w2 = make_layer(4160, H, I, E, K, hot=list(range(E)), seed=4)
-    check_layer_against_c_oracle(m, wr, w13, w2, *acts(4160, H, 6), K)
+@pytest.mark.parametrize("more", [1, 6200, 30000])
+def test_row_blocks_at_their_edges(more):
+    """Experts whose row counts lie on the edges of row blocks, in passes of few, of some and of many rows, with an odd number of w13
+    slices."""
+    from tests.test_gpu_fabric_moe import BLOCK_EDGES, directed
+    H, I, E = 256, 192, len(BLOCK_EDGES) + 1
+    counts = BLOCK_EDGES + [more]
+    T = sum(counts)
+    m, wr, w13, w2 = make_layer(T, H, I, E, 1, hot=list(range(E)), seed=4)
+    xn, _ = directed(counts, wr, 6)
+    check_layer_against_c_oracle(m, wr, w13, w2, xn, acts(T, H, 7)[1], 1)
+    assert m.workspace("counts")[:E].tolist() == counts
     m.close()
