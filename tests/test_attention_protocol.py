@@ -526,3 +526,184 @@ def test_without_the_common_exit_decision_a_thread_can_be_left_at_a_barrier():
 def test_failure_model_runs_clean_chains_to_the_end():
     for seed in range(20):
         assert run_failure([("alt", 5), ("rep", 3), ("alt", 2), ("rep", 0), ("alt", 0)], seed, abort_step=-1) is None
+
+
+# ----------------------------------------------------------------------------------------------------------
+# The fabric worker's hand-over of records (fabric_device.cu): one softmax group, one P buffer, S freed by P of its tile, and a producer
+# that waits until every earlier record is finished, except between one attention item and the next where the first is not
+# replicated.  Kinds: 'rows' (output rows leave through P's memory), 'rep' (merges in the memory of K and V), 'other' (a record that uses the
+# whole ring).
+
+def run_records(items, seed, drain_behind_rep=True, q_waits=True):
+    rnd = random.Random(seed)
+    bar = {n: [Phase(1), Phase(1)] for n in ("k_full", "v_full", "k_empty", "v_empty", "s_full", "o_full")}
+    bar["p_full"] = [Phase(THREADS), Phase(THREADS)]
+    q_full, q_empty = Phase(1), Phase(1)
+    S, K, V, O, Q, P = [None, None], [None, None], [None, None], [None], [None], {}
+    unread_s, errors, done = [set(), set()], [], {"exec": 0, "mma": 0, "load": 0}
+    together, exec_left = Meet(THREADS), [THREADS] * len(items)
+
+    def parity(base, j):
+        return (base[j & 1] + (j >> 1)) & 1
+
+    def advance(n, st):
+        st[0] += 1
+        st[1][0] += (n + 1) >> 1
+        st[1][1] += n >> 1
+
+    def wait(b, par, who):
+        while not b.done(par):
+            yield who
+
+    def producer():
+        st, prev_attn, prev_rows = [0, [0, 0]], False, False
+        for rec, (kind, n) in enumerate(items):
+            attn = kind != "other"
+            behind = prev_rows or (not drain_behind_rep and prev_attn)
+            if (attn or prev_attn) and not (attn and behind):
+                while done["exec"] < rec or done["mma"] < rec:
+                    yield f"producer: earlier records, {rec}"
+            prev_attn, prev_rows = True, kind == "rows"
+            if not attn:
+                Q[0] = K[0] = K[1] = V[0] = V[1] = rec
+                P.update({t: rec for t in range(THREADS)})
+                done["load"] = rec + 1
+                yield None
+                continue
+            base = list(st[1])
+            if st[0] > 0 and q_waits:
+                yield from wait(q_empty, (st[0] - 1) & 1, f"producer: Q of {rec}")
+            Q[0] = rec
+            q_full.arrive()
+            for step in range(n + 1):
+                for buf, name, j in ((K, "k", step), (V, "v", step - 1)):
+                    if not 0 <= j < n:
+                        continue
+                    s = j & 1
+                    uses = base[s] + (j >> 1)
+                    if uses > 0:
+                        yield from wait(bar[name + "_empty"][s], (uses - 1) & 1, f"producer: {name} of {rec} tile {j}")
+                    buf[s] = (rec, j)
+                    bar[name + "_full"][s].arrive()
+                yield None
+            advance(n, st)
+
+    def mma():
+        st = [0, [0, 0]]
+        for rec, (kind, n) in enumerate(items):
+            if kind != "other":
+                base = list(st[1])
+                yield from wait(q_full, st[0] & 1, f"mma: Q of {rec}")
+
+                def mma_s(j):
+                    s = j & 1
+                    yield from wait(bar["k_full"][s], parity(base, j), f"mma: K, {rec} tile {j}")
+                    uses = base[s] + (j >> 1)
+                    if uses > 0:
+                        yield from wait(bar["p_full"][s], (uses - 1) & 1, f"mma: S free, {rec} tile {j}")
+                    if K[s] != (rec, j) or Q[0] != rec:
+                        errors.append(f"S of {rec} tile {j} reads K {K[s]}, Q {Q[0]}")
+                    if unread_s[s]:
+                        errors.append(f"S[{s}] overwritten by {rec} tile {j}")
+                    S[s], unread_s[s] = (rec, j), set(range(THREADS))
+                    bar["s_full"][s].arrive()
+                    bar["k_empty"][s].arrive()
+                    if j == n - 1:
+                        q_empty.arrive()
+
+                if n == 0:
+                    q_empty.arrive()
+                for j in range(min(n, 2)):
+                    yield from mma_s(j)
+                for j in range(n):
+                    s = j & 1
+                    yield from wait(bar["v_full"][s], parity(base, j), f"mma: V, {rec} tile {j}")
+                    yield from wait(bar["p_full"][s], parity(base, j), f"mma: P, {rec} tile {j}")
+                    if V[s] != (rec, j) or any(P.get(t) != (rec, j) for t in range(THREADS)):
+                        errors.append(f"P V of {rec} tile {j} reads V {V[s]}, P {P}")
+                    O[0] = (rec, j)
+                    bar["o_full"][s].arrive()
+                    bar["v_empty"][s].arrive()
+                    if j + 2 < n:
+                        yield from mma_s(j + 2)
+                    yield None
+                for j in range(max(0, n - 2), n):
+                    yield from wait(bar["k_empty"][j & 1], parity(base, j), f"mma: tail K, {rec}")
+                    yield from wait(bar["v_empty"][j & 1], parity(base, j), f"mma: tail V, {rec}")
+                advance(n, st)
+            done["mma"] = rec + 1
+
+    def softmax(tid):
+        st = [0, [0, 0]]
+        me = f"softmax {tid}"
+        for rec, (kind, n) in enumerate(items):
+            if kind != "other":
+                base = list(st[1])
+                for j in range(n):
+                    s = j & 1
+                    yield from wait(bar["s_full"][s], parity(base, j), f"{me}: S, {rec} tile {j}")
+                    if S[s] != (rec, j):
+                        errors.append(f"{me} reads S {S[s]}, wants {rec} tile {j}")
+                    if j >= 1:   # one P buffer
+                        yield from wait(bar["o_full"][(j - 1) & 1], parity(base, j - 1), f"{me}: P free, {rec} tile {j}")
+                    unread_s[s].discard(tid)
+                    P[tid] = (rec, j)
+                    bar["p_full"][s].arrive()
+                    yield None
+                if n > 0:
+                    yield from wait(bar["o_full"][(n - 1) & 1], parity(base, n - 1), f"{me}: last P V, {rec}")
+                    if O[0] != (rec, n - 1):
+                        errors.append(f"{me} reads O {O[0]}, wants {rec} tile {n - 1}")
+                if kind == "rep":
+                    yield from together.wait(f"{me}: before the merge, {rec}")
+                    K[tid & 1] = V[tid & 1] = ("merge", rec)
+                    yield from together.wait(f"{me}: merge, {rec}")
+                    for _ in range(3):
+                        yield None
+                    if (K[tid & 1], V[tid & 1]) != (("merge", rec),) * 2:
+                        errors.append(f"{me} merges {K[tid & 1]}, {V[tid & 1]} in {rec}")
+                else:
+                    P[tid] = ("out", rec)
+                    yield None
+                    if P[tid] != ("out", rec):
+                        errors.append(f"{me} stores {P[tid]} for {rec}")
+                advance(n, st)
+            else:
+                while done["load"] <= rec:   # it works on what the producer brings
+                    yield f"{me}: record {rec}"
+            exec_left[rec] -= 1
+            yield from together.wait(f"{me}: end of {rec}")
+            if exec_left[rec] == 0:
+                done["exec"] = max(done["exec"], rec + 1)
+
+    procs = {"producer": producer(), "mma": mma(), **{f"softmax {t}": softmax(t) for t in range(THREADS)}}
+    idle = 0
+    while procs:
+        name = rnd.choice(list(procs))
+        try:
+            idle = 0 if next(procs[name]) is None else idle + 1
+        except StopIteration:
+            del procs[name]
+            idle = 0
+        if idle > 20000:
+            return f"deadlock: {list(procs)}"
+    return errors[0] if errors else None
+
+
+def records():
+    rnd = random.Random(2)
+    out = [[("rows", n)] * 4 for n in range(6)] + [[("rep", n), ("rows", n), ("other", 0)] * 2 for n in (0, 1, 2, 5)]
+    return out + [[(rnd.choice(["rows", "rows", "rep", "other"]), rnd.choice([0, 1, 2, 3, 5])) for _ in range(7)] for _ in range(40)]
+
+
+def test_records_of_a_fabric_worker():
+    for items in records():
+        for seed in range(15):
+            assert run_records(items, seed) is None, (items, seed)
+
+
+def test_the_record_model_sees_what_the_waits_are_for():
+    merges = [run_records(items, seed, drain_behind_rep=False) for items in records() for seed in range(15)]
+    assert any(r and "merges" in r for r in merges)
+    queries = [run_records(items, seed, q_waits=False) for items in records() for seed in range(15)]
+    assert any(r and "Q" in r for r in queries)
