@@ -98,7 +98,7 @@ __device__ __noinline__ void gated_rows(const TileDesc& t, int tid, uint8_t* rin
     float u[2][CB][4];
     GatedMemoryArgs args;                                      // read again for each chunk rather than kept in registers
   };
-  static_assert(sizeof(Shared) <= 216 * 1024, "the operand ring");
+  static_assert(sizeof(Shared) <= kWideRingBytes, "the operand ring");
   __builtin_assume(__isShared(ring));
   Shared& sh = *reinterpret_cast<Shared*>(ring);
   GatedMemoryArgs& A = sh.args;
@@ -445,7 +445,7 @@ __device__ __noinline__ bool gated_step(const TileDesc& t, int tid, const LayerC
   using T = typename std::conditional<F32, float, __nv_bfloat16>::type;
   constexpr int kSide = 32 / G, kWarp = NC * kSide, kBlock = 4 * kWarp;   // columns side by side in a warp; of a warp; of a block
   constexpr int kDepth = 6, kStageBytes = kWarp * G * ND * 16;
-  static_assert(4 * kDepth * kStageBytes <= 216 * 1024 && kStageBytes % 128 == 0, "the operand ring");
+  static_assert(4 * kDepth * kStageBytes <= kWideRingBytes && kStageBytes % 128 == 0, "the operand ring");
   __builtin_assume(__isShared(ctx.ring));
   __builtin_assume(__isShared(ctx.scratch));
   struct Head {

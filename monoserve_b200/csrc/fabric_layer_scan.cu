@@ -146,7 +146,7 @@ __device__ __noinline__ void scan_rows(const TileDesc& t, int tid, uint8_t* ring
     Chunk in[2];
     T y[kScanTokens][kScanChannels];
   };
-  static_assert(sizeof(Shared) <= 216 * 1024, "the operand ring");
+  static_assert(sizeof(Shared) <= kWideRingBytes, "the operand ring");
   __builtin_assume(__isShared(ring));
   Shared& sh = *reinterpret_cast<Shared*>(ring);
   ScanArgs A;

@@ -13,11 +13,13 @@
 // the matching up feature, so the epilogue pairs them with a warp shuffle instead
 // of a trip through shared memory (with the rows on M they are columns of one lane).
 //
-// What bounds the products of prompts (cycles a K step and SM, loads from the L2): the MMAs are 512 of a 128 x 256
-// tile and 1024 of 256 x 256, and the SM can read twice what either needs.  In the way were, one after the other, the
-// producer's loop (770 a stage, now 550; a small tile's two K steps a stage, 650 a step, now 310), weights evicted
-// from the L2 before their other row blocks read them, and the epilogue, 13000 cycles of a 256 x 256 tile.  4096 x 12288 x
-// 2048: 221 -> 159 us a stage of the fabric; 8192 tokens over 128 experts, hidden 2048, width 768: 1180 -> 1108 us a layer.
+// What bounds the products of prompts: with all SMs at it, the operands.  8192 tokens over 128 experts, hidden 2048, width 768, cut into
+// tiles of 128 x 256 only: 997 K steps a CTA in 880 thousand cycles, 880 a step, of which the MMAs are 512 and the MMA warp waits for
+// operands (48 KB a step) 300; in tiles of 256 x 256 (64 KB a step) 605 K steps of 1024 cycles of MMA take 890 thousand,
+// the rest in epilogues that nothing hides, under the power cap (1.47 GHz).  In the way before were the producer's loop (a stage by itself 770
+// cycles, now 550; a small tile's two K steps a stage, 650 a step, now 310), weights evicted from the L2 before their other row
+// blocks read them, and an epilogue of 13000 cycles a 256 x 256 tile.  4096 x 12288 x 2048: 221 -> 159 us a stage of the fabric; those
+// experts and all around them: 1180 -> 1108 us a layer, with the row blocks of row_blocks.h 1010.
 //
 // Roles: produce() runs in one warp (an elected lane issues TMA), mma() in one warp (one lane
 // issues tcgen05.mma / tcgen05.commit), epilogue() in the four warps whose
@@ -37,11 +39,10 @@ constexpr int kBlockK = 64;                      // elements per K step (128 byt
 constexpr int kATileBytes = 128 * kBlockK * 2;   // 16 KB
 constexpr int kGemmMaxN = 256;
 // Operand stages live in one byte ring: a stage takes 16 KB for the weight tile
-// plus n * 128 bytes for the activation tile: eleven stages of a decode tile, four of 128 x 256.  Behind
-// the ring, 4 KB for each epilogue warp, through which rows leave in whole lines (epilogue_rows).
-constexpr int kRingBytes = 200 * 1024;
-constexpr int kOutBytes = 4 * 4096;
-constexpr int kGemmStages = 12;                  // most stages in flight (barrier pairs)
+// plus n * 128 bytes for the activation tile a K step: five stages of two K steps of a decode tile of 16 rows, four of 64 rows and of
+// 128 x 256, three of 256 x 256; six of 32 KB at most.  Twelve barrier pairs: a stage's pair has long been let go when its turn comes.
+constexpr int kGemmStages = 12;
+static_assert(kRingBytes / (32 * 1024) < kGemmStages, "barrier pairs are never what a stage waits for");
 constexpr int kGemmSmemBytes = kRingBytes + kOutBytes + 1024;
 constexpr int kTmemCols = 512;
 constexpr int kAccCols = 256;                    // TMEM columns per accumulator buffer (two buffers)
@@ -137,8 +138,6 @@ struct GemmInflight {
   uint32_t tail_parity = 0;
 };
 
-// Bytes of one stage: weight tile (bf16), activation tile, and for FP8 weights the
-// raw e4m3 tile the converter warps expand.
 // Which tiles put the activation rows on the MMA's M dimension (TMEM lanes): those of at least 128 rows whose epilogue stores,
 // of bf16 weights.  A lane then owns a row of the output and stores its 32 columns as whole 32-byte sectors, and gate and up of
 // a feature lie in one lane; with the weights on M a warp's store covers one feature of 32 lanes, 2 bytes each, and a
@@ -196,8 +195,8 @@ __device__ __forceinline__ void gemm_barriers_init(GemmBarriers& b) {
 // TMA issue for one tile.  The WHOLE producer warp calls it in step: every lane keeps the same bookkeeping, and one elected
 // lane arms the barrier and issues the copies of a stage (one or two weight boxes and the activation rows).  Weights that are
 // gathered from eight 16-row boxes go out as a single warp-wide instruction (lanes 0..7 the boxes, lane 8 the activation box,
-// lanes 16..23 the second slice's).  What a stage costs here bounds every tile whose MMAs take less: 770 cycles for 128 x 256
-// with an array of stages in flight and lanes in roles, now 548 (its MMAs are 512), 650 -> 520 for 16 rows.
+// lanes 16..23 the second slice's).  What a stage costs here bounds every tile whose MMAs and loads take less: 770 cycles for 128 x 256
+// with an array of stages in flight and lanes in roles, now 548 (of a tile that waits for nothing else), 650 -> 520 for 16 rows.
 // Returns false when a wait was abandoned.
 template <bool kFetch = true>
 __device__ __forceinline__ bool gemm_produce(const GemmWork& w, uint8_t* ring, GemmBarriers& bar, GemmPipe& pipe,

@@ -44,6 +44,10 @@ struct GemmQueues {
 };
 static_assert(sizeof(GemmQueues) == 64, "GemmQueues is 64 bytes");
 
+// Shared memory of a GEMM worker: the ring of operand stages, and behind it 4 KB for each epilogue warp, through which rows leave in whole
+// lines.  Wide tiles of the fabric use both.
+constexpr int kRingBytes = 200 * 1024, kOutBytes = 4 * 4096;
+
 constexpr int kActBoxes = 5;      // activation tensor maps with box heights 16, 32, 64, 128, 256
 
 struct GemmPhaseParams {

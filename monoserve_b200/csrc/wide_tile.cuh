@@ -3,6 +3,7 @@
 #pragma once
 #include "fabric_layer_tiles.cuh"
 #include "ptx.cuh"
+#include "types.h"
 
 namespace mf {
 namespace fab {
@@ -111,7 +112,7 @@ __device__ __forceinline__ void mbar_inval(uint64_t* bar) {
 // The rows of a row-wise tile, one after the other through stages of the operand ring.  128 threads cannot hold enough loads
 // of their own in flight to draw an SM's share of the memory bandwidth; bulk copies, issued by thread 0 as far ahead as the
 // ring holds rows, can.  Barriers in the first 2 kRowStages ints of the scratch.
-constexpr uint32_t kWideRingBytes = 216 * 1024;
+constexpr uint32_t kWideRingBytes = kRingBytes + kOutBytes;
 constexpr int kRowStages = 12;
 struct RowStages {
   uint8_t* ring;

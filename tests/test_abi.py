@@ -100,3 +100,11 @@ def test_releases_wait_for_a_resident_fabric():
     _C.lib.monofab_release_debug(1, dev, None)                         # the last one stops: drained
     assert state() == [0, done0 + 4, 0]
     assert _C.lib.monofab_release_debug(3, 64, None) != 0              # device index out of range
+
+
+def test_the_ring_of_a_wide_tile_is_what_the_host_plans_with():
+    """layer_list.py sizes tiles for the shared memory that csrc/types.h sets apart."""
+    from monoserve_b200.layer_list import RING_BYTES
+    text = open(os.path.join(ROOT, "monoserve_b200", "csrc", "types.h")).read()
+    ring, out = re.search(r"kRingBytes = (\d+) \* 1024, kOutBytes = (\d+) \* 4096;", text).groups()
+    assert int(ring) * 1024 + int(out) * 4096 == RING_BYTES
