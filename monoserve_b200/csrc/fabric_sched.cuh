@@ -674,7 +674,7 @@ __device__ __forceinline__ uint32_t schedule(DeviceState& S, WorkerState& ws, Sm
   __syncwarp();
   if (of_lane && (which == kWSlots || which == kWGen)) words &= 0xffffffffull;
   if (of_lane && which == kWRunning) words >>= 32;
-  const bool changed = __any_sync(kWarp, words != seen && !(of_lane && which >= kWHead));
+  const bool changed = __any_sync(kWarp, words != seen && !(of_lane && which == kWHead));
   auto idle = [&](bool found_nothing, bool more = false) {
     const bool busy = __any_sync(kWarp, of_lane && which == kWRunning && words != 0);
     const uint32_t cap = max(64u, static_cast<uint32_t>(__shfl_sync(kWarp, words, kStopLane) >> 32)), most = busy ? max(32u, cap >> kBusyCapLog2) : cap;

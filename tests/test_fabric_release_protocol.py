@@ -283,3 +283,44 @@ def test_the_run_time_limit_is_looked_at_whatever_lies_between_claims():
     device = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "monoserve_b200", "csrc", "fabric_device.cu")).read()
     assert "(ws.polls & 15) == 0 && must_leave(false)" in device
     assert not re.search(r"ws\.polls = 0", SCHED)   # set where the worker starts, and only there
+
+
+def woken(seed, watches_program):
+    """The same lane; a worker that found nothing looks again once one of the words it watches has changed.  True: it finds the entry."""
+    rnd = random.Random(seed)
+    mem = Memory(prog=1, gen=1, head=4, tail=4)
+    found = []
+
+    def lane():
+        th = Thread(mem, rnd)
+        th.store("prog", 2, release=True)
+        yield
+        th.store("gen", 2, release=True)
+        yield
+        th.store("tail", 5, release=True)
+
+    def worker():
+        th, before = Thread(mem, rnd), None
+        for _ in range(200):
+            words = ["prog", "gen", "tail"]
+            rnd.shuffle(words)
+            seen = {}
+            for w in words:
+                seen[w] = th.load(w, acquire=True)
+                yield
+            watched = {w: v for w, v in seen.items() if w != "prog" or watches_program}
+            if watched == before:
+                continue
+            before = watched
+            if seen["tail"] > 4 and seen["prog"] == 2:
+                found.append(1)
+                return
+
+    assert interleave(rnd, [lane(), worker()])
+    return bool(found)
+
+
+def test_a_worker_looks_again_when_the_program_has_changed():
+    assert all(woken(seed, watches_program=True) for seed in range(2000))
+    assert not all(woken(seed, watches_program=False) for seed in range(2000))
+    assert "words != seen && !(of_lane && which == kWHead)" in body_of("uint32_t schedule")
