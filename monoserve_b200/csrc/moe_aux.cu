@@ -276,7 +276,7 @@ __device__ __forceinline__ void make_plan(const PlanParams& A) {
     tier = A.table[2 * expert] == 0 ? kTierHost : kTierHot;
     z = A.table[2 * expert + 1];
     if (tier == kTierHost) bh = A.form ? A.form : 256;
-    else if (A.slices > 1 && cnt > kNarrowRows) wide_blocks = row_blocks(cnt, total);
+    else if (A.slices > 1) wide_blocks = row_blocks(cnt, total);
     nb = wide_blocks.n ? wide_blocks.n + (wide_blocks.rest > 0) : (cnt + bh - 1) / bh;
   }
   const int nw = wide_blocks.n;

@@ -30,8 +30,9 @@ struct RowBlocks {
   int rest;      // rows of a block behind them with tiles of one, or 0
 };
 
-// rows > kNarrowRows, of `total` rows of the pass; `tall`: blocks of more than 128 rows can be taken.
+// Of `total` rows of the pass; `tall`: blocks of more than 128 rows can be taken.
 __host__ __device__ __forceinline__ RowBlocks row_blocks(int rows, int total, bool tall = true) {
+  if (rows <= kNarrowRows) return RowBlocks{0, 0, rows};
   if (!tall || total < kSomeRows) {
     const int n = (rows + 128 - kNarrowRows - 1) / 128, rest = rows - 128 * n;
     return RowBlocks{n, 0, rest > 0 ? rest : 0};

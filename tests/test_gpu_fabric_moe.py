@@ -388,3 +388,34 @@ def test_row_blocks_in_passes_of_some_and_many_rows(more):
     finally:
         fab.stop()
         fab.close()
+
+
+def test_a_dynamic_region_without_room_is_reported(monkeypatch):
+    """The expand tile finds no room for its tiles: no expert stage gets any, and the error bit is set; the host stops the fabric."""
+    from monoserve_b200.fabric import Fabric
+    from monoserve_b200.lane import MoELane
+    counts = [300, 200, 70, 1100]
+    H, I, E, T = 256, 192, len(counts), sum(counts)
+    wr, w13, w2 = weights(H, I, E, 41)
+    xn, _ = directed(counts, wr, 42)
+    fab = Fabric(pool_bytes=128 << 20)
+    fab.set_max_run(20)
+    try:
+        lane = MoELane(fab, 0, H, I, E, 1, T, wr, w13, w2, hot=list(range(E)))
+        lane.set_input(xn.cuda())
+        monkeypatch.setattr(lane, "dynamic_tiles", lambda T: 8)
+        before = lane.y.clone()
+        h = lane.build(T, iterations=1)
+        fab.start()
+        fab.publish(map=[0] * fab.num_workers, caps=[4], order=[0], programs=[h])
+        t0 = time.time()
+        while not fab.progress()["error"]:
+            assert time.time() - t0 < 10
+            time.sleep(1e-3)
+        time.sleep(0.05)
+        fab.stop()
+        assert fab.progress()["error"] == 32
+        assert torch.equal(lane.y, before)
+    finally:
+        fab.stop()
+        fab.close()
